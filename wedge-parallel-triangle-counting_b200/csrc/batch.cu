@@ -483,10 +483,10 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
                                                          pw.ptr);
     WETRIC_LAUNCH_CHECK();
     WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, is_pair.ptr,
-                                                         ppos.ptr, NT)));
+                                                         ppos.ptr, NT, err.ptr)));
   }
   WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, active.ptr,
-                                                       pos.ptr, NT)));
+                                                       pos.ptr, NT, err.ptr)));
   uint64_t K = 0, Kp = 0;
   unsigned long long maxdeg = 0, Wp = 0;
   WETRIC_CUDA_TRY(cudaMemcpyAsync(&K, pos.ptr + NT, 8, cudaMemcpyDeviceToHost, st));
@@ -521,7 +521,8 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
     k_active_graph<<<grid_for(ctx, NT), 256, 0, st>>>(is_pair.ptr, NT, ppos.ptr, d_vbase.ptr,
                                                       G, b->pg.ptr);
     WETRIC_LAUNCH_CHECK();
-    WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, lens.ptr, b->ps.ptr, Kp)));
+    WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, lens.ptr, b->ps.ptr, Kp,
+                                                         err.ptr)));
     Scratch<unsigned long long> gw;
     WETRIC_TRY(gw.alloc(ctx, st, G));
     WETRIC_CUDA_TRY(cudaMemsetAsync(gw.ptr, 0, G * 8ull, st));
@@ -565,7 +566,7 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
     WETRIC_LAUNCH_CHECK();
   }
   WETRIC_TRY((prim::exclusive_scan<uint64_t, uint64_t>(ctx, st, b->act_wp.ptr,
-                                                       b->act_wp.ptr, K)));
+                                                       b->act_wp.ptr, K, err.ptr)));
   Scratch<uint64_t> d_wbase;
   WETRIC_TRY(d_wbase.alloc(ctx, st, G + 1));
   k_graph_wedge_base<<<grid_for(ctx, G + 1), 256, 0, st>>>(
@@ -642,11 +643,17 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
           b->csr.row_ptr, NT, d_vbase.ptr, G, b->bm_first.ptr, nb.ptr);
     WETRIC_LAUNCH_CHECK();
     WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, nb.ptr,
-                                                         b->hoff.ptr, NT)));
+                                                         b->hoff.ptr, NT, err.ptr)));
     uint64_t buckets = 0;
+    uint32_t herr = 0;
     WETRIC_CUDA_TRY(cudaMemcpyAsync(&buckets, b->hoff.ptr + NT, 8,
                                     cudaMemcpyDeviceToHost, st));
+    WETRIC_CUDA_TRY(cudaMemcpyAsync(&herr, err.ptr, 4, cudaMemcpyDeviceToHost, st));
     WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+    if (herr == kDevLookbackTimeout) {
+      set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
+      return WETRIC_ETIMEDOUT;
+    }
     nb.release();
     // The sets stay resident with the batch: take at most half of the
     // device memory that is free now.

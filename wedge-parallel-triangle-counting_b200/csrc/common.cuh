@@ -162,6 +162,8 @@ enum DeviceError : uint32_t {
   kDevColumnRange = 3,
   kDevDegreeRange = 4,
   kDevRowPtrRange = 5,
+  kDevStageTimeout = 6,     // a shared-memory staging copy did not complete
+  kDevLookbackTimeout = 7,  // a scan's or sort's look-back ran out
 };
 
 }  // namespace wetric

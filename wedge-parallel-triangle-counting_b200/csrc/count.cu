@@ -54,6 +54,7 @@
 #include "count_kernels.cuh"
 #include "pair_streams.cuh"
 #include "primitives.cuh"
+#include "readback.cuh"
 
 namespace wetric {
 
@@ -84,81 +85,6 @@ struct EventPair {
     return WETRIC_OK;
   }
 };
-
-// Host read-backs: one gather kernel collects the values into a device
-// array and one copy brings them to pinned host memory. A copy into
-// pageable memory (a stack variable) returns only when it is done, so one
-// copy per value cost a round trip each while the device sat idle.
-struct ReadSpan {
-  const void *src;
-  uint32_t count, bytes;  // elements of 4 or 8 bytes
-};
-constexpr uint32_t kReadSpans = 12;
-constexpr uint32_t kReadWords = 128;
-struct ReadPlan {
-  ReadSpan s[kReadSpans];
-  uint32_t n = 0, total = 0;
-  // Returns the first word of the span in the gathered array.
-  uint32_t add(const void *src, uint32_t count, uint32_t bytes) {
-    s[n++] = ReadSpan{src, count, bytes};
-    total += count;
-    return total - count;
-  }
-};
-__global__ void k_read_gather(ReadPlan p, uint64_t *__restrict__ out) {
-  uint32_t base = 0;
-  for (uint32_t i = 0; i < p.n; ++i) {
-    const ReadSpan sp = p.s[i];
-    for (uint32_t j = threadIdx.x; j < sp.count; j += blockDim.x)
-      out[base + j] = sp.bytes == 4 ? (uint64_t)static_cast<const uint32_t *>(sp.src)[j]
-                                    : static_cast<const uint64_t *>(sp.src)[j];
-    base += sp.count;
-  }
-}
-// Pinned words for the calling thread's read-backs (portable: any device),
-// made on first use and freed when the thread ends; null if pinned memory
-// cannot be had (the caller then reads into its own array).
-uint64_t *readback_words() {
-  struct Holder {
-    uint64_t *p = nullptr;
-    bool tried = false;
-    ~Holder() {
-      if (p) cudaFreeHost(p);
-    }
-  };
-  thread_local Holder h;
-  if (!h.tried) {
-    h.tried = true;
-    if (cudaHostAlloc(reinterpret_cast<void **>(&h.p), kReadWords * sizeof(uint64_t),
-                      cudaHostAllocPortable) != cudaSuccess) {
-      h.p = nullptr;
-      cudaGetLastError();
-    }
-  }
-  return h.p;
-}
-// Gathers plan's values on st, copies them to the host and waits (for
-// `done`, recorded after the copy, when given); *words points at them
-// afterwards (valid until the calling thread's next read).
-int read_back(DeviceContext *ctx, cudaStream_t st, const ReadPlan &plan, uint64_t *local,
-              const uint64_t **words, cudaEvent_t done = nullptr) {
-  Scratch<uint64_t> dev;
-  WETRIC_TRY(dev.alloc(ctx, st, plan.total));
-  k_read_gather<<<1, 128, 0, st>>>(plan, dev.ptr);
-  WETRIC_LAUNCH_CHECK();
-  uint64_t *host = readback_words();
-  if (!host) host = local;
-  WETRIC_CUDA_TRY(cudaMemcpyAsync(host, dev.ptr, plan.total * sizeof(uint64_t),
-                                  cudaMemcpyDeviceToHost, st));
-  if (done) {
-    WETRIC_CUDA_TRY(cudaEventRecord(done, st));
-    WETRIC_CUDA_TRY(cudaEventSynchronize(done));
-  } else {
-    WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
-  }
-  *words = host;
-  return WETRIC_OK;
-}
 
 template <typename Off>
 int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
@@ -243,7 +169,7 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
   }
 
   WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, active.ptr,
-                                                       pos.ptr, n)));
+                                                       pos.ptr, n, small.ptr)));
   launches += 3;
 
   // Active-vertex arrays sized for all n vertices, so nothing waits for K:
@@ -260,7 +186,7 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
   WETRIC_LAUNCH_CHECK();
   ++launches;
   WETRIC_TRY((prim::exclusive_scan<uint64_t, uint64_t>(ctx, st, act_wp.ptr,
-                                                       act_wp.ptr, n)));
+                                                       act_wp.ptr, n, small.ptr)));
   launches += 3;
 
   // Bucket counts of the per-row hash sets (kernels 6-8) from the row
@@ -283,7 +209,7 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
         nb.ptr);
     WETRIC_LAUNCH_CHECK();
     WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, nb.ptr,
-                                                         hoff.ptr, n)));
+                                                         hoff.ptr, n, small.ptr)));
     launches += 4;
     if (ncount) {
       WETRIC_TRY(noff.alloc(ctx, st, ncount + 1));
@@ -292,7 +218,7 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
           nb.ptr);
       WETRIC_LAUNCH_CHECK();
       WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, nb.ptr,
-                                                           noff.ptr, ncount)));
+                                                           noff.ptr, ncount, small.ptr)));
       launches += 4;
     }
   }
@@ -379,6 +305,10 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
       for (uint32_t i = 0; i < 2 * kCoreNumCandidates; ++i) plan[i] = w[iL + i];
     if (cstart.ptr)
       for (uint32_t i = 0; i < 2 * cs.c; ++i) starts[i] = w[iS + i];
+  }
+  if (err == kDevLookbackTimeout) {
+    set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
+    return WETRIC_ETIMEDOUT;
   }
   if (err != kDevOk) {
     set_error(WETRIC_EINVAL, "oriented CSR check failed (device code %u)", err);
@@ -680,7 +610,7 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
     const uint64_t Tp = pair_tile_cols(Rp, ctx->sm_count);
     const uint64_t ptiles = ceil_div(Rp, Tp);
     WETRIC_TRY(ps.alloc(ctx, st, Kp + 1));
-    WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, pl.ptr, ps.ptr, Kp)));
+    WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, pl.ptr, ps.ptr, Kp, small.ptr)));
     WETRIC_TRY(ptile.alloc(ctx, st, ptiles + 1));
     k_tile_map<<<grid_for(ctx, ptiles + 1), 256, 0, st>>>(ps.ptr, Kp, 0, Rp, Tp, ptiles,
                                                           ptile.ptr);
@@ -878,8 +808,8 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
     WETRIC_CUDA_TRY(cudaEventElapsedTime(&ms, ev_pair.a, ev_pair.b));
     pair_ms = ms;
   }
-  if (err_after == kDevStageTimeout) {
-    set_error(WETRIC_ETIMEDOUT, "a shared-memory staging copy did not complete in time");
+  if (err_after == kDevStageTimeout || err_after == kDevLookbackTimeout) {
+    set_error(WETRIC_ETIMEDOUT, "a bounded wait on the device ran out (code %u)", err_after);
     return WETRIC_ETIMEDOUT;
   }
   r->triangles = tri;
@@ -946,7 +876,7 @@ static int wedge_total_impl(DeviceContext *ctx, cudaStream_t st,
     WETRIC_LAUNCH_CHECK();
     // Reuse: wc[v] = C(d, 2) for all v (compact with pos == identity).
     WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, active.ptr,
-                                                         wc.ptr, n)));
+                                                         wc.ptr, n, err.ptr)));
   }
   uint64_t K = 0;
   uint32_t herr = 0;
@@ -971,13 +901,19 @@ static int wedge_total_impl(DeviceContext *ctx, cudaStream_t st,
     WETRIC_LAUNCH_CHECK();
   }
   WETRIC_TRY((prim::exclusive_scan<uint64_t, uint64_t>(ctx, st, act_wp.ptr,
-                                                       act_wp.ptr, K)));
+                                                       act_wp.ptr, K, err.ptr)));
   unsigned long long hmd = 0;
+  WETRIC_CUDA_TRY(cudaMemcpyAsync(&herr, err.ptr, sizeof(uint32_t),
+                                  cudaMemcpyDeviceToHost, st));
   WETRIC_CUDA_TRY(cudaMemcpyAsync(W, act_wp.ptr + K, sizeof(uint64_t),
                                   cudaMemcpyDeviceToHost, st));
   WETRIC_CUDA_TRY(cudaMemcpyAsync(&hmd, md.ptr, sizeof(hmd),
                                   cudaMemcpyDeviceToHost, st));
   WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  if (herr != kDevOk) {
+    set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
+    return WETRIC_ETIMEDOUT;
+  }
   *maxdeg = hmd;
   return WETRIC_OK;
 }

@@ -1572,7 +1572,6 @@ __global__ void k_core_prefix(const uint64_t *__restrict__ act_wp,
 // false.
 constexpr uint32_t kStageCols = 2048;
 constexpr uint32_t kStageSpin = 1u << 22;
-constexpr uint32_t kDevStageTimeout = 6;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -1620,7 +1619,7 @@ __device__ __forceinline__ bool stage_row(const uint32_t *__restrict__ ci, uint6
   for (uint64_t j = a1 + threadIdx.x; j < rb + d; j += blockDim.x) stage[j - a0] = __ldg(ci + j);
   const bool ok = mbar_wait(mbar, 0, kStageSpin);
   if (!ok) {
-    if (threadIdx.x == 0 && err) atomicCAS(err, 0u, kDevStageTimeout);
+    if (threadIdx.x == 0 && err) atomicCAS(err, 0u, (uint32_t)kDevStageTimeout);
     mbar_wait(mbar, 0, kStageSpin);  // the copy this block started, once more
   }
   __syncthreads();

@@ -66,27 +66,26 @@ struct Arena {
   }
 };
 
-// Exclusive scan with its block sums taken from the arena (same kernels as
-// the allocating scan in primitives.cuh).
+// Exclusive scan with its look-back words taken from the arena (same kernel
+// as the allocating scan in primitives.cuh).
 template <typename InT, typename OutT>
 int scan_in_arena(Arena *ar, cudaStream_t st, const InT *in, OutT *out,
-                  uint64_t n) {
+                  uint64_t n, uint32_t *err) {
   using namespace wetric::prim;
-  const uint64_t blocks = n == 0 ? 1 : wetric::ceil_div(n, kScanChunk);
-  if (blocks == 1) {
-    scan_apply_kernel<InT, OutT><<<1, kScanThreads, 0, st>>>(in, n, out, nullptr);
+  const uint64_t tiles = n == 0 ? 1 : wetric::ceil_div(n, kScanChunk);
+  if (tiles == 1) {
+    k_scan<InT, OutT><<<1, kScanThreads, 0, st>>>(in, n, out, nullptr, nullptr, err);
     WETRIC_LAUNCH_CHECK();
     return WETRIC_OK;
   }
-  OutT *sums = ar->take<OutT>(blocks + 1);
-  if (!sums) {
+  uint64_t *state = ar->take<uint64_t>(tiles + 1);
+  if (!state) {
     wetric::set_error(WETRIC_ERANGE, "graph too large for the no-allocation scratch");
     return WETRIC_ERANGE;
   }
-  scan_reduce_kernel<InT, OutT><<<(unsigned)blocks, kScanThreads, 0, st>>>(in, n, sums);
-  WETRIC_LAUNCH_CHECK();
-  WETRIC_TRY((scan_in_arena<OutT, OutT>(ar, st, sums, sums, blocks)));
-  scan_apply_kernel<InT, OutT><<<(unsigned)blocks, kScanThreads, 0, st>>>(in, n, out, sums);
+  WETRIC_CUDA_TRY(cudaMemsetAsync(state, 0, (tiles + 1) * sizeof(uint64_t), st));
+  k_scan<InT, OutT><<<(unsigned)tiles, kScanThreads, 0, st>>>(
+      in, n, out, state + 1, reinterpret_cast<uint32_t *>(state), err);
   WETRIC_LAUNCH_CHECK();
   return WETRIC_OK;
 }
@@ -185,7 +184,7 @@ int count_noalloc_impl(int device, cudaStream_t st, const Off *rp,
   WETRIC_CUDA_TRY(cudaMemsetAsync(acc, 0, 4 * sizeof(unsigned long long), st));
   k_vertex_wedges<Off><<<grid_cap(sms, n), 256, 0, st>>>(rp, n, m, active, acc, small);
   WETRIC_LAUNCH_CHECK();
-  WETRIC_TRY((scan_in_arena<uint32_t, uint64_t>(&ar, st, active, pos, n)));
+  WETRIC_TRY((scan_in_arena<uint32_t, uint64_t>(&ar, st, active, pos, n, small)));
   uint64_t K = 0;
   unsigned long long maxdeg = 0;
   uint32_t err = 0;
@@ -193,6 +192,10 @@ int count_noalloc_impl(int device, cudaStream_t st, const Off *rp,
   WETRIC_CUDA_TRY(cudaMemcpyAsync(&maxdeg, acc, 8, cudaMemcpyDeviceToHost, st));
   WETRIC_CUDA_TRY(cudaMemcpyAsync(&err, small, 4, cudaMemcpyDeviceToHost, st));
   WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  if (err == kDevLookbackTimeout) {
+    set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
+    return WETRIC_ETIMEDOUT;
+  }
   if (err != kDevOk) {
     set_error(WETRIC_EINVAL, "oriented CSR check failed (device code %u)", err);
     return WETRIC_EINVAL;
@@ -210,10 +213,15 @@ int count_noalloc_impl(int device, cudaStream_t st, const Off *rp,
                                                            act_rb, act_d);
     WETRIC_LAUNCH_CHECK();
   }
-  WETRIC_TRY((scan_in_arena<uint64_t, uint64_t>(&ar, st, act_wp, act_wp, K)));
+  WETRIC_TRY((scan_in_arena<uint64_t, uint64_t>(&ar, st, act_wp, act_wp, K, small)));
   uint64_t W = 0;
   WETRIC_CUDA_TRY(cudaMemcpyAsync(&W, act_wp + K, 8, cudaMemcpyDeviceToHost, st));
+  WETRIC_CUDA_TRY(cudaMemcpyAsync(&err, small, 4, cudaMemcpyDeviceToHost, st));
   WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  if (err != kDevOk) {
+    set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
+    return WETRIC_ETIMEDOUT;
+  }
   if (W == 0) return WETRIC_OK;
 
   const uint64_t T = 256ull * s;

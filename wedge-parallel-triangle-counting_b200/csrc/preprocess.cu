@@ -7,29 +7,32 @@
 // (763-784). Here all of that runs on the GPU with this library's own radix
 // sort:
 //
-//   raw pairs --canonical (min,max) key--> sort --> unique --> degrees
+//   raw pairs --canonical (min,max) key--> sort --> unique + degrees
 //     --> stable (degree, id) rank --> (rank lo, rank hi) key --> sort
 //     --> oriented CSR (u64 row offsets, u32 columns)
 //
 // Keys pack two ids of b = bits(n-1) bits each into 2b bits, so a sort
 // costs ceil(2b / 8) digit passes. Canonicalising to (min, max) before the
 // first sort halves the keys compared with the reference's symmetrised
-// list. The vertex order equals that of the reference's stable CUB sort
-// (its -p 1 / -p 2 styles): ascending degree, ties by ascending id.
+// list. The passes take their keys where they arise: the first sort reads
+// the pairs, the degree sort the degrees, the symmetric sort the unique
+// keys, and none of them stores an unsorted copy. The vertex order equals
+// that of the reference's stable CUB sort (its -p 1 / -p 2 styles):
+// ascending degree, ties by ascending id.
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "common.cuh"
 #include "preprocess.cuh"
 #include "primitives.cuh"
+#include "readback.cuh"
 
 namespace wetric {
 
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kItems = 8;
-constexpr int kTile = kThreads * kItems;
 
 __device__ __forceinline__ uint64_t pack_key(uint32_t lo, uint32_t hi,
                                              uint32_t b) {
@@ -58,152 +61,207 @@ __global__ void k_max_id(const uint32_t *__restrict__ src,
   }
 }
 
-// keys[i] = (min, max) packed, or the all-ones sentinel for a self-loop or
-// an id >= n (the latter also raises *err).
-__global__ void k_canon_keys(const uint32_t *__restrict__ src,
-                             const uint32_t *__restrict__ dst, uint64_t P,
-                             uint32_t b, uint64_t n, uint64_t sentinel,
-                             uint64_t *__restrict__ keys, uint32_t *err) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t s = src[i], d = dst[i];
-    uint64_t k = sentinel;
-    if (s != d) {
-      if ((uint64_t)s >= n || (uint64_t)d >= n) {
-        atomicCAS(err, 0u, (uint32_t)kDevColumnRange);
-      } else {
-        k = pack_key(min(s, d), max(s, d), b);
-      }
-    }
-    keys[i] = k;
+// Key of raw pair i: (min, max) packed, or the all-ones sentinel for a
+// self-loop or an id >= n. kCheck (the first reading) also raises *err for
+// such an id; without it the reading has no branch, so a thread's loads go
+// out together.
+template <bool kCheck>
+struct CanonPairs {
+  const uint32_t *__restrict__ src, *__restrict__ dst;
+  uint32_t b;
+  uint64_t n, sentinel;
+  uint32_t *err;
+  __device__ __forceinline__ uint64_t operator()(uint64_t i) const {
+    const uint32_t s = __ldg(src + i), d = __ldg(dst + i);
+    const uint32_t lo = min(s, d), hi = max(s, d);
+    if (kCheck && s != d && (uint64_t)hi >= n) atomicCAS(err, 0u, (uint32_t)kDevColumnRange);
+    return s == d || (uint64_t)hi >= n ? sentinel : pack_key(lo, hi, b);
   }
-}
+};
 
-// Per-tile count of keys that are not the sentinel and differ from their
-// predecessor (keys sorted).
+// Sorted keys -> the unique ones (no sentinel) in order, their number, and
+// the degree of every vertex, in one pass: a warp's keys are consecutive,
+// the block's offset comes by look-back. deg[hi] takes one atomic per edge
+// and deg[lo] one per run of equal lo in a warp's 32 keys (equal addresses
+// serialise: with one atomic per edge each side, in a kernel of its own
+// after two more passes over the keys, this took 2.16 + 0.69 ms on R-MAT
+// scale 22; now 0.77 ms, bound by the atomics on deg[hi]).
+constexpr int kUniqueItems = 16;
+constexpr int kUniqueTile = kThreads * kUniqueItems;
 __global__ void __launch_bounds__(kThreads)
-    k_unique_count(const uint64_t *__restrict__ keys, uint64_t N,
-                   uint64_t sentinel, uint32_t *__restrict__ tile_counts) {
-  __shared__ uint32_t warp_sums[kThreads / 32];
-  const uint64_t base =
-      (uint64_t)blockIdx.x * kTile + (uint64_t)threadIdx.x * kItems;
-  uint32_t c = 0;
+    k_unique_degrees(const uint64_t *__restrict__ keys, uint64_t N, uint64_t sentinel,
+                     uint32_t b, uint64_t *__restrict__ out, uint32_t *__restrict__ deg,
+                     uint64_t *__restrict__ state, uint32_t *__restrict__ ticket,
+                     uint64_t *__restrict__ m_out, uint32_t *err) {
+  __shared__ uint32_t s_warp[kThreads / 32];
+  __shared__ uint64_t s_excl;
+  __shared__ uint32_t s_ticket, s_ok;
+  if (threadIdx.x == 0) s_ticket = atomicAdd(ticket, 1u);
+  __syncthreads();
+  const uint64_t tile = s_ticket;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t sub = tile * kUniqueTile + (uint64_t)warp * 32 * kUniqueItems;
+  const uint64_t mask = (1ull << b) - 1;
+  uint64_t k[kUniqueItems];
+  uint32_t keep[kUniqueItems];
 #pragma unroll
-  for (int j = 0; j < kItems; ++j) {
-    const uint64_t i = base + j;
-    if (i < N) {
-      const uint64_t k = keys[i];
-      c += (k != sentinel && (i == 0 || keys[i - 1] != k)) ? 1u : 0u;
+  for (int j = 0; j < kUniqueItems; ++j) {
+    const uint64_t i = sub + (uint64_t)j * 32 + lane;
+    k[j] = i < N ? keys[i] : sentinel;
+  }
+  // the key before the warp's first (any key but it when there is none)
+  uint64_t last = sub > 0 && sub - 1 < N ? keys[sub - 1] : ~k[0];
+  last = __shfl_sync(0xffffffffu, last, 0);
+  uint32_t mine = 0;
+#pragma unroll
+  for (int j = 0; j < kUniqueItems; ++j) {
+    uint64_t prev = __shfl_up_sync(0xffffffffu, k[j], 1);
+    if (lane == 0) prev = last;
+    last = __shfl_sync(0xffffffffu, k[j], 31);
+    keep[j] = __ballot_sync(0xffffffffu, k[j] != sentinel && k[j] != prev);
+    mine += __popc(keep[j]);
+  }
+  if (lane == 0) s_warp[warp] = mine;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t c = lane < kThreads / 32 ? s_warp[lane] : 0u;
+    const uint32_t total = __reduce_add_sync(0xffffffffu, c);
+    uint64_t excl = 0;
+    const bool ok = prim::tile_prefix(state, tile, total, err, &excl);
+    if (lane == 0) {
+      s_excl = excl;
+      s_ok = ok;
+      if (ok && (tile + 1) * kUniqueTile >= N) *m_out = excl + total;
     }
   }
-  uint32_t total;
-  prim::block_inclusive_scan<uint32_t>(c, warp_sums, &total);
-  if (threadIdx.x == 0) tile_counts[blockIdx.x] = total;
+  __syncthreads();
+  if (!s_ok) return;
+  uint64_t pos = s_excl;
+  for (uint32_t w = 0; w < warp; ++w) pos += s_warp[w];
+  const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+  for (int j = 0; j < kUniqueItems; ++j) {
+    const bool mykeep = (keep[j] >> lane) & 1u;
+    const uint32_t lo = (uint32_t)(k[j] >> b);
+    if (mykeep) {
+      out[pos + __popc(keep[j] & lt)] = k[j];
+      atomicAdd(&deg[(uint32_t)(k[j] & mask)], 1u);
+    }
+    pos += __popc(keep[j]);
+    // runs of equal lo: the run's first lane adds its kept keys
+    const uint32_t before = __shfl_up_sync(0xffffffffu, lo, 1);
+    const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || lo != before);
+    if ((heads >> lane) & 1u) {
+      const uint32_t later = heads & ~(lt | (1u << lane));
+      const uint32_t upto = later ? (1u << (__ffs(later) - 1)) - 1u : 0xFFFFFFFFu;
+      const uint32_t c = __popc(keep[j] & upto & ~lt);
+      if (c) atomicAdd(&deg[lo], c);
+    }
+  }
 }
 
 __global__ void __launch_bounds__(kThreads)
-    k_unique_write(const uint64_t *__restrict__ keys, uint64_t N,
-                   uint64_t sentinel, const uint64_t *__restrict__ tile_off,
-                   uint64_t *__restrict__ out) {
-  __shared__ uint32_t warp_sums[kThreads / 32];
-  const uint64_t base =
-      (uint64_t)blockIdx.x * kTile + (uint64_t)threadIdx.x * kItems;
-  uint32_t keep_mask = 0, c = 0;
-  uint64_t k[kItems];
-#pragma unroll
-  for (int j = 0; j < kItems; ++j) {
-    const uint64_t i = base + j;
-    k[j] = 0;
-    if (i < N) {
-      k[j] = keys[i];
-      if (k[j] != sentinel && (i == 0 || keys[i - 1] != k[j])) {
-        keep_mask |= 1u << j;
-        ++c;
-      }
-    }
-  }
-  uint32_t total;
-  const uint32_t incl = prim::block_inclusive_scan<uint32_t>(c, warp_sums, &total);
-  uint64_t pos = tile_off[blockIdx.x] + (incl - c);
-#pragma unroll
-  for (int j = 0; j < kItems; ++j)
-    if (keep_mask & (1u << j)) out[pos++] = k[j];
-}
-
-__global__ void k_degree_undirected(const uint64_t *__restrict__ ukeys,
-                                    uint64_t m, uint32_t b,
-                                    uint32_t *__restrict__ deg) {
-  const uint64_t mask = (b >= 64) ? ~0ull : ((1ull << b) - 1);
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = ukeys[i];
-    atomicAdd(&deg[(uint32_t)(k >> b)], 1u);
-    atomicAdd(&deg[(uint32_t)(k & mask)], 1u);
-  }
-}
-
-__global__ void k_max_u32(const uint32_t *__restrict__ a, uint64_t n,
-                          uint32_t *out) {
+    k_max_u32(const uint32_t *__restrict__ a, uint64_t n, uint64_t *out) {
   uint32_t local = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x)
     local = max(local, a[i]);
   local = __reduce_max_sync(0xffffffffu, local);
-  if ((threadIdx.x & 31) == 0) atomicMax(out, local);
-}
-
-__global__ void k_iota(uint32_t *__restrict__ v, uint64_t n) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    v[i] = (uint32_t)i;
-}
-
-__global__ void k_rank_from_order(const uint32_t *__restrict__ order,
-                                  uint64_t n, uint32_t *__restrict__ rank) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    rank[order[i]] = (uint32_t)i;
-}
-
-__global__ void k_orient_keys(const uint64_t *ukeys, uint64_t m, uint32_t b,
-                              const uint32_t *__restrict__ rank,
-                              uint64_t *okeys) {
-  const uint64_t mask = (1ull << b) - 1;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = ukeys[i];
-    const uint32_t ra = rank[(uint32_t)(k >> b)];
-    const uint32_t rb = rank[(uint32_t)(k & mask)];
-    okeys[i] = pack_key(min(ra, rb), max(ra, rb), b);
+  __shared__ uint32_t s_max[kThreads / 32];
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = local;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (uint32_t w = 1; w < kThreads / 32; ++w) local = max(local, s_max[w]);
+    atomicMax(reinterpret_cast<unsigned long long *>(out), (unsigned long long)local);
   }
 }
 
-__global__ void k_both_directions(const uint64_t *__restrict__ ukeys,
-                                  uint64_t m, uint32_t b,
-                                  uint64_t *__restrict__ dkeys) {
-  const uint64_t mask = (1ull << b) - 1;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = ukeys[i];
-    const uint32_t lo = (uint32_t)(k >> b), hi = (uint32_t)(k & mask);
-    dkeys[2 * i] = pack_key(lo, hi, b);
-    dkeys[2 * i + 1] = pack_key(hi, lo, b);
+// The degree sort's keys (degree above, id below: the ids ride along) and
+// what it is for: rank[id] = position.
+struct DegreeKeys {
+  const uint32_t *__restrict__ deg;
+  __device__ __forceinline__ uint64_t operator()(uint64_t i) const {
+    return ((uint64_t)deg[i] << 32) | i;
   }
-}
+};
+struct RankTo {
+  uint32_t *__restrict__ rank;
+  __device__ __forceinline__ void operator()(uint64_t i, uint64_t k) const {
+    rank[(uint32_t)k] = (uint32_t)i;
+  }
+};
 
-__global__ void k_row_histogram(const uint64_t *__restrict__ keys, uint64_t m,
-                                uint32_t b, uint32_t *__restrict__ cnt) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    atomicAdd(&cnt[(uint32_t)(keys[i] >> b)], 1u);
-}
+// Keys of the oriented edges, (rank lower, rank higher), made and stored
+// while their digits are counted.
+struct OrientedKeys {
+  const uint64_t *__restrict__ keys;
+  const uint32_t *__restrict__ rank;
+  uint64_t *__restrict__ out;
+  uint32_t b;
+  __device__ __forceinline__ uint64_t operator()(uint64_t i) const {
+    const uint64_t k = __ldg(keys + i);
+    const uint32_t ra = __ldg(rank + (uint32_t)(k >> b));
+    const uint32_t rb = __ldg(rank + (uint32_t)(k & ((1ull << b) - 1)));
+    const uint64_t o = pack_key(min(ra, rb), max(ra, rb), b);
+    out[i] = o;
+    return o;
+  }
+};
 
-__global__ void k_low_bits(const uint64_t *__restrict__ keys, uint64_t m,
-                           uint32_t b, uint32_t *__restrict__ col) {
+// Both directions of every unique key.
+struct BothDirections {
+  const uint64_t *__restrict__ keys;
+  uint32_t b;
+  __device__ __forceinline__ uint64_t operator()(uint64_t i) const {
+    const uint64_t k = keys[i >> 1];
+    return (i & 1) ? pack_key((uint32_t)(k & ((1ull << b) - 1)), (uint32_t)(k >> b), b) : k;
+  }
+};
+
+// Sorted (row, col) keys -> columns and row offsets in one pass: the offset
+// of every row in (row of key i - 1, row of key i] is i. The rows before the
+// first key's (isolated vertices come first in the degree order) and after
+// the last key's are filled by the whole grid; longer gaps in between by
+// the whole block. Replaces a histogram by one atomic per edge on the row
+// (equal addresses for a whole row: 0.73 ms on R-MAT scale 22), a scan and
+// a pass for the columns: 0.93 -> 0.24 ms there.
+constexpr uint32_t kGapByThread = 8;
+__global__ void __launch_bounds__(kThreads)
+    k_keys_to_csr(const uint64_t *__restrict__ keys, uint64_t m, uint64_t n, uint32_t b,
+                  uint64_t *__restrict__ rp, uint32_t *__restrict__ ci) {
+  __shared__ uint32_t s_from[kThreads], s_to[kThreads], s_gaps;
   const uint64_t mask = (1ull << b) - 1;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    col[i] = (uint32_t)(keys[i] & mask);
+  const uint64_t gid = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+  const uint64_t stride = (uint64_t)gridDim.x * kThreads;
+  const uint64_t first = keys[0] >> b, end = keys[m - 1] >> b;
+  for (uint64_t r = gid; r <= first; r += stride) rp[r] = 0;
+  for (uint64_t r = end + 1 + gid; r <= n; r += stride) rp[r] = m;
+  for (uint64_t i0 = (uint64_t)blockIdx.x * kThreads; i0 < m; i0 += stride) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_gaps = 0;
+    __syncthreads();
+    const uint64_t i = i0 + threadIdx.x;
+    if (i < m) {
+      const uint64_t k = keys[i];
+      ci[i] = (uint32_t)(k & mask);
+      if (i > 0) {
+        const uint32_t row = (uint32_t)(k >> b), prev = (uint32_t)(keys[i - 1] >> b);
+        if (row - prev <= kGapByThread) {
+          for (uint32_t r = prev; r < row; ++r) rp[r + 1] = i;
+        } else {
+          const uint32_t g = atomicAdd(&s_gaps, 1u);
+          s_from[g] = prev;
+          s_to[g] = threadIdx.x;
+        }
+      }
+    }
+    __syncthreads();
+    for (uint32_t g = 0; g < s_gaps; ++g) {
+      const uint64_t at = i0 + s_to[g];
+      const uint64_t row = keys[at] >> b;
+      for (uint64_t r = (uint64_t)s_from[g] + 1 + threadIdx.x; r <= row; r += kThreads) rp[r] = at;
+    }
+  }
 }
 
 // Degrees of a CSR given by row offsets (the reference's num_edges of
@@ -288,145 +346,103 @@ unsigned grid_for(DeviceContext *ctx, uint64_t work) {
   return (unsigned)g;
 }
 
-int read_u32(cudaStream_t st, const uint32_t *d, uint32_t *h) {
-  WETRIC_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(uint32_t),
-                                  cudaMemcpyDeviceToHost, st));
+// Grid of a kernel that ends in one atomic per block.
+unsigned max_grid(DeviceContext *ctx, uint64_t n) {
+  const uint64_t cap = (uint64_t)ctx->sm_count * 4;
+  const uint64_t g = ceil_div(n, kThreads * 4);
+  return (unsigned)(g == 0 ? 1 : g < cap ? g : cap);
+}
+
+// Words that the pipeline leaves for the host: read by one copy into pinned
+// memory, so a read costs one round trip.
+struct PrepWords {
+  uint64_t m;       // unique (or kept) edges
+  uint64_t maxdeg;  // largest degree
+  uint32_t err, pad;
+  uint32_t max_id, any_edge;
+};
+int read_words(cudaStream_t st, const PrepWords *d, PrepWords *h) {
+  uint64_t *host = readback_words();
+  if (!host) host = reinterpret_cast<uint64_t *>(h);
+  WETRIC_CUDA_TRY(cudaMemcpyAsync(host, d, sizeof(PrepWords), cudaMemcpyDeviceToHost, st));
   WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  memcpy(h, host, sizeof(PrepWords));
   return WETRIC_OK;
 }
 
-int read_u64(cudaStream_t st, const uint64_t *d, uint64_t *h) {
-  WETRIC_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(uint64_t),
-                                  cudaMemcpyDeviceToHost, st));
-  WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
-  return WETRIC_OK;
-}
-
-int dev_error(cudaStream_t st, const uint32_t *d_err, const char *what) {
-  uint32_t e = 0;
-  WETRIC_TRY(read_u32(st, d_err, &e));
-  if (e != kDevOk) {
-    set_error(WETRIC_EINVAL, "%s: invalid input (device check %u)", what, e);
+// Reads the words and turns a device error into a status.
+int checked_words(cudaStream_t st, const PrepWords *d, const char *what, PrepWords *h) {
+  WETRIC_TRY(read_words(st, d, h));
+  if (h->err == kDevLookbackTimeout) {
+    set_error(WETRIC_ETIMEDOUT, "%s: a look-back did not complete in time", what);
+    return WETRIC_ETIMEDOUT;
+  }
+  if (h->err != kDevOk) {
+    set_error(WETRIC_EINVAL, "%s: invalid input (device check %u)", what, h->err);
     return WETRIC_EINVAL;
   }
   return WETRIC_OK;
 }
 
-// Sorted, deduplicated compaction of `keys` (sorted, with sentinel) into
-// `out`; returns the number kept in *m.
-int unique_sorted(DeviceContext *ctx, cudaStream_t st, const uint64_t *keys,
-                  uint64_t N, uint64_t sentinel, uint64_t *out, uint64_t *m) {
-  const uint64_t tiles = N == 0 ? 1 : ceil_div(N, kTile);
-  Scratch<uint32_t> counts;
-  Scratch<uint64_t> offs;
-  WETRIC_TRY(counts.alloc(ctx, st, tiles));
-  WETRIC_TRY(offs.alloc(ctx, st, tiles + 1));
-  k_unique_count<<<(unsigned)tiles, kThreads, 0, st>>>(keys, N, sentinel,
-                                                       counts.ptr);
-  WETRIC_LAUNCH_CHECK();
-  WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, counts.ptr,
-                                                       offs.ptr, tiles)));
-  k_unique_write<<<(unsigned)tiles, kThreads, 0, st>>>(keys, N, sentinel,
-                                                       offs.ptr, out);
-  WETRIC_LAUNCH_CHECK();
-  return read_u64(st, offs.ptr + tiles, m);
+int alloc_words(DeviceContext *ctx, cudaStream_t st, Scratch<PrepWords> *w) {
+  WETRIC_TRY(w->alloc(ctx, st, 1));
+  WETRIC_CUDA_TRY(cudaMemsetAsync(w->ptr, 0, sizeof(PrepWords), st));
+  return WETRIC_OK;
 }
 
-// Group of every vertex of a disjoint union: key = (group << dbits) | deg,
-// group = the g with group_base[g] <= v < group_base[g + 1].
-__global__ void k_group_keys(const uint32_t *__restrict__ deg, uint64_t n,
-                             const uint64_t *__restrict__ group_base,
-                             uint32_t G, uint32_t dbits,
-                             uint64_t *__restrict__ keys) {
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
-       v += (uint64_t)gridDim.x * blockDim.x) {
+// The group sort's keys, in degree order: group above (the g with
+// group_base[g] <= v < group_base[g + 1]), id below.
+struct GroupKeys {
+  const uint64_t *__restrict__ by_degree;
+  const uint64_t *__restrict__ group_base;
+  uint32_t G;
+  __device__ __forceinline__ uint64_t operator()(uint64_t i) const {
+    const uint32_t v = (uint32_t)by_degree[i];
     uint32_t lo = 0, len = G;
     while (len > 1) {
       const uint32_t h = len >> 1;
       if (group_base[lo + h] <= v) lo += h;
       len -= h;
     }
-    keys[v] = ((uint64_t)lo << dbits) | deg[v];
+    return ((uint64_t)lo << 32) | v;
   }
-}
+};
 
-// Within-group rank: vertices of a disjoint union ordered by (group,
-// degree, id), so every group keeps its id range and the order inside a
-// group is the stable ascending-degree order of that group alone.
-int grouped_degree_rank(DeviceContext *ctx, cudaStream_t st,
-                        const uint32_t *deg, uint64_t n,
-                        const uint64_t *group_base, uint32_t G,
-                        uint32_t *rank) {
-  Scratch<uint64_t> k0, k1;
-  Scratch<uint32_t> v0, v1, dmax;
-  WETRIC_TRY(k0.alloc(ctx, st, n));
-  WETRIC_TRY(k1.alloc(ctx, st, n));
-  WETRIC_TRY(v0.alloc(ctx, st, n));
-  WETRIC_TRY(v1.alloc(ctx, st, n));
-  WETRIC_TRY(dmax.alloc(ctx, st, 1));
-  WETRIC_CUDA_TRY(cudaMemsetAsync(dmax.ptr, 0, sizeof(uint32_t), st));
-  k_max_u32<<<grid_for(ctx, n), 256, 0, st>>>(deg, n, dmax.ptr);
-  WETRIC_LAUNCH_CHECK();
-  uint32_t maxdeg = 0;
-  WETRIC_TRY(read_u32(st, dmax.ptr, &maxdeg));
+// rank[v] = position of v in the stable ascending-degree order. With groups
+// (a disjoint union of G graphs) the order is (group, degree, id), so every
+// group keeps its id range and the order inside a group is that of the
+// group alone.
+int degree_rank(DeviceContext *ctx, cudaStream_t st, const uint32_t *deg, uint64_t n,
+                uint64_t maxdeg, uint32_t *rank, uint32_t *err,
+                const uint64_t *group_base = nullptr, uint32_t G = 0) {
   const uint32_t dbits = bits_for(maxdeg);
-  const uint32_t gbits = bits_for(G ? G - 1 : 0);
-  k_group_keys<<<grid_for(ctx, n), 256, 0, st>>>(deg, n, group_base, G, dbits,
-                                                 k0.ptr);
-  WETRIC_LAUNCH_CHECK();
-  k_iota<<<grid_for(ctx, n), 256, 0, st>>>(v0.ptr, n);
-  WETRIC_LAUNCH_CHECK();
-  bool alt = false;
-  WETRIC_TRY((prim::radix_sort<uint64_t, uint32_t>(
-      ctx, st, k0.ptr, k1.ptr, v0.ptr, v1.ptr, n, dbits + gbits, &alt)));
-  const uint32_t *order = alt ? v1.ptr : v0.ptr;
-  k_rank_from_order<<<grid_for(ctx, n), 256, 0, st>>>(order, n, rank);
-  WETRIC_LAUNCH_CHECK();
-  return WETRIC_OK;
-}
-
-// rank[v] = position of v in the stable ascending-degree order.
-int degree_rank(DeviceContext *ctx, cudaStream_t st, const uint32_t *deg,
-                uint64_t n, uint32_t *rank) {
-  Scratch<uint32_t> k0, k1, v0, v1, dmax;
-  WETRIC_TRY(k0.alloc(ctx, st, n));
-  WETRIC_TRY(k1.alloc(ctx, st, n));
-  WETRIC_TRY(v0.alloc(ctx, st, n));
-  WETRIC_TRY(v1.alloc(ctx, st, n));
-  WETRIC_TRY(dmax.alloc(ctx, st, 1));
-  WETRIC_CUDA_TRY(cudaMemsetAsync(dmax.ptr, 0, sizeof(uint32_t), st));
-  WETRIC_CUDA_TRY(cudaMemcpyAsync(k0.ptr, deg, n * sizeof(uint32_t),
-                                  cudaMemcpyDeviceToDevice, st));
-  k_max_u32<<<grid_for(ctx, n), 256, 0, st>>>(deg, n, dmax.ptr);
-  WETRIC_LAUNCH_CHECK();
-  k_iota<<<grid_for(ctx, n), 256, 0, st>>>(v0.ptr, n);
-  WETRIC_LAUNCH_CHECK();
-  uint32_t maxdeg = 0;
-  WETRIC_TRY(read_u32(st, dmax.ptr, &maxdeg));
-  bool alt = false;
-  WETRIC_TRY((prim::radix_sort<uint32_t, uint32_t>(
-      ctx, st, k0.ptr, k1.ptr, v0.ptr, v1.ptr, n, bits_for(maxdeg), &alt)));
-  const uint32_t *order = alt ? v1.ptr : v0.ptr;
-  k_rank_from_order<<<grid_for(ctx, n), 256, 0, st>>>(order, n, rank);
-  WETRIC_LAUNCH_CHECK();
-  return WETRIC_OK;
+  const bool groups = group_base != nullptr && G > 1;
+  const uint32_t passes = prim::digit_plan(32, dbits ? dbits : 1).passes;
+  Scratch<uint64_t> a, b;
+  if (groups || passes > 1) WETRIC_TRY(a.alloc(ctx, st, n));
+  if (groups || passes > 2) WETRIC_TRY(b.alloc(ctx, st, n));
+  const DegreeKeys keys{deg};
+  if (!groups)
+    return prim::radix_sort_into(ctx, st, keys, keys, a.ptr, b.ptr, RankTo{rank}, n, 32, dbits,
+                                 err);
+  uint64_t *by_degree = prim::sorted_buffer(a.ptr, b.ptr, 32, dbits);
+  WETRIC_TRY((prim::radix_sort_into(ctx, st, keys, keys, a.ptr, b.ptr, prim::KeysTo{by_degree}, n,
+                                    32, dbits, err)));
+  const GroupKeys gkeys{by_degree, group_base, G};
+  return prim::radix_sort_into(ctx, st, gkeys, gkeys, by_degree == a.ptr ? b.ptr : a.ptr,
+                               by_degree, RankTo{rank}, n, 32, bits_for(G - 1), err);
 }
 
 // Sorted packed (row, col) keys -> CSR arrays.
 int keys_to_csr(DeviceContext *ctx, cudaStream_t st, const uint64_t *keys,
                 uint64_t m, uint64_t n, uint32_t b, uint64_t *row_ptr,
                 uint32_t *col_ind) {
-  Scratch<uint32_t> cnt;
-  WETRIC_TRY(cnt.alloc(ctx, st, n));
-  WETRIC_CUDA_TRY(cudaMemsetAsync(cnt.ptr, 0, n * sizeof(uint32_t), st));
-  if (m > 0) {
-    k_row_histogram<<<grid_for(ctx, m), 256, 0, st>>>(keys, m, b, cnt.ptr);
-    WETRIC_LAUNCH_CHECK();
-    k_low_bits<<<grid_for(ctx, m), 256, 0, st>>>(keys, m, b, col_ind);
-    WETRIC_LAUNCH_CHECK();
+  if (m == 0) {
+    WETRIC_CUDA_TRY(cudaMemsetAsync(row_ptr, 0, (n + 1) * sizeof(uint64_t), st));
+    return WETRIC_OK;
   }
-  WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, cnt.ptr,
-                                                       row_ptr, n)));
+  k_keys_to_csr<<<grid_for(ctx, m), kThreads, 0, st>>>(keys, m, n, b, row_ptr, col_ind);
+  WETRIC_LAUNCH_CHECK();
   return WETRIC_OK;
 }
 
@@ -462,26 +478,22 @@ static int alloc_csr(DeviceContext *ctx, cudaStream_t st, uint64_t n,
   return WETRIC_OK;
 }
 
-// Raw pairs -> unique undirected edges as sorted canonical keys.
-static int unique_edges(DeviceContext *ctx, cudaStream_t st,
-                        const uint32_t *src, const uint32_t *dst, uint64_t P,
-                        uint64_t n_hint, uint64_t *n_out, uint32_t *b_out,
-                        Scratch<uint64_t> *ukeys, uint64_t *m_out) {
-  Scratch<uint32_t> small;
-  WETRIC_TRY(small.alloc(ctx, st, 4));
-  WETRIC_CUDA_TRY(cudaMemsetAsync(small.ptr, 0, 4 * sizeof(uint32_t), st));
+// Raw pairs -> unique undirected edges as sorted canonical keys (P slots,
+// words->m of them used) and the degrees of the n vertices. Reads m, the
+// largest degree and the checks back.
+static int unique_edges(DeviceContext *ctx, cudaStream_t st, const uint32_t *src,
+                        const uint32_t *dst, uint64_t P, uint64_t n_hint,
+                        const Scratch<PrepWords> &words, uint64_t *n_out, uint32_t *b_out,
+                        Scratch<uint64_t> *ukeys, Scratch<uint32_t> *deg, PrepWords *h) {
   uint64_t n = n_hint;
   if (n == 0) {
     if (P > 0) {
-      k_max_id<<<grid_for(ctx, P), 256, 0, st>>>(src, dst, P, small.ptr,
-                                                 small.ptr + 1);
+      k_max_id<<<grid_for(ctx, P), 256, 0, st>>>(src, dst, P, &words.ptr->max_id,
+                                                 &words.ptr->any_edge);
       WETRIC_LAUNCH_CHECK();
     }
-    uint32_t h[2] = {0, 0};
-    WETRIC_CUDA_TRY(cudaMemcpyAsync(h, small.ptr, 2 * sizeof(uint32_t),
-                                    cudaMemcpyDeviceToHost, st));
-    WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
-    n = (uint64_t)h[0] + 1;  // tc.cu:625, max_vertex starts at 0
+    WETRIC_TRY(read_words(st, words.ptr, h));
+    n = (uint64_t)h->max_id + 1;  // tc.cu:625, max_vertex starts at 0
   }
   if (n > (1ull << 32)) {
     set_error(WETRIC_ERANGE, "n = %llu exceeds 2^32", (unsigned long long)n);
@@ -493,36 +505,36 @@ static int unique_edges(DeviceContext *ctx, cudaStream_t st,
   Scratch<uint64_t> keys, alt;
   WETRIC_TRY(keys.alloc(ctx, st, P));
   WETRIC_TRY(alt.alloc(ctx, st, P));
+  WETRIC_TRY(deg->alloc(ctx, st, n));
+  WETRIC_CUDA_TRY(cudaMemsetAsync(deg->ptr, 0, n * sizeof(uint32_t), st));
+  const CanonPairs<true> counted{src, dst, b, n, sentinel, &words.ptr->err};
+  const CanonPairs<false> canon{src, dst, b, n, sentinel, nullptr};
+  uint64_t *sorted = prim::sorted_buffer(keys.ptr, alt.ptr, 0, 2 * b);
+  WETRIC_TRY((prim::radix_sort_into(ctx, st, counted, canon, keys.ptr, alt.ptr,
+                                    prim::KeysTo{sorted}, P, 0, 2 * b, &words.ptr->err)));
+  uint64_t *spare = sorted == keys.ptr ? alt.ptr : keys.ptr;
   if (P > 0) {
-    k_canon_keys<<<grid_for(ctx, P), 256, 0, st>>>(src, dst, P, b, n, sentinel,
-                                                   keys.ptr, small.ptr + 2);
+    const uint64_t tiles = ceil_div(P, kUniqueTile);
+    Scratch<uint64_t> state;  // [0] the ticket, then one word per tile
+    WETRIC_TRY(state.alloc(ctx, st, tiles + 1));
+    WETRIC_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (tiles + 1) * sizeof(uint64_t), st));
+    k_unique_degrees<<<(unsigned)tiles, kThreads, 0, st>>>(
+        sorted, P, sentinel, b, spare, deg->ptr, state.ptr + 1,
+        reinterpret_cast<uint32_t *>(state.ptr), &words.ptr->m, &words.ptr->err);
     WETRIC_LAUNCH_CHECK();
   }
-  WETRIC_TRY(dev_error(st, small.ptr + 2, "edge ids"));
-  bool in_alt = false;
-  WETRIC_TRY((prim::radix_sort<uint64_t, uint32_t>(
-      ctx, st, keys.ptr, alt.ptr, nullptr, nullptr, P, 2 * b, &in_alt)));
-  uint64_t *sorted = in_alt ? alt.ptr : keys.ptr;
-  uint64_t *spare = in_alt ? keys.ptr : alt.ptr;
-  uint64_t m = 0;
-  WETRIC_TRY(unique_sorted(ctx, st, sorted, P, sentinel, spare, &m));
+  k_max_u32<<<max_grid(ctx, n), kThreads, 0, st>>>(deg->ptr, n, &words.ptr->maxdeg);
+  WETRIC_LAUNCH_CHECK();
   // Keep the buffer that holds the unique keys; release the other.
-  if (in_alt) {
-    alt.release();
-    ukeys->ctx = keys.ctx;
-    ukeys->stream = keys.stream;
-    ukeys->bytes = keys.bytes;
-    ukeys->ptr = keys.detach();
-  } else {
-    keys.release();
-    ukeys->ctx = alt.ctx;
-    ukeys->stream = alt.stream;
-    ukeys->bytes = alt.bytes;
-    ukeys->ptr = alt.detach();
-  }
+  Scratch<uint64_t> &kept = spare == keys.ptr ? keys : alt;
+  (spare == keys.ptr ? alt : keys).release();
+  ukeys->ctx = kept.ctx;
+  ukeys->stream = kept.stream;
+  ukeys->bytes = kept.bytes;
+  ukeys->ptr = kept.detach();
+  WETRIC_TRY(checked_words(st, words.ptr, "edge ids", h));
   *n_out = n;
   *b_out = b;
-  *m_out = m;
   return WETRIC_OK;
 }
 
@@ -530,69 +542,58 @@ int orient_pairs(DeviceContext *ctx, cudaStream_t st, const uint32_t *src,
                  const uint32_t *dst, uint64_t P, uint64_t n_hint,
                  DeviceCsr *out, const uint64_t *group_base, uint32_t G) {
   NvtxRange nvtx_("wetric orient");
-  uint64_t n = 0, m = 0;
+  uint64_t n = 0;
   uint32_t b = 0;
+  PrepWords h{};
+  Scratch<PrepWords> words;
   Scratch<uint64_t> ukeys;
-  WETRIC_TRY(unique_edges(ctx, st, src, dst, P, n_hint, &n, &b, &ukeys, &m));
   Scratch<uint32_t> deg, rank;
-  WETRIC_TRY(deg.alloc(ctx, st, n));
+  WETRIC_TRY(alloc_words(ctx, st, &words));
+  WETRIC_TRY(unique_edges(ctx, st, src, dst, P, n_hint, words, &n, &b, &ukeys, &deg, &h));
+  const uint64_t m = h.m;
+  uint32_t *err = &words.ptr->err;
   WETRIC_TRY(rank.alloc(ctx, st, n));
-  WETRIC_CUDA_TRY(cudaMemsetAsync(deg.ptr, 0, n * sizeof(uint32_t), st));
-  if (m > 0) {
-    k_degree_undirected<<<grid_for(ctx, m), 256, 0, st>>>(ukeys.ptr, m, b,
-                                                          deg.ptr);
-    WETRIC_LAUNCH_CHECK();
-  }
-  if (group_base != nullptr && G > 1) {
-    WETRIC_TRY(grouped_degree_rank(ctx, st, deg.ptr, n, group_base, G, rank.ptr));
-  } else {
-    WETRIC_TRY(degree_rank(ctx, st, deg.ptr, n, rank.ptr));
-  }
+  WETRIC_TRY(degree_rank(ctx, st, deg.ptr, n, h.maxdeg, rank.ptr, err, group_base, G));
   deg.release();
-  // Orientation rewrites each unique key in place (element i reads and
-  // writes only position i), so only the sort's second buffer is new: the
-  // peak stays at input pairs + 2 key buffers (m > 2^32 fits 180 GB).
-  if (m > 0) {
-    k_orient_keys<<<grid_for(ctx, m), 256, 0, st>>>(ukeys.ptr, m, b, rank.ptr,
-                                                    ukeys.ptr);
-    WETRIC_LAUNCH_CHECK();
-  }
+  // The oriented keys go to the sort's second buffer, so the peak stays at
+  // input pairs + 2 key buffers (m > 2^32 fits 180 GB).
+  Scratch<uint64_t> okeys;
+  WETRIC_TRY(okeys.alloc(ctx, st, m));
+  uint64_t *sorted = prim::sorted_buffer(ukeys.ptr, okeys.ptr, 0, 2 * b);
+  WETRIC_TRY((prim::radix_sort_into(
+      ctx, st, OrientedKeys{ukeys.ptr, rank.ptr, okeys.ptr, b}, prim::KeysFrom{okeys.ptr},
+      ukeys.ptr, okeys.ptr, prim::KeysTo{sorted}, m, 0, 2 * b, err)));
   rank.release();
-  Scratch<uint64_t> oalt;
-  WETRIC_TRY(oalt.alloc(ctx, st, m));
-  bool in_alt = false;
-  WETRIC_TRY((prim::radix_sort<uint64_t, uint32_t>(
-      ctx, st, ukeys.ptr, oalt.ptr, nullptr, nullptr, m, 2 * b, &in_alt)));
-  const uint64_t *sorted = in_alt ? oalt.ptr : ukeys.ptr;
   WETRIC_TRY(alloc_csr(ctx, st, n, m, out));
   WETRIC_TRY(keys_to_csr(ctx, st, sorted, m, n, b, out->row_ptr, out->col_ind));
-  return WETRIC_OK;
+  return checked_words(st, words.ptr, "orientation", &h);
 }
 
 int symmetric_from_pairs(DeviceContext *ctx, cudaStream_t st,
                          const uint32_t *src, const uint32_t *dst, uint64_t P,
                          uint64_t n_hint, DeviceCsr *out) {
-  uint64_t n = 0, m = 0;
+  uint64_t n = 0;
   uint32_t b = 0;
+  PrepWords h{};
+  Scratch<PrepWords> words;
   Scratch<uint64_t> ukeys;
-  WETRIC_TRY(unique_edges(ctx, st, src, dst, P, n_hint, &n, &b, &ukeys, &m));
+  Scratch<uint32_t> deg;
+  WETRIC_TRY(alloc_words(ctx, st, &words));
+  WETRIC_TRY(unique_edges(ctx, st, src, dst, P, n_hint, words, &n, &b, &ukeys, &deg, &h));
+  deg.release();
+  const uint64_t m = h.m;
   Scratch<uint64_t> dkeys, dalt;
   WETRIC_TRY(dkeys.alloc(ctx, st, 2 * m));
   WETRIC_TRY(dalt.alloc(ctx, st, 2 * m));
-  if (m > 0) {
-    k_both_directions<<<grid_for(ctx, m), 256, 0, st>>>(ukeys.ptr, m, b,
-                                                        dkeys.ptr);
-    WETRIC_LAUNCH_CHECK();
-  }
+  const BothDirections both{ukeys.ptr, b};
+  uint64_t *sorted = prim::sorted_buffer(dkeys.ptr, dalt.ptr, 0, 2 * b);
+  WETRIC_TRY((prim::radix_sort_into(ctx, st, both, both, dkeys.ptr, dalt.ptr,
+                                    prim::KeysTo{sorted}, 2 * m, 0, 2 * b, &words.ptr->err)));
   ukeys.release();
-  bool in_alt = false;
-  WETRIC_TRY((prim::radix_sort<uint64_t, uint32_t>(
-      ctx, st, dkeys.ptr, dalt.ptr, nullptr, nullptr, 2 * m, 2 * b, &in_alt)));
-  const uint64_t *sorted = in_alt ? dalt.ptr : dkeys.ptr;
   WETRIC_TRY(alloc_csr(ctx, st, n, 2 * m, out));
   WETRIC_TRY(
       keys_to_csr(ctx, st, sorted, 2 * m, n, b, out->row_ptr, out->col_ind));
-  return WETRIC_OK;
+  return checked_words(st, words.ptr, "symmetric CSR", &h);
 }
 
 int orient_csr(DeviceContext *ctx, cudaStream_t st, const uint64_t *rp,
@@ -606,21 +607,23 @@ int orient_csr(DeviceContext *ctx, cudaStream_t st, const uint64_t *rp,
     set_error(WETRIC_ERANGE, "n = %llu exceeds 2^32", (unsigned long long)n);
     return WETRIC_ERANGE;
   }
-  Scratch<uint32_t> err;
-  WETRIC_TRY(err.alloc(ctx, st, 1));
-  WETRIC_CUDA_TRY(cudaMemsetAsync(err.ptr, 0, sizeof(uint32_t), st));
-  k_check_ids<<<grid_for(ctx, m > n ? m : n), 256, 0, st>>>(rp, ci, n, m,
-                                                           err.ptr);
-  WETRIC_LAUNCH_CHECK();
-  WETRIC_TRY(dev_error(st, err.ptr, "csr"));
-  uint32_t b = bits_for(n - 1);
-  if (b == 0) b = 1;
+  PrepWords h{};
+  Scratch<PrepWords> words;
   Scratch<uint32_t> deg, rank;
+  WETRIC_TRY(alloc_words(ctx, st, &words));
+  uint32_t *err = &words.ptr->err;
+  k_check_ids<<<grid_for(ctx, m > n ? m : n), 256, 0, st>>>(rp, ci, n, m, err);
+  WETRIC_LAUNCH_CHECK();
   WETRIC_TRY(deg.alloc(ctx, st, n));
   WETRIC_TRY(rank.alloc(ctx, st, n));
   k_row_lengths<<<grid_for(ctx, n), 256, 0, st>>>(rp, n, deg.ptr);
   WETRIC_LAUNCH_CHECK();
-  WETRIC_TRY(degree_rank(ctx, st, deg.ptr, n, rank.ptr));
+  k_max_u32<<<max_grid(ctx, n), kThreads, 0, st>>>(deg.ptr, n, &words.ptr->maxdeg);
+  WETRIC_LAUNCH_CHECK();
+  WETRIC_TRY(checked_words(st, words.ptr, "csr", &h));
+  uint32_t b = bits_for(n - 1);
+  if (b == 0) b = 1;
+  WETRIC_TRY(degree_rank(ctx, st, deg.ptr, n, h.maxdeg, rank.ptr, err));
   // deg is reused as the per-row kept count.
   const unsigned warps_grid = grid_for(ctx, n * 32);
   k_kept_per_row<<<warps_grid, 256, 0, st>>>(rp, ci, n, rank.ptr, deg.ptr);
@@ -628,9 +631,11 @@ int orient_csr(DeviceContext *ctx, cudaStream_t st, const uint64_t *rp,
   Scratch<uint64_t> off;
   WETRIC_TRY(off.alloc(ctx, st, n + 1));
   WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, deg.ptr,
-                                                       off.ptr, n)));
-  uint64_t kept = 0;
-  WETRIC_TRY(read_u64(st, off.ptr + n, &kept));
+                                                       off.ptr, n, err)));
+  WETRIC_CUDA_TRY(cudaMemcpyAsync(&words.ptr->m, off.ptr + n, sizeof(uint64_t),
+                                  cudaMemcpyDeviceToDevice, st));
+  WETRIC_TRY(checked_words(st, words.ptr, "csr", &h));
+  const uint64_t kept = h.m;
   Scratch<uint64_t> okeys, oalt;
   WETRIC_TRY(okeys.alloc(ctx, st, kept));
   WETRIC_TRY(oalt.alloc(ctx, st, kept));
@@ -640,14 +645,14 @@ int orient_csr(DeviceContext *ctx, cudaStream_t st, const uint64_t *rp,
   deg.release();
   rank.release();
   off.release();
-  bool in_alt = false;
-  WETRIC_TRY((prim::radix_sort<uint64_t, uint32_t>(
-      ctx, st, okeys.ptr, oalt.ptr, nullptr, nullptr, kept, 2 * b, &in_alt)));
-  const uint64_t *sorted = in_alt ? oalt.ptr : okeys.ptr;
+  const prim::KeysFrom from{okeys.ptr};
+  uint64_t *sorted = prim::sorted_buffer(oalt.ptr, okeys.ptr, 0, 2 * b);
+  WETRIC_TRY((prim::radix_sort_into(ctx, st, from, from, oalt.ptr, okeys.ptr,
+                                    prim::KeysTo{sorted}, kept, 0, 2 * b, err)));
   WETRIC_TRY(alloc_csr(ctx, st, n, kept, out));
   WETRIC_TRY(
       keys_to_csr(ctx, st, sorted, kept, n, b, out->row_ptr, out->col_ind));
-  return WETRIC_OK;
+  return checked_words(st, words.ptr, "csr", &h);
 }
 
 }  // namespace wetric

@@ -2,9 +2,15 @@
 // written for this library in place of the CUB calls of the reference
 // (DeviceRadixSort / DeviceSegmentedSort, tc.cu:500-558).
 //
-// Neither primitive waits on another block: the scan is reduce-then-scan
-// (three launches) and the sort is histogram / scan / scatter per digit,
-// so no kernel here can spin.
+// Both are single pass over the data per step: a block takes its tile from a
+// ticket counter, publishes its totals and looks back over its
+// predecessors' published totals for its offset ("decoupled look-back",
+// Merrill and Garland, "Single-pass parallel prefix scan with decoupled
+// look-back", 2016; for the sort, Adinets and Merrill, "Onesweep", 2022).
+// Tickets are handed out in order to running blocks, so a block only ever
+// waits on blocks that are already running. Every wait is bounded all the
+// same: on running out it records kDevLookbackTimeout, publishes a poison
+// word that ends its successors' waits, and the block leaves.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -14,14 +20,101 @@
 namespace wetric {
 namespace prim {
 
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
-constexpr int kScanChunk = kScanThreads * kScanItems;
+// Published words: value in the low 48 bits, (epoch << 2 | flag) above it.
+// A word of another epoch reads as "not published yet", so one clearing of
+// the words serves every pass of a sort.
+constexpr uint32_t kTileAgg = 1, kTileIncl = 2, kTilePoison = 3;
+constexpr uint64_t kTileValueMask = (1ull << 48) - 1;
+constexpr uint32_t kLookbackSpins = 1u << 22;
 
-// Inclusive scan of one value per thread across a 256-thread block.
-// Returns the inclusive prefix; *total receives the block total.
-template <typename T>
+__device__ __forceinline__ uint64_t tile_word(uint32_t epoch, uint32_t flag, uint64_t value) {
+  return ((uint64_t)(epoch << 2 | flag) << 48) | value;
+}
+__device__ __forceinline__ uint32_t tile_flag(uint64_t w, uint32_t epoch) {
+  const uint32_t tag = (uint32_t)(w >> 48);
+  return (tag >> 2) == epoch ? (tag & 3u) : 0u;
+}
+__device__ __forceinline__ uint64_t ld_tile(const uint64_t *p) {
+  uint64_t v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_tile(uint64_t *p, uint64_t v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// Exclusive prefix of `agg` over the tiles before `tile` (a whole warp
+// calls it; one word per tile). A step looks at 128 predecessors, four per
+// lane: all tiles of a short scan start together, so the last one walks back
+// over all of them. Returns false when a wait ran out.
+constexpr int kLookWide = 4;
+__device__ __forceinline__ bool tile_prefix(uint64_t *state, uint64_t tile, uint64_t agg,
+                                            uint32_t *err, uint64_t *excl) {
+  const uint32_t lane = threadIdx.x & 31;
+  *excl = 0;
+  if (tile == 0) {
+    if (lane == 0) st_tile(state, tile_word(0, kTileIncl, agg));
+    return true;
+  }
+  if (lane == 0) st_tile(state + tile, tile_word(0, kTileAgg, agg));
+  uint64_t sum = 0;
+  for (int64_t hi = (int64_t)tile - 1;; hi -= 32 * kLookWide) {
+    // word j of the lane: predecessor j * 32 + lane of the window
+    uint64_t w[kLookWide];
+    uint32_t spins = 0;
+    bool bad = false;
+    for (;;) {
+      bool ready = true;
+#pragma unroll
+      for (int j = 0; j < kLookWide; ++j) {
+        const int64_t at = hi - j * 32 - lane;
+        w[j] = at >= 0 ? ld_tile(state + at) : tile_word(0, kTileIncl, 0);
+      }
+#pragma unroll
+      for (int j = 0; j < kLookWide; ++j) {
+        const uint32_t f = tile_flag(w[j], 0);
+        ready = ready && f != 0;
+        bad = bad || f == kTilePoison;
+      }
+      if (__any_sync(0xffffffffu, bad) || __all_sync(0xffffffffu, ready)) break;
+      if (++spins > kLookbackSpins) {
+        bad = true;
+        break;
+      }
+    }
+    if (__any_sync(0xffffffffu, bad)) {
+      if (lane == 0) {
+        atomicCAS(err, 0u, (uint32_t)kDevLookbackTimeout);
+        st_tile(state + tile, tile_word(0, kTilePoison, 0));
+      }
+      return false;
+    }
+    // up to the nearest inclusive word
+    bool found = false;
+    uint64_t v = 0;
+#pragma unroll
+    for (int j = 0; j < kLookWide; ++j) {
+      const uint32_t incl = __ballot_sync(0xffffffffu, tile_flag(w[j], 0) == kTileIncl);
+      const uint32_t last = incl ? __ffs(incl) - 1 : 31;
+      if (!found && lane <= last) v += w[j] & kTileValueMask;
+      found = found || incl;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    sum += v;
+    if (found) break;
+  }
+  if (lane == 0) st_tile(state + tile, tile_word(0, kTileIncl, sum + agg));
+  *excl = sum;
+  return true;
+}
+
+// Inclusive scan of one value per thread across a block of kThreads.
+// Returns the inclusive prefix; *total receives the block total. smem_warp
+// holds kThreads / 32 values.
+template <int kThreads, typename T>
 __device__ __forceinline__ T block_inclusive_scan(T v, T *smem_warp, T *total) {
+  constexpr int kWarps = kThreads / 32;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
 #pragma unroll
@@ -32,236 +125,458 @@ __device__ __forceinline__ T block_inclusive_scan(T v, T *smem_warp, T *total) {
   if (lane == 31) smem_warp[warp] = v;
   __syncthreads();
   if (warp == 0) {
-    T w = lane < (kScanThreads / 32) ? smem_warp[lane] : T(0);
+    T w = lane < kWarps ? smem_warp[lane] : T(0);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       T y = __shfl_up_sync(0xffffffffu, w, o);
       if (lane >= o) w += y;
     }
-    if (lane < (kScanThreads / 32)) smem_warp[lane] = w;
+    if (lane < kWarps) smem_warp[lane] = w;
   }
   __syncthreads();
   if (warp > 0) v += smem_warp[warp - 1];
-  *total = smem_warp[kScanThreads / 32 - 1];
+  *total = smem_warp[kWarps - 1];
   return v;
 }
 
-template <typename InT, typename OutT>
-__global__ void __launch_bounds__(kScanThreads)
-    scan_reduce_kernel(const InT *__restrict__ in, uint64_t n,
-                       OutT *__restrict__ block_sums) {
-  __shared__ OutT warp_sums[kScanThreads / 32];
-  const uint64_t base =
-      (uint64_t)blockIdx.x * kScanChunk + (uint64_t)threadIdx.x * kScanItems;
-  OutT s = 0;
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    const uint64_t i = base + j;
-    if (i < n) s += (OutT)in[i];
-  }
-  OutT total;
-  block_inclusive_scan<OutT>(s, warp_sums, &total);
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
+// ------------------------------------------------------------------- scan
 
-// out[i] = offset(block) + exclusive prefix within the block. When
-// block_offsets is null the offset is 0. The block that owns element n-1
-// (or block 0 when n == 0) also writes out[n] = total.
+constexpr int kScanThreads = 256;
+constexpr int kScanItems = 16;
+constexpr int kScanChunk = kScanThreads * kScanItems;
+
+// out[i] = exclusive prefix of in, out[n] = total, in one pass, the tile's
+// offset by look-back (state null: a single tile). Item j of lane l is
+// element j * 32 + l of the warp's 512, so loads and stores are whole lines
+// and each item is a warp scan on top of the last one's total. Bound
+// by the latency of the look-back (4.2M u32 -> u64: 27 us): on the device
+// it takes as long as the reduce, scan and apply launches it replaces, and
+// saves the host two launches of three.
 template <typename InT, typename OutT>
 __global__ void __launch_bounds__(kScanThreads)
-    scan_apply_kernel(const InT *in, uint64_t n, OutT *out,
-                      const OutT *__restrict__ block_offsets) {
-  __shared__ OutT warp_sums[kScanThreads / 32];
-  const uint64_t base =
-      (uint64_t)blockIdx.x * kScanChunk + (uint64_t)threadIdx.x * kScanItems;
+    k_scan(const InT *in, uint64_t n, OutT *out, uint64_t *state, uint32_t *ticket,
+           uint32_t *err) {
+  __shared__ OutT s_warp[kScanThreads / 32];
+  __shared__ uint64_t s_excl;
+  __shared__ uint32_t s_tile, s_ok;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t tile = 0;
+  if (state) {
+    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    __syncthreads();
+    tile = s_tile;
+  }
+  const uint64_t base = tile * kScanChunk + (uint64_t)warp * 32 * kScanItems + lane;
   OutT vals[kScanItems];
-  OutT s = 0;
 #pragma unroll
   for (int j = 0; j < kScanItems; ++j) {
-    const uint64_t i = base + j;
+    const uint64_t i = base + (uint64_t)j * 32;
     vals[j] = i < n ? (OutT)in[i] : OutT(0);
-    s += vals[j];
   }
-  OutT total;
-  OutT incl = block_inclusive_scan<OutT>(s, warp_sums, &total);
-  OutT run = incl - s + (block_offsets ? block_offsets[blockIdx.x] : OutT(0));
+  OutT run = 0;  // of the warp's items so far
 #pragma unroll
   for (int j = 0; j < kScanItems; ++j) {
-    const uint64_t i = base + j;
-    if (i < n) out[i] = run;
-    run += vals[j];
+    OutT x = vals[j];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const OutT y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    vals[j] = run + x - vals[j];
+    run += __shfl_sync(0xffffffffu, x, 31);
   }
-  const uint64_t block_end = (uint64_t)(blockIdx.x + 1) * kScanChunk;
-  if (threadIdx.x == kScanThreads - 1 && block_end >= n) {
-    out[n] = (block_offsets ? block_offsets[blockIdx.x] : OutT(0)) + total;
+  if (lane == 0) s_warp[warp] = run;
+  __syncthreads();
+  OutT off = 0, total = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < kScanThreads / 32; ++w) {
+    if (w < warp) off += s_warp[w];
+    total += s_warp[w];
   }
+  uint64_t before = 0;
+  if (state) {
+    if (warp == 0) {
+      uint64_t excl = 0;
+      const bool ok = tile_prefix(state, tile, (uint64_t)total, err, &excl);
+      if (lane == 0) {
+        s_excl = excl;
+        s_ok = ok;
+      }
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    before = s_excl;
+  }
+  off += (OutT)before;
+#pragma unroll
+  for (int j = 0; j < kScanItems; ++j) {
+    const uint64_t i = base + (uint64_t)j * 32;
+    if (i < n) out[i] = off + vals[j];
+  }
+  if (threadIdx.x == 0 && (tile + 1) * kScanChunk >= n) out[n] = (OutT)before + total;
 }
 
 // out[0..n] = exclusive prefix of in[0..n-1]; out[n] = total. out may alias
-// in when InT == OutT.
+// in when InT == OutT (a tile reads its items before it writes them). A
+// look-back that runs out is recorded in *err (device).
 template <typename InT, typename OutT>
 int exclusive_scan(DeviceContext *ctx, cudaStream_t st, const InT *in,
-                   OutT *out, uint64_t n) {
-  const uint64_t blocks = n == 0 ? 1 : ceil_div(n, kScanChunk);
-  if (blocks == 1) {
-    scan_apply_kernel<InT, OutT><<<1, kScanThreads, 0, st>>>(in, n, out,
-                                                             nullptr);
+                   OutT *out, uint64_t n, uint32_t *err) {
+  const uint64_t tiles = n == 0 ? 1 : ceil_div(n, kScanChunk);
+  if (tiles == 1) {
+    k_scan<InT, OutT><<<1, kScanThreads, 0, st>>>(in, n, out, nullptr, nullptr, err);
     WETRIC_LAUNCH_CHECK();
     return WETRIC_OK;
   }
-  Scratch<OutT> sums;
-  WETRIC_TRY(sums.alloc(ctx, st, blocks + 1));
-  scan_reduce_kernel<InT, OutT><<<(unsigned)blocks, kScanThreads, 0, st>>>(
-      in, n, sums.ptr);
-  WETRIC_LAUNCH_CHECK();
-  WETRIC_TRY((exclusive_scan<OutT, OutT>(ctx, st, sums.ptr, sums.ptr, blocks)));
-  scan_apply_kernel<InT, OutT><<<(unsigned)blocks, kScanThreads, 0, st>>>(
-      in, n, out, sums.ptr);
+  Scratch<uint64_t> state;  // [0] the ticket, then one word per tile
+  WETRIC_TRY(state.alloc(ctx, st, tiles + 1));
+  WETRIC_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (tiles + 1) * sizeof(uint64_t), st));
+  k_scan<InT, OutT><<<(unsigned)tiles, kScanThreads, 0, st>>>(
+      in, n, out, state.ptr + 1, reinterpret_cast<uint32_t *>(state.ptr), err);
   WETRIC_LAUNCH_CHECK();
   return WETRIC_OK;
 }
 
 // ------------------------------------------------------------ radix sort
 
-constexpr int kSortThreads = 256;
+constexpr int kSortThreads = 384;
+constexpr int kSortBlocks = 3;  // per SM
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 8;  // per lane
+constexpr int kSortItems = 16;  // per thread
 constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
+constexpr int kMaxPasses = 8;
 
-// Tile layout (shared by the histogram and scatter kernels, which is what
-// keeps the sort stable): warp w of tile t owns the contiguous keys
-// [t*Tile + w*32*Items, +32*Items); item j of lane l is key
-// [that base + j*32 + l], so every load is coalesced and the order
-// (warp, item, lane) is the input order.
-template <typename K>
-__global__ void __launch_bounds__(kSortThreads)
-    radix_hist_kernel(const K *__restrict__ keys, uint64_t n, uint32_t shift,
-                      uint64_t num_tiles, uint32_t *__restrict__ counts) {
-  __shared__ uint32_t hist[kRadix];
-  for (int d = threadIdx.x; d < kRadix; d += kSortThreads) hist[d] = 0;
+// The passes of a sort over `bits` key bits from bit `lo`: as few as
+// 8-bit digits allow, of even widths (narrow digits make longer runs).
+struct DigitPlan {
+  uint32_t passes;
+  uint32_t shift[kMaxPasses], bits[kMaxPasses];
+};
+inline DigitPlan digit_plan(uint32_t lo, uint32_t bits) {
+  DigitPlan p{};
+  p.passes = (bits + kRadixBits - 1) / kRadixBits;
+  uint32_t at = lo;
+  for (uint32_t i = 0; i < p.passes; ++i) {
+    p.bits[i] = (lo + bits - at + (p.passes - i) - 1) / (p.passes - i);
+    p.shift[i] = at;
+    at += p.bits[i];
+  }
+  return p;
+}
+
+// Where a pass takes its keys from and what it does with each at its sorted
+// position.
+struct KeysFrom {
+  const uint64_t *__restrict__ keys;
+  __device__ __forceinline__ uint64_t operator()(uint64_t i) const { return keys[i]; }
+};
+struct KeysTo {
+  uint64_t *__restrict__ keys;
+  __device__ __forceinline__ void operator()(uint64_t i, uint64_t k) const { keys[i] = k; }
+};
+
+// Histograms of every digit in one read of the keys (bound by the
+// shared-memory atomics: 0.26 ms for 67M keys of six digits). Four copies per block
+// in shared memory (lane & 3 picks one), since the digits of graph keys are
+// skewed and a warp's equal digits serialise on one counter.
+constexpr int kHistCopies = 4;
+constexpr int kHistAhead = 4;
+template <class Load>
+__global__ void __launch_bounds__(256)
+    k_radix_hist(Load load, uint64_t n, const __grid_constant__ DigitPlan plan,
+                 unsigned long long *__restrict__ hist) {
+  extern __shared__ uint32_t s_hist[];  // [pass][digit][copy]
+  const uint32_t total = plan.passes * kRadix * kHistCopies;
+  for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) s_hist[i] = 0;
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const uint64_t sub = (uint64_t)blockIdx.x * kSortTile +
-                       (uint64_t)warp * 32 * kSortItems;
+  const uint32_t copy = threadIdx.x & (kHistCopies - 1);
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  auto add = [&](uint64_t k) {
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const uint64_t i = sub + (uint64_t)j * 32 + lane;
-    if (i < n) {
-      const uint32_t d = (uint32_t)(keys[i] >> shift) & (kRadix - 1);
-      atomicAdd(&hist[d], 1u);
+    for (int p = 0; p < kMaxPasses; ++p)
+      if (p < plan.passes) {
+        const uint32_t d = (uint32_t)(k >> plan.shift[p]) & ((1u << plan.bits[p]) - 1u);
+        atomicAdd(&s_hist[(p * kRadix + d) * kHistCopies + copy], 1u);
+      }
+  };
+  // several keys' loads in flight per thread
+  for (; i + (kHistAhead - 1) * stride < n; i += kHistAhead * stride) {
+    uint64_t k[kHistAhead];
+#pragma unroll
+    for (int j = 0; j < kHistAhead; ++j) k[j] = load(i + j * stride);
+#pragma unroll
+    for (int j = 0; j < kHistAhead; ++j) add(k[j]);
+  }
+  for (; i < n; i += stride) add(load(i));
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < plan.passes * kRadix; i += blockDim.x) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int j = 0; j < kHistCopies; ++j) c += s_hist[i * kHistCopies + j];
+    if (c) atomicAdd(&hist[i], (unsigned long long)c);
+  }
+}
+
+// The digit of a key: bits [shift, shift + kBits) of its 64, masked to the
+// pass's width. kHigh: shift >= 32.
+template <bool kHigh>
+__device__ __forceinline__ uint32_t key_digit(uint64_t k, uint32_t shift, uint32_t mask) {
+  const uint32_t lo = (uint32_t)k, hi = (uint32_t)(k >> 32);
+  return (kHigh ? hi >> (shift - 32) : __funnelshift_r(lo, hi, shift)) & mask;
+}
+
+// Lanes of `valid` with the same digit, by one ballot per digit bit: the
+// cost does not depend on the digits (match.any took two to three times as
+// long on digits with many values as on skewed ones).
+template <int kBits>
+__device__ __forceinline__ uint32_t match_digit(uint32_t d, uint32_t valid) {
+  uint32_t m = valid;
+#pragma unroll
+  for (int b = 0; b < kBits; ++b) {
+    const bool bit = (d >> b) & 1u;
+    const uint32_t bal = __ballot_sync(0xffffffffu, bit);
+    m &= bit ? bal : ~bal;
+  }
+  return m;
+}
+
+// One pass: a block ranks its tile's keys by digit (warp w owns the
+// contiguous keys [w*32*Items, +32*Items) of the tile, item j of lane l is
+// key j*32 + l of them, so (warp, item, lane) is the input order and the
+// sort is stable), publishes the tile's digit counts, orders the keys in
+// shared memory, finds each digit's global offset by look-back (thread d
+// walks digit d, four predecessors at a time) and writes whole runs. Bound
+// by instruction issue (about 100 warp instructions per 32 keys, a third of
+// them the ballots): 0.36 ms per pass of 64M keys, 8-bit digits, where the
+// histogram, scan and scatter it replaces took 0.6-0.8 ms with scattered
+// 8-byte stores. Tile shape from a sweep at 64M 44-bit keys, whole sort: 384
+// threads x 16 keys x 3 blocks 2.46 ms, 512 x 16 x 2 2.48, 256 x 16 x 4 2.84,
+// 1024 x 12 x 1 2.97, 512 x 8 x 3 2.92; five 9-bit passes 2.61 (512 x 16).
+constexpr size_t kSortSmem = kSortTile * sizeof(uint64_t) +
+                             kSortWarps * kRadix * sizeof(uint32_t) +
+                             kRadix * (sizeof(uint64_t) + sizeof(uint32_t));
+constexpr int kLookAhead = 4;
+template <int kBits, bool kHigh, class Load, class Sink>
+__global__ void __launch_bounds__(kSortThreads, kSortBlocks)
+    k_onesweep(Load load, Sink sink, uint64_t n, uint32_t shift, uint32_t bits, uint32_t epoch,
+               const unsigned long long *__restrict__ hist, uint64_t *__restrict__ state,
+               uint32_t *__restrict__ ticket, uint32_t *err) {
+  static_assert(kSortThreads >= kRadix, "thread d owns digit d");
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  uint64_t *s_key = reinterpret_cast<uint64_t *>(s_raw);
+  uint64_t *s_goff = s_key + kSortTile;
+  uint32_t *s_toff = reinterpret_cast<uint32_t *>(s_goff + kRadix);
+  uint32_t *s_whist = s_toff + kRadix;
+  __shared__ uint32_t s_warp[kSortWarps];
+  __shared__ unsigned long long s_warp64[kSortWarps];
+  __shared__ uint32_t s_ticket, s_bad;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    s_ticket = atomicAdd(ticket, 1u);
+    s_bad = 0;
+  }
+  for (uint32_t i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads) s_whist[i] = 0;
+  __syncthreads();
+  const uint64_t tile = s_ticket;
+  const uint64_t base = tile * kSortTile;
+  const uint32_t count = n - base < kSortTile ? (uint32_t)(n - base) : kSortTile;
+  const uint32_t mask = (1u << bits) - 1u;
+  const uint32_t sub = warp * 32 * kSortItems + lane;
+  uint32_t *wh = s_whist + warp * kRadix;
+  uint64_t k[kSortItems];
+  uint16_t rank[kSortItems];  // below 32 * kSortItems
+  const uint32_t lt = (1u << lane) - 1u;
+  if (count == kSortTile) {
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j) k[j] = load(base + sub + j * 32);
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j) {
+      const uint32_t d = key_digit<kHigh>(k[j], shift, mask);
+      const uint32_t peers = match_digit<kBits>(d, 0xffffffffu);
+      const uint32_t leader = __ffs(peers) - 1;
+      uint32_t before = 0;
+      if (lane == leader) before = atomicAdd(&wh[d], (uint32_t)__popc(peers));
+      rank[j] = (uint16_t)(__shfl_sync(0xffffffffu, before, leader) + __popc(peers & lt));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j)
+      k[j] = sub + j * 32 < count ? load(base + sub + j * 32) : 0;
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j) {
+      const bool valid = sub + j * 32 < count;
+      const uint32_t d = key_digit<kHigh>(k[j], shift, mask);
+      const uint32_t peers = match_digit<kBits>(d, __ballot_sync(0xffffffffu, valid));
+      const uint32_t leader = valid ? __ffs(peers) - 1 : lane;
+      uint32_t before = 0;
+      if (valid && lane == leader) before = atomicAdd(&wh[d], (uint32_t)__popc(peers));
+      rank[j] = (uint16_t)(__shfl_sync(0xffffffffu, before, leader) + __popc(peers & lt));
     }
   }
   __syncthreads();
-  for (int d = threadIdx.x; d < kRadix; d += kSortThreads)
-    counts[(uint64_t)d * num_tiles + blockIdx.x] = hist[d];
-}
-
-template <typename K, typename V, bool kHasValues>
-__global__ void __launch_bounds__(kSortThreads)
-    radix_scatter_kernel(const K *__restrict__ keys_in,
-                         const V *__restrict__ vals_in, uint64_t n,
-                         uint32_t shift, uint64_t num_tiles,
-                         const uint64_t *__restrict__ offsets,
-                         K *__restrict__ keys_out, V *__restrict__ vals_out) {
-  __shared__ uint32_t whist[kSortWarps][kRadix];
-  __shared__ uint64_t goff[kRadix];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  for (int d = threadIdx.x; d < kRadix; d += kSortThreads) {
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) whist[w][d] = 0;
-    goff[d] = offsets[(uint64_t)d * num_tiles + blockIdx.x];
-  }
-  __syncthreads();
-
-  const uint64_t sub = (uint64_t)blockIdx.x * kSortTile +
-                       (uint64_t)warp * 32 * kSortItems;
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  K k[kSortItems];
-  V v[kSortItems];
-  uint32_t rank[kSortItems];
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const uint64_t i = sub + (uint64_t)j * 32 + lane;
-    const bool valid = i < n;
-    k[j] = valid ? keys_in[i] : K(0);
-    if (kHasValues) v[j] = valid ? vals_in[i] : V(0);
-    const uint32_t d = (uint32_t)(k[j] >> shift) & (kRadix - 1);
-    const uint32_t tag = valid ? d : 0xFFFFFFFFu;
-    const uint32_t peers = __match_any_sync(0xffffffffu, tag);
-    uint32_t before = 0;
-    if (valid) before = whist[warp][d];
-    __syncwarp();
-    if (valid && lane == __ffs(peers) - 1) whist[warp][d] = before + __popc(peers);
-    __syncwarp();
-    rank[j] = before + __popc(peers & lt_mask);
-  }
-  __syncthreads();
-  for (int d = threadIdx.x; d < kRadix; d += kSortThreads) {
-    uint32_t run = 0;
+  // digit d's count in the tile, its warps' offsets within it
+  uint32_t c = 0;
+  if (threadIdx.x < kRadix) {
 #pragma unroll
     for (int w = 0; w < kSortWarps; ++w) {
-      const uint32_t c = whist[w][d];
-      whist[w][d] = run;
-      run += c;
+      const uint32_t x = s_whist[w * kRadix + threadIdx.x];
+      s_whist[w * kRadix + threadIdx.x] = c;
+      c += x;
     }
   }
+  uint64_t *word = state + tile * kRadix + threadIdx.x;
+  if (threadIdx.x < kRadix && tile > 0) st_tile(word, tile_word(epoch, kTileAgg, c));
+  uint32_t total;
+  const uint32_t incl = block_inclusive_scan<kSortThreads, uint32_t>(c, s_warp, &total);
+  if (threadIdx.x < kRadix) s_toff[threadIdx.x] = incl - c;
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j) {
-    const uint64_t i = sub + (uint64_t)j * 32 + lane;
-    if (i < n) {
-      const uint32_t d = (uint32_t)(k[j] >> shift) & (kRadix - 1);
-      const uint64_t pos = goff[d] + whist[warp][d] + rank[j];
-      keys_out[pos] = k[j];
-      if (kHasValues) vals_out[pos] = v[j];
+    if (sub + j * 32 < count) {
+      const uint32_t d = key_digit<kHigh>(k[j], shift, mask);
+      s_key[s_toff[d] + wh[d] + rank[j]] = k[j];
     }
+  }
+  if (tile == 0) {
+    // the first tile's inclusive words carry the digits' global starts
+    unsigned long long t64;
+    const unsigned long long h = threadIdx.x < kRadix ? hist[threadIdx.x] : 0;
+    const unsigned long long i64 =
+        block_inclusive_scan<kSortThreads, unsigned long long>(h, s_warp64, &t64);
+    if (threadIdx.x < kRadix) {
+      st_tile(word, tile_word(epoch, kTileIncl, i64 - h + c));
+      s_goff[threadIdx.x] = i64 - h - (incl - c);
+    }
+  } else if (threadIdx.x < kRadix) {
+    uint64_t sum = 0;
+    uint32_t spins = 0, done = 0;  // done: 1 = reached an inclusive word, 2 = gave up
+    for (uint64_t at = tile; !done;) {
+      // the words of the kLookAhead tiles before `at` (tile 0's is inclusive)
+      uint64_t w[kLookAhead];
+#pragma unroll
+      for (int j = 0; j < kLookAhead; ++j) {
+        const uint64_t q = at > (uint64_t)j ? at - 1 - j : 0;
+        w[j] = ld_tile(state + q * kRadix + threadIdx.x);
+      }
+#pragma unroll
+      for (int j = 0; j < kLookAhead; ++j) {
+        const uint32_t f = tile_flag(w[j], epoch);
+        if (f == 0) {
+          if (++spins > kLookbackSpins) done = 2;
+          break;
+        }
+        if (f == kTilePoison) {
+          done = 2;
+          break;
+        }
+        sum += w[j] & kTileValueMask;
+        --at;
+        if (f == kTileIncl) {
+          done = 1;
+          break;
+        }
+      }
+    }
+    if (done == 2) {
+      atomicCAS(err, 0u, (uint32_t)kDevLookbackTimeout);
+      s_bad = 1;
+      st_tile(word, tile_word(epoch, kTilePoison, 0));
+    } else {
+      st_tile(word, tile_word(epoch, kTileIncl, sum + c));
+      s_goff[threadIdx.x] = sum - (incl - c);
+    }
+  }
+  __syncthreads();
+  if (s_bad) return;
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < count; i += kSortThreads) {
+    const uint64_t key = s_key[i];
+    sink(s_goff[key_digit<kHigh>(key, shift, mask)] + i, key);
   }
 }
 
-// Stable LSD sort of keys (and optional values) on their low `bits` bits.
-// Ping-pongs between (keys, keys_alt); *result_in_alt tells which buffer
-// holds the sorted output.
-template <typename K, typename V>
-int radix_sort(DeviceContext *ctx, cudaStream_t st, K *keys, K *keys_alt,
-               V *vals, V *vals_alt, uint64_t n, uint32_t bits,
-               bool *result_in_alt) {
-  *result_in_alt = false;
-  if (n <= 1 || bits == 0) return WETRIC_OK;
-  const uint64_t num_tiles = ceil_div(n, kSortTile);
-  const uint64_t ncounts = (uint64_t)kRadix * num_tiles;
-  Scratch<uint32_t> counts;
-  Scratch<uint64_t> offsets;
-  WETRIC_TRY(counts.alloc(ctx, st, ncounts));
-  WETRIC_TRY(offsets.alloc(ctx, st, ncounts + 1));
-  K *kin = keys, *kout = keys_alt;
-  V *vin = vals, *vout = vals_alt;
-  bool in_alt = false;
-  for (uint32_t shift = 0; shift < bits; shift += kRadixBits) {
-    radix_hist_kernel<K><<<(unsigned)num_tiles, kSortThreads, 0, st>>>(
-        kin, n, shift, num_tiles, counts.ptr);
-    WETRIC_LAUNCH_CHECK();
-    WETRIC_TRY((exclusive_scan<uint32_t, uint64_t>(ctx, st, counts.ptr,
-                                                   offsets.ptr, ncounts)));
-    if (vals != nullptr) {
-      radix_scatter_kernel<K, V, true>
-          <<<(unsigned)num_tiles, kSortThreads, 0, st>>>(
-              kin, vin, n, shift, num_tiles, offsets.ptr, kout, vout);
-    } else {
-      radix_scatter_kernel<K, V, false>
-          <<<(unsigned)num_tiles, kSortThreads, 0, st>>>(
-              kin, vin, n, shift, num_tiles, offsets.ptr, kout, vout);
-    }
-    WETRIC_LAUNCH_CHECK();
-    K *tk = kin; kin = kout; kout = tk;
-    V *tv = vin; vin = vout; vout = tv;
-    in_alt = !in_alt;
+// Workspace of one sort: the digits' histograms, the passes' tickets and the
+// look-back words, cleared at once.
+struct SortSpace {
+  Scratch<uint64_t> buf;
+  unsigned long long *hist = nullptr;
+  uint32_t *tickets = nullptr;
+  uint64_t *state = nullptr;
+  int alloc(DeviceContext *ctx, cudaStream_t st, uint64_t n) {
+    const uint64_t head = (uint64_t)kMaxPasses * kRadix + kMaxPasses;
+    const uint64_t words = head + ceil_div(n, kSortTile) * kRadix;
+    WETRIC_TRY(buf.alloc(ctx, st, words));
+    WETRIC_CUDA_TRY(cudaMemsetAsync(buf.ptr, 0, words * sizeof(uint64_t), st));
+    hist = reinterpret_cast<unsigned long long *>(buf.ptr);
+    tickets = reinterpret_cast<uint32_t *>(buf.ptr + kMaxPasses * kRadix);
+    state = buf.ptr + head;
+    return WETRIC_OK;
   }
-  *result_in_alt = in_alt;
+};
+
+template <int kBits, bool kHigh, class Load, class Sink>
+int onesweep_launch(cudaStream_t st, const Load &load, const Sink &sink, uint64_t n,
+                    const DigitPlan &plan, uint32_t p, const SortSpace &ws, uint32_t *err) {
+  const auto fn = k_onesweep<kBits, kHigh, Load, Sink>;
+  WETRIC_CUDA_TRY(
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortSmem));
+  fn<<<(unsigned)ceil_div(n, kSortTile), kSortThreads, kSortSmem, st>>>(
+      load, sink, n, plan.shift[p], plan.bits[p], p + 1, ws.hist + (uint64_t)p * kRadix, ws.state,
+      ws.tickets + p, err);
+  WETRIC_LAUNCH_CHECK();
   return WETRIC_OK;
+}
+
+template <class Load, class Sink>
+int onesweep_pass(cudaStream_t st, const Load &load, const Sink &sink, uint64_t n,
+                  const DigitPlan &plan, uint32_t p, const SortSpace &ws, uint32_t *err) {
+  const bool high = plan.shift[p] >= 32;
+  if (plan.bits[p] > 7)
+    return high ? onesweep_launch<8, true>(st, load, sink, n, plan, p, ws, err)
+                : onesweep_launch<8, false>(st, load, sink, n, plan, p, ws, err);
+  return high ? onesweep_launch<7, true>(st, load, sink, n, plan, p, ws, err)
+              : onesweep_launch<7, false>(st, load, sink, n, plan, p, ws, err);
+}
+
+// Stable LSD sort of n keys on their bits [lo, lo + bits). `counted` gives
+// the keys to the histogram pass (it may build and store them), `first` to
+// the first pass, whose output goes to a; the passes then alternate between
+// a and b, and the last one hands (position, key) to `sink`. Pass count:
+// digit_plan(lo, bits).passes, at least 1 (bits >= 1). *err (device) receives
+// a look-back that ran out.
+template <class Counted, class First, class Sink>
+int radix_sort_into(DeviceContext *ctx, cudaStream_t st, const Counted &counted,
+                    const First &first, uint64_t *a, uint64_t *b, const Sink &sink, uint64_t n,
+                    uint32_t lo, uint32_t bits, uint32_t *err) {
+  if (n == 0) return WETRIC_OK;
+  const DigitPlan plan = digit_plan(lo, bits ? bits : 1);
+  SortSpace ws;
+  WETRIC_TRY(ws.alloc(ctx, st, n));
+  uint64_t blocks = ceil_div(n, 256 * 16);
+  const uint64_t cap = (uint64_t)ctx->sm_count * 8;
+  if (blocks > cap) blocks = cap;
+  const size_t hs = (size_t)plan.passes * kRadix * kHistCopies * sizeof(uint32_t);
+  k_radix_hist<Counted><<<(unsigned)blocks, 256, hs, st>>>(counted, n, plan, ws.hist);
+  WETRIC_LAUNCH_CHECK();
+  if (plan.passes == 1) return onesweep_pass(st, first, sink, n, plan, 0, ws, err);
+  WETRIC_TRY((onesweep_pass(st, first, KeysTo{a}, n, plan, 0, ws, err)));
+  uint64_t *from = a, *to = b;
+  for (uint32_t p = 1; p + 1 < plan.passes; ++p) {
+    WETRIC_TRY((onesweep_pass(st, KeysFrom{from}, KeysTo{to}, n, plan, p, ws, err)));
+    uint64_t *x = from;
+    from = to;
+    to = x;
+  }
+  return onesweep_pass(st, KeysFrom{from}, sink, n, plan, plan.passes - 1, ws, err);
+}
+
+// The buffer (a or b) that the sort above leaves its keys in when the last
+// sink is KeysTo: the one its last pass does not read.
+inline uint64_t *sorted_buffer(uint64_t *a, uint64_t *b, uint32_t lo, uint32_t bits) {
+  return digit_plan(lo, bits ? bits : 1).passes % 2 == 1 ? a : b;
 }
 
 }  // namespace prim

@@ -263,7 +263,8 @@ int serve_prepare(DeviceContext *ctx, cudaStream_t st, uint32_t spread,
                                                   acc.ptr + 2);
     WETRIC_LAUNCH_CHECK();
   }
-  WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, active.ptr, pos.ptr, n)));
+  WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, active.ptr, pos.ptr, n,
+                                                       small.ptr)));
   WETRIC_TRY(p->act_wp.alloc(ctx, st, n + 1));
   WETRIC_TRY(p->act_rb.alloc(ctx, st, n));
   WETRIC_TRY(p->act_d.alloc(ctx, st, n));
@@ -272,7 +273,7 @@ int serve_prepare(DeviceContext *ctx, cudaStream_t st, uint32_t spread,
       rp, n, active.ptr, pos.ptr, p->act_wp.ptr, p->act_rb.ptr, p->act_d.ptr);
   WETRIC_LAUNCH_CHECK();
   WETRIC_TRY((prim::exclusive_scan<uint64_t, uint64_t>(ctx, st, p->act_wp.ptr,
-                                                       p->act_wp.ptr, n)));
+                                                       p->act_wp.ptr, n, small.ptr)));
   // Edge-check structures of kernel 8: bitmap over the last a vertices,
   // 16-bit near sets for the rows with d+ >= 16 within 65536 of the end,
   // 32-bit hash sets for the other rows with d+ >= 16.
@@ -285,13 +286,15 @@ int serve_prepare(DeviceContext *ctx, cudaStream_t st, uint32_t spread,
   k_hash_sizes<uint32_t><<<grid_for(ctx, n), 256, 0, st>>>(
       rp, n, ncount ? nfirst : bm_first, kHashMinDegree, kHashKeysPerBucket, nb.ptr);
   WETRIC_LAUNCH_CHECK();
-  WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, nb.ptr, hoff.ptr, n)));
+  WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, nb.ptr, hoff.ptr, n,
+                                                       small.ptr)));
   if (ncount) {
     WETRIC_TRY(noff.alloc(ctx, st, ncount + 1));
     k_hash_sizes<uint32_t><<<grid_for(ctx, ncount), 256, 0, st>>>(
         rp + nfirst, ncount, ncount, kHashMinDegree, kNearKeysPerBucket, nb.ptr);
     WETRIC_LAUNCH_CHECK();
-    WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, nb.ptr, noff.ptr, ncount)));
+    WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, nb.ptr, noff.ptr, ncount,
+                                                         small.ptr)));
   }
   // Dense core and shell (as count_oriented): candidate sizes from the row
   // offsets and the first core / shell wedge of each, in the same read-back.
@@ -337,6 +340,10 @@ int serve_prepare(DeviceContext *ctx, cudaStream_t st, uint32_t spread,
                                     cudaMemcpyDeviceToHost, st));
   }
   WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  if (err == kDevLookbackTimeout) {
+    set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
+    return WETRIC_ETIMEDOUT;
+  }
   if (err != kDevOk) {
     set_error(WETRIC_EINVAL, "oriented CSR check failed (device code %u)", err);
     return WETRIC_EINVAL;
@@ -356,7 +363,14 @@ int serve_prepare(DeviceContext *ctx, cudaStream_t st, uint32_t spread,
   nb.release();
   if (Rp) {
     WETRIC_TRY(p->ps.alloc(ctx, st, Kp + 1));
-    WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, pl.ptr, p->ps.ptr, Kp)));
+    WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, pl.ptr, p->ps.ptr, Kp,
+                                                         small.ptr)));
+    WETRIC_CUDA_TRY(cudaMemcpyAsync(&err, small.ptr, 4, cudaMemcpyDeviceToHost, st));
+    WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+    if (err == kDevLookbackTimeout) {
+      set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
+      return WETRIC_ETIMEDOUT;
+    }
   }
   pl.release();
   if (W == 0 && !Rp) return WETRIC_OK;
