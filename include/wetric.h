@@ -182,7 +182,10 @@ typedef struct {
   uint64_t wedge_end;     /*   wedge_end == 0 means "to the end"          */
   int32_t device;         /* CUDA device ordinal                          */
   uint32_t l2_persist;    /* != 0: pin the bitmap in L2 (access window)   */
-  uint32_t kernel;        /* count kernel: 0 = default (8), 1 = block-tile,
+  uint32_t kernel;        /* count kernel: 0 = default (whole graphs with
+                             offsets of 32 bits by row intersections, the
+                             column walk and the core; the rest by 8),
+                             1 = block-tile,
                              2 = warp-staged, 3 = row-walk with the
                              shared-memory stage, 4 = row-walk, 5 = 4 at
                              6 blocks/SM, 6 = 5 with per-row hash sets
@@ -222,12 +225,14 @@ typedef struct {
  * of a persistent grid, so work on other streams gets SMs as the count's
  * blocks finish (the serving lanes use this). */
 #define WETRIC_OPT_ONE_PASS 0x2u
-/* No pair streams for short rows. By default a whole-graph count (kernel
- * 8, 32-bit offsets, columns not copied in row chunks) counts each vertex
- * with d+ <= 64 whose neighbours' rows are short too the other way round:
- * its out-neighbours go into a shared-memory set and the rows of those
- * neighbours stream through it (k_count_pairs), instead of one set lookup
- * per wedge. The count is the same either way. */
+/* No row-by-row counting of short rows. By default a whole-graph count (m <
+ * 2^31) intersects each edge's tail with its end's short row and streams
+ * the others through the long rows' sets, and kernel 8 (32-bit offsets,
+ * columns not copied in row chunks) counts each vertex with d+ <= 64 whose
+ * neighbours' rows are short by pair streams: its out-neighbours go into a
+ * shared-memory set and the rows of those neighbours stream through it.
+ * With this flag every wedge below the core is one set lookup of kernel 8.
+ * The count is the same either way. */
 #define WETRIC_OPT_NO_PAIR_STREAMS 0x4u
 
 typedef struct {
@@ -252,10 +257,13 @@ typedef struct {
   uint64_t shell_len;     /* shell vertices used (0: none)                */
   uint64_t shell_wedges;  /* wedges counted by the shell kernel           */
   double shell_ms;        /* the shell kernel alone (part of count_ms)    */
-  uint64_t pair_rows;     /* vertices counted by pair streams (0: none)   */
-  uint64_t pair_wedges;   /* their wedges (part of wedges_counted)        */
-  double pair_ms;         /* the pair-stream kernel alone (part of
-                             count_ms)                                    */
+  uint64_t pair_rows;     /* vertices whose wedges the kernel of the short
+                             rows took, in whole or in part (row
+                             intersections; with kernel 8, pair streams,
+                             in whole); 0: none                           */
+  uint64_t pair_wedges;   /* the wedges it counted (part of
+                             wedges_counted)                              */
+  double pair_ms;         /* that kernel alone (part of count_ms)         */
 } wetric_stats;
 
 /* Cap the device memory this library may hold on `device` (0 = no cap).

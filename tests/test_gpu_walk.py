@@ -1,0 +1,139 @@
+"""GPU tests of the column walk (csrc/walk.cuh): the wedges below the core
+counted by middle vertex, at the sizes where its pieces change -- rows past
+one hash set's columns, vertices past one piece of entries, light vertices at
+their limits, no core and cores of several lengths, wedge ranges that cut
+rows and tails, and host input in row chunks. Counts are exact: every one
+equals the oracle's.
+"""
+import numpy as np
+import pytest
+
+from conftest import complete_graph, comb3
+
+pytestmark = pytest.mark.gpu
+
+
+def graph(oracle_mod, kind):
+    rng = np.random.default_rng(77)
+    if kind == "rmat":
+        import wetric
+
+        src, dst = wetric.gen_rmat(16, 16 << 16, seed=5)
+    elif kind == "dense":  # rows of 700 to 2,600 columns: several set sizes, two parts
+        n = 3000
+        i, j = np.triu_indices(n, 1)
+        keep = rng.random(i.size) < np.where(i < 400, 0.97, 0.45)
+        src, dst = i[keep], j[keep]
+    elif kind == "hub":  # short rows all ending in a few hubs: many pieces per w
+        m = 120_000
+        leaf = np.repeat(np.arange(m), 32)
+        src, dst = leaf, m + rng.integers(0, 90, leaf.size)
+        i, j = np.triu_indices(90, 1)
+        src, dst = np.concatenate([src, m + i]), np.concatenate([dst, m + j])
+    else:  # "light": d+ around 64 and entries around 128
+        n = 20_000
+        src = rng.integers(0, n, 64 * n)
+        dst = (src + rng.integers(1, 130, src.size)) % n
+    return oracle_mod.oriented_from_pairs(src.astype(np.uint32), dst.astype(np.uint32))
+
+
+@pytest.mark.parametrize("kind", ["rmat", "dense", "hub", "light"])
+def test_walk_parity(wetric_mod, oracle_mod, kind):
+    import torch
+
+    g = graph(oracle_mod, kind)
+    want = oracle_mod.count_merge(g)
+    W = oracle_mod.wedge_total(g)
+    assert W >= 4 * g.m + (16 << 20), (W, g.m)  # enough wedges for the walk
+    rp = torch.from_numpy(g.row_ptr.view(np.int64)).cuda()
+    rp32 = rp.int()
+    ci = torch.from_numpy(g.col_ind.view(np.int32)).cuda()
+    for core in (wetric_mod.CORE_OFF, 0, 32, 1000):
+        for kw in ({}, {"pair_streams": False}, {"one_pass": True}, {"validate": True},
+                   {"keep_u64_offsets": True}, {"kernel": 8}):
+            got, st = wetric_mod.count(rp, ci, 5, 8192, core_len=core, **kw)
+            assert got == want, (kind, core, kw)
+            assert st.wedges == W and st.wedges_counted == W
+        assert wetric_mod.count(rp32, ci, 1, 0, core_len=core)[0] == want
+
+
+@pytest.mark.parametrize("kind", ["rmat", "dense"])
+def test_walk_wedge_ranges(wetric_mod, oracle_mod, kind):
+    """Ranges large enough to walk, their ends inside rows and tails."""
+    g = graph(oracle_mod, kind)
+    W = oracle_mod.wedge_total(g)
+    rng = np.random.default_rng(3)
+    need = 4 * g.m + (16 << 20)
+    for core in (wetric_mod.CORE_OFF, 500):
+        for _ in range(4):
+            b = int(rng.integers(0, W - need))
+            e = int(rng.integers(b + need, W + 1))
+            got, st = wetric_mod.count(g.row_ptr, g.col_ind, 5, 8192, wedge_begin=b,
+                                       wedge_end=e, core_len=core)
+            rest = [wetric_mod.count(g.row_ptr, g.col_ind, 5, 8192, wedge_begin=x, wedge_end=y,
+                                     core_len=core, kernel=8)[0]
+                    for x, y in ((b, b + 7), (b + 7, e - 5), (e - 5, e))]
+            assert st.wedges_counted == e - b
+            assert got == sum(rest), (core, b, e)
+
+
+def test_walk_host_row_chunks(wetric_mod, oracle_mod):
+    src, dst = wetric_mod.gen_rmat(19, 16 << 19, seed=21)
+    g = oracle_mod.oriented_from_pairs(src, dst)
+    assert g.m >= 1 << 22
+    want = oracle_mod.count_merge(g)
+    for core in (wetric_mod.CORE_OFF, 0, 4096):
+        assert wetric_mod.count(g.row_ptr, g.col_ind, 5, 8192, core_len=core)[0] == want
+
+
+def test_walk_on_a_clique(wetric_mod, oracle_mod):
+    """Rows of up to 2,199 columns, every wedge closed: hash sets in two
+    parts (no core) and the whole graph in the core."""
+    k = 2200
+    g = oracle_mod.oriented_from_pairs(*complete_graph(k))
+    for core in (wetric_mod.CORE_OFF, 40, 0):
+        assert wetric_mod.count(g.row_ptr, g.col_ind, 5, 64, core_len=core)[0] == comb3(k)
+
+
+def test_walk_without_room_falls_back(wetric_mod, oracle_mod):
+    """Under a budget that has no room for the walk's entries the count takes
+    the wedge-check path and is the same."""
+    import torch
+
+    g = graph(oracle_mod, "rmat")
+    want = oracle_mod.count_merge(g)
+    rp = torch.from_numpy(g.row_ptr.astype(np.int32)).cuda()
+    ci = torch.from_numpy(g.col_ind.view(np.int32)).cuda()
+    try:
+        wetric_mod.set_hbm_budget(12 << 20)
+        assert wetric_mod.count(rp, ci, 5, 0, core_len=wetric_mod.CORE_OFF)[0] == want
+    finally:
+        wetric_mod.set_hbm_budget(0)
+
+
+def test_small_graphs_in_one_pass(wetric_mod, oracle_mod):
+    """Graphs below the size of a core and a walk, with rows longer than a
+    short row, at the edges of the tiles, u64 and u32 offsets, columns at
+    every alignment, and offsets that do not fit them."""
+    import torch
+
+    rng = np.random.default_rng(8)
+    for n, pairs in ((2, 1), (3, 3), (40, 700), (33, 31), (300, 4000), (700, 100000),
+                     (5000, 20001)):
+        src, dst = (rng.integers(0, n, pairs).astype(np.uint32) for _ in range(2))
+        g = oracle_mod.oriented_from_pairs(src, dst)
+        want, W = oracle_mod.count_merge(g), oracle_mod.wedge_total(g)
+        d = np.diff(g.row_ptr.astype(np.int64))
+        for off in range(8 if n == 300 else 2):
+            ci = torch.zeros(g.m + off, dtype=torch.int32, device="cuda")[off:]
+            ci.copy_(torch.from_numpy(g.col_ind.view(np.int32)))
+            for dt in (np.int32, np.int64):
+                rp = torch.from_numpy(g.row_ptr.astype(dt)).cuda()
+                got, st = wetric_mod.count(rp, ci, 5, 8192)
+                assert (got, st.wedges) == (want, W)
+                assert st.max_out_degree == (d.max() if d.size else 0)
+                if g.m > 2:
+                    bad = rp.clone()
+                    bad[1] = g.m + 5
+                    with pytest.raises(wetric_mod.WetricError):
+                        wetric_mod.count(bad, ci, 5, 8192)

@@ -556,8 +556,20 @@ int count_ex_impl(const wetric_csr *csr, const wetric_opts *o,
   // 3. u32 row offsets for the count when m < 2^32 (halves the offset
   //    bytes of every edge check).
   Scratch<uint32_t> narrow;
+  CountArgs a;
+  a.n = cn;
+  a.m = cm;
+  a.bitmap_len = o->bitmap_len;
+  a.wedge_begin = o->wedge_begin;
+  a.wedge_end = o->wedge_end;
+  a.l2_persist = o->l2_persist != 0;
+  a.kernel = o->kernel;
+  a.core_len = o->core_len;
+  a.shell_len = o->shell_len;
+  a.pair_streams = !(o->opt_flags & WETRIC_OPT_NO_PAIR_STREAMS);
+  // (a small whole graph is counted on whatever offsets it has)
   if (!c_off32 && cm < (1ull << 32) && cn > 0 &&
-      !(o->opt_flags & WETRIC_OPT_KEEP_U64_OFFSETS)) {
+      !(o->opt_flags & WETRIC_OPT_KEEP_U64_OFFSETS) && !count_whole_takes(a)) {
     WETRIC_TRY(narrow.alloc(ctx, st, cn + 1));
     WETRIC_TRY(narrow_offsets(ctx, st, static_cast<const uint64_t *>(rp), cn,
                               narrow.ptr));
@@ -565,24 +577,13 @@ int count_ex_impl(const wetric_csr *csr, const wetric_opts *o,
     c_off32 = true;
   }
 
-  CountArgs a;
-  a.n = cn;
-  a.m = cm;
   a.row_ptr = rp;
   a.offsets32 = c_off32;
   a.col_ind = ci;
   a.spread = o->spread;
-  a.bitmap_len = o->bitmap_len;
   a.block = o->block;
-  a.wedge_begin = o->wedge_begin;
-  a.wedge_end = o->wedge_end;
   a.validate = o->validate != 0;
-  a.l2_persist = o->l2_persist != 0;
-  a.kernel = o->kernel;
-  a.core_len = o->core_len;
-  a.shell_len = o->shell_len;
   a.persistent = !(o->opt_flags & WETRIC_OPT_ONE_PASS);
-  a.pair_streams = !(o->opt_flags & WETRIC_OPT_NO_PAIR_STREAMS);
   a.ci_ready = ci_ready;
   if (nchunks > 1) {
     a.col_chunks = nchunks;

@@ -846,8 +846,15 @@ int count_oriented(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
     set_error(WETRIC_ERANGE, "u32 offsets with m >= 2^32");
     return WETRIC_ERANGE;
   }
-  if (a.offsets32) return count_impl<uint32_t>(ctx, st, a, r);
-  return count_impl<uint64_t>(ctx, st, a, r);
+  CountArgs b = a;
+  if (count_whole_takes(a)) {
+    bool declined = false;
+    const int rc = count_whole(ctx, st, a, r, &declined);
+    if (rc != WETRIC_OK || !declined) return rc;
+    if (r->copies_issued) b.issue_copies = nullptr;
+  }
+  if (a.offsets32) return count_impl<uint32_t>(ctx, st, b, r);
+  return count_impl<uint64_t>(ctx, st, b, r);
 }
 
 template <typename Off>

@@ -48,12 +48,12 @@ struct CountArgs {
   // Shell below the core (with the core matrix as the bitmap): 0 or
   // kCoreOff = none, else that many vertices.
   uint32_t shell_len = 0;
-  // Pair streams for short rows (kernel 8, whole-graph counts with 32-bit
-  // offsets whose columns are not copied in row chunks): vertices with d+ <= 64
-  // whose pair streams cost less than their wedge checks are counted by
-  // k_count_pairs instead (pair_streams.cuh). The count does not change.
+  // Short rows counted by row intersections (count_whole.cu, kernel 0) or,
+  // with kernel 8, by pair streams (pair_streams.cuh; 32-bit offsets, columns
+  // not copied in row chunks). The count does not change.
   bool pair_streams = true;
-  uint32_t kernel = 0;  // 0 = default (8), 1 = block-tile, 2 = warp-staged,
+  uint32_t kernel = 0;  // 0 = default (count_whole.cu where it takes the
+                        // call, else 8), 1 = block-tile, 2 = warp-staged,
                         // 3 = row-walk with the shared-memory stage,
                         // 4 = row-walk, 5 = row-walk at 6 blocks/SM,
                         // 6 = 5 with per-row hash sets, 7 = 6 with
@@ -77,7 +77,8 @@ struct CountResult {
   double shell_ms = 0.0;     // the shell kernel alone
   uint64_t pair_rows = 0;    // vertices counted by pair streams
   uint64_t pair_wedges = 0;  // their wedges
-  double pair_ms = 0.0;      // the pair-stream kernel alone
+  double pair_ms = 0.0;      // the kernel of the short rows alone
+  bool copies_issued = false;  // CountArgs::issue_copies has been called
 };
 
 constexpr uint32_t kCoreOff = 0xFFFFFFFFu;
@@ -86,6 +87,13 @@ constexpr uint32_t kCoreOff = 0xFFFFFFFFu;
 // oriented CSR. Synchronous on `st` (it reads W back to size the launch).
 int count_oriented(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
                    CountResult *r);
+
+// The default count of a whole graph (count_whole.cu). count_oriented sends
+// the calls it takes there; *declined: not counted (no room, or too many
+// entries), the wedge-check path takes the call.
+bool count_whole_takes(const CountArgs &a);
+int count_whole(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
+                CountResult *r, bool *declined);
 
 // W and the max out-degree of an oriented CSR.
 int wedge_total(DeviceContext *ctx, cudaStream_t st, const void *row_ptr,

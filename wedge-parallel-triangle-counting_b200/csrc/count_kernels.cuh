@@ -1526,16 +1526,17 @@ __global__ void k_core_plan(const Off *__restrict__ rp, uint64_t n,
 
 // The automatic core from k_core_plan's read-back (plan[2c] = wedges,
 // plan[2c + 1] = words of candidate c): among the eligible candidates, the
-// least words - kCoreWordsPerCheck * wedges (the row ANDs' reads against
+// least words - words_per_check * wedges (the row ANDs' reads against
 // the wedge checks they save); -1 = no core. Candidates that n caps to the
 // same length tie, and the first of them is kept.
-inline int core_pick(const unsigned long long *plan) {
+inline int core_pick(const unsigned long long *plan,
+                     double words_per_check = kCoreWordsPerCheck) {
   int pick = -1;
   double best = 0.0;
   for (uint32_t c = 0; c < kCoreNumCandidates; ++c) {
     const unsigned long long wedges = plan[2 * c], words = plan[2 * c + 1];
     if (wedges < kCoreMinWedges || words > kCoreWordsPerWedge * wedges) continue;
-    const double score = (double)words - kCoreWordsPerCheck * (double)wedges;
+    const double score = (double)words - words_per_check * (double)wedges;
     if (pick < 0 || score < best) {
       pick = (int)c;
       best = score;
@@ -1652,7 +1653,9 @@ __device__ __forceinline__ uint32_t masked_popc(uint32_t x, uint32_t jj,
 // warps): the row loads mostly hit L2 and more warps in flight hide their
 // latency (R-MAT scale 22, core of 32,768, before the strided pairs: 1.55
 // ms at 8 blocks per SM, 1.86 ms at 6).
-template <typename Off>
+// kRows: one block per core vertex from row0 on, straight from the row
+// offsets, all its wedges.
+template <typename Off, bool kRows = false>
 __global__ void __launch_bounds__(kCoreBlock, 8)
     k_core_count(const uint32_t *__restrict__ ci,
                  const uint32_t *__restrict__ core, uint64_t v0, uint32_t h,
@@ -1660,18 +1663,20 @@ __global__ void __launch_bounds__(kCoreBlock, 8)
                  const uint64_t *__restrict__ act_rb,
                  const uint32_t *__restrict__ act_d, uint64_t Kc, uint64_t K,
                  uint64_t lo, uint64_t hi, unsigned long long *__restrict__ out,
-                 bool tma_ok = false, uint32_t *err = nullptr) {
+                 bool tma_ok = false, uint32_t *err = nullptr,
+                 const Off *__restrict__ rows = nullptr, uint64_t row0 = 0) {
   __shared__ __align__(16) uint32_t rv[kCoreMaxH4];
   __shared__ __align__(128) uint32_t stage[kStageCols];
   __shared__ __align__(8) unsigned long long mbar;
   __shared__ unsigned long long warp_acc[kCoreBlock / 32];
   const uint64_t k = Kc + blockIdx.x;
-  if (k >= K) return;
-  const uint64_t P = __ldg(act_wp + k);
-  const uint32_t d = __ldg(act_d + k);
+  if (!kRows && k >= K) return;
+  const uint64_t P = kRows ? 0 : __ldg(act_wp + k);
+  const uint64_t rb = kRows ? ld_off(rows, row0 + blockIdx.x) : __ldg(act_rb + k);
+  const uint32_t d =
+      kRows ? (uint32_t)(ld_off(rows, row0 + blockIdx.x + 1) - rb) : __ldg(act_d + k);
   const uint64_t Wv = (uint64_t)d * (d - 1) / 2;
-  if (P + Wv <= lo || P >= hi) return;  // block-uniform
-  const uint64_t rb = __ldg(act_rb + k);
+  if (kRows ? d < 2 : P + Wv <= lo || P >= hi) return;  // block-uniform
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (uint32_t i = tid; i < H4; i += kCoreBlock) rv[i] = 0;
   // N+(v), read twice below: staged in shared memory when it fits
@@ -1683,7 +1688,7 @@ __global__ void __launch_bounds__(kCoreBlock, 8)
     if (c < h) atomicOr(&rv[c >> 5], 1u << (c & 31));
   }
   __syncthreads();
-  const bool whole = P >= lo && P + Wv <= hi;
+  const bool whole = kRows || (P >= lo && P + Wv <= hi);
   uint32_t acc = 0;
   // Warp q takes the pairs wi = q, q + 8, q + 16, ...: the rows of w get
   // shorter as wi grows (w's stored row starts at its own column), so

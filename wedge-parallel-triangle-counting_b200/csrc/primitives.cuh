@@ -546,15 +546,17 @@ int onesweep_pass(cudaStream_t st, const Load &load, const Sink &sink, uint64_t 
 // the first pass, whose output goes to a; the passes then alternate between
 // a and b, and the last one hands (position, key) to `sink`. Pass count:
 // digit_plan(lo, bits).passes, at least 1 (bits >= 1). *err (device) receives
-// a look-back that ran out.
+// a look-back that ran out. space: a workspace for n keys or more, fresh from
+// alloc (none: the sort takes its own).
 template <class Counted, class First, class Sink>
 int radix_sort_into(DeviceContext *ctx, cudaStream_t st, const Counted &counted,
                     const First &first, uint64_t *a, uint64_t *b, const Sink &sink, uint64_t n,
-                    uint32_t lo, uint32_t bits, uint32_t *err) {
+                    uint32_t lo, uint32_t bits, uint32_t *err, const SortSpace *space = nullptr) {
   if (n == 0) return WETRIC_OK;
   const DigitPlan plan = digit_plan(lo, bits ? bits : 1);
-  SortSpace ws;
-  WETRIC_TRY(ws.alloc(ctx, st, n));
+  SortSpace own;
+  if (!space) WETRIC_TRY(own.alloc(ctx, st, n));
+  const SortSpace &ws = space ? *space : own;
   uint64_t blocks = ceil_div(n, 256 * 16);
   const uint64_t cap = (uint64_t)ctx->sm_count * 8;
   if (blocks > cap) blocks = cap;

@@ -16,7 +16,7 @@ struct ReadSpan {
   const void *src;
   uint32_t count, bytes;  // elements of 4 or 8 bytes
 };
-constexpr uint32_t kReadSpans = 12;
+constexpr uint32_t kReadSpans = 24;
 constexpr uint32_t kReadWords = 128;
 struct ReadPlan {
   ReadSpan s[kReadSpans];
@@ -28,16 +28,16 @@ struct ReadPlan {
     return total - count;
   }
 };
-__global__ void k_read_gather(ReadPlan p, uint64_t *__restrict__ out) {
-  uint32_t base = 0;
-  for (uint32_t i = 0; i < p.n; ++i) {
-    const ReadSpan sp = p.s[i];
-    for (uint32_t j = threadIdx.x; j < sp.count; j += blockDim.x)
-      out[base + j] = sp.bytes == 4 ? (uint64_t)static_cast<const uint32_t *>(sp.src)[j]
-                                    : static_cast<const uint64_t *>(sp.src)[j];
-    base += sp.count;
-  }
+__global__ void k_read_gather(const __grid_constant__ ReadPlan p, uint64_t *__restrict__ out) {
+  uint32_t j = threadIdx.x;  // one word per thread: its span, its element
+  if (j >= p.total) return;
+  uint32_t i = 0;
+  while (j >= p.s[i].count) j -= p.s[i++].count;
+  const ReadSpan &sp = p.s[i];
+  out[threadIdx.x] = sp.bytes == 4 ? (uint64_t)static_cast<const uint32_t *>(sp.src)[j]
+                                   : static_cast<const uint64_t *>(sp.src)[j];
 }
+static_assert(kReadWords <= 128, "one word per thread of the gather's block");
 // Pinned words for the calling thread's read-backs (portable: any device),
 // made on first use and freed when the thread ends; null if pinned memory
 // cannot be had (the caller then reads into its own array).

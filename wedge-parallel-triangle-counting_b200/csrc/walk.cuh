@@ -1,0 +1,894 @@
+// walk.cuh -- the default count of whole graphs: every edge (v, w) of the
+// oriented CSR closes its wedges (v; w, u) -- u in the tail of row v behind w
+// -- by one of three ways, chosen by w's row and v's place:
+//
+//   v in the dense core  row ANDs (k_core_count, count_kernels.cuh)
+//   d+(w) <= 48          the edge's own thread intersects the tail with the
+//                        short row of w, a sector of each at a time
+//                        (k_edge_merge)
+//   longer rows          the column walk: the edges are sorted by w, a block
+//                        builds N+(w) once in shared memory and the tails of
+//                        all rows v stream through it (k_walk_count)
+//
+// The wedge-check kernel (count_kernels.cuh), which serves the other calls,
+// looks every u up in a set of N+(w): one random 32-byte sector of L2 or DRAM
+// for each wedge. Here a wedge costs the four bytes of its u, read with the
+// rest of the tail, and a compare or a shared-memory lookup.
+//
+// In the walk, columns of the last 65,536 vertices (the window: most columns
+// of a graph with hubs) and the others are kept apart, so that the window's
+// set is a plain bit row: the i-th long row stands for two middle vertices,
+// 2i + 1 with its window columns and 2i with the rest, and a tail that has
+// both is two entries.
+//
+//   k_edge_vertices  row checks, W, the longest row, core sizing, and the
+//                    numbers of the long rows
+//   k_walk_split     where a row's window columns start
+//   k_edge_merge     the short rows' edges counted, the others' entries:
+//                    middle vertex, the tail's first column index and its
+//                    length in 64 bits
+//   radix sort       by middle vertex (primitives.cuh)
+//   k_walk_starts    the first entry of every middle vertex
+//   k_walk_plan      work items: a vertex, a piece of its entries
+//   k_walk_count     a block per item: the bit row, or a hash set
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "common.cuh"
+#include "count_kernels.cuh"
+#include "primitives.cuh"
+#include "readback.cuh"
+
+namespace wetric {
+namespace {
+
+constexpr uint32_t kWalkWindow = 65536;
+
+// Fields of an entry, low to high: tail length, first column index, middle
+// vertex.
+struct WalkBits {
+  uint32_t w, start, len;
+  __host__ __device__ uint32_t shift() const { return start + len; }
+};
+
+constexpr uint32_t kWalkBlock = 256;
+constexpr uint32_t kWalkEmpty = 0xFFFFFFFFu;
+constexpr uint32_t kWalkShort = 0xFFFFFFFFu;  // number of a row that is not long
+constexpr uint32_t kWalkShortCols = 48;       // columns of a short row at most
+constexpr uint32_t kMergeTile = 512;          // edges per warp at most
+constexpr uint32_t kMergeStage = 128;         // entries a warp gathers (64 or more)
+constexpr uint32_t kWalkBig = 64;             // entries from which a block takes a vertex
+constexpr uint32_t kWalkBigCols = 128;        // or columns
+constexpr uint32_t kWalkPiece = 2048;         // entries per item of a block
+constexpr uint32_t kWalkPer = 4;              // entries per thread streamed at once
+constexpr uint32_t kWalkBigBlock = 128, kWalkSmallBlock = 32;
+constexpr int kWalkBigBlocks = 10, kWalkSmallBlocks = 28;  // per SM
+constexpr uint32_t kWalkSmallSlots = 512;
+constexpr uint32_t kWalkSetCols = 1024;  // columns per hash set
+constexpr uint32_t kWalkSetSlots = 2048;
+constexpr int kWalkCarveout = 70;  // percent of an SM's memory that is shared
+
+// Inclusive scan over the warp.
+__device__ __forceinline__ uint32_t walk_scan(uint32_t x, uint32_t lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  return x;
+}
+
+// Core lengths to size up, at most n each.
+struct EdgeCores {
+  uint32_t len[kCoreNumCandidates];
+  uint32_t count;
+};
+
+// Totals of the rows: [0] W, [1] longest row, [2] rows with wedges, [3] long
+// rows, then per core candidate its wedges, AND words (k_core_plan) and rows
+// with wedges.
+constexpr uint32_t kEdgeTotals = 4 + 3 * kCoreNumCandidates;
+template <typename Off>
+__global__ void __launch_bounds__(kWalkBlock)
+    k_edge_vertices(const Off *__restrict__ rp, uint64_t n, uint64_t m,
+                    const __grid_constant__ EdgeCores cores, unsigned long long *__restrict__ totals, uint32_t *__restrict__ number,
+                    uint32_t *__restrict__ long_rows, uint32_t *err) {
+  const uint32_t lane = threadIdx.x & 31;
+  unsigned long long W = 0, rows = 0, longest = 0;
+  unsigned long long plan[3 * kCoreNumCandidates] = {};
+  const uint64_t top = cores.count ? cores.len[0] : 0u;  // the longest
+  bool in_top = false;
+  for (uint64_t v0 = (uint64_t)blockIdx.x * kWalkBlock + threadIdx.x - lane; v0 < n;
+       v0 += (uint64_t)gridDim.x * kWalkBlock) {
+    const uint64_t v = v0 + lane;
+    uint64_t d = 0;
+    if (v < n) {
+      const uint64_t b = ld_off(rp, v), e = ld_off(rp, v + 1);
+      if (e < b || e > m)
+        atomicCAS(err, 0u, (uint32_t)kDevRowPtrRange);
+      else
+        d = e - b;
+    }
+    const unsigned long long w = d >= 2 ? d * (d - 1) / 2 : 0;
+    W += w;
+    rows += d >= 2;
+    longest = longest > d ? longest : d;
+    if (v < n && v >= n - top) {
+      in_top = true;
+#pragma unroll
+      for (uint32_t c = 0; c < kCoreNumCandidates; ++c) {
+        const uint64_t hc = c < cores.count ? cores.len[c] : 0u;
+        if (v >= n - hc) {
+          plan[3 * c] += w;
+          plan[3 * c + 1] += d * (hc - (v - (n - hc))) / 64 + d;
+          plan[3 * c + 2] += d >= 2;
+        }
+      }
+    }
+    if (number) {
+      const bool is_long = d > kWalkShortCols;
+      const uint32_t mask = __ballot_sync(0xffffffffu, is_long);
+      uint32_t id = 0;
+      if (mask && lane == 0) id = (uint32_t)atomicAdd(totals + 3, (unsigned long long)__popc(mask));
+      id = __shfl_sync(0xffffffffu, id, 0) + __popc(mask & ((1u << lane) - 1u));
+      if (v < n) number[v] = is_long ? id : kWalkShort;
+      if (is_long) long_rows[id] = (uint32_t)v;
+    }
+  }
+  __shared__ unsigned long long s_sum[3], s_plan[3 * kCoreNumCandidates];
+  if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+  if (threadIdx.x < 3 * kCoreNumCandidates) s_plan[threadIdx.x] = 0;
+  __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) {
+    W += __shfl_down_sync(0xffffffffu, W, o);
+    rows += __shfl_down_sync(0xffffffffu, rows, o);
+    const unsigned long long x = __shfl_down_sync(0xffffffffu, longest, o);
+    longest = longest > x ? longest : x;
+  }
+  if (lane == 0) {
+    atomicAdd(&s_sum[0], W);
+    atomicMax(&s_sum[1], longest);
+    atomicAdd(&s_sum[2], rows);
+  }
+  if (__any_sync(0xffffffffu, in_top)) {
+#pragma unroll
+    for (uint32_t c = 0; c < 3 * kCoreNumCandidates; ++c) {
+      unsigned long long x = plan[c];
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0 && x) atomicAdd(&s_plan[c], x);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (s_sum[0]) atomicAdd(totals, s_sum[0]);
+    atomicMax(totals + 1, s_sum[1]);
+    if (s_sum[2]) atomicAdd(totals + 2, s_sum[2]);
+  }
+  if (threadIdx.x < 3 * kCoreNumCandidates && s_plan[threadIdx.x])
+    atomicAdd(totals + 4 + threadIdx.x, s_plan[threadIdx.x]);
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    if (ld_off(rp, 0) != 0 || ld_off(rp, n) != m) atomicCAS(err, 0u, (uint32_t)kDevRowPtrRange);
+}
+
+// split[v] = index of row v's first window column (rows are sorted), rows
+// [lo, hi).
+__global__ void __launch_bounds__(kWalkBlock)
+    k_walk_split(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ci, uint64_t n,
+                 uint64_t lo_row, uint64_t hi_row, uint32_t *__restrict__ split) {
+  const uint32_t t0 = n > kWalkWindow ? (uint32_t)(n - kWalkWindow) : 0u;
+  for (uint64_t v = lo_row + (uint64_t)blockIdx.x * kWalkBlock + threadIdx.x; v < hi_row;
+       v += (uint64_t)gridDim.x * kWalkBlock) {
+    uint32_t lo = rp[v], hi = rp[v + 1];
+    if (v >= t0) hi = lo;  // every column is above its row
+    while (lo < hi) {
+      const uint32_t mid = lo + (hi - lo) / 2;
+      if (__ldg(ci + mid) >= t0) hi = mid;
+      else lo = mid + 1;
+    }
+    split[v] = lo;
+  }
+}
+
+// start[x] = the first of the sorted entries of middle vertex x or more, x in
+// [0, n].
+// A lane fills a gap of up to 8 vertices, the warp a longer one.
+__global__ void __launch_bounds__(kWalkBlock)
+    k_walk_starts(const uint64_t *__restrict__ keys, uint32_t m, uint32_t n, uint32_t shift,
+                  uint32_t *__restrict__ start) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t stride = (uint64_t)gridDim.x * kWalkBlock;
+  const uint64_t gid = (uint64_t)blockIdx.x * kWalkBlock + threadIdx.x;
+  const uint64_t first = keys[0] >> shift, end = keys[m - 1] >> shift;
+  for (uint64_t w = gid; w <= first && w <= n; w += stride) start[w] = 0;
+  for (uint64_t w = end + 1 + gid; w <= n; w += stride) start[w] = m;
+  for (uint64_t i0 = gid - lane; i0 < m; i0 += stride) {
+    const uint64_t i = i0 + lane;
+    uint32_t w = 0, prev = 0;
+    if (i < m) {
+      w = (uint32_t)(keys[i] >> shift);
+      prev = i ? (uint32_t)(keys[i - 1] >> shift) : w;
+      if (w > n) w = n;
+      if (prev > n) prev = n;
+    }
+    const bool wide = w - prev > 8u;
+    if (!wide)
+      for (uint32_t r = prev; r < w; ++r) start[r + 1] = (uint32_t)i;
+    for (uint32_t mask = __ballot_sync(0xffffffffu, wide); mask; mask &= mask - 1) {
+      const int l = __ffs(mask) - 1;
+      const uint32_t from = __shfl_sync(0xffffffffu, prev, l), to = __shfl_sync(0xffffffffu, w, l);
+      for (uint32_t r = from + 1 + lane; r <= to; r += 32) start[r] = (uint32_t)(i0 + l);
+    }
+  }
+}
+
+// The set columns of middle vertex x: its row's window columns or the rest.
+__device__ __forceinline__ uint2 walk_set(const uint32_t *__restrict__ rp,
+                                          const uint32_t *__restrict__ split,
+                                          const uint32_t *__restrict__ long_rows, uint32_t x) {
+  const uint32_t w = __ldg(long_rows + (x >> 1)), s = __ldg(split + w);
+  return x & 1 ? make_uint2(s, __ldg(rp + w + 1)) : make_uint2(__ldg(rp + w), s);
+}
+
+// The work items over the x_end middle vertices: counts[0] pieces of those
+// with more than kWalkBig entries or kWalkBigCols columns, counts[1] of the
+// others (whole).
+__global__ void __launch_bounds__(kWalkBlock)
+    k_walk_plan(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ split,
+                const uint32_t *__restrict__ long_rows, const uint32_t *__restrict__ start,
+                uint32_t x_end, uint2 *__restrict__ big, uint2 *__restrict__ small,
+                uint32_t *__restrict__ counts) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t stride = (uint64_t)gridDim.x * kWalkBlock;
+  for (uint64_t x0 = (uint64_t)blockIdx.x * kWalkBlock + threadIdx.x - lane; x0 < x_end;
+       x0 += stride) {
+    const uint64_t x = x0 + lane;
+    const uint32_t E = x < x_end ? start[x + 1] - start[x] : 0u;
+    bool few = false;
+    if (E && E <= kWalkBig) {
+      const uint2 set = walk_set(rp, split, long_rows, (uint32_t)x);
+      few = set.y - set.x <= kWalkBigCols;
+    }
+    const uint32_t pieces = E && !few ? (E + kWalkPiece - 1) / kWalkPiece : 0u;
+    const uint32_t incl = walk_scan(pieces, lane);
+    const uint32_t sm = __ballot_sync(0xffffffffu, few);
+    const uint32_t sum = __shfl_sync(0xffffffffu, incl, 31);
+    const uint32_t add = lane == 0 ? sum : __popc(sm);
+    uint32_t got = 0;
+    if (lane < 2 && add) got = atomicAdd(counts + lane, add);
+    const uint32_t base = __shfl_sync(0xffffffffu, got, 0) + incl - pieces;
+    const uint32_t at = __shfl_sync(0xffffffffu, got, 1) + __popc(sm & ((1u << lane) - 1u));
+    for (uint32_t p = 0; p < pieces; ++p) big[base + p] = make_uint2((uint32_t)x, p);
+    if (few) small[at] = make_uint2((uint32_t)x, 0u);
+  }
+}
+
+// The columns as the streams read them: in 32-byte sectors, whole ones by
+// one load, those that stick out of the array by single loads. `mis` is the
+// column array's offset in its first sector; indices carry it.
+struct WalkColumns {
+  const uint32_t *base;  // 32-byte aligned, mis columns before the array
+  uint32_t mis, end;     // columns [mis, end) exist (end <= 2^32 - 8)
+};
+inline WalkColumns walk_columns(const uint32_t *ci, uint64_t m) {
+  WalkColumns c;
+  c.mis = (uint32_t)((reinterpret_cast<uintptr_t>(ci) & 31) / 4);
+  c.base = ci - c.mis;
+  c.end = (uint32_t)(m + c.mis);
+  return c;
+}
+
+// The sector at (mis-carrying) index a; where it sticks out of the array,
+// only the columns of [lo, hi).
+__device__ __forceinline__ void walk_sector(const WalkColumns &cols, uint32_t a, uint32_t lo,
+                                            uint32_t hi, uint32_t (&x)[8]) {
+  if (a >= cols.mis && a + 8 <= cols.end) {
+    const Bucket b = ld_bucket(cols.base + a);
+    x[0] = b.s0, x[1] = b.s1, x[2] = b.s2, x[3] = b.s3;
+    x[4] = b.s4, x[5] = b.s5, x[6] = b.s6, x[7] = b.s7;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = a + j >= lo && a + j < hi ? __ldg(cols.base + a + j) : 0u;
+  }
+}
+
+// Half a sector, likewise.
+__device__ __forceinline__ void walk_half(const WalkColumns &cols, uint32_t a, uint32_t lo,
+                                          uint32_t hi, uint32_t (&x)[4]) {
+  if (a >= cols.mis && a + 4 <= cols.end) {
+    const uint4 b = __ldg(reinterpret_cast<const uint4 *>(cols.base + a));
+    x[0] = b.x, x[1] = b.y, x[2] = b.z, x[3] = b.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = a + j >= lo && a + j < hi ? __ldg(cols.base + a + j) : 0u;
+  }
+}
+
+// |[t0, t1) & [s0, s1)| of the column array (both sorted, indices with mis,
+// neither empty), four columns of each at a time: all pairs of them, then
+// the four with the smaller last column move on. (Eight at a time: fewer
+// loads, four times the pairs; Erdos-Renyi, 13.3M edges: 670 us against
+// 551.)
+struct MergeTask {
+  uint32_t t0, t1, t_last, s0, s1;  // t_last: the column at t1 - 1
+};
+__device__ __forceinline__ uint32_t merge_rows(const WalkColumns &cols, const MergeTask &task) {
+  const uint32_t t0 = task.t0, t1 = task.t1, t_last = task.t_last, s0 = task.s0, s1 = task.s1;
+  const uint32_t s_last = __ldg(cols.base + s1 - 1);
+  uint32_t a = t0 & ~3u, b = s0 & ~3u, hits = 0;
+  uint32_t x[4], y[4];
+  walk_half(cols, a, t0, t1, x);
+  walk_half(cols, b, s0, s1, y);
+  uint32_t xm = a + 4 < t1 ? x[3] : t_last, ym = b + 4 < s1 ? y[3] : s_last;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {  // columns that are not the rows' match nothing
+    if (a + j < t0 || a + j >= t1) x[j] = 0xFFFFFFFFu;
+    if (b + j < s0 || b + j >= s1) y[j] = 0xFFFFFFFEu;
+  }
+  for (;;) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      hits += x[i] == y[0] || x[i] == y[1] || x[i] == y[2] || x[i] == y[3];
+    const bool tail = xm <= ym;
+    const uint32_t p = (tail ? a : b) + 4, end = tail ? t1 : s1;
+    if (p >= end) break;
+    uint32_t z[4];
+    walk_half(cols, p, p, end, z);
+    const uint32_t zm = p + 4 < end ? z[3] : tail ? t_last : s_last;
+    const uint32_t none = tail ? 0xFFFFFFFFu : 0xFFFFFFFEu;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t c = p + j < end ? z[j] : none;
+      x[j] = tail ? c : x[j];
+      y[j] = tail ? y[j] : c;
+    }
+    if (tail) a = p, xm = zm;
+    else b = p, ym = zm;
+  }
+  return hits;
+}
+
+// Row of edge j: the last row r in [lo, hi) with rp[r] <= j (a warp together,
+// 32 probes a step).
+template <typename Off>
+__device__ __forceinline__ uint64_t row_of_edge(const Off *__restrict__ rp, uint64_t lo,
+                                                uint64_t hi, uint64_t j, uint32_t lane) {
+  uint64_t count = hi - lo;
+  while (count > 1) {
+    const uint64_t step = (count + 31) / 32, at = (lane + 1) * step;
+    const bool below = at < count && ld_off(rp, lo + at) <= j;
+    const uint64_t k = __popc(__ballot_sync(0xffffffffu, below));
+    lo += k * step;
+    count = min(step, count - k * step);
+  }
+  return lo;
+}
+
+// The edges [rp[row_lo], rp[row_hi]), T per warp, one thread each: edges to
+// short rows are counted here (their wedges added to out[1], triangles to
+// out[0]); with kEmit, edges to long rows become entries for the walk,
+// appended in any order (*made of them, those past cap are only counted) --
+// but for the tail's part outside the window, which is intersected here when
+// the long row has few columns there -- and without it they are counted here
+// too. Nothing is done when *err is set: the
+// row offsets cannot be trusted.
+// Bound by instruction issue: a step intersects 4 by 4 columns of each of 32
+// edges in about 50 instructions. Erdos-Renyi with 700,001 vertices and 13.3M
+// edges: 551 us where the pair streams took 584 after a plan of 131 us and
+// 152 us of hash sets; R-MAT scale 22: 0.79 ms (1.27 ms before the few
+// edges that intersect rows there were gathered to fill the warp).
+template <typename Off, bool kEmit>
+__global__ void __launch_bounds__(kWalkBlock, 4)
+    k_edge_merge(const Off *__restrict__ rp, const __grid_constant__ WalkColumns cols, uint64_t n,
+                 uint64_t row_lo, uint64_t row_hi, uint32_t T,
+                 const uint32_t *__restrict__ number, const uint32_t *__restrict__ split,
+                 const WalkBits bits, uint64_t *__restrict__ entries, uint32_t cap,
+                 uint32_t *__restrict__ made, unsigned long long *__restrict__ out,
+                 const uint32_t *__restrict__ err) {
+  __shared__ uint32_t s_start[kWalkBlock / 32][32], s_row[kWalkBlock / 32][32];
+  __shared__ uint64_t s_entry[kEmit ? kWalkBlock / 32 : 1][kEmit ? kMergeStage : 1];
+  __shared__ MergeTask s_task[kEmit ? kWalkBlock / 32 : 1][64];
+  if (*err != kDevOk) return;
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u, le = 0xFFFFFFFFu >> (31 - lane);
+  const uint32_t *ci = cols.base + cols.mis;
+  const uint32_t j_end = (uint32_t)ld_off(rp, row_hi);
+  const uint64_t t = (uint64_t)blockIdx.x * (kWalkBlock / 32) + wid;
+  const uint64_t from = ld_off(rp, row_lo) + t * T;
+  if (from >= j_end) return;
+  const uint32_t j1 = j_end - from < T ? j_end : (uint32_t)from + T;
+  unsigned long long wedges = 0;
+  uint32_t hits = 0;
+  // A warp's entries gather in shared memory and go out together: one atomic
+  // on the common counter for up to 128 of them (one per round of 32 edges
+  // took longer than the rest of the kernel).
+  uint32_t staged = 0, tasks = 0;
+  uint64_t *stage = s_entry[kEmit ? wid : 0];
+  auto flush = [&]() {
+    __syncwarp();
+    uint32_t x = 0;
+    if (lane == 0) x = atomicAdd(made, staged);
+    x = __shfl_sync(0xffffffffu, x, 0);
+    for (uint32_t i = lane; i < staged; i += 32)
+      if (x + i < cap) entries[x + i] = stage[i];
+    staged = 0;
+    __syncwarp();
+  };
+  for (uint32_t j = (uint32_t)from; j < j1;) {
+    const uint64_t r = row_of_edge(rp, row_lo, row_hi, j, lane);
+    const uint64_t v = r + lane < row_hi ? r + lane : row_hi;
+    const uint32_t b = (uint32_t)ld_off(rp, v);
+    const uint32_t e = v < row_hi ? (uint32_t)ld_off(rp, v + 1) : b;
+    const uint32_t last = e > b ? __ldg(ci + e - 1) : 0u;
+    uint32_t mid = b, rest_last = 0;
+    if (kEmit && v < row_hi) {
+      mid = split[v];
+      if (mid > b) rest_last = __ldg(ci + mid - 1);
+    }
+    const uint32_t stop = min(j1, __shfl_sync(0xffffffffu, e, 31));
+    const uint32_t rows = __ballot_sync(0xffffffffu, e > b);
+    __syncwarp();
+    if (e > b) {
+      s_start[wid][__popc(rows & lt)] = max(b, j) - j;
+      s_row[wid][__popc(rows & lt)] = lane;
+    }
+    __syncwarp();
+    const uint32_t c = lane < __popc(rows) ? s_start[wid][lane] : 0xFFFFFFFFu;
+    uint32_t before = 0;
+    for (uint32_t q0 = 0; q0 < stop - j; q0 += 32) {
+      const uint32_t starts = __reduce_or_sync(0xffffffffu, c - q0 < 32u ? 1u << (c - q0) : 0u);
+      const uint32_t at = before + __popc(starts & le) - 1;
+      before += __popc(starts);
+      const uint32_t edge = j + q0 + lane;
+      const uint32_t row = s_row[wid][at & 31];
+      const uint32_t end = __shfl_sync(0xffffffffu, e, row);
+      const uint32_t first = edge + 1;
+      const bool on = edge < stop && first < end;
+      const uint32_t w = on ? __ldg(ci + edge) : 0u;
+      const bool ok = on && w < n;
+      uint32_t id = kWalkShort, t1 = end, t_last = __shfl_sync(0xffffffffu, last, row);
+      uint32_t s0 = 0, s1 = 0;
+      if (kEmit) {
+        const uint32_t cut = __shfl_sync(0xffffffffu, mid, row);
+        const uint32_t rl = __shfl_sync(0xffffffffu, rest_last, row);
+        if (ok) id = __ldg(number + w);
+        const bool is_long = id != kWalkShort;
+        const bool win = is_long && cut < end;
+        bool rest = is_long && first < cut;
+        if (rest) {
+          s0 = (uint32_t)ld_off(rp, w);
+          s1 = split[w];
+          if (s1 - s0 <= kWalkShortCols) {
+            rest = false;
+            t1 = cut;
+            t_last = rl;
+            wedges += cut - first;
+          } else {
+            s1 = s0;
+          }
+        }
+        const uint32_t rm = __ballot_sync(0xffffffffu, rest);
+        const uint32_t wm = __ballot_sync(0xffffffffu, win);
+        if (rm | wm) {
+          const uint32_t add = __popc(rm) + __popc(wm);
+          if (staged + add > kMergeStage) flush();
+          const uint32_t xr = staged + __popc(rm & lt);
+          const uint32_t xw = staged + __popc(rm) + __popc(wm & lt);
+          const uint64_t key = (uint64_t)id << (bits.shift() + 1);
+          const uint32_t wf = max(first, cut);
+          if (rest) stage[xr] = key | ((uint64_t)first << bits.len) | (cut - first);
+          if (win)
+            stage[xw] = key | (1ull << bits.shift()) | ((uint64_t)wf << bits.len) | (end - wf);
+          staged += add;
+        }
+      }
+      if (ok && id == kWalkShort) {
+        wedges += end - first;
+        s0 = (uint32_t)ld_off(rp, w), s1 = (uint32_t)ld_off(rp, w + 1);
+      }
+      const MergeTask task{first + cols.mis, t1 + cols.mis, t_last, s0 + cols.mis, s1 + cols.mis};
+      if (!kEmit) {
+        if (s0 < s1) hits += merge_rows(cols, task);
+      } else {
+        // few of the edges intersect rows here: they gather until there is
+        // one for every lane
+        const uint32_t mm = __ballot_sync(0xffffffffu, s0 < s1);
+        if (s0 < s1) s_task[wid][tasks + __popc(mm & lt)] = task;
+        tasks += __popc(mm);
+        __syncwarp();
+        if (tasks >= 32) {
+          hits += merge_rows(cols, s_task[wid][lane]);
+          tasks -= 32;
+          const MergeTask moved = s_task[wid][32 + lane];
+          __syncwarp();
+          if (lane < tasks) s_task[wid][lane] = moved;
+          __syncwarp();
+        }
+      }
+    }
+    j = stop;
+  }
+  if (kEmit && lane < tasks) hits += merge_rows(cols, s_task[kEmit ? wid : 0][lane]);
+  if (kEmit && staged) flush();
+  unsigned long long h = hits;
+  for (int o = 16; o > 0; o >>= 1) {
+    h += __shfl_down_sync(0xffffffffu, h, o);
+    wedges += __shfl_down_sync(0xffffffffu, wedges, o);
+  }
+  if (lane == 0) {
+    if (h) atomicAdd(out, h);
+    if (wedges) atomicAdd(out + 1, wedges);
+  }
+}
+
+// Edges per warp: kMergeTile, or fewer (whole rounds) when that leaves the
+// device's warps less than two tiles each.
+inline uint32_t merge_tile(uint64_t edges, int sms) {
+  const uint64_t per = ceil_div(ceil_div(edges, 2ull * sms * 32), 32) * 32;
+  return per < kMergeTile ? (uint32_t)(per ? per : 32) : kMergeTile;
+}
+
+// The 32-byte sectors that a tail [first, first + len) touches.
+__device__ __forceinline__ uint32_t walk_sectors(uint32_t first, uint32_t len) {
+  return len ? ((first + len + 7) >> 3) - (first >> 3) : 0u;
+}
+
+// Streams the tails of k <= kGroup entries through test(columns, entry,
+// mask), which returns how many of the masked 8 columns it finds. The
+// tails' sectors lie one after another in s_pre's numbering (exclusive
+// prefix of their counts, S in all), and thread `id` of kLanes takes sectors
+// id, id + kLanes, ...: every thread does the same number of rounds, a round
+// is 8 columns for one load, and neighbouring threads read neighbouring
+// sectors. A sector's entry is the number of tails that start at or before
+// it: s_head marks the starts, s_cnt counts those before each of its words.
+// Steps on the way, R-MAT scale 22: a warp's 32 lanes packed over the
+// columns (a reduction, popcounts and shuffles a round: 61 instructions per
+// 32 columns) 4.0 ms; spans of consecutive sectors per thread (no lookup,
+// but 32 lines a load) 2.3 ms; this with blocks of two sizes 2.1 ms. The next sector's load is
+// out while one is tested. sync() is the threads' barrier.
+template <uint32_t kGroup, uint32_t kLanes, uint32_t kWords, class Entry, class Sync, class Test>
+__device__ __forceinline__ uint32_t walk_tails(const WalkColumns &cols, const Entry *s_e,
+                                               const uint32_t *s_pre, uint32_t *s_head,
+                                               uint32_t *s_cnt, uint32_t k, uint32_t S,
+                                               uint32_t id, const Sync &sync, const Test &test) {
+  static_assert(kLanes >= kWords, "a thread per word of s_head");
+  const uint32_t le = 0xFFFFFFFFu >> (31 - (id & 31));
+  uint32_t hits = 0;
+  for (uint32_t s0 = 0; s0 < S; s0 += 32 * kWords) {
+    const uint32_t s1 = min(S, s0 + 32 * kWords);
+    if (s0) sync();
+    if (id < kWords && 32 * id < s1 - s0) {
+      s_head[id] = 0;
+      uint32_t c = 0;  // entries that start before word id: the first at or past it
+#pragma unroll
+      for (uint32_t o = kGroup / 2; o; o >>= 1)
+        if (c + o <= k && s_pre[c + o - 1] < s0 + 32 * id) c += o;
+      if (c < k && s_pre[c] < s0 + 32 * id) ++c;
+      s_cnt[id] = c;
+    }
+    sync();
+    for (uint32_t i = id; i < k; i += kLanes) {
+      const uint32_t at = s_pre[i] - s0;
+      if (at < s1 - s0) atomicOr(&s_head[at >> 5], 1u << (at & 31));
+    }
+    sync();
+    auto fetch = [&](uint32_t s, uint32_t(&x)[8], Entry &en) {
+      uint32_t mask = 0;
+      if (s < s1) {
+        const uint32_t word = (s - s0) >> 5;
+        const uint32_t e = s_cnt[word] + __popc(s_head[word] & le) - 1;
+        en = s_e[e];
+        const uint32_t a = (en.first & ~7u) + 8 * (s - s_pre[e]);
+        const uint32_t end = en.first + en.len;
+        mask = (0xFFu >> (en.first > a ? en.first - a : 0u)) &
+               (0xFFu << (end < a + 8 ? a + 8 - end : 0u));
+        walk_sector(cols, a, en.first, end, x);
+      }
+      return mask;
+    };
+    uint32_t x[8] = {}, y[8] = {};
+    Entry ex{}, ey{};
+    uint32_t mx = fetch(s0 + id, x, ex);
+    for (uint32_t s = s0 + id; s - id < s1; s += 2 * kLanes) {
+      const uint32_t my = fetch(s + kLanes, y, ey);
+      hits += test(x, ex, mx);
+      mx = fetch(s + 2 * kLanes, x, ex);
+      hits += test(y, ey, my);
+    }
+  }
+  return hits;
+}
+
+__device__ __forceinline__ void walk_insert(uint32_t *set, uint32_t slots, uint32_t x,
+                                            uint32_t shift) {
+  uint32_t h = (x * kHashMul) >> shift;
+  for (;;) {
+    const uint32_t old = atomicCAS(set + h, kWalkEmpty, x);
+    if (old == kWalkEmpty || old == x) return;
+    h = (h + 1) & (slots - 1);
+  }
+}
+// How many of the masked columns are in the set: every column's home slot
+// first, then the few that it does not decide.
+__device__ __forceinline__ uint32_t walk_find8(const uint32_t *set, uint32_t slots, uint32_t shift,
+                                               const uint32_t (&x)[8], uint32_t mask) {
+  uint32_t found = 0, open = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t key = set[(x[j] * kHashMul) >> shift];
+    found |= key == x[j] ? 128u >> j : 0u;
+    open |= key != x[j] && key != kWalkEmpty ? 128u >> j : 0u;
+  }
+  uint32_t hits = __popc(found & mask);
+  open &= mask;
+  if (open) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (!((open >> (7 - j)) & 1u)) continue;
+      uint32_t h = (x[j] * kHashMul) >> shift;
+      for (;;) {
+        h = (h + 1) & (slots - 1);
+        const uint32_t key = set[h];
+        if (key == x[j]) ++hits;
+        if (key == x[j] || key == kWalkEmpty) break;
+      }
+    }
+  }
+  return hits;
+}
+
+// One block per item: taken from a counter (per_block == 0), or per_block
+// consecutive ones per block. Window columns are bits of a 65,536 bit row,
+// cleared column by column when the item is done; others a hash set at most
+// half full (longer rows: 1,024 columns at a time, the tails streamed again
+// for each part). The block's threads share the sectors of up to four tails
+// each equally, so they meet at the barriers together: with tails handed to
+// warps in groups of 64 the kernel spent half its time there. Vertices of up
+// to 256 entries have blocks of one warp: most of the vertices of R-MAT scale
+// 22, whose set-up by four warps took two thirds of the instructions.
+// WALK_FIGURES
+template <uint32_t kThreads, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks)
+    k_walk_count(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ split,
+                 const uint32_t *__restrict__ long_rows, const __grid_constant__ WalkColumns cols,
+                 uint32_t t0, const uint64_t *__restrict__ keys,
+                 const uint32_t *__restrict__ start, const WalkBits bits,
+                 const uint2 *__restrict__ items, const uint32_t *__restrict__ count,
+                 uint32_t *__restrict__ ticket, uint32_t per_block,
+                 unsigned long long *__restrict__ out) {
+  struct Entry {
+    uint32_t first, len;
+  };
+  static_assert(kWalkSetSlots * 32 == kWalkWindow, "the bit row and the set share memory");
+  constexpr bool kBits = kThreads > 32;  // small vertices have hash sets only
+  constexpr uint32_t kSlots = kBits ? kWalkSetSlots : kWalkSmallSlots;
+  constexpr uint32_t kWarps = kThreads / 32, kGroup = kWalkPer * kThreads;
+  __shared__ __align__(16) uint32_t s_set[kSlots];
+  __shared__ Entry s_e[kGroup];
+  __shared__ uint32_t s_pre[kGroup];
+  __shared__ uint32_t s_head[kThreads], s_cnt[kThreads];
+  __shared__ uint32_t s_warp[kWarps], s_item;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t *ci = cols.base + cols.mis;
+  const uint32_t n_items = *count;
+  const uint32_t not_t0 = t0 - 1;
+  const char *row = reinterpret_cast<const char *>(s_set);
+  constexpr uint32_t word_mask = (kWalkSetSlots - 1) * 4;
+  const uint64_t start_mask = (1ull << bits.start) - 1, len_mask = (1ull << bits.len) - 1;
+  auto fill = [&](uint32_t slots, uint32_t with) {
+    for (uint32_t i = tid; i < slots / 4; i += kThreads)
+      reinterpret_cast<uint4 *>(s_set)[i] = make_uint4(with, with, with, with);
+  };
+  if (kBits) fill(kWalkSetSlots, 0u);
+  unsigned long long hits = 0;
+  uint32_t turn = 0, next = 0;
+  if (tid == 0) next = per_block ? blockIdx.x * per_block : atomicAdd(ticket, 1u);
+  for (;;) {
+    if (tid == 0) s_item = next;
+    __syncthreads();
+    const uint32_t it = s_item;
+    if (it >= n_items) break;
+    ++turn;
+    if (tid == 0)  // the next item, ahead of its use
+      next = per_block ? (turn < per_block ? it + 1 : n_items) : atomicAdd(ticket, 1u);
+    const uint2 item = items[it];
+    const uint32_t x = item.x;
+    const uint32_t e0 = start[x] + item.y * kWalkPiece;
+    const uint32_t e1 = min(start[x + 1], e0 + kWalkPiece);
+    const uint2 set = walk_set(rp, split, long_rows, x);
+    const uint32_t d = set.y - set.x;
+    const bool window = kBits && (x & 1);
+    for (uint32_t part = 0; part < d; part += window || !kBits ? d : kWalkSetCols) {
+      const uint32_t ncols = window || !kBits ? d : min(d - part, kWalkSetCols);
+      const uint32_t slots = min(1u << (32 - __clz(max(ncols * 4u, 256u) - 1u)), kSlots);
+      const uint32_t shift = __clz(slots - 1);
+      for (uint32_t at = e0; at < e1; at += kGroup) {
+        if (part || at > e0) __syncthreads();  // the last group is done with
+        const bool fresh = at == e0;           // the set is built with the first group
+        if (fresh && !window) fill(slots, kWalkEmpty);
+        Entry en[kWalkPer];
+        uint32_t sec[kWalkPer], mine = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kWalkPer; ++j) {
+          const uint32_t i = at + tid * kWalkPer + j;
+          const uint64_t k = i < e1 ? __ldg(keys + i) : 0;
+          en[j] = Entry{(uint32_t)((k >> bits.len) & start_mask) + cols.mis,
+                        (uint32_t)(k & len_mask)};
+          sec[j] = mine;
+          mine += walk_sectors(en[j].first, en[j].len);
+        }
+        const uint32_t incl = walk_scan(mine, lane);
+        uint32_t before = incl - mine, S = 0;
+        if (kWarps > 1) {
+          if (lane == 31) s_warp[warp] = incl;
+          __syncthreads();
+#pragma unroll
+          for (uint32_t q = 0; q < kWarps; ++q) {
+            if (q < warp) before += s_warp[q];
+            S += s_warp[q];
+          }
+        } else {
+          S = __shfl_sync(0xffffffffu, incl, 31);
+          __syncwarp();
+        }
+        const uint32_t k = min(e1 - at, kGroup);
+        if (tid * kWalkPer < k) {
+#pragma unroll
+          for (uint32_t j = 0; j < kWalkPer; ++j) {
+            s_e[tid * kWalkPer + j] = en[j];
+            s_pre[tid * kWalkPer + j] = before + sec[j];
+          }
+        }
+        if (fresh)
+          for (uint32_t i = tid; i < ncols; i += kThreads) {
+            const uint32_t u = __ldg(ci + set.x + part + i), c = u - t0;
+            if (!window)
+              walk_insert(s_set, slots, u, shift);
+            else if (c < kWalkWindow)
+              atomicOr(&s_set[c >> 5], 1u << (c & 31));
+          }
+        __syncthreads();
+        if (window)
+          hits += walk_tails<kGroup, kThreads, kThreads>(
+              cols, s_e, s_pre, s_head, s_cnt, k, S, tid, [] { __syncthreads(); },
+              [&](const uint32_t(&x)[8], const Entry &, uint32_t mask) {
+                // bit c of the row, c = x - t0, at the top of its word
+                // shifted left by ~c (the byte offset wraps, for columns
+                // that are not the tail's)
+                uint32_t b = 0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  const uint32_t nc = not_t0 - x[j];
+                  const uint32_t word =
+                      *reinterpret_cast<const uint32_t *>(row + (~(nc >> 3) & word_mask));
+                  b = __funnelshift_l(word << (nc & 31), b, 1);
+                }
+                return (uint32_t)__popc(b & mask);
+              });
+        else
+          hits += walk_tails<kGroup, kThreads, kThreads>(
+              cols, s_e, s_pre, s_head, s_cnt, k, S, tid, [] { __syncthreads(); },
+              [&](const uint32_t(&x)[8], const Entry &, uint32_t mask) {
+                return walk_find8(s_set, slots, shift, x, mask);
+              });
+      }
+    }
+    __syncthreads();
+    if (window) {
+      for (uint32_t i = tid; i < d; i += kThreads) {
+        const uint32_t c = __ldg(ci + set.x + i) - t0;
+        if (c < kWalkWindow) s_set[c >> 5] = 0;
+      }
+    } else if (kBits) {
+      fill(kWalkSetSlots, 0u);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, o);
+  if (lane == 0 && hits) atomicAdd(out, hits);
+}
+
+// Room for at least x elements, in eighths of a power of two: graphs of one
+// kind then ask the pool for the same sizes and find the blocks that the last
+// count freed (with exact sizes the pool went to the driver now and then:
+// 33-51 ms a count on R-MAT scale 24 for 32).
+inline uint64_t walk_room(uint64_t x) {
+  if (x < 4096) return 4096;
+  const uint64_t step = 1ull << (bits_for(x) - 4);
+  return ceil_div(x, step) * step;
+}
+
+// The walk of one count: its buffers and launches.
+struct WalkRun {
+  WalkBits bits{};
+  uint64_t n = 0, m = 0, rows = 0, cap = 0, entries = 0, big_cap = 0;
+  Scratch<uint64_t> keys, alt;
+  Scratch<uint32_t> split, start, counts;  // entries made, big, small items, tickets
+  Scratch<uint2> big, small;
+  prim::SortSpace ws;
+  const uint64_t *sorted = nullptr;
+
+  static unsigned grid(DeviceContext *ctx, uint64_t threads) {
+    const uint64_t most = (uint64_t)ctx->sm_count * 32, g = ceil_div(threads, kWalkBlock);
+    return (unsigned)(g == 0 ? 1 : g < most ? g : most);
+  }
+  // Whether an entry fits 64 bits.
+  bool fits(uint64_t n_, uint64_t m_, uint64_t long_rows, uint64_t longest) {
+    n = n_;
+    m = m_;
+    rows = long_rows;
+    bits.w = 1 + (rows > 1 ? bits_for(rows - 1) : 1);
+    bits.start = bits_for(m);
+    bits.len = bits_for(longest);
+    return n < (1ull << 31) && m < (1ull << 31) && bits.w + bits.start + bits.len <= 64;
+  }
+  // Room for `most` entries.
+  int alloc(DeviceContext *ctx, cudaStream_t st, uint64_t most) {
+    cap = walk_room(most);
+    const uint64_t room = walk_room(2 * rows);
+    WETRIC_TRY(split.alloc(ctx, st, n));
+    WETRIC_TRY(keys.alloc(ctx, st, cap));
+    WETRIC_TRY(alt.alloc(ctx, st, cap));
+    WETRIC_TRY(counts.alloc(ctx, st, 8));
+    WETRIC_CUDA_TRY(cudaMemsetAsync(counts.ptr, 0, 8 * sizeof(uint32_t), st));
+    big_cap = cap / kWalkPiece + cap / kWalkBig + m / kWalkBigCols + 1;
+    WETRIC_TRY(start.alloc(ctx, st, room + 1));
+    WETRIC_TRY(small.alloc(ctx, st, room));
+    WETRIC_TRY(ws.alloc(ctx, st, cap));
+    return big.alloc(ctx, st, big_cap);
+  }
+  // The entries made, sorted by middle vertex, and the work items.
+  int sort(DeviceContext *ctx, cudaStream_t st, const uint32_t *rp, const uint32_t *long_rows,
+           uint64_t made, uint32_t *err, uint32_t *launches) {
+    entries = made;
+    const prim::KeysFrom from{keys.ptr};
+    uint64_t *to = prim::sorted_buffer(alt.ptr, keys.ptr, bits.shift(), bits.w);
+    WETRIC_TRY((prim::radix_sort_into(ctx, st, from, from, alt.ptr, keys.ptr, prim::KeysTo{to},
+                                      entries, bits.shift(), bits.w, err, &ws)));
+    sorted = to;
+    k_walk_starts<<<grid(ctx, entries), kWalkBlock, 0, st>>>(
+        sorted, (uint32_t)entries, (uint32_t)(2 * rows), bits.shift(), start.ptr);
+    WETRIC_LAUNCH_CHECK();
+    k_walk_plan<<<grid(ctx, 2 * rows), kWalkBlock, 0, st>>>(
+        rp, split.ptr, long_rows, start.ptr, (uint32_t)(2 * rows), big.ptr, small.ptr,
+        counts.ptr + 1);
+    WETRIC_LAUNCH_CHECK();
+    *launches += 3 + prim::digit_plan(bits.shift(), bits.w).passes;
+    return WETRIC_OK;
+  }
+  // The count. Persistent: one wave of blocks, items from a counter; otherwise
+  // short blocks, so other streams' blocks get SMs in between.
+  int count(DeviceContext *ctx, cudaStream_t st, const uint32_t *rp, const uint32_t *ci,
+            const uint32_t *long_rows, bool persistent, unsigned long long *out, uint64_t *most,
+            uint32_t *launches) {
+    constexpr uint32_t kPerBlock = 16;
+    const auto big_fn = k_walk_count<kWalkBigBlock, kWalkBigBlocks>;
+    const auto small_fn = k_walk_count<kWalkSmallBlock, kWalkSmallBlocks>;
+    const uint64_t g = persistent ? (uint64_t)ctx->sm_count * kWalkBigBlocks
+                                  : ceil_div(big_cap, kPerBlock);
+    const uint64_t gs = persistent ? (uint64_t)ctx->sm_count * kWalkSmallBlocks
+                                   : ceil_div(2 * rows, kPerBlock);
+    const WalkColumns cols = walk_columns(ci, m);
+    const uint32_t t0 = n > kWalkWindow ? (uint32_t)(n - kWalkWindow) : 0u;
+    // The sector loads need L1 lines for the data in flight: with the shared
+    // memory of as many blocks as fit (218 KB) about 80 lines were left and
+    // the kernel ran at 1.2 TB/s of sectors.
+    WETRIC_CUDA_TRY(cudaFuncSetAttribute(
+        big_fn, cudaFuncAttributePreferredSharedMemoryCarveout, kWalkCarveout));
+    WETRIC_CUDA_TRY(cudaFuncSetAttribute(
+        small_fn, cudaFuncAttributePreferredSharedMemoryCarveout, kWalkCarveout));
+    big_fn<<<(unsigned)g, kWalkBigBlock, 0, st>>>(
+        rp, split.ptr, long_rows, cols, t0, sorted, start.ptr, bits, big.ptr, counts.ptr + 1,
+        counts.ptr + 3, persistent ? 0 : kPerBlock, out);
+    WETRIC_LAUNCH_CHECK();
+    small_fn<<<(unsigned)gs, kWalkSmallBlock, 0, st>>>(
+        rp, split.ptr, long_rows, cols, t0, sorted, start.ptr, bits, small.ptr, counts.ptr + 2,
+        counts.ptr + 4, persistent ? 0 : kPerBlock, out);
+    WETRIC_LAUNCH_CHECK();
+    *launches += 2;
+    if (g > *most) *most = g;
+    return WETRIC_OK;
+  }
+};
+
+}  // namespace
+}  // namespace wetric

@@ -445,12 +445,13 @@ def count(row_ptr, col_ind, s: int = 5, a: int = 8192, *, oriented: bool = True,
     wedge range only the triangles closed by those wedges are counted.
     ``stream`` is a ``torch.cuda.Stream`` (or raw handle) to run on.
     ``kernel`` picks the count kernel (``wetric_opts.kernel``: 0 = the
-    default, 8, the row walk with long-row segments and 16-bit near hash
+    default, row intersections and the column walk for whole graphs and 8 for
+    the rest; 8 = the row walk with long-row segments and 16-bit near hash
     sets; 1-7 the earlier variants). ``core_len`` sizes the dense core
     (``wetric_opts.core_len``: 0 = chosen by the library, :data:`CORE_OFF` =
     none, else that many top vertices counted by row ANDs) and ``shell_len``
-    the shell below it (0 = none). ``pair_streams=False`` turns off the
-    pair streams for short rows (``WETRIC_OPT_NO_PAIR_STREAMS``). A host CSR of
+    the shell below it (0 = none). ``pair_streams=False`` counts every wedge
+    below the core by a set lookup (``WETRIC_OPT_NO_PAIR_STREAMS``). A host CSR of
     2^22 columns or more is copied in row chunks, highest rows first, and
     counted as it arrives.
     """
