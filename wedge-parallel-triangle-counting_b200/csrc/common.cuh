@@ -9,6 +9,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -90,6 +91,16 @@ int set_budget(int device, uint64_t bytes);
 // Stream-ordered device scratch owned by a context.
 int dev_alloc(DeviceContext *ctx, cudaStream_t s, size_t bytes, void **p);
 void dev_free(DeviceContext *ctx, cudaStream_t s, void *p, size_t bytes);
+
+// Loads kernels (their first launch would): a kernel that is first launched
+// while another one runs may have to wait for it to end.
+inline int load_kernels(std::initializer_list<const void *> kernels) {
+  for (const void *k : kernels) {
+    cudaFuncAttributes at;
+    WETRIC_CUDA_TRY(cudaFuncGetAttributes(&at, k));
+  }
+  return WETRIC_OK;
+}
 
 // RAII holder for one scratch allocation.
 template <typename T>

@@ -569,6 +569,24 @@ int orient_pairs(DeviceContext *ctx, cudaStream_t st, const uint32_t *src,
   return checked_words(st, words.ptr, "orientation", &h);
 }
 
+int load_orient_kernels() {
+  using prim::KeysFrom;
+  using prim::KeysTo;
+  WETRIC_TRY((prim::load_onesweep<CanonPairs<false>, KeysTo>()));
+  WETRIC_TRY((prim::load_onesweep<KeysFrom, KeysTo>()));
+  WETRIC_TRY((prim::load_onesweep<DegreeKeys, KeysTo>()));
+  WETRIC_TRY((prim::load_onesweep<DegreeKeys, RankTo>()));
+  WETRIC_TRY((prim::load_onesweep<KeysFrom, RankTo>()));
+  WETRIC_TRY((prim::load_onesweep<GroupKeys, KeysTo>()));
+  WETRIC_TRY((prim::load_onesweep<GroupKeys, RankTo>()));
+  return load_kernels({(const void *)k_max_id, (const void *)k_unique_degrees,
+                       (const void *)k_max_u32, (const void *)k_keys_to_csr,
+                       (const void *)prim::k_radix_hist<CanonPairs<true>>,
+                       (const void *)prim::k_radix_hist<DegreeKeys>,
+                       (const void *)prim::k_radix_hist<GroupKeys>,
+                       (const void *)prim::k_radix_hist<OrientedKeys>});
+}
+
 int symmetric_from_pairs(DeviceContext *ctx, cudaStream_t st,
                          const uint32_t *src, const uint32_t *dst, uint64_t P,
                          uint64_t n_hint, DeviceCsr *out) {

@@ -31,6 +31,9 @@ int orient_pairs(DeviceContext *ctx, cudaStream_t st, const uint32_t *src,
                  DeviceCsr *out, const uint64_t *group_base = nullptr,
                  uint32_t G = 0);
 
+// Loads the kernels of orient_pairs.
+int load_orient_kernels();
+
 // Raw pairs -> symmetric deduplicated CSR without self-loops (the CSR that
 // read_graph returns, tc.cu:561-685).
 int symmetric_from_pairs(DeviceContext *ctx, cudaStream_t st,

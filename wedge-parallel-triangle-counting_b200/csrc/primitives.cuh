@@ -243,7 +243,22 @@ constexpr int kSortThreads = 384;
 constexpr int kSortBlocks = 3;  // per SM
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortItems = 16;  // per thread
-constexpr int kSortTile = kSortThreads * kSortItems;
+// Few keys: a pass is one block's latency, and a tile of a quarter shortens
+// it while every tile still has an SM and the look-back stays short
+// (orientation of 2,000 pairs 162 -> 149 us, of 200,000 221 -> 197 us; with
+// 4 tiles per SM 400,000 pairs took 247 us against 243). Its 27 KB of shared memory
+// also fit beside the resident serving kernel, whose SMs keep the
+// shared-memory split they were started with: a large tile could wait there
+// until that kernel ended.
+constexpr int kSortFewItems = 4;
+constexpr uint64_t kSortFewTiles = 148;
+constexpr uint64_t kSortFewKeys = kSortFewTiles * kSortThreads * kSortFewItems;
+// Most tiles of a sort of up to n keys.
+inline uint64_t sort_tiles(uint64_t n) {
+  if (n <= kSortFewKeys) return ceil_div(n, kSortThreads * kSortFewItems);
+  const uint64_t tiles = ceil_div(n, kSortThreads * kSortItems);
+  return tiles > kSortFewTiles ? tiles : kSortFewTiles;
+}
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
 constexpr int kMaxPasses = 8;
@@ -355,19 +370,21 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d, uint32_t valid) {
 // 8-byte stores. Tile shape from a sweep at 64M 44-bit keys, whole sort: 384
 // threads x 16 keys x 3 blocks 2.46 ms, 512 x 16 x 2 2.48, 256 x 16 x 4 2.84,
 // 1024 x 12 x 1 2.97, 512 x 8 x 3 2.92; five 9-bit passes 2.61 (512 x 16).
-constexpr size_t kSortSmem = kSortTile * sizeof(uint64_t) +
-                             kSortWarps * kRadix * sizeof(uint32_t) +
-                             kRadix * (sizeof(uint64_t) + sizeof(uint32_t));
+constexpr size_t sort_smem(int items) {
+  return kSortThreads * items * sizeof(uint64_t) + kSortWarps * kRadix * sizeof(uint32_t) +
+         kRadix * (sizeof(uint64_t) + sizeof(uint32_t));
+}
 constexpr int kLookAhead = 4;
-template <int kBits, bool kHigh, class Load, class Sink>
+template <int kBits, bool kHigh, int kItems, class Load, class Sink>
 __global__ void __launch_bounds__(kSortThreads, kSortBlocks)
     k_onesweep(Load load, Sink sink, uint64_t n, uint32_t shift, uint32_t bits, uint32_t epoch,
                const unsigned long long *__restrict__ hist, uint64_t *__restrict__ state,
                uint32_t *__restrict__ ticket, uint32_t *err) {
+  constexpr int kTile = kSortThreads * kItems;
   static_assert(kSortThreads >= kRadix, "thread d owns digit d");
   extern __shared__ __align__(16) unsigned char s_raw[];
   uint64_t *s_key = reinterpret_cast<uint64_t *>(s_raw);
-  uint64_t *s_goff = s_key + kSortTile;
+  uint64_t *s_goff = s_key + kTile;
   uint32_t *s_toff = reinterpret_cast<uint32_t *>(s_goff + kRadix);
   uint32_t *s_whist = s_toff + kRadix;
   __shared__ uint32_t s_warp[kSortWarps];
@@ -381,19 +398,19 @@ __global__ void __launch_bounds__(kSortThreads, kSortBlocks)
   for (uint32_t i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads) s_whist[i] = 0;
   __syncthreads();
   const uint64_t tile = s_ticket;
-  const uint64_t base = tile * kSortTile;
-  const uint32_t count = n - base < kSortTile ? (uint32_t)(n - base) : kSortTile;
+  const uint64_t base = tile * kTile;
+  const uint32_t count = n - base < kTile ? (uint32_t)(n - base) : kTile;
   const uint32_t mask = (1u << bits) - 1u;
-  const uint32_t sub = warp * 32 * kSortItems + lane;
+  const uint32_t sub = warp * 32 * kItems + lane;
   uint32_t *wh = s_whist + warp * kRadix;
-  uint64_t k[kSortItems];
-  uint16_t rank[kSortItems];  // below 32 * kSortItems
+  uint64_t k[kItems];
+  uint16_t rank[kItems];  // below 32 * kItems
   const uint32_t lt = (1u << lane) - 1u;
-  if (count == kSortTile) {
+  if (count == kTile) {
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j) k[j] = load(base + sub + j * 32);
+    for (int j = 0; j < kItems; ++j) k[j] = load(base + sub + j * 32);
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
+    for (int j = 0; j < kItems; ++j) {
       const uint32_t d = key_digit<kHigh>(k[j], shift, mask);
       const uint32_t peers = match_digit<kBits>(d, 0xffffffffu);
       const uint32_t leader = __ffs(peers) - 1;
@@ -403,10 +420,10 @@ __global__ void __launch_bounds__(kSortThreads, kSortBlocks)
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j)
+    for (int j = 0; j < kItems; ++j)
       k[j] = sub + j * 32 < count ? load(base + sub + j * 32) : 0;
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
+    for (int j = 0; j < kItems; ++j) {
       const bool valid = sub + j * 32 < count;
       const uint32_t d = key_digit<kHigh>(k[j], shift, mask);
       const uint32_t peers = match_digit<kBits>(d, __ballot_sync(0xffffffffu, valid));
@@ -434,7 +451,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortBlocks)
   if (threadIdx.x < kRadix) s_toff[threadIdx.x] = incl - c;
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
+  for (int j = 0; j < kItems; ++j) {
     if (sub + j * 32 < count) {
       const uint32_t d = key_digit<kHigh>(k[j], shift, mask);
       s_key[s_toff[d] + wh[d] + rank[j]] = k[j];
@@ -507,7 +524,7 @@ struct SortSpace {
   uint64_t *state = nullptr;
   int alloc(DeviceContext *ctx, cudaStream_t st, uint64_t n) {
     const uint64_t head = (uint64_t)kMaxPasses * kRadix + kMaxPasses;
-    const uint64_t words = head + ceil_div(n, kSortTile) * kRadix;
+    const uint64_t words = head + sort_tiles(n) * kRadix;
     WETRIC_TRY(buf.alloc(ctx, st, words));
     WETRIC_CUDA_TRY(cudaMemsetAsync(buf.ptr, 0, words * sizeof(uint64_t), st));
     hist = reinterpret_cast<unsigned long long *>(buf.ptr);
@@ -517,28 +534,51 @@ struct SortSpace {
   }
 };
 
-template <int kBits, bool kHigh, class Load, class Sink>
+template <int kBits, bool kHigh, int kItems, class Load, class Sink>
 int onesweep_launch(cudaStream_t st, const Load &load, const Sink &sink, uint64_t n,
                     const DigitPlan &plan, uint32_t p, const SortSpace &ws, uint32_t *err) {
-  const auto fn = k_onesweep<kBits, kHigh, Load, Sink>;
-  WETRIC_CUDA_TRY(
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortSmem));
-  fn<<<(unsigned)ceil_div(n, kSortTile), kSortThreads, kSortSmem, st>>>(
+  const auto fn = k_onesweep<kBits, kHigh, kItems, Load, Sink>;
+  constexpr size_t smem = sort_smem(kItems);
+  if (smem > 48 * 1024)
+    WETRIC_CUDA_TRY(
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  fn<<<(unsigned)ceil_div(n, kSortThreads * kItems), kSortThreads, smem, st>>>(
       load, sink, n, plan.shift[p], plan.bits[p], p + 1, ws.hist + (uint64_t)p * kRadix, ws.state,
       ws.tickets + p, err);
   WETRIC_LAUNCH_CHECK();
   return WETRIC_OK;
 }
 
+template <int kItems, class Load, class Sink>
+int onesweep_items(cudaStream_t st, const Load &load, const Sink &sink, uint64_t n,
+                   const DigitPlan &plan, uint32_t p, const SortSpace &ws, uint32_t *err) {
+  const bool high = plan.shift[p] >= 32;
+  if (plan.bits[p] > 7)
+    return high ? onesweep_launch<8, true, kItems>(st, load, sink, n, plan, p, ws, err)
+                : onesweep_launch<8, false, kItems>(st, load, sink, n, plan, p, ws, err);
+  return high ? onesweep_launch<7, true, kItems>(st, load, sink, n, plan, p, ws, err)
+              : onesweep_launch<7, false, kItems>(st, load, sink, n, plan, p, ws, err);
+}
+
 template <class Load, class Sink>
 int onesweep_pass(cudaStream_t st, const Load &load, const Sink &sink, uint64_t n,
                   const DigitPlan &plan, uint32_t p, const SortSpace &ws, uint32_t *err) {
-  const bool high = plan.shift[p] >= 32;
-  if (plan.bits[p] > 7)
-    return high ? onesweep_launch<8, true>(st, load, sink, n, plan, p, ws, err)
-                : onesweep_launch<8, false>(st, load, sink, n, plan, p, ws, err);
-  return high ? onesweep_launch<7, true>(st, load, sink, n, plan, p, ws, err)
-              : onesweep_launch<7, false>(st, load, sink, n, plan, p, ws, err);
+  return n <= kSortFewKeys
+             ? onesweep_items<kSortFewItems>(st, load, sink, n, plan, p, ws, err)
+             : onesweep_items<kSortItems>(st, load, sink, n, plan, p, ws, err);
+}
+
+// Loads the forms of a pass.
+template <class Load, class Sink>
+int load_onesweep() {
+  return load_kernels({(const void *)k_onesweep<7, false, kSortItems, Load, Sink>,
+                       (const void *)k_onesweep<7, true, kSortItems, Load, Sink>,
+                       (const void *)k_onesweep<8, false, kSortItems, Load, Sink>,
+                       (const void *)k_onesweep<8, true, kSortItems, Load, Sink>,
+                       (const void *)k_onesweep<7, false, kSortFewItems, Load, Sink>,
+                       (const void *)k_onesweep<7, true, kSortFewItems, Load, Sink>,
+                       (const void *)k_onesweep<8, false, kSortFewItems, Load, Sink>,
+                       (const void *)k_onesweep<8, true, kSortFewItems, Load, Sink>});
 }
 
 // Stable LSD sort of n keys on their bits [lo, lo + bits). `counted` gives
@@ -557,7 +597,7 @@ int radix_sort_into(DeviceContext *ctx, cudaStream_t st, const Counted &counted,
   SortSpace own;
   if (!space) WETRIC_TRY(own.alloc(ctx, st, n));
   const SortSpace &ws = space ? *space : own;
-  uint64_t blocks = ceil_div(n, 256 * 16);
+  uint64_t blocks = ceil_div(n, 256 * (n <= kSortFewKeys ? kSortFewItems : kSortItems));
   const uint64_t cap = (uint64_t)ctx->sm_count * 8;
   if (blocks > cap) blocks = cap;
   const size_t hs = (size_t)plan.passes * kRadix * kHistCopies * sizeof(uint32_t);

@@ -6,6 +6,30 @@
 #include "common.cuh"
 
 namespace wetric {
+
+constexpr uint32_t kReadWords = 128;
+// Pinned words for the calling thread's read-backs (portable: any device),
+// made on first use and freed when the thread ends; null if pinned memory
+// cannot be had (the caller then reads into its own array).
+inline uint64_t *readback_words() {
+  struct Holder {
+    uint64_t *p = nullptr;
+    bool tried = false;
+    ~Holder() {
+      if (p) cudaFreeHost(p);
+    }
+  };
+  thread_local Holder h;
+  if (!h.tried) {
+    h.tried = true;
+    if (cudaHostAlloc(reinterpret_cast<void **>(&h.p), kReadWords * sizeof(uint64_t),
+                      cudaHostAllocPortable) != cudaSuccess) {
+      h.p = nullptr;
+      cudaGetLastError();
+    }
+  }
+  return h.p;
+}
 namespace {
 
 // Host read-backs: one gather kernel collects the values into a device
@@ -17,7 +41,6 @@ struct ReadSpan {
   uint32_t count, bytes;  // elements of 4 or 8 bytes
 };
 constexpr uint32_t kReadSpans = 24;
-constexpr uint32_t kReadWords = 128;
 struct ReadPlan {
   ReadSpan s[kReadSpans];
   uint32_t n = 0, total = 0;
@@ -38,28 +61,6 @@ __global__ void k_read_gather(const __grid_constant__ ReadPlan p, uint64_t *__re
                                    : static_cast<const uint64_t *>(sp.src)[j];
 }
 static_assert(kReadWords <= 128, "one word per thread of the gather's block");
-// Pinned words for the calling thread's read-backs (portable: any device),
-// made on first use and freed when the thread ends; null if pinned memory
-// cannot be had (the caller then reads into its own array).
-uint64_t *readback_words() {
-  struct Holder {
-    uint64_t *p = nullptr;
-    bool tried = false;
-    ~Holder() {
-      if (p) cudaFreeHost(p);
-    }
-  };
-  thread_local Holder h;
-  if (!h.tried) {
-    h.tried = true;
-    if (cudaHostAlloc(reinterpret_cast<void **>(&h.p), kReadWords * sizeof(uint64_t),
-                      cudaHostAllocPortable) != cudaSuccess) {
-      h.p = nullptr;
-      cudaGetLastError();
-    }
-  }
-  return h.p;
-}
 // Gathers plan's values on st, copies them to the host and waits (for
 // `done`, recorded after the copy, when given); *words points at them
 // afterwards (valid until the calling thread's next read).

@@ -220,6 +220,19 @@ void *host_mapped(size_t bytes, void **dev) {
 
 // ------------------------------------------------------------ preparation
 
+int serve_load_kernels() {
+  return load_kernels(
+      {(const void *)k_vertex_wedges<uint32_t>, (const void *)k_pair_plan<false>,
+       (const void *)k_compact_active<uint32_t>, (const void *)k_hash_sizes<uint32_t>,
+       (const void *)k_core_plan<uint32_t>, (const void *)k_core_prefix,
+       (const void *)k_tile_map, (const void *)k_bitmap<uint32_t>, (const void *)k_hash_rows,
+       (const void *)k_hash_build<uint32_t>, (const void *)k_near_build<uint32_t>,
+       (const void *)k_core_bitmap<uint32_t>, (const void *)k_core_count<uint32_t>,
+       (const void *)k_shell_count<uint32_t, true>, (const void *)k_count_pairs<false>,
+       (const void *)prim::k_scan<uint32_t, uint64_t>,
+       (const void *)prim::k_scan<uint64_t, uint64_t>});
+}
+
 int serve_prepare(DeviceContext *ctx, cudaStream_t st, uint32_t spread,
                   uint32_t bitmap_len, ServePlan *p) {
   NvtxRange nvtx_("wetric serve prepare");

@@ -47,6 +47,9 @@ struct ServePlan {
   }
 };
 
+// Loads the kernels that requests launch while the resident one runs.
+int serve_load_kernels();
+
 // Builds every structure of plan->csr's count on `st` and waits for them:
 // the work of count_oriented up to (not including) the count launch.
 int serve_prepare(DeviceContext *ctx, cudaStream_t st, uint32_t spread,

@@ -40,6 +40,7 @@
 #include "common.cuh"
 #include "count.cuh"
 #include "preprocess.cuh"
+#include "readback.cuh"
 #include "serve.cuh"
 
 namespace wetric {
@@ -137,6 +138,7 @@ struct Server {
   uint64_t items_reserved = 0;              // items live requests will still publish
   uint64_t freed_seen = 0, recycles = 0;
   int lanes_running = 0;
+  int lanes_ready = 0;  // resident workers that have their pinned words
   uint32_t lane_phase[2] = {0, 0};  // see wetric_server_stats::lane_phase
   Lane lanes[2];  // 0: small requests, 1: large requests
   std::unordered_map<uint64_t, Result> results;
@@ -423,6 +425,14 @@ void lane_loop_resident(Lane *ln, cudaStream_t wst) {
   Server *s = ln->srv;
   cudaSetDevice(s->ctx->device);
   const int li = ln == &s->lanes[1] ? 1 : 0;
+  // pinned memory is allocated before any request: beside the resident
+  // kernel the allocation would wait for it to go idle
+  readback_words();
+  {
+    std::lock_guard<std::mutex> lk(s->mu);
+    ++s->lanes_ready;
+    s->cv_done.notify_all();
+  }
   for (;;) {
     Request r;
     {
@@ -695,9 +705,23 @@ int wetric_server_create(int device, const wetric_server_opts *opts,
       return WETRIC_ECUDA;
     }
   }
-  // Warm-up before the first request: every lane runs a tiny graph through
-  // both paths (loads the kernels, sets up the streams) and grows the memory
-  // pool by reserve_bytes once, so no request pays for either.
+  // Warm-up before the first request: the kernels that graphs of any size
+  // use in preprocessing are loaded (beside the resident kernel a first
+  // launch would wait for it to go idle), every lane runs a tiny graph through
+  // both paths (which sets up the streams) and grows the memory pool by
+  // reserve_bytes once, so no request pays for either.
+  {
+    int lst = load_orient_kernels();
+    if (lst == WETRIC_OK)
+      lst = load_kernels({(const void *)k_csr_to_pairs<uint32_t>,
+                          (const void *)k_csr_to_pairs<uint64_t>});
+    if (lst == WETRIC_OK && o.resident) lst = serve_load_kernels();
+    if (lst != WETRIC_OK) {
+      for (Lane &l2 : h->s.lanes) cudaStreamDestroy(l2.stream);
+      delete h;
+      return lst;
+    }
+  }
   for (Lane &ln : h->s.lanes) {
     const int wst = warm_up_lane(&h->s, &ln);
     if (wst != WETRIC_OK) {
@@ -743,6 +767,10 @@ int wetric_server_create(int device, const wetric_server_opts *opts,
     for (Lane &ln : h->s.lanes) {
       ln.worker = std::thread(lane_loop_resident, &ln, ln.stream);
       for (cudaStream_t x : ln.more_streams) ln.more.emplace_back(lane_loop_resident, &ln, x);
+    }
+    {
+      std::unique_lock<std::mutex> lk(h->s.mu);
+      h->s.cv_done.wait(lk, [&] { return h->s.lanes_ready == workers; });
     }
     h->s.monitor = std::thread(monitor_loop, &h->s);
   } else {
