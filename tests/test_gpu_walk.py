@@ -137,3 +137,34 @@ def test_small_graphs_in_one_pass(wetric_mod, oracle_mod):
                     bad[1] = g.m + 5
                     with pytest.raises(wetric_mod.WetricError):
                         wetric_mod.count(bad, ci, 5, 8192)
+
+
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_batch_walk(wetric_mod, oracle_mod, use_graph):
+    """A batch whose long rows are walked per graph: graphs past one
+    65,536-bit window beside tiny and empty ones, so that graph boundaries
+    fall inside windows, tiles and groups of entries; every count repeated."""
+    rng = np.random.default_rng(3)
+    parts, n = [], []
+    for kind in ("rmat", "dense", "hub"):
+        g = graph(oracle_mod, kind)
+        i = np.repeat(np.arange(g.n), np.diff(g.row_ptr.astype(np.int64)))
+        parts.append((i.astype(np.uint32), g.col_ind.astype(np.uint32)))
+        n.append(g.n)
+        for size in (1, 3, 40, 700):
+            e = 0 if size == 1 else 6 * size
+            parts.append(tuple(rng.integers(0, size, e).astype(np.uint32) for _ in "sd"))
+            n.append(size)
+    order = rng.permutation(len(parts))
+    parts, n = [parts[i] for i in order], [n[i] for i in order]
+    want = [oracle_mod.count_merge(oracle_mod.oriented_from_pairs(*p)) if p[0].size else 0
+            for p in parts]
+    src, dst = (np.concatenate([p[k] for p in parts]) for k in (0, 1))
+    off = np.concatenate([[0], np.cumsum([p[0].size for p in parts])]).astype(np.uint64)
+    args = (src, dst, off, np.array(n, np.uint64))
+    b = wetric_mod.Batch(*args, use_cuda_graph=use_graph)
+    for _ in range(3):
+        got, _ = b.count()
+        assert [int(x) for x in got] == want
+    got, _ = wetric_mod.Batch(*args, use_cuda_graph=use_graph, pair_streams=False).count()
+    assert [int(x) for x in got] == want

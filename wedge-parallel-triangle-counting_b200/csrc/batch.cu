@@ -1,23 +1,31 @@
-// batch.cu -- many graphs of uneven sizes counted in one persistent launch.
+// batch.cu -- many graphs of uneven sizes counted together.
 //
 // The reference counts one graph per process run (tc.cu:896-913). Here a
 // batch of G graphs is preprocessed once as a disjoint union (graph g owns
 // ids [vbase[g], vbase[g+1]) and is ranked inside its own range, so its
 // oriented CSR equals the one it gets alone), kept resident on the device,
-// and counted by the row-walk kernel over the union's wedge space: every
-// tile the persistent warps pull from the device work counter is a
+// and counted like a single graph, per graph (walk.cuh): the edges intersect
+// short rows in tiles over the union, and the entries of the edges to long
+// rows, sorted when the batch is made, stream through those rows' sets.
+//
+// A batch of 2^31 columns or more, without room for the entries, or with pair
+// streams off is counted by the row-walk kernel over the union's wedge space:
+// every tile the persistent warps pull from the device work counter is a
 // (graph, wedge-range) piece, and hits accumulate per graph. Each graph has
 // its own bitmap over its last min(a, n_g) vertices and per-row hash sets
 // for its longer rows below the bitmap; graph g's tiles hold 256 * s_g
 // wedges, s_g from the autotuner's per-device table of size/skew buckets
-// (or a size table); the count is captured once in a CUDA graph and
-// replayed per count.
+// (or a size table).
+//
+// The count is captured once in a CUDA graph and replayed per count.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
 
 #include <algorithm>
 #include <map>
+#include <memory>
+#include <new>
 #include <numeric>
 #include <vector>
 
@@ -27,8 +35,17 @@
 #include "pair_streams.cuh"
 #include "preprocess.cuh"
 #include "primitives.cuh"
+#include "readback.cuh"
+#include "walk.cuh"
 
 namespace wetric {
+
+struct BatchWalk {
+  WalkRun run;
+  Scratch<uint32_t> number, long_rows, long_graph;
+  Scratch<unsigned long long> words;  // [0] unused, [1] wedges of short rows, [2] error
+  bool entries = false;
+};
 
 namespace {
 
@@ -162,6 +179,64 @@ __global__ void k_pair_graph_wedges(const uint32_t *__restrict__ rp,
   }
 }
 
+// The batch's rows: W per graph, totals ([0] longest row, [1] rows with wedges,
+// [2] long rows, [3] the long rows' wedges), and the long rows with their
+// graphs. A warp takes 32 rows; mostly they are one graph's.
+__global__ void __launch_bounds__(kWalkBlock)
+    k_batch_rows(const uint32_t *__restrict__ rp, uint64_t n, uint64_t m, const WalkGroups groups,
+                 unsigned long long *__restrict__ W, unsigned long long *__restrict__ totals,
+                 uint32_t *__restrict__ number, uint32_t *__restrict__ long_rows,
+                 uint32_t *__restrict__ long_graph, uint32_t *err) {
+  const uint32_t lane = threadIdx.x & 31;
+  unsigned long long rows = 0, longest = 0, long_w = 0;
+  for (uint64_t v0 = (uint64_t)blockIdx.x * kWalkBlock + threadIdx.x - lane; v0 < n;
+       v0 += (uint64_t)gridDim.x * kWalkBlock) {
+    const uint64_t v = v0 + lane;
+    const uint32_t g0 = (uint32_t)row_of_edge(groups.base, 0, groups.G, v0, lane);
+    const bool same = v0 + 32 <= groups.base[g0 + 1];
+    uint64_t d = 0;
+    if (v < n) {
+      const uint32_t b = rp[v], e = rp[v + 1];
+      if (e < b || e > m)
+        atomicCAS(err, 0u, (uint32_t)kDevRowPtrRange);
+      else
+        d = e - b;
+    }
+    unsigned long long w = d >= 2 ? d * (d - 1) / 2 : 0;
+    rows += d >= 2;
+    longest = longest > d ? longest : d;
+    const bool is_long = d > kWalkShortCols;
+    if (is_long) long_w += w;
+    const uint32_t g = same || v >= n ? g0 : walk_group(groups, v);
+    const uint32_t mask = __ballot_sync(0xffffffffu, is_long);
+    uint32_t id = 0;
+    if (mask && lane == 0) id = (uint32_t)atomicAdd(totals + 2, (unsigned long long)__popc(mask));
+    id = __shfl_sync(0xffffffffu, id, 0) + __popc(mask & ((1u << lane) - 1u));
+    if (v < n) number[v] = is_long ? id : kWalkShort;
+    if (is_long) {
+      long_rows[id] = (uint32_t)v;
+      long_graph[id] = g;
+    }
+    if (same) {
+      for (int o = 16; o > 0; o >>= 1) w += __shfl_down_sync(0xffffffffu, w, o);
+      if (lane == 0 && w) atomicAdd(W + g0, w);
+    } else if (w) {
+      atomicAdd(W + g, w);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    rows += __shfl_down_sync(0xffffffffu, rows, o);
+    long_w += __shfl_down_sync(0xffffffffu, long_w, o);
+    const unsigned long long x = __shfl_down_sync(0xffffffffu, longest, o);
+    longest = longest > x ? longest : x;
+  }
+  if (lane == 0) {
+    atomicMax(totals, longest);
+    if (rows) atomicAdd(totals + 1, rows);
+    if (long_w) atomicAdd(totals + 3, long_w);
+  }
+}
+
 // out[g] = row offset of graph g's first id (g <= G), so out[g+1] - out[g]
 // is graph g's oriented edge count.
 __global__ void k_first_offsets(const uint64_t *__restrict__ rp,
@@ -198,6 +273,7 @@ void Batch::release_all() {
   graph = nullptr;
 }
 
+Batch::Batch() = default;
 Batch::~Batch() { release_all(); }
 
 // Sizes the per-graph bitmaps: a_g = min(a, n_g rounded up to 32), and no
@@ -360,6 +436,101 @@ static int autotune_spreads(Batch *b, std::vector<uint32_t> *sg, cudaStream_t st
   return WETRIC_OK;
 }
 
+// Rows and, where they pay, the long rows' entries of a batch counted by row
+// intersections and the walk; b->whole stays false when there is no room.
+static int make_whole(Batch *b, cudaStream_t st) {
+  DeviceContext *ctx = b->ctx;
+  const uint32_t G = b->G;
+  const uint64_t n = b->vbase[G], m = b->m_total;
+  WETRIC_TRY(b->vbase_d.alloc(ctx, st, G + 1));
+  WETRIC_TRY(b->counts.alloc(ctx, st, G));
+  WETRIC_CUDA_TRY(cudaMemcpyAsync(b->vbase_d.ptr, b->vbase.data(), (G + 1) * 8,
+                                  cudaMemcpyHostToDevice, st));
+  std::unique_ptr<BatchWalk> w(new (std::nothrow) BatchWalk());
+  if (!w) {
+    set_error(WETRIC_ENOMEM, "host allocation failed");
+    return WETRIC_ENOMEM;
+  }
+  constexpr uint32_t kWords = 8;  // BatchWalk::words, then k_batch_rows' totals
+  WETRIC_TRY(w->words.alloc(ctx, st, kWords + G));
+  WETRIC_CUDA_TRY(cudaMemsetAsync(w->words.ptr, 0, (kWords + G) * 8ull, st));
+  uint32_t *err = reinterpret_cast<uint32_t *>(w->words.ptr + 2);
+  if (w->number.alloc(ctx, st, n) != WETRIC_OK ||
+      w->long_rows.alloc(ctx, st, m / (kWalkShortCols + 1) + 1) != WETRIC_OK ||
+      w->long_graph.alloc(ctx, st, m / (kWalkShortCols + 1) + 1) != WETRIC_OK) {
+    clear_error();
+    return WETRIC_OK;
+  }
+  const WalkGroups groups{b->vbase_d.ptr, G, b->counts.ptr};
+  k_batch_rows<<<WalkRun::grid(ctx, n), kWalkBlock, 0, st>>>(
+      b->rp32.ptr, n, m, groups, w->words.ptr + kWords, w->words.ptr + 4, w->number.ptr,
+      w->long_rows.ptr, w->long_graph.ptr, err);
+  WETRIC_LAUNCH_CHECK();
+  std::vector<uint64_t> host(kWords + G);
+  WETRIC_CUDA_TRY(cudaMemcpyAsync(host.data(), w->words.ptr, (kWords + G) * 8ull,
+                                  cudaMemcpyDeviceToHost, st));
+  WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  if ((uint32_t)host[2] != kDevOk) {
+    set_error(WETRIC_EINVAL, "batch row check failed (device code %u)", (uint32_t)host[2]);
+    return WETRIC_EINVAL;
+  }
+  const uint64_t longest = host[4], rows = host[5], long_rows = host[6], long_w = host[7];
+  if (longest >= (1ull << 30)) {
+    set_error(WETRIC_ERANGE, "max out-degree %llu >= 2^30", (unsigned long long)longest);
+    return WETRIC_ERANGE;
+  }
+  b->wbase.assign(G + 1, 0);
+  for (uint32_t g = 0; g < G; ++g) b->wbase[g + 1] = b->wbase[g] + host[kWords + g];
+  b->W = b->wbase[G];
+  b->max_out_degree = longest;
+  b->Kp = rows;
+  b->pair_wedges = b->W;
+  if (walk_wanted(long_rows, longest, long_w, m) && w->run.fits(n, m, long_rows, longest)) {
+    WalkRun &run = w->run;
+    if (run.alloc(ctx, st, m + m / 4) != WETRIC_OK) {
+      clear_error();
+      return WETRIC_OK;
+    }
+    k_walk_split<true><<<WalkRun::grid(ctx, n), kWalkBlock, 0, st>>>(
+        b->rp32.ptr, b->csr.col_ind, n, 0, n, run.split.ptr, groups);
+    WETRIC_LAUNCH_CHECK();
+    const uint32_t T = merge_tile(m, ctx->sm_count);
+    k_edge_merge<uint32_t, true, true>
+        <<<(unsigned)ceil_div(ceil_div(m, T), kWalkBlock / 32), kWalkBlock, 0, st>>>(
+            b->rp32.ptr, walk_columns(b->csr.col_ind, m), n, 0, n, T, w->number.ptr,
+            run.split.ptr, run.bits, run.keys.ptr, (uint32_t)run.cap, run.counts.ptr,
+            w->words.ptr, err, groups, kMergeEmit);
+    WETRIC_LAUNCH_CHECK();
+    uint64_t local[kReadWords];
+    const uint64_t *got = nullptr;
+    ReadPlan rd;
+    rd.add(run.counts.ptr, 1, 4);
+    rd.add(w->words.ptr + 1, 1, 8);
+    WETRIC_TRY(read_back(ctx, st, rd, local, &got));
+    const uint64_t made = got[0];
+    b->pair_wedges = got[1];
+    if (made > run.cap) return WETRIC_OK;
+    w->entries = made > 0;
+    uint32_t launches = 0;
+    if (made) {
+      WETRIC_TRY(run.sort(ctx, st, b->rp32.ptr, w->long_rows.ptr, made, err, &launches));
+      uint32_t herr = 0;
+      WETRIC_CUDA_TRY(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
+      WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+      if (herr != kDevOk) {
+        set_error(WETRIC_ETIMEDOUT, "a look-back did not complete in time");
+        return WETRIC_ETIMEDOUT;
+      }
+      (run.sorted == run.keys.ptr ? run.alt : run.keys).release();
+      run.ws.buf.release();
+    }
+  }
+  b->W -= b->pair_wedges;  // (the statistics add the two)
+  b->walk = std::move(w);
+  b->whole = true;
+  return WETRIC_OK;
+}
+
 int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
                  const uint64_t *pair_off, const uint64_t *n, uint32_t G,
                  bool on_device, const BatchOptions &opt, Batch *b,
@@ -446,6 +617,25 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
   if (b->off32) {
     WETRIC_TRY(b->rp32.alloc(ctx, st, NT + 1));
     WETRIC_TRY(narrow_offsets(ctx, st, b->csr.row_ptr, NT, b->rp32.ptr));
+  }
+
+  auto spreads = [&]() {
+    std::vector<uint32_t> sg(G, opt.spread);
+    for (uint32_t g = 0; g < G; ++g) {
+      const uint64_t Wg = b->wbase[g + 1] - b->wbase[g];
+      uint32_t s1 = opt.spread_for ? opt.spread_for(b->n[g], Wg, opt.tune_ctx) : opt.spread;
+      sg[g] = s1 ? s1 : opt.spread;
+    }
+    return sg;
+  };
+  if (b->off32 && m < (1ull << 31) && opt.pair_streams && m > 0) {
+    WETRIC_TRY(make_whole(b, st));
+    if (b->whole) {  // (its spreads are what the wedge check would take)
+      b->spread_of = spreads();
+      return WETRIC_OK;
+    }
+    b->counts.release();
+    b->vbase_d.release();
   }
 
   // 4. Active vertices of the union with their graph.
@@ -700,12 +890,7 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
         &occ, k_count_rows<uint64_t, true, false, kBatchMinBlocks, true, true>, kWarpsPerBlock * 32, 0));
   b->grid_max = (uint64_t)ctx->sm_count * (occ < 1 ? 1 : occ);
 
-  std::vector<uint32_t> sg(G, opt.spread);
-  for (uint32_t g = 0; g < G; ++g) {
-    const uint64_t Wg = b->wbase[g + 1] - b->wbase[g];
-    uint32_t s1 = opt.spread_for ? opt.spread_for(b->n[g], Wg, opt.tune_ctx) : opt.spread;
-    sg[g] = s1 ? s1 : opt.spread;
-  }
+  std::vector<uint32_t> sg = spreads();
   if (opt.autotune) WETRIC_TRY(autotune_spreads(b, &sg, st));
   WETRIC_TRY(build_tile_space(b, sg, st));
   WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
@@ -716,6 +901,34 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
 // one persistent launch over the batch's whole tile space.
 static int batch_enqueue(Batch *b, cudaStream_t st, uint32_t *launches) {
   WETRIC_CUDA_TRY(cudaMemsetAsync(b->counts.ptr, 0, b->G * 8ull, st));
+  if (b->whole) {
+    BatchWalk &w = *b->walk;
+    DeviceContext *ctx = b->ctx;
+    const uint64_t n = b->vbase[b->G], m = b->m_total;
+    const WalkGroups groups{b->vbase_d.ptr, b->G, b->counts.ptr};
+    const uint32_t T = merge_tile(m, ctx->sm_count);
+    const unsigned grid = (unsigned)ceil_div(ceil_div(m, T), kWalkBlock / 32);
+    uint32_t *err = reinterpret_cast<uint32_t *>(w.words.ptr + 2);
+    const WalkColumns cols = walk_columns(b->csr.col_ind, m);
+    *launches = 1;
+    uint64_t most = 0;
+    if (!w.entries) {
+      k_edge_merge<uint32_t, false, true><<<grid, kWalkBlock, 0, st>>>(
+          b->rp32.ptr, cols, n, 0, n, T, nullptr, nullptr, WalkBits{}, nullptr, 0, nullptr,
+          w.words.ptr, err, groups);
+      WETRIC_LAUNCH_CHECK();
+      return WETRIC_OK;
+    }
+    k_edge_merge<uint32_t, true, true><<<grid, kWalkBlock, 0, st>>>(
+        b->rp32.ptr, cols, n, 0, n, T, w.number.ptr, w.run.split.ptr, w.run.bits, nullptr, 0,
+        nullptr, w.words.ptr, err, groups, kMergeCount);
+    WETRIC_LAUNCH_CHECK();
+    // the walk's item counters (counts[3], counts[4])
+    WETRIC_CUDA_TRY(cudaMemsetAsync(w.run.counts.ptr + 3, 0, 2 * sizeof(uint32_t), st));
+    return w.run.count<true>(ctx, st, b->rp32.ptr, b->csr.col_ind, w.long_rows.ptr,
+                             b->opt.persistent, nullptr, &most, launches, groups,
+                             w.long_graph.ptr);
+  }
   WETRIC_CUDA_TRY(cudaMemsetAsync(b->total.ptr, 0, 8, st));
   WETRIC_CUDA_TRY(cudaMemsetAsync(b->next_tile.ptr, 0, 8, st));
   *launches = 0;

@@ -25,10 +25,13 @@ struct BatchOptions {
   // Optional tuner: spread for a graph with n vertices and W wedges.
   uint32_t (*spread_for)(uint64_t n, uint64_t W, const void *ctx) = nullptr;
   const void *tune_ctx = nullptr;
-  // Pair streams for the short rows of every graph (32-bit offsets only):
-  // counted by k_count_pairs beside the wedge check (pair_streams.cuh).
+  // Count by row intersections and the column walk (walk.cuh; batches of
+  // fewer than 2^31 columns that have room for it) instead of wedge checks
+  // and, on 32-bit offsets, pair streams.
   bool pair_streams = true;
 };
+
+struct BatchWalk;  // the long rows' entries (batch.cu)
 
 struct Batch {
   DeviceContext *ctx = nullptr;
@@ -68,10 +71,15 @@ struct Batch {
   Scratch<uint32_t> pv, pg, ptile_k;
   Scratch<uint64_t> ps;
   std::vector<uint64_t> pair_w;
+  // Counted by row intersections and the walk: no wedge tiles, bitmaps or
+  // hash sets then.
+  bool whole = false;
+  std::unique_ptr<BatchWalk> walk;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   cudaStream_t graph_stream = nullptr;
   uint32_t graph_launches = 0;
+  Batch();
   void release_all();
   ~Batch();
 };

@@ -35,9 +35,6 @@ namespace {
 // Below this many columns a graph takes no core and no walk: one kernel
 // intersects the rows of all its edges, and the count is read back once.
 constexpr uint64_t kSmallColumns = 1ull << 17;
-// Below this many columns under the core the long rows' edges are not worth
-// a sort (about 60 us of launches).
-constexpr uint64_t kWalkMinEdges = 1ull << 19;
 
 // A word read by the core's row ANDs against a wedge counted below it (R-MAT
 // scale 22, between neighbouring lengths: 0.21 ps per estimated word, 0.8 ps
@@ -186,8 +183,8 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
     } else if (cores.count) {
       unsigned long long plan[2 * kCoreNumCandidates];
       for (uint32_t c = 0; c < kCoreNumCandidates; ++c) {
-        plan[2 * c] = tot[4 + 3 * c];
-        plan[2 * c + 1] = tot[5 + 3 * c];
+        plan[2 * c] = tot[kEdgeCand + 3 * c];
+        plan[2 * c + 1] = tot[kEdgeCand + 3 * c + 1];
       }
       pick = core_pick(plan, kCoreWordsPerWalked);
     }
@@ -195,11 +192,11 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
       core_h = cores.len[pick];
       core_v0 = n - core_h;
       below_m = w[kWords + pick];
-      r->core_wedges = tot[4 + 3 * pick];
-      core_rows = tot[6 + 3 * pick];
+      r->core_wedges = tot[kEdgeCand + 3 * pick];
+      core_rows = tot[kEdgeCand + 3 * pick + 2];
       r->core_len = (uint32_t)core_h;
     }
-    emit = tot[3] > 0 && below_m >= kWalkMinEdges && walk.fits(n, m, tot[3], tot[1]);
+    emit = walk_wanted(tot[3], tot[1], tot[4], below_m) && walk.fits(n, m, tot[3], tot[1]);
     // Room for an entry per edge below the core and a quarter more: tails
     // with two entries are rare (they need a long row with more than 48
     // columns outside the window), and a graph with more of them starts over
@@ -242,8 +239,8 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
     const cudaEvent_t ready = C_in ? a.chunk_ready[i] : a.ci_ready;
     if (ready && !small) WETRIC_CUDA_TRY(cudaStreamWaitEvent(st, ready, 0));
     if (emit) {
-      k_walk_split<<<WalkRun::grid(ctx, hi - lo), kWalkBlock, 0, st>>>(rp32, a.col_ind, n, lo, hi,
-                                                                       walk.split.ptr);
+      k_walk_split<false><<<WalkRun::grid(ctx, hi - lo), kWalkBlock, 0, st>>>(
+          rp32, a.col_ind, n, lo, hi, walk.split.ptr, WalkGroups{});
       WETRIC_LAUNCH_CHECK();
       ++launches;
     }

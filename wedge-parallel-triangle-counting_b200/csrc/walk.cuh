@@ -85,17 +85,40 @@ struct EdgeCores {
   uint32_t count;
 };
 
+// The graphs of a batch: graph g owns rows [base[g], base[g + 1]) of the
+// disjoint union and counts into counts[g].
+struct WalkGroups {
+  const uint64_t *base = nullptr;
+  uint32_t G = 0;
+  unsigned long long *counts = nullptr;
+};
+__device__ __forceinline__ uint32_t walk_group(const WalkGroups &gr, uint64_t row) {
+  uint32_t lo = 0, len = gr.G;
+  while (len > 1) {
+    const uint32_t h = len >> 1;
+    if (__ldg(gr.base + lo + h) <= row) lo += h;
+    len -= h;
+  }
+  return lo;
+}
+// First window column of graph g's rows.
+__device__ __forceinline__ uint32_t walk_window(const WalkGroups &gr, uint32_t g) {
+  const uint64_t b = __ldg(gr.base + g), e = __ldg(gr.base + g + 1);
+  return (uint32_t)(e - b > kWalkWindow ? e - kWalkWindow : b);
+}
+
 // Totals of the rows: [0] W, [1] longest row, [2] rows with wedges, [3] long
-// rows, then per core candidate its wedges, AND words (k_core_plan) and rows
-// with wedges.
-constexpr uint32_t kEdgeTotals = 4 + 3 * kCoreNumCandidates;
+// rows, [4] their wedges, then per core candidate its wedges, AND words
+// (k_core_plan) and rows with wedges.
+constexpr uint32_t kEdgeCand = 5;
+constexpr uint32_t kEdgeTotals = kEdgeCand + 3 * kCoreNumCandidates;
 template <typename Off>
 __global__ void __launch_bounds__(kWalkBlock)
     k_edge_vertices(const Off *__restrict__ rp, uint64_t n, uint64_t m,
                     const __grid_constant__ EdgeCores cores, unsigned long long *__restrict__ totals, uint32_t *__restrict__ number,
                     uint32_t *__restrict__ long_rows, uint32_t *err) {
   const uint32_t lane = threadIdx.x & 31;
-  unsigned long long W = 0, rows = 0, longest = 0;
+  unsigned long long W = 0, rows = 0, longest = 0, long_w = 0;
   unsigned long long plan[3 * kCoreNumCandidates] = {};
   const uint64_t top = cores.count ? cores.len[0] : 0u;  // the longest
   bool in_top = false;
@@ -133,20 +156,25 @@ __global__ void __launch_bounds__(kWalkBlock)
       if (mask && lane == 0) id = (uint32_t)atomicAdd(totals + 3, (unsigned long long)__popc(mask));
       id = __shfl_sync(0xffffffffu, id, 0) + __popc(mask & ((1u << lane) - 1u));
       if (v < n) number[v] = is_long ? id : kWalkShort;
-      if (is_long) long_rows[id] = (uint32_t)v;
+      if (is_long) {
+        long_rows[id] = (uint32_t)v;
+        long_w += w;
+      }
     }
   }
-  __shared__ unsigned long long s_sum[3], s_plan[3 * kCoreNumCandidates];
-  if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+  __shared__ unsigned long long s_sum[4], s_plan[3 * kCoreNumCandidates];
+  if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
   if (threadIdx.x < 3 * kCoreNumCandidates) s_plan[threadIdx.x] = 0;
   __syncthreads();
   for (int o = 16; o > 0; o >>= 1) {
     W += __shfl_down_sync(0xffffffffu, W, o);
     rows += __shfl_down_sync(0xffffffffu, rows, o);
+    long_w += __shfl_down_sync(0xffffffffu, long_w, o);
     const unsigned long long x = __shfl_down_sync(0xffffffffu, longest, o);
     longest = longest > x ? longest : x;
   }
   if (lane == 0) {
+    atomicAdd(&s_sum[3], long_w);
     atomicAdd(&s_sum[0], W);
     atomicMax(&s_sum[1], longest);
     atomicAdd(&s_sum[2], rows);
@@ -164,21 +192,25 @@ __global__ void __launch_bounds__(kWalkBlock)
     if (s_sum[0]) atomicAdd(totals, s_sum[0]);
     atomicMax(totals + 1, s_sum[1]);
     if (s_sum[2]) atomicAdd(totals + 2, s_sum[2]);
+    if (s_sum[3]) atomicAdd(totals + 4, s_sum[3]);
   }
   if (threadIdx.x < 3 * kCoreNumCandidates && s_plan[threadIdx.x])
-    atomicAdd(totals + 4 + threadIdx.x, s_plan[threadIdx.x]);
+    atomicAdd(totals + kEdgeCand + threadIdx.x, s_plan[threadIdx.x]);
   if (blockIdx.x == 0 && threadIdx.x == 0)
     if (ld_off(rp, 0) != 0 || ld_off(rp, n) != m) atomicCAS(err, 0u, (uint32_t)kDevRowPtrRange);
 }
 
 // split[v] = index of row v's first window column (rows are sorted), rows
-// [lo, hi).
+// [lo, hi). kBatch: of the row's own graph.
+template <bool kBatch>
 __global__ void __launch_bounds__(kWalkBlock)
     k_walk_split(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ci, uint64_t n,
-                 uint64_t lo_row, uint64_t hi_row, uint32_t *__restrict__ split) {
-  const uint32_t t0 = n > kWalkWindow ? (uint32_t)(n - kWalkWindow) : 0u;
+                 uint64_t lo_row, uint64_t hi_row, uint32_t *__restrict__ split,
+                 const WalkGroups groups) {
+  uint32_t t0 = n > kWalkWindow ? (uint32_t)(n - kWalkWindow) : 0u;
   for (uint64_t v = lo_row + (uint64_t)blockIdx.x * kWalkBlock + threadIdx.x; v < hi_row;
        v += (uint64_t)gridDim.x * kWalkBlock) {
+    if (kBatch) t0 = walk_window(groups, walk_group(groups, v));
     uint32_t lo = rp[v], hi = rp[v + 1];
     if (v >= t0) hi = lo;  // every column is above its row
     while (lo < hi) {
@@ -370,21 +402,26 @@ __device__ __forceinline__ uint64_t row_of_edge(const Off *__restrict__ rp, uint
 // appended in any order (*made of them, those past cap are only counted) --
 // but for the tail's part outside the window, which is intersected here when
 // the long row has few columns there -- and without it they are counted here
-// too. Nothing is done when *err is set: the
-// row offsets cannot be trusted.
+// too. Nothing is done when *err is set: the row offsets cannot be trusted.
 // Bound by instruction issue: a step intersects 4 by 4 columns of each of 32
 // edges in about 50 instructions. Erdos-Renyi with 700,001 vertices and 13.3M
 // edges: 551 us where the pair streams took 584 after a plan of 131 us and
 // 152 us of hash sets; R-MAT scale 22: 0.79 ms (1.27 ms before the few
 // edges that intersect rows there were gathered to fill the warp).
-template <typename Off, bool kEmit>
+// kBatch: the rows are a batch's, the triangles go to their graphs' counts;
+// with kEmit, `what` says whether it is the count (the long rows' entries
+// were made before) or the making of the entries.
+enum MergeWhat : uint32_t { kMergeCount = 1, kMergeEmit = 2 };
+template <typename Off, bool kEmit, bool kBatch = false>
 __global__ void __launch_bounds__(kWalkBlock, 4)
     k_edge_merge(const Off *__restrict__ rp, const __grid_constant__ WalkColumns cols, uint64_t n,
                  uint64_t row_lo, uint64_t row_hi, uint32_t T,
                  const uint32_t *__restrict__ number, const uint32_t *__restrict__ split,
                  const WalkBits bits, uint64_t *__restrict__ entries, uint32_t cap,
                  uint32_t *__restrict__ made, unsigned long long *__restrict__ out,
-                 const uint32_t *__restrict__ err) {
+                 const uint32_t *__restrict__ err,
+                 const __grid_constant__ WalkGroups groups = WalkGroups{},
+                 uint32_t what = kMergeCount | kMergeEmit) {
   __shared__ uint32_t s_start[kWalkBlock / 32][32], s_row[kWalkBlock / 32][32];
   __shared__ uint64_t s_entry[kEmit ? kWalkBlock / 32 : 1][kEmit ? kMergeStage : 1];
   __shared__ MergeTask s_task[kEmit ? kWalkBlock / 32 : 1][64];
@@ -414,14 +451,32 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
     staged = 0;
     __syncwarp();
   };
+  uint32_t g = 0;
+  auto drain = [&]() {  // kBatch: the graph's hits so far
+    if (kEmit && lane < tasks) hits += merge_rows(cols, s_task[kEmit ? wid : 0][lane]);
+    tasks = 0;
+    const uint32_t c = __reduce_add_sync(0xffffffffu, hits);
+    if (lane == 0 && c) atomicAdd(groups.counts + g, (unsigned long long)c);
+    hits = 0;
+    __syncwarp();
+  };
   for (uint32_t j = (uint32_t)from; j < j1;) {
     const uint64_t r = row_of_edge(rp, row_lo, row_hi, j, lane);
-    const uint64_t v = r + lane < row_hi ? r + lane : row_hi;
+    uint64_t rows_end = row_hi;
+    if (kBatch) {  // the rows at hand are one graph's
+      const uint32_t now = (uint32_t)row_of_edge(groups.base, 0, groups.G, r, lane);
+      if (now != g) {
+        drain();
+        g = now;
+      }
+      rows_end = __ldg(groups.base + g + 1);
+    }
+    const uint64_t v = r + lane < rows_end ? r + lane : rows_end;
     const uint32_t b = (uint32_t)ld_off(rp, v);
-    const uint32_t e = v < row_hi ? (uint32_t)ld_off(rp, v + 1) : b;
+    const uint32_t e = v < rows_end ? (uint32_t)ld_off(rp, v + 1) : b;
     const uint32_t last = e > b ? __ldg(ci + e - 1) : 0u;
     uint32_t mid = b, rest_last = 0;
-    if (kEmit && v < row_hi) {
+    if (kEmit && v < rows_end) {
       mid = split[v];
       if (mid > b) rest_last = __ldg(ci + mid - 1);
     }
@@ -469,7 +524,7 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
         }
         const uint32_t rm = __ballot_sync(0xffffffffu, rest);
         const uint32_t wm = __ballot_sync(0xffffffffu, win);
-        if (rm | wm) {
+        if ((rm | wm) && (!kBatch || (what & kMergeEmit))) {
           const uint32_t add = __popc(rm) + __popc(wm);
           if (staged + add > kMergeStage) flush();
           const uint32_t xr = staged + __popc(rm & lt);
@@ -492,6 +547,7 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
       } else {
         // few of the edges intersect rows here: they gather until there is
         // one for every lane
+        if (kBatch && !(what & kMergeCount)) s1 = s0;
         const uint32_t mm = __ballot_sync(0xffffffffu, s0 < s1);
         if (s0 < s1) s_task[wid][tasks + __popc(mm & lt)] = task;
         tasks += __popc(mm);
@@ -508,6 +564,7 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
     }
     j = stop;
   }
+  if (kBatch) drain();
   if (kEmit && lane < tasks) hits += merge_rows(cols, s_task[kEmit ? wid : 0][lane]);
   if (kEmit && staged) flush();
   unsigned long long h = hits;
@@ -519,6 +576,19 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
     if (h) atomicAdd(out, h);
     if (wedges) atomicAdd(out + 1, wedges);
   }
+}
+
+// Whether the edges to long rows (more than 48 columns) are worth sorting for
+// the walk, against intersecting every row where its edge is: intersections
+// with rows of up to 128 columns waste at most 32 steps, and below 2^25
+// wedges of long rows the sort's launches and passes cost more than they save
+// (Chung-Lu, 100,000 vertices, mean degree 40, longest row 97: 0.24 ms
+// without, 0.31 with; 300,000 and 60, longest 218: 1.42 against 0.87; with
+// 1,000,000 and 40, exponent 2.8, longest 51: 0.86 against 1.04).
+constexpr uint64_t kWalkMinEdges = 1ull << 19;
+inline bool walk_wanted(uint64_t long_rows, uint64_t longest, uint64_t long_wedges,
+                        uint64_t edges) {
+  return long_rows > 0 && edges >= kWalkMinEdges && (longest > 128 || long_wedges >= (1ull << 25));
 }
 
 // Edges per warp: kMergeTile, or fewer (whole rounds) when that leaves the
@@ -647,7 +717,7 @@ __device__ __forceinline__ uint32_t walk_find8(const uint32_t *set, uint32_t slo
 // to 256 entries have blocks of one warp: most of the vertices of R-MAT scale
 // 22, whose set-up by four warps took two thirds of the instructions.
 // WALK_FIGURES
-template <uint32_t kThreads, int kBlocks>
+template <uint32_t kThreads, int kBlocks, bool kBatch>
 __global__ void __launch_bounds__(kThreads, kBlocks)
     k_walk_count(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ split,
                  const uint32_t *__restrict__ long_rows, const __grid_constant__ WalkColumns cols,
@@ -655,7 +725,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
                  const uint32_t *__restrict__ start, const WalkBits bits,
                  const uint2 *__restrict__ items, const uint32_t *__restrict__ count,
                  uint32_t *__restrict__ ticket, uint32_t per_block,
-                 unsigned long long *__restrict__ out) {
+                 unsigned long long *__restrict__ out, const __grid_constant__ WalkGroups groups,
+                 const uint32_t *__restrict__ long_graph) {
   struct Entry {
     uint32_t first, len;
   };
@@ -671,7 +742,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t *ci = cols.base + cols.mis;
   const uint32_t n_items = *count;
-  const uint32_t not_t0 = t0 - 1;
+  uint32_t not_t0 = t0 - 1, g = 0;
   const char *row = reinterpret_cast<const char *>(s_set);
   constexpr uint32_t word_mask = (kWalkSetSlots - 1) * 4;
   const uint64_t start_mask = (1ull << bits.start) - 1, len_mask = (1ull << bits.len) - 1;
@@ -697,6 +768,17 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
     const uint32_t e1 = min(start[x + 1], e0 + kWalkPiece);
     const uint2 set = walk_set(rp, split, long_rows, x);
     const uint32_t d = set.y - set.x;
+    if (kBatch) {
+      const uint32_t now = __ldg(long_graph + (x >> 1));
+      if (now != g) {
+        const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)hits);
+        if (lane == 0 && c) atomicAdd(groups.counts + g, (unsigned long long)c);
+        hits = 0;
+        g = now;
+      }
+      t0 = walk_window(groups, g);
+      not_t0 = t0 - 1;
+    }
     const bool window = kBits && (x & 1);
     for (uint32_t part = 0; part < d; part += window || !kBits ? d : kWalkSetCols) {
       const uint32_t ncols = window || !kBits ? d : min(d - part, kWalkSetCols);
@@ -784,7 +866,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
     }
   }
   for (int o = 16; o > 0; o >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, o);
-  if (lane == 0 && hits) atomicAdd(out, hits);
+  if (lane == 0 && hits) atomicAdd(kBatch ? groups.counts + g : out, hits);
 }
 
 // Room for at least x elements, in eighths of a power of two: graphs of one
@@ -856,13 +938,16 @@ struct WalkRun {
     return WETRIC_OK;
   }
   // The count. Persistent: one wave of blocks, items from a counter; otherwise
-  // short blocks, so other streams' blocks get SMs in between.
+  // short blocks, so other streams' blocks get SMs in between. The counters
+  // start at zero (alloc) and are the caller's to clear for another count.
+  template <bool kBatch = false>
   int count(DeviceContext *ctx, cudaStream_t st, const uint32_t *rp, const uint32_t *ci,
             const uint32_t *long_rows, bool persistent, unsigned long long *out, uint64_t *most,
-            uint32_t *launches) {
+            uint32_t *launches, const WalkGroups &groups = WalkGroups{},
+            const uint32_t *long_graph = nullptr) {
     constexpr uint32_t kPerBlock = 16;
-    const auto big_fn = k_walk_count<kWalkBigBlock, kWalkBigBlocks>;
-    const auto small_fn = k_walk_count<kWalkSmallBlock, kWalkSmallBlocks>;
+    const auto big_fn = k_walk_count<kWalkBigBlock, kWalkBigBlocks, kBatch>;
+    const auto small_fn = k_walk_count<kWalkSmallBlock, kWalkSmallBlocks, kBatch>;
     const uint64_t g = persistent ? (uint64_t)ctx->sm_count * kWalkBigBlocks
                                   : ceil_div(big_cap, kPerBlock);
     const uint64_t gs = persistent ? (uint64_t)ctx->sm_count * kWalkSmallBlocks
@@ -878,11 +963,11 @@ struct WalkRun {
         small_fn, cudaFuncAttributePreferredSharedMemoryCarveout, kWalkCarveout));
     big_fn<<<(unsigned)g, kWalkBigBlock, 0, st>>>(
         rp, split.ptr, long_rows, cols, t0, sorted, start.ptr, bits, big.ptr, counts.ptr + 1,
-        counts.ptr + 3, persistent ? 0 : kPerBlock, out);
+        counts.ptr + 3, persistent ? 0 : kPerBlock, out, groups, long_graph);
     WETRIC_LAUNCH_CHECK();
     small_fn<<<(unsigned)gs, kWalkSmallBlock, 0, st>>>(
         rp, split.ptr, long_rows, cols, t0, sorted, start.ptr, bits, small.ptr, counts.ptr + 2,
-        counts.ptr + 4, persistent ? 0 : kPerBlock, out);
+        counts.ptr + 4, persistent ? 0 : kPerBlock, out, groups, long_graph);
     WETRIC_LAUNCH_CHECK();
     *launches += 2;
     if (g > *most) *most = g;
