@@ -168,3 +168,35 @@ def test_batch_walk(wetric_mod, oracle_mod, use_graph):
         assert [int(x) for x in got] == want
     got, _ = wetric_mod.Batch(*args, use_cuda_graph=use_graph, pair_streams=False).count()
     assert [int(x) for x in got] == want
+
+
+@pytest.mark.parametrize("degree", [17, 20, 31, 33, 48, 49, 63, 66])
+@pytest.mark.parametrize("window", [70, 4000])
+def test_row_sets_parity(wetric_mod, oracle_mod, degree, window):
+    """Rows around one warp, a set's 64 columns and the short rows' 48: enough
+    edges per row for the sets, columns close together (`window`: neighbours
+    among the next ids, so shared columns and triangles are many) and spread."""
+    rng = np.random.default_rng(degree * 31 + window)
+    n = 2_000_000 // degree
+    src = np.repeat(np.arange(n), degree)
+    dst = (src + 1 + rng.integers(0, window, src.size)) % n
+    g = oracle_mod.oriented_from_pairs(src.astype(np.uint32), dst.astype(np.uint32))
+    want = oracle_mod.count_merge(g)
+    W = oracle_mod.wedge_total(g)
+    assert g.m >= 1 << 20 and W >= 8 * g.m  # enough for the sets
+    import torch
+
+    rp = torch.from_numpy(g.row_ptr.view(np.int64)).cuda()
+    ci = torch.from_numpy(g.col_ind.view(np.int32)).cuda()
+    for core in (wetric_mod.CORE_OFF, 0):
+        got, st = wetric_mod.count(rp, ci, 5, 8192, core_len=core)
+        assert got == want and st.wedges == W and st.wedges_counted == W
+    # the same columns at an odd place in their sector
+    ci1 = torch.cat([ci[:3], ci])[3:]
+    assert wetric_mod.count(rp, ci1, 5, 8192)[0] == want
+    # twice in a batch, with a small graph between
+    off = np.array([0, src.size, src.size + 3, 2 * src.size + 3], np.uint64)
+    s = np.concatenate([src, [0, 1, 2], src]).astype(np.uint32)
+    d = np.concatenate([dst, [1, 2, 0], dst]).astype(np.uint32)
+    counts, _ = wetric_mod.Batch(s, d, off, np.array([n, 3, n], np.uint64)).count()
+    assert [int(x) for x in counts] == [want, 1, want]

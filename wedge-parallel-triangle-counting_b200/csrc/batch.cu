@@ -44,7 +44,7 @@ struct BatchWalk {
   WalkRun run;
   Scratch<uint32_t> number, long_rows, long_graph;
   Scratch<unsigned long long> words;  // [0] unused, [1] wedges of short rows, [2] error
-  bool entries = false;
+  bool entries = false, sets = false;
 };
 
 namespace {
@@ -495,8 +495,8 @@ static int make_whole(Batch *b, cudaStream_t st) {
         b->rp32.ptr, b->csr.col_ind, n, 0, n, run.split.ptr, groups);
     WETRIC_LAUNCH_CHECK();
     const uint32_t T = merge_tile(m, ctx->sm_count);
-    k_edge_merge<uint32_t, true, true>
-        <<<(unsigned)ceil_div(ceil_div(m, T), kWalkBlock / 32), kWalkBlock, 0, st>>>(
+    k_edge_merge<uint32_t, true, true, false>
+        <<<(unsigned)ceil_div(ceil_div(m, T), kMergeBlock / 32), kMergeBlock, 0, st>>>(
             b->rp32.ptr, walk_columns(b->csr.col_ind, m), n, 0, n, T, w->number.ptr,
             run.split.ptr, run.bits, run.keys.ptr, (uint32_t)run.cap, run.counts.ptr,
             w->words.ptr, err, groups, kMergeEmit);
@@ -526,6 +526,7 @@ static int make_whole(Batch *b, cudaStream_t st) {
     }
   }
   b->W -= b->pair_wedges;  // (the statistics add the two)
+  w->sets = row_sets_wanted(m, b->W + b->pair_wedges, longest, b->W);
   b->walk = std::move(w);
   b->whole = true;
   return WETRIC_OK;
@@ -907,22 +908,26 @@ static int batch_enqueue(Batch *b, cudaStream_t st, uint32_t *launches) {
     const uint64_t n = b->vbase[b->G], m = b->m_total;
     const WalkGroups groups{b->vbase_d.ptr, b->G, b->counts.ptr};
     const uint32_t T = merge_tile(m, ctx->sm_count);
-    const unsigned grid = (unsigned)ceil_div(ceil_div(m, T), kWalkBlock / 32);
+    const unsigned grid = (unsigned)ceil_div(ceil_div(m, T), kMergeBlock / 32);
     uint32_t *err = reinterpret_cast<uint32_t *>(w.words.ptr + 2);
     const WalkColumns cols = walk_columns(b->csr.col_ind, m);
     *launches = 1;
     uint64_t most = 0;
-    if (!w.entries) {
-      k_edge_merge<uint32_t, false, true><<<grid, kWalkBlock, 0, st>>>(
-          b->rp32.ptr, cols, n, 0, n, T, nullptr, nullptr, WalkBits{}, nullptr, 0, nullptr,
-          w.words.ptr, err, groups);
-      WETRIC_LAUNCH_CHECK();
-      return WETRIC_OK;
-    }
-    k_edge_merge<uint32_t, true, true><<<grid, kWalkBlock, 0, st>>>(
-        b->rp32.ptr, cols, n, 0, n, T, w.number.ptr, w.run.split.ptr, w.run.bits, nullptr, 0,
-        nullptr, w.words.ptr, err, groups, kMergeCount);
+    const auto merge = [&](auto kernel) {
+      kernel<<<grid, kMergeBlock, 0, st>>>(b->rp32.ptr, cols, n, 0, n, T, w.number.ptr,
+                                           w.run.split.ptr, w.run.bits, nullptr, 0, nullptr,
+                                           w.words.ptr, err, groups, kMergeCount);
+    };
+    if (w.entries && w.sets)
+      merge(k_edge_merge<uint32_t, true, true, true>);
+    else if (w.entries)
+      merge(k_edge_merge<uint32_t, true, true, false>);
+    else if (w.sets)
+      merge(k_edge_merge<uint32_t, false, true, true>);
+    else
+      merge(k_edge_merge<uint32_t, false, true, false>);
     WETRIC_LAUNCH_CHECK();
+    if (!w.entries) return WETRIC_OK;
     // the walk's item counters (counts[3], counts[4])
     WETRIC_CUDA_TRY(cudaMemsetAsync(w.run.counts.ptr + 3, 0, 2 * sizeof(uint32_t), st));
     return w.run.count<true>(ctx, st, b->rp32.ptr, b->csr.col_ind, w.long_rows.ptr,

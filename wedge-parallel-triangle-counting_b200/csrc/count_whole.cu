@@ -164,7 +164,7 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
   uint64_t core_h = 0, core_v0 = n, below_m = m, core_rows = 0;
   uint64_t local[kReadWords];
   uint64_t W = 0, rows = 0;
-  bool emit = false;
+  bool emit = false, sets = false;
   WalkRun walk;
   if (!small) {
     ReadPlan rd;
@@ -197,6 +197,7 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
       r->core_len = (uint32_t)core_h;
     }
     emit = walk_wanted(tot[3], tot[1], tot[4], below_m) && walk.fits(n, m, tot[3], tot[1]);
+    sets = row_sets_wanted(below_m, W - r->core_wedges, tot[1], emit ? tot[4] : 0);
     // Room for an entry per edge below the core and a quarter more: tails
     // with two entries are rare (they need a long row with more than 48
     // columns outside the window), and a graph with more of them starts over
@@ -248,17 +249,23 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
     if (top > lo && below_m > 0) {
       // the chunk's share of the edges: at most all of them
       const uint32_t T = merge_tile(below_m, ctx->sm_count);
-      const uint64_t g = ceil_div(ceil_div(below_m, T), kWalkBlock / 32);
+      const uint64_t g = ceil_div(ceil_div(below_m, T), kMergeBlock / 32);
       if (g > grid) grid = g;
       WETRIC_TRY(ev_merge[i].start(st));
-      if (emit)
-        k_edge_merge<uint32_t, true><<<(unsigned)g, kWalkBlock, 0, st>>>(
-            rp32, cols, n, lo, top, T, number.ptr, walk.split.ptr, walk.bits, walk.keys.ptr,
-            (uint32_t)walk.cap, walk.counts.ptr, words.ptr, err);
+      const auto merge = [&](auto kernel, const auto *offsets) {
+        kernel<<<(unsigned)g, kMergeBlock, 0, st>>>(
+            offsets, cols, n, lo, top, T, number.ptr, walk.split.ptr, walk.bits, walk.keys.ptr,
+            (uint32_t)walk.cap, walk.counts.ptr, words.ptr, err, WalkGroups{},
+            kMergeCount | kMergeEmit);
+      };
+      if (emit && sets)
+        merge(k_edge_merge<uint32_t, true, false, true>, rp32);
+      else if (emit)
+        merge(k_edge_merge<uint32_t, true, false, false>, rp32);
+      else if (sets)
+        merge(k_edge_merge<uint32_t, false, false, true>, rp32);
       else
-        k_edge_merge<Off, false><<<(unsigned)g, kWalkBlock, 0, st>>>(
-            rp, cols, n, lo, top, T, nullptr, nullptr, WalkBits{}, nullptr, 0, nullptr, words.ptr,
-            err);
+        merge(k_edge_merge<Off, false, false, false>, rp);
       WETRIC_LAUNCH_CHECK();
       ++launches;
       WETRIC_TRY(ev_merge[i].stop(st));

@@ -56,7 +56,15 @@ constexpr uint32_t kWalkBlock = 256;
 constexpr uint32_t kWalkEmpty = 0xFFFFFFFFu;
 constexpr uint32_t kWalkShort = 0xFFFFFFFFu;  // number of a row that is not long
 constexpr uint32_t kWalkShortCols = 48;       // columns of a short row at most
+constexpr uint32_t kMergeBlock = 128;
 constexpr uint32_t kMergeTile = 512;          // edges per warp at most
+constexpr uint32_t kRowSetCols = 64;          // columns in a warp's set at most
+constexpr uint32_t kRowSetSlots = 1024;
+constexpr uint32_t kRowSetFill = 24;          // edges of whole rows that fill a warp
+constexpr uint32_t kRowSetRows = 4;
+constexpr uint32_t kRowSetTries = 8;
+constexpr uint32_t kRowSetMin = 8;            // edges that are worth a set
+constexpr uint32_t kRowSetLong = 64;          // columns of a row w streamed at most
 constexpr uint32_t kMergeStage = 128;         // entries a warp gathers (64 or more)
 constexpr uint32_t kWalkBig = 64;             // entries from which a block takes a vertex
 constexpr uint32_t kWalkBigCols = 128;        // or columns
@@ -342,11 +350,11 @@ __device__ __forceinline__ void walk_half(const WalkColumns &cols, uint32_t a, u
 // loads, four times the pairs; Erdos-Renyi, 13.3M edges: 670 us against
 // 551.)
 struct MergeTask {
-  uint32_t t0, t1, t_last, s0, s1;  // t_last: the column at t1 - 1
+  uint32_t t0, t1, s0, s1;
 };
 __device__ __forceinline__ uint32_t merge_rows(const WalkColumns &cols, const MergeTask &task) {
-  const uint32_t t0 = task.t0, t1 = task.t1, t_last = task.t_last, s0 = task.s0, s1 = task.s1;
-  const uint32_t s_last = __ldg(cols.base + s1 - 1);
+  const uint32_t t0 = task.t0, t1 = task.t1, s0 = task.s0, s1 = task.s1;
+  const uint32_t t_last = __ldg(cols.base + t1 - 1), s_last = __ldg(cols.base + s1 - 1);
   uint32_t a = t0 & ~3u, b = s0 & ~3u, hits = 0;
   uint32_t x[4], y[4];
   walk_half(cols, a, t0, t1, x);
@@ -380,6 +388,14 @@ __device__ __forceinline__ uint32_t merge_rows(const WalkColumns &cols, const Me
   return hits;
 }
 
+// A set of (row, column) pairs in a warp's table: the pair lies at
+// (column * seed) / 2^22 ^ row * 32, so that no two rows share a slot for
+// the same column and a slot that holds the column answers exactly; the
+// warp looks for a seed under which no two pairs share a slot.
+__device__ __forceinline__ uint32_t row_set_at(uint32_t c, uint32_t seed, uint32_t key) {
+  return (((c * seed) >> 20) & (4 * kRowSetSlots - 4)) ^ key;  // bytes from the tables' start
+}
+
 // Row of edge j: the last row r in [lo, hi) with rp[r] <= j (a warp together,
 // 32 probes a step).
 template <typename Off>
@@ -403,17 +419,25 @@ __device__ __forceinline__ uint64_t row_of_edge(const Off *__restrict__ rp, uint
 // but for the tail's part outside the window, which is intersected here when
 // the long row has few columns there -- and without it they are counted here
 // too. Nothing is done when *err is set: the row offsets cannot be trusted.
-// Bound by instruction issue: a step intersects 4 by 4 columns of each of 32
-// edges in about 50 instructions. Erdos-Renyi with 700,001 vertices and 13.3M
-// edges: 551 us where the pair streams took 584 after a plan of 131 us and
-// 152 us of hash sets; R-MAT scale 22: 0.79 ms (1.27 ms before the few
-// edges that intersect rows there were gathered to fill the warp).
+// An edge intersects its tail with its short row (merge_rows: 4 by 4 columns
+// in about 50 instructions, with 57% of the lanes busy), or, with kSets, the
+// columns of the chunk's rows become an exact set in shared memory and the
+// short rows stream through it, a 32-byte sector per lane (8 columns in
+// about 85 instructions, nearly all lanes busy). Bound by instruction issue
+// and the shared-memory pipe (65% each). Erdos-Renyi with 700,001 vertices
+// and 13.3M edges: 427 us by sets, 533 by intersections (pair streams: 584
+// after a plan of 131 us and 152 us of hash sets); R-MAT scale 22: 0.76 ms
+// by intersections (1.27 ms before the few edges that intersect rows there
+// were gathered to fill the warp). A chunk ends with a row when that leaves
+// fewer than 8 lanes idle (a batch of 96 graphs: 6.63 ms; always 32 edges:
+// 6.94; whole rows only: 7.5); chunks of more than 4 rows, 64 columns or
+// fewer than 8 edges to short rows intersect.
 // kBatch: the rows are a batch's, the triangles go to their graphs' counts;
 // with kEmit, `what` says whether it is the count (the long rows' entries
 // were made before) or the making of the entries.
 enum MergeWhat : uint32_t { kMergeCount = 1, kMergeEmit = 2 };
-template <typename Off, bool kEmit, bool kBatch = false>
-__global__ void __launch_bounds__(kWalkBlock, 4)
+template <typename Off, bool kEmit, bool kBatch, bool kSets>
+__global__ void __launch_bounds__(kMergeBlock, kSets ? 7 : 8)
     k_edge_merge(const Off *__restrict__ rp, const __grid_constant__ WalkColumns cols, uint64_t n,
                  uint64_t row_lo, uint64_t row_hi, uint32_t T,
                  const uint32_t *__restrict__ number, const uint32_t *__restrict__ split,
@@ -422,18 +446,28 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
                  const uint32_t *__restrict__ err,
                  const __grid_constant__ WalkGroups groups = WalkGroups{},
                  uint32_t what = kMergeCount | kMergeEmit) {
-  __shared__ uint32_t s_start[kWalkBlock / 32][32], s_row[kWalkBlock / 32][32];
-  __shared__ uint64_t s_entry[kEmit ? kWalkBlock / 32 : 1][kEmit ? kMergeStage : 1];
-  __shared__ MergeTask s_task[kEmit ? kWalkBlock / 32 : 1][64];
+  __shared__ uint32_t s_start[kMergeBlock / 32][32], s_row[kMergeBlock / 32][32];
+  __shared__ uint64_t s_entry[kEmit ? kMergeBlock / 32 : 1][kEmit ? kMergeStage : 1];
+  constexpr bool kGather = kEmit || kSets;
+  __shared__ MergeTask s_task[kGather ? kMergeBlock / 32 : 1][64];
+  __shared__ __align__(16) uint32_t s_set[kSets ? kMergeBlock / 32 * kRowSetSlots : 4];
+  __shared__ uint4 s_unit[kSets ? kMergeBlock / 32 : 1][32];
   if (*err != kDevOk) return;
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u, le = 0xFFFFFFFFu >> (31 - lane);
   const uint32_t *ci = cols.base + cols.mis;
   const uint32_t j_end = (uint32_t)ld_off(rp, row_hi);
-  const uint64_t t = (uint64_t)blockIdx.x * (kWalkBlock / 32) + wid;
+  const uint64_t t = (uint64_t)blockIdx.x * (kMergeBlock / 32) + wid;
   const uint64_t from = ld_off(rp, row_lo) + t * T;
   if (from >= j_end) return;
   const uint32_t j1 = j_end - from < T ? j_end : (uint32_t)from + T;
+  auto slot = [&](uint32_t at) -> uint32_t & {
+    return *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(s_set) + at);
+  };
+  if (kSets)
+    for (uint32_t i = lane; i < kRowSetSlots; i += 32) s_set[wid * kRowSetSlots + i] = kWalkEmpty;
+  __syncwarp();
+  uint32_t seed = 0x9E3779B1u;
   unsigned long long wedges = 0;
   uint32_t hits = 0;
   // A warp's entries gather in shared memory and go out together: one atomic
@@ -453,7 +487,7 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
   };
   uint32_t g = 0;
   auto drain = [&]() {  // kBatch: the graph's hits so far
-    if (kEmit && lane < tasks) hits += merge_rows(cols, s_task[kEmit ? wid : 0][lane]);
+    if (kGather && lane < tasks) hits += merge_rows(cols, s_task[kGather ? wid : 0][lane]);
     tasks = 0;
     const uint32_t c = __reduce_add_sync(0xffffffffu, hits);
     if (lane == 0 && c) atomicAdd(groups.counts + g, (unsigned long long)c);
@@ -474,12 +508,7 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
     const uint64_t v = r + lane < rows_end ? r + lane : rows_end;
     const uint32_t b = (uint32_t)ld_off(rp, v);
     const uint32_t e = v < rows_end ? (uint32_t)ld_off(rp, v + 1) : b;
-    const uint32_t last = e > b ? __ldg(ci + e - 1) : 0u;
-    uint32_t mid = b, rest_last = 0;
-    if (kEmit && v < rows_end) {
-      mid = split[v];
-      if (mid > b) rest_last = __ldg(ci + mid - 1);
-    }
+    const uint32_t mid = kEmit && v < rows_end ? split[v] : b;
     const uint32_t stop = min(j1, __shfl_sync(0xffffffffu, e, 31));
     const uint32_t rows = __ballot_sync(0xffffffffu, e > b);
     __syncwarp();
@@ -490,22 +519,37 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
     __syncwarp();
     const uint32_t c = lane < __popc(rows) ? s_start[wid][lane] : 0xFFFFFFFFu;
     uint32_t before = 0;
-    for (uint32_t q0 = 0; q0 < stop - j; q0 += 32) {
-      const uint32_t starts = __reduce_or_sync(0xffffffffu, c - q0 < 32u ? 1u << (c - q0) : 0u);
+    uint32_t w_next = j + lane < stop ? __ldg(ci + j + lane) : 0u, s0_next = 0, s1_next = 0;
+    auto next_row = [&](bool in) {
+      s0_next = in && w_next < n ? (uint32_t)ld_off(rp, w_next) : 0u;
+      s1_next = in && w_next < n ? (uint32_t)ld_off(rp, w_next + 1) : 0u;
+    };
+    if (!kEmit) next_row(j + lane < stop);
+    for (uint32_t q0 = 0, len; q0 < stop - j; q0 += len) {
+      const uint32_t p = j + q0;
+      len = min(32u, stop - p);
+      if (kSets) {  // a set of whole rows when that leaves few lanes idle
+        const uint32_t whole = __reduce_max_sync(0xffffffffu, e <= p + 32 ? e : 0u);
+        if (whole >= p + kRowSetFill) len = min(len, whole - p);
+      }
+      const uint32_t starts =
+          __reduce_or_sync(0xffffffffu, c - q0 < len ? 1u << (c - q0) : 0u);
       const uint32_t at = before + __popc(starts & le) - 1;
       before += __popc(starts);
-      const uint32_t edge = j + q0 + lane;
+      const uint32_t edge = p + lane;
       const uint32_t row = s_row[wid][at & 31];
       const uint32_t end = __shfl_sync(0xffffffffu, e, row);
       const uint32_t first = edge + 1;
-      const bool on = edge < stop && first < end;
-      const uint32_t w = on ? __ldg(ci + edge) : 0u;
+      const bool on = lane < len && first < end;
+      // the next edges' columns and the offsets of their rows are under way
+      // while these are counted
+      const uint32_t w = w_next, r0 = s0_next, r1 = s1_next;
+      w_next = edge + len < stop ? __ldg(ci + edge + len) : 0u;
       const bool ok = on && w < n;
-      uint32_t id = kWalkShort, t1 = end, t_last = __shfl_sync(0xffffffffu, last, row);
+      uint32_t id = kWalkShort, t1 = end;
       uint32_t s0 = 0, s1 = 0;
       if (kEmit) {
         const uint32_t cut = __shfl_sync(0xffffffffu, mid, row);
-        const uint32_t rl = __shfl_sync(0xffffffffu, rest_last, row);
         if (ok) id = __ldg(number + w);
         const bool is_long = id != kWalkShort;
         const bool win = is_long && cut < end;
@@ -516,7 +560,6 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
           if (s1 - s0 <= kWalkShortCols) {
             rest = false;
             t1 = cut;
-            t_last = rl;
             wedges += cut - first;
           } else {
             s1 = s0;
@@ -537,35 +580,116 @@ __global__ void __launch_bounds__(kWalkBlock, 4)
           staged += add;
         }
       }
+      bool task_on = s0 < s1;  // the rest of a tail
       if (ok && id == kWalkShort) {
         wedges += end - first;
-        s0 = (uint32_t)ld_off(rp, w), s1 = (uint32_t)ld_off(rp, w + 1);
+        s0 = kEmit ? (uint32_t)ld_off(rp, w) : r0;
+        s1 = kEmit ? (uint32_t)ld_off(rp, w + 1) : r1;
       }
-      const MergeTask task{first + cols.mis, t1 + cols.mis, t_last, s0 + cols.mis, s1 + cols.mis};
-      if (!kEmit) {
+      if (kBatch && !(what & kMergeCount)) continue;
+      const MergeTask task{first + cols.mis, t1 + cols.mis, s0 + cols.mis, s1 + cols.mis};
+      if (!kGather) {
         if (s0 < s1) hits += merge_rows(cols, task);
-      } else {
-        // few of the edges intersect rows here: they gather until there is
-        // one for every lane
-        if (kBatch && !(what & kMergeCount)) s1 = s0;
-        const uint32_t mm = __ballot_sync(0xffffffffu, s0 < s1);
-        if (s0 < s1) s_task[wid][tasks + __popc(mm & lt)] = task;
-        tasks += __popc(mm);
-        __syncwarp();
-        if (tasks >= 32) {
-          hits += merge_rows(cols, s_task[wid][lane]);
-          tasks -= 32;
-          const MergeTask moved = s_task[wid][32 + lane];
+        if (!kEmit) next_row(edge + len < stop);
+        continue;
+      }
+      const uint32_t set_end = __shfl_sync(0xffffffffu, end, len - 1);
+      bool unit = !task_on && s0 < s1 && s1 - s0 <= kRowSetLong;
+      task_on = s0 < s1;
+      bool fetched = false;
+      const uint32_t um = __ballot_sync(0xffffffffu, unit);
+      if (kSets && __popc(starts) <= kRowSetRows && set_end - p <= kRowSetCols && __popc(um) >= kRowSetMin) {
+        // the chunk's rows as a set, two columns a lane: those of its edges,
+        // and the last row's behind them
+        const uint32_t x4 =
+            ((__popc(starts & le) - (starts & 1u)) * 32 | wid * kRowSetSlots) * 4;
+        const uint32_t x2 = __shfl_sync(0xffffffffu, x4, len - 1);
+        const bool in1 = edge < set_end, in2 = edge + 32 < set_end;
+        const uint32_t x1 = lane < len ? x4 : x2;
+        const uint32_t w1 = lane < len ? w : in1 ? __ldg(ci + edge) : 0u;
+        const uint32_t w2 = in2 ? __ldg(ci + edge + 32) : 0u;
+        bool found = false;
+        for (uint32_t tries = 0; tries < kRowSetTries; ++tries) {
+          const uint32_t a1 = row_set_at(w1, seed, x1), a2 = row_set_at(w2, seed, x2);
+          if (in1) slot(a1) = w1;
+          if (in2) slot(a2) = w2;
           __syncwarp();
-          if (lane < tasks) s_task[wid][lane] = moved;
+          const bool lost = (in1 && slot(a1) != w1) || (in2 && slot(a2) != w2);
+          found = !__any_sync(0xffffffffu, lost);
+          if (found) break;
+          if (in1) slot(a1) = kWalkEmpty;
+          if (in2) slot(a2) = kWalkEmpty;
+          __syncwarp();
+          seed = seed * 0x2C9277B5u + 2u;  // odd stays odd
+        }
+        if (found) {
+          // the sectors of the rows of w, one per lane and round
+          const uint32_t f = (s0 + cols.mis) >> 3;
+          const uint32_t sectors = unit ? ((s1 + cols.mis + 7) >> 3) - f : 0u;
+          const uint32_t incl = walk_scan(sectors, lane), pre = incl - sectors;
+          const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+          if (unit)
+            s_unit[kSets ? wid : 0][__popc(um & lt)] =
+                make_uint4(f - pre, s0 + cols.mis, s1 + cols.mis, x4);
+          __syncwarp();
+          uint32_t units = 0, key = wid * kRowSetSlots * 4, valid = 0, x[8] = {};
+          auto fetch = [&](uint32_t u0) {
+            const uint32_t heads = __reduce_or_sync(
+                0xffffffffu, unit && pre - u0 < 32u ? 1u << (pre - u0) : 0u);
+            const uint4 u = s_unit[kSets ? wid : 0][(units + __popc(heads & le) - 1) & 31];
+            units += __popc(heads);
+            valid = 0;
+            if (u0 + lane < total) {
+              const uint32_t sa = (u.x + u0 + lane) << 3;
+              walk_sector(cols, sa, u.y, u.z, x);
+              const uint32_t lo = u.y > sa ? u.y - sa : 0u;
+              const uint32_t hi = sa + 8 > u.z ? sa + 8 - u.z : 0u;
+              valid = (0xFFu << lo) & (0xFFu >> hi);
+              key = u.w;
+            }
+          };
+          fetch(0);
+          if (!kEmit) next_row(edge + len < stop);
+          fetched = true;
+          for (uint32_t u0 = 0; u0 < total; u0 += 32) {
+            uint32_t y[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = x[i];
+            const uint32_t in = valid, k = key;
+            if (u0 + 32 < total) fetch(u0 + 32);
+            uint32_t got = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              if (slot(row_set_at(y[i], seed, k)) == y[i]) got |= 1u << i;
+            hits += __popc(got & in);
+          }
+          task_on = task_on && !unit;
+          __syncwarp();
+          if (in1) slot(row_set_at(w1, seed, x1)) = kWalkEmpty;
+          if (in2) slot(row_set_at(w2, seed, x2)) = kWalkEmpty;
           __syncwarp();
         }
+      }
+      // the others gather until there is one for every lane
+      if (!kEmit && !fetched) next_row(edge + len < stop);
+      const uint32_t mm = __ballot_sync(0xffffffffu, task_on);
+      if (!mm) continue;
+      if (task_on) s_task[wid][tasks + __popc(mm & lt)] = task;
+      tasks += __popc(mm);
+      __syncwarp();
+      if (tasks >= 32) {
+        hits += merge_rows(cols, s_task[wid][lane]);
+        tasks -= 32;
+        const MergeTask moved = s_task[wid][32 + lane];
+        __syncwarp();
+        if (lane < tasks) s_task[wid][lane] = moved;
+        __syncwarp();
       }
     }
     j = stop;
   }
   if (kBatch) drain();
-  if (kEmit && lane < tasks) hits += merge_rows(cols, s_task[kEmit ? wid : 0][lane]);
+  if (kGather && lane < tasks) hits += merge_rows(cols, s_task[kGather ? wid : 0][lane]);
   if (kEmit && staged) flush();
   unsigned long long h = hits;
   for (int o = 16; o > 0; o >>= 1) {
@@ -589,6 +713,19 @@ constexpr uint64_t kWalkMinEdges = 1ull << 19;
 inline bool walk_wanted(uint64_t long_rows, uint64_t longest, uint64_t long_wedges,
                         uint64_t edges) {
   return long_rows > 0 && edges >= kWalkMinEdges && (longest > 128 || long_wedges >= (1ull << 25));
+}
+
+// Whether k_edge_merge counts by sets: a set pays when many wedges share it,
+// that is from some mean tail (wedges per edge) on. Measured, sets /
+// intersections in us: Erdos-Renyi, 6M edges, tail 4.2 207 / 192, 5.4 200 /
+// 198, 6.6 195 / 208; 13.3M, 9.2 427 / 533; 2M, 6.6 86 / 82, 8.5 79 / 80, 16
+// 105 / 128. Rows of uneven lengths leave more lanes of the intersections
+// idle: Chung-Lu, 6M edges, longest row 47, 3.4 184 / 196, 6.7 231 / 273.
+// Fewer than 2^20 edges take 20-32 either way. Not where the walk takes most
+// wedges (R-MAT scale 22: 906 / 759).
+inline bool row_sets_wanted(uint64_t edges, uint64_t wedges, uint64_t longest, uint64_t walked) {
+  const uint64_t tail = edges < (1ull << 22) ? 8 : longest > 40 ? 3 : 6;
+  return edges >= (1ull << 20) && wedges >= tail * edges && walked < wedges / 2;
 }
 
 // Edges per warp: kMergeTile, or fewer (whole rounds) when that leaves the
