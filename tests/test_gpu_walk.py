@@ -200,3 +200,40 @@ def test_row_sets_parity(wetric_mod, oracle_mod, degree, window):
     d = np.concatenate([dst, [1, 2, 0], dst]).astype(np.uint32)
     counts, _ = wetric_mod.Batch(s, d, off, np.array([n, 3, n], np.uint64)).count()
     assert [int(x) for x in counts] == [want, 1, want]
+
+
+@pytest.mark.parametrize("n,edges", [(2, 1), (33, 400), (70, 2000), (9000, 131_000),
+                                     (60_000, 131_071), (60_000, 131_072), (1 << 20, 60_000),
+                                     ((1 << 20) + 1, 60_000)])
+def test_small_graph_parity(wetric_mod, oracle_mod, n, edges):
+    """Around the single launch's limits: its columns (2^17), its rows (2^20),
+    fewer edges than a warp, long runs of empty rows, a row of every edge."""
+    import torch
+
+    rng = np.random.default_rng(n + edges)
+    for hub in (False, True):
+        if hub:  # one row past several warps' edges
+            k = min(n - 1, edges)
+            src = np.zeros(k, np.int64)
+            dst = 1 + np.arange(k)
+            extra = rng.integers(0, n, (2, max(0, edges - k)))
+            src, dst = np.concatenate([src, extra[0]]), np.concatenate([dst, extra[1]])
+            key = np.unique(np.minimum(src, dst) * n + np.maximum(src, dst))
+        else:
+            pair = rng.integers(0, n, (2, 2 * edges + 20)) if n > 2 else np.array([[0], [1]])
+            key = np.unique(pair.min(0) * n + pair.max(0))
+            key = rng.permutation(key[key // n != key % n])[:edges]
+        key = np.sort(key[key // n != key % n])
+        rp = np.zeros(n + 1, np.uint64)  # an oriented CSR in id order
+        rp[1:] = np.cumsum(np.bincount(key // n, minlength=n))
+        ci = (key % n).astype(np.uint32)
+        g = oracle_mod.CSR(rp, ci)
+        want, W = oracle_mod.count_merge(g), oracle_mod.wedge_total(g)
+        rp64 = torch.from_numpy(rp.view(np.int64)).cuda()
+        col = torch.from_numpy(ci.view(np.int32)).cuda()
+        odd = torch.cat([col[:1], col])[1:]
+        for r, c in ((rp64, col), (rp64.int(), col), (rp64.int(), odd)):
+            for kw in ({}, {"validate": True}):
+                got, st = wetric_mod.count(r, c, 5, 8192, **kw)
+                assert got == want and st.wedges == st.wedges_counted == W
+                assert st.max_out_degree == int(np.diff(rp.astype(np.int64)).max())

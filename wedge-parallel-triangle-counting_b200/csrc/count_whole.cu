@@ -5,11 +5,9 @@
 // The reference counts every wedge by one edge check (tc.cu:173-293); here
 // every edge (v, w) takes the cheapest of three forms of the same
 // intersection, so nothing needs the wedge prefix, the tiles over it or
-// per-row hash sets. A small graph is two kernels and one read-back:
-//
-//   k_edge_vertices  k_edge_merge                                 [read]
-//
-// and a large one
+// per-row hash sets. A small graph is one kernel that writes its results to
+// the host (k_small_count; with validation k_edge_vertices, k_validate,
+// k_edge_merge and a copy), a large one
 //
 //   k_edge_vertices                                               [read]
 //   per row chunk: k_walk_split k_edge_merge k_core_bitmap k_core_count
@@ -33,8 +31,9 @@ namespace wetric {
 namespace {
 
 // Below this many columns a graph takes no core and no walk: one kernel
-// intersects the rows of all its edges, and the count is read back once.
+// intersects the rows of all its edges.
 constexpr uint64_t kSmallColumns = 1ull << 17;
+constexpr uint64_t kSmallRows = 1ull << 20;  // and this many rows at most: one launch
 
 // A word read by the core's row ANDs against a wedge counted below it (R-MAT
 // scale 22, between neighbouring lengths: 0.21 ps per estimated word, 0.8 ps
@@ -95,6 +94,50 @@ bool count_whole_takes(const CountArgs &a) {
          (a.offsets32 || (a.m < kSmallColumns && (a.core_len == 0 || a.core_len == kCoreOff)));
 }
 
+// The small graph's single launch (k_small_count); false: no pinned words.
+template <typename Off>
+static int small_count(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, CountResult *r,
+                       bool *done) {
+  static_assert(kSmallBlocks * kSmallWords <= kPinnedWords, "one word group per block");
+  const unsigned long long *out = reinterpret_cast<unsigned long long *>(readback_words());
+  *done = out != nullptr;
+  if (!out) return WETRIC_OK;
+  EventPair ev_all;
+  WETRIC_TRY(ev_all.start(st));
+  if (a.ci_ready) WETRIC_CUDA_TRY(cudaStreamWaitEvent(st, a.ci_ready, 0));
+  const uint32_t n = (uint32_t)a.n, m = (uint32_t)a.m, warps = kWalkBlock / 32;
+  const uint32_t T = 32 * (uint32_t)ceil_div(m ? m : 1, 32ull * warps * kSmallBlocks);
+  const uint64_t for_rows = ceil_div(n, kWalkBlock), for_edges = ceil_div(m, T * warps);
+  uint64_t grid = for_rows > for_edges ? for_rows : for_edges;
+  if (grid > kSmallBlocks) grid = kSmallBlocks;
+  k_small_count<Off><<<(unsigned)grid, kWalkBlock, 0, st>>>(
+      static_cast<const Off *>(a.row_ptr), walk_columns(a.col_ind, m), n, m, T,
+      const_cast<unsigned long long *>(out));
+  WETRIC_LAUNCH_CHECK();
+  WETRIC_TRY(ev_all.stop(st));
+  WETRIC_CUDA_TRY(cudaEventSynchronize(ev_all.b));
+  unsigned long long sum[3] = {}, longest = 0, bad = 0;
+  for (uint64_t i = 0; i < grid; ++i) {
+    const unsigned long long *w = out + i * kSmallWords;
+    sum[0] += w[0];
+    sum[1] += w[1];
+    sum[2] += w[2] & ((1ull << 40) - 1);
+    bad |= w[2] >> 40;
+    longest = longest > w[3] ? longest : w[3];
+  }
+  r->max_out_degree = longest;
+  WETRIC_TRY(check_words(bad ? (uint64_t)kDevRowPtrRange : 0, longest));
+  r->triangles = sum[0];
+  r->wedges = r->wedges_counted = r->pair_wedges = sum[1];
+  r->pair_rows = sum[2];
+  WETRIC_TRY(ev_all.add_to(&r->exec_ms));
+  r->count_ms = r->pair_ms = r->exec_ms;
+  r->block = kWalkBlock;
+  r->grid = (uint32_t)grid;
+  r->launches = 1;
+  return WETRIC_OK;
+}
+
 template <typename Off>
 static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, CountResult *r,
                       bool *declined) {
@@ -114,6 +157,12 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
       return WETRIC_EINVAL;
     }
   }
+  const bool small = m < kSmallColumns && (a.core_len == 0 || a.core_len == kCoreOff);
+  if (small && !a.validate && !C_in && n > 0 && n <= kSmallRows) {
+    bool done = false;
+    WETRIC_TRY(small_count<Off>(ctx, st, a, r, &done));
+    if (done) return WETRIC_OK;
+  }
   EventPair ev_all;
   WETRIC_TRY(ev_all.start(st));
   uint32_t launches = 0;
@@ -127,7 +176,6 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
   WETRIC_CUDA_TRY(cudaMemsetAsync(words.ptr, 0, kWords * sizeof(uint64_t), st));
   uint32_t *err = reinterpret_cast<uint32_t *>(words.ptr + 2);
 
-  const bool small = m < kSmallColumns && (a.core_len == 0 || a.core_len == kCoreOff);
   EdgeCores cores{};
   if (!small && a.core_len != kCoreOff && n >= 64) {
     if (a.core_len == 0)

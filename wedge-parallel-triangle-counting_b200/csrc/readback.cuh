@@ -7,7 +7,8 @@
 
 namespace wetric {
 
-constexpr uint32_t kReadWords = 128;
+constexpr uint32_t kReadWords = 128;     // values of one read-back at most
+constexpr uint32_t kPinnedWords = 1024;  // of a thread
 // Pinned words for the calling thread's read-backs (portable: any device),
 // made on first use and freed when the thread ends; null if pinned memory
 // cannot be had (the caller then reads into its own array).
@@ -22,7 +23,7 @@ inline uint64_t *readback_words() {
   thread_local Holder h;
   if (!h.tried) {
     h.tried = true;
-    if (cudaHostAlloc(reinterpret_cast<void **>(&h.p), kReadWords * sizeof(uint64_t),
+    if (cudaHostAlloc(reinterpret_cast<void **>(&h.p), kPinnedWords * sizeof(uint64_t),
                       cudaHostAllocPortable) != cudaSuccess) {
       h.p = nullptr;
       cudaGetLastError();
@@ -60,7 +61,8 @@ __global__ void k_read_gather(const __grid_constant__ ReadPlan p, uint64_t *__re
   out[threadIdx.x] = sp.bytes == 4 ? (uint64_t)static_cast<const uint32_t *>(sp.src)[j]
                                    : static_cast<const uint64_t *>(sp.src)[j];
 }
-static_assert(kReadWords <= 128, "one word per thread of the gather's block");
+
+static_assert(kReadWords <= 128 && kReadWords <= kPinnedWords, "a thread of the gather per word");
 // Gathers plan's values on st, copies them to the host and waits (for
 // `done`, recorded after the copy, when given); *words points at them
 // afterwards (valid until the calling thread's next read).

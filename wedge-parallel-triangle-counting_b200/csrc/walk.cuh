@@ -702,6 +702,95 @@ __global__ void __launch_bounds__(kMergeBlock, kSets ? 7 : 8)
   }
 }
 
+// A small graph's whole count in one launch: the row checks and totals of
+// k_edge_vertices and the intersections of k_edge_merge, T edges per warp,
+// block b's results in out[4b, 4b + 4) -- triangles, W, rows with wedges (and
+// bit 40: bad offsets), longest row -- which may be host memory, so nothing is
+// cleared before or copied after. Offsets are not trusted: each row's are
+// checked before it is read. Bound by the call around it (launch, events,
+// wait): 2,000 vertices, 57 -> 33 us against the two kernels, a memset and a
+// copy.
+constexpr uint32_t kSmallBlocks = 256;
+constexpr uint32_t kSmallWords = 4;
+template <typename Off>
+__global__ void __launch_bounds__(kWalkBlock)
+    k_small_count(const Off *__restrict__ rp, const __grid_constant__ WalkColumns cols, uint32_t n,
+                  uint32_t m, uint32_t T, unsigned long long *__restrict__ out) {
+  __shared__ uint32_t s_start[kWalkBlock / 32][32], s_row[kWalkBlock / 32][32];
+  __shared__ unsigned long long s_sum[kSmallWords];
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u, le = 0xFFFFFFFFu >> (31 - lane);
+  if (threadIdx.x < kSmallWords) s_sum[threadIdx.x] = 0;
+  __syncthreads();
+  bool bad = blockIdx.x == 0 && threadIdx.x == 0 &&
+             (ld_off(rp, 0) != 0 || ld_off(rp, (uint64_t)n) != m);
+  unsigned long long W = 0;
+  uint32_t rows = 0, longest = 0, hits = 0;
+  for (uint32_t v = blockIdx.x * kWalkBlock + threadIdx.x; v < n; v += gridDim.x * kWalkBlock) {
+    const uint64_t b = ld_off(rp, (uint64_t)v), e = ld_off(rp, (uint64_t)v + 1);
+    if (e < b || e > m) {
+      bad = true;
+    } else {
+      const uint32_t d = (uint32_t)(e - b);
+      W += d >= 2 ? (unsigned long long)d * (d - 1) / 2 : 0;
+      rows += d >= 2;
+      longest = max(longest, d);
+    }
+  }
+  const uint32_t *ci = cols.base + cols.mis;
+  const uint64_t from = (uint64_t)(blockIdx.x * (kWalkBlock / 32) + wid) * T;
+  const uint32_t j1 = (uint32_t)min((uint64_t)m, from + T);
+  for (uint32_t j = (uint32_t)min(from, (uint64_t)m); j < j1;) {
+    const uint64_t v = row_of_edge(rp, 0, n, j, lane) + lane;
+    uint64_t b64 = m, e64 = m;
+    if (v < n) b64 = ld_off(rp, v), e64 = ld_off(rp, v + 1);
+    if (e64 < b64 || e64 > m) b64 = e64 = 0;  // counted as bad above
+    const uint32_t b = (uint32_t)b64, e = (uint32_t)e64;
+    const uint32_t stop = min(j1, __shfl_sync(0xffffffffu, e, 31));
+    if (stop <= j) break;  // not with good offsets
+    const uint32_t some = __ballot_sync(0xffffffffu, e > b);
+    __syncwarp();
+    if (e > b) {
+      s_start[wid][__popc(some & lt)] = max(b, j) - j;
+      s_row[wid][__popc(some & lt)] = lane;
+    }
+    __syncwarp();
+    const uint32_t c = lane < __popc(some) ? s_start[wid][lane] : 0xFFFFFFFFu;
+    uint32_t before = 0;
+    for (uint32_t q0 = 0; q0 < stop - j; q0 += 32) {
+      const uint32_t starts = __reduce_or_sync(0xffffffffu, c - q0 < 32u ? 1u << (c - q0) : 0u);
+      const uint32_t at = before + __popc(starts & le) - 1;
+      before += __popc(starts);
+      const uint32_t edge = j + q0 + lane;
+      const uint32_t end = __shfl_sync(0xffffffffu, e, s_row[wid][at & 31]);
+      if (edge < stop && edge + 1 < end) {
+        const uint32_t w = __ldg(ci + edge);
+        if (w < n) {
+          const uint64_t s0 = ld_off(rp, (uint64_t)w), s1 = ld_off(rp, (uint64_t)w + 1);
+          if (s0 < s1 && s1 <= m)
+            hits += merge_rows(cols, MergeTask{edge + 1 + cols.mis, end + cols.mis,
+                                               (uint32_t)s0 + cols.mis, (uint32_t)s1 + cols.mis});
+        }
+      }
+    }
+    j = stop;
+  }
+  for (int o = 16; o > 0; o >>= 1) W += __shfl_down_sync(0xffffffffu, W, o);
+  hits = __reduce_add_sync(0xffffffffu, hits);
+  rows = __reduce_add_sync(0xffffffffu, rows);
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  bad = __any_sync(0xffffffffu, bad);
+  if (lane == 0) {
+    if (hits) atomicAdd(&s_sum[0], (unsigned long long)hits);
+    if (W) atomicAdd(&s_sum[1], W);
+    if (rows) atomicAdd(&s_sum[2], (unsigned long long)rows);
+    if (bad) atomicOr(&s_sum[2], 1ull << 40);
+    if (longest) atomicMax(&s_sum[3], (unsigned long long)longest);
+  }
+  __syncthreads();
+  if (threadIdx.x < kSmallWords) out[blockIdx.x * kSmallWords + threadIdx.x] = s_sum[threadIdx.x];
+}
+
 // Whether the edges to long rows (more than 48 columns) are worth sorting for
 // the walk, against intersecting every row where its edge is: intersections
 // with rows of up to 128 columns waste at most 32 steps, and below 2^25
