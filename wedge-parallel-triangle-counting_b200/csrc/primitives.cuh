@@ -515,21 +515,25 @@ __global__ void __launch_bounds__(kSortThreads, kSortBlocks)
   }
 }
 
-// Workspace of one sort: the digits' histograms, the passes' tickets and the
-// look-back words, cleared at once.
+// Workspace of one sort of up to n keys, cleared: the digits' histograms, the
+// passes' tickets and the look-back words. A part of a larger one (at), or
+// its own (alloc).
 struct SortSpace {
   Scratch<uint64_t> buf;
   unsigned long long *hist = nullptr;
   uint32_t *tickets = nullptr;
   uint64_t *state = nullptr;
+  static constexpr uint64_t kHead = (uint64_t)kMaxPasses * kRadix + kMaxPasses;
+  static uint64_t words(uint64_t n) { return kHead + sort_tiles(n) * kRadix; }
+  void at(uint64_t *p) {
+    hist = reinterpret_cast<unsigned long long *>(p);
+    tickets = reinterpret_cast<uint32_t *>(p + kMaxPasses * kRadix);
+    state = p + kHead;
+  }
   int alloc(DeviceContext *ctx, cudaStream_t st, uint64_t n) {
-    const uint64_t head = (uint64_t)kMaxPasses * kRadix + kMaxPasses;
-    const uint64_t words = head + sort_tiles(n) * kRadix;
-    WETRIC_TRY(buf.alloc(ctx, st, words));
-    WETRIC_CUDA_TRY(cudaMemsetAsync(buf.ptr, 0, words * sizeof(uint64_t), st));
-    hist = reinterpret_cast<unsigned long long *>(buf.ptr);
-    tickets = reinterpret_cast<uint32_t *>(buf.ptr + kMaxPasses * kRadix);
-    state = buf.ptr + head;
+    WETRIC_TRY(buf.alloc(ctx, st, words(n)));
+    WETRIC_CUDA_TRY(cudaMemsetAsync(buf.ptr, 0, words(n) * sizeof(uint64_t), st));
+    at(buf.ptr);
     return WETRIC_OK;
   }
 };
