@@ -24,3 +24,28 @@ def test_orientation_at_tile_edges(wetric_mod, oracle_mod, pairs, n):
     g.free()
     assert np.array_equal(got.row_ptr, want.row_ptr)
     assert np.array_equal(got.col_ind, want.col_ind)
+
+
+@pytest.mark.parametrize("size", [2, 5, 32, 33, 34, 130, 512, 513, 514, 600])
+def test_symmetric_rows_around_the_row_sort(wetric_mod, oracle_mod, size):
+    """A clique of `size` gives an oriented row of size - 1 columns: around a
+    warp's and the in-place rows' 512, where the radix sort takes over; with
+    a sparse graph, hubs and isolated vertices beside it, host and device."""
+    import torch
+
+    rng = np.random.default_rng(size)
+    n = 4000
+    i, j = np.triu_indices(size, 1)
+    ids = rng.permutation(n - 500)  # the last 500 stay isolated
+    src = np.concatenate([ids[i], rng.integers(0, n - 500, 9000), np.full(900, ids[700])])
+    dst = np.concatenate([ids[j], rng.integers(0, n - 500, 9000), ids[1000:1900]])
+    sym = oracle_mod.csr_from_pairs(src.astype(np.uint32), dst.astype(np.uint32), n)
+    want = oracle_mod.preprocess(sym)
+    got = wetric_mod.preprocess(wetric_mod.Graph(sym.row_ptr, sym.col_ind))
+    assert np.array_equal(got.row_ptr, want.row_ptr)
+    assert np.array_equal(got.col_ind, want.col_ind)
+    tri = oracle_mod.count_merge(want)
+    rp = torch.from_numpy(sym.row_ptr.view(np.int64)).cuda()
+    ci = torch.from_numpy(sym.col_ind.view(np.int32)).cuda()
+    assert wetric_mod.count(rp, ci, 5, 64, oriented=False)[0] == tri
+    assert wetric_mod.count(rp.int(), ci, 5, 64, oriented=False)[0] == tri
