@@ -260,7 +260,7 @@ def run_ours(args):
     ci32_np = ci32.numpy().view(np.uint32)
     for _ in range(args.warmup):
         wetric.count(rp32_np, ci32_np, args.s, args.a, device=dev, wedge_begin=lo,
-                     wedge_end=hi, kernel=args.kernel, core_len=args.core_len)
+                     wedge_end=hi_arg, kernel=args.kernel, core_len=args.core_len)
     if world > 1:
         dist.barrier()
     torch.cuda.synchronize()
@@ -271,7 +271,7 @@ def run_ours(args):
     for _ in range(args.steps):
         t1 = time.perf_counter()
         c, st = wetric.count(rp32_np, ci32_np, args.s, args.a, device=dev,
-                             wedge_begin=lo, wedge_end=hi, kernel=args.kernel,
+                             wedge_begin=lo, wedge_end=hi_arg, kernel=args.kernel,
                              core_len=args.core_len)
         e2e_steps.append((time.perf_counter() - t1) * 1e3)
         e2e_launches += st.launches
@@ -295,14 +295,14 @@ def run_ours(args):
     ci_pg = np.array(host.col_ind, dtype=np.uint32, copy=True)
     for _ in range(args.warmup):
         wetric.count(rp_pg, ci_pg, args.s, args.a, device=dev, wedge_begin=lo,
-                     wedge_end=hi, kernel=args.kernel, core_len=args.core_len)
+                     wedge_end=hi_arg, kernel=args.kernel, core_len=args.core_len)
     if world > 1:
         dist.barrier()
     torch.cuda.synchronize()
     t0 = time.perf_counter()
     for _ in range(args.steps):
         c, st = wetric.count(rp_pg, ci_pg, args.s, args.a, device=dev,
-                             wedge_begin=lo, wedge_end=hi, kernel=args.kernel,
+                             wedge_begin=lo, wedge_end=hi_arg, kernel=args.kernel,
                              core_len=args.core_len)
         if world > 1:
             t = torch.tensor([c], dtype=torch.int64, device=f"cuda:{dev}")
