@@ -227,7 +227,7 @@ typedef struct {
 #define WETRIC_OPT_ONE_PASS 0x2u
 /* No row-by-row counting of short rows. By default a whole-graph count (m <
  * 2^31) intersects each edge's tail with its end's short row and streams
- * the others through the long rows' sets, and kernel 8 (32-bit offsets,
+ * the tails of the others through the long rows' sets, and kernel 8 (32-bit offsets,
  * columns not copied in row chunks) counts each vertex with d+ <= 64 whose
  * neighbours' rows are short by pair streams: its out-neighbours go into a
  * shared-memory set and the rows of those neighbours stream through it.
@@ -346,9 +346,11 @@ int wetric_count_noalloc(const wetric_csr *csr, uint32_t s, uint32_t a,
  * the reference counts one graph per run, tc.cu:896-913). The batch is
  * preprocessed once on the device as a disjoint union in which every graph
  * keeps its own id range and its own degree order (so each graph's oriented
- * CSR equals the one it gets alone), stays resident, and is counted by a
- * persistent kernel that pulls (graph, wedge-range) tiles from a device work
- * counter; the launches are captured in a CUDA graph and replayed. */
+ * CSR equals the one it gets alone), stays resident, and is counted by the
+ * kernels of a single graph over the union (with no_pair_streams, m >= 2^31 or
+ * no room: by a persistent kernel that pulls (graph, wedge-range) tiles from a
+ * device work counter; spread, bitmap and autotune are that kernel's); the
+ * launches are captured in a CUDA graph and replayed. */
 typedef struct wetric_batch_s *wetric_batch;
 
 typedef struct {
@@ -359,7 +361,7 @@ typedef struct {
                               for each size/skew bucket of graphs not yet in
                               this device's tuning table, and use the table */
   uint64_t bitmap_cap_bytes; /* total bitmap memory (0 = 2 GiB)             */
-  uint32_t no_pair_streams;  /* != 0: no pair streams for the short rows
+  uint32_t no_pair_streams;  /* != 0: every wedge by a set lookup
                                 (WETRIC_OPT_NO_PAIR_STREAMS for a batch)   */
 } wetric_batch_opts;
 
@@ -379,8 +381,8 @@ int wetric_batch_count(wetric_batch b, uint64_t *counts, wetric_stats *stats);
 /* Per-graph W and oriented edge counts (host arrays of G entries; either
  * may be NULL). */
 int wetric_batch_info(wetric_batch b, uint64_t *wedges, uint64_t *edges);
-/* The spread s_g each graph is counted with (host array of G entries):
- * tiles of 256 * s_g wedges. */
+/* The spread s_g of each graph's tiles of 256 * s_g wedges (host array of G
+ * entries; where the wedges are not tiled, the one its size would get). */
 int wetric_batch_spreads(wetric_batch b, uint32_t *spread);
 void wetric_batch_free(wetric_batch b);
 
