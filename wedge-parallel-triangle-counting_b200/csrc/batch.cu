@@ -214,8 +214,12 @@ __global__ void __launch_bounds__(kWalkBlock)
     id = __shfl_sync(0xffffffffu, id, 0) + __popc(mask & ((1u << lane) - 1u));
     if (v < n) number[v] = is_long ? id : kWalkShort;
     if (is_long) {
-      long_rows[id] = (uint32_t)v;
-      long_graph[id] = g;
+      if (id < long_rows_room(m)) {
+        long_rows[id] = (uint32_t)v;
+        long_graph[id] = g;
+      } else {
+        atomicCAS(err, 0u, (uint32_t)kDevRowPtrRange);
+      }
     }
     if (same) {
       for (int o = 16; o > 0; o >>= 1) w += __shfl_down_sync(0xffffffffu, w, o);
@@ -456,8 +460,8 @@ static int make_whole(Batch *b, cudaStream_t st) {
   WETRIC_CUDA_TRY(cudaMemsetAsync(w->words.ptr, 0, (kWords + G) * 8ull, st));
   uint32_t *err = reinterpret_cast<uint32_t *>(w->words.ptr + 2);
   if (w->number.alloc(ctx, st, n) != WETRIC_OK ||
-      w->long_rows.alloc(ctx, st, m / (kWalkShortCols + 1) + 1) != WETRIC_OK ||
-      w->long_graph.alloc(ctx, st, m / (kWalkShortCols + 1) + 1) != WETRIC_OK) {
+      w->long_rows.alloc(ctx, st, long_rows_room(m)) != WETRIC_OK ||
+      w->long_graph.alloc(ctx, st, long_rows_room(m)) != WETRIC_OK) {
     clear_error();
     return WETRIC_OK;
   }

@@ -191,7 +191,7 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
   Scratch<uint32_t> number, long_rows;
   if (!small) {
     WETRIC_TRY(number.alloc(ctx, st, n));
-    WETRIC_TRY(long_rows.alloc(ctx, st, m / (kWalkShortCols + 1) + 1));
+    WETRIC_TRY(long_rows.alloc(ctx, st, long_rows_room(m)));
   }
   if (n > 0) {
     const uint64_t most = (uint64_t)ctx->sm_count * 8, need = ceil_div(n, kWalkBlock);

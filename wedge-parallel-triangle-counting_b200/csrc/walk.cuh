@@ -122,6 +122,14 @@ __device__ __forceinline__ uint32_t walk_window(const WalkGroups &gr, uint32_t g
 // (k_core_plan) and rows with wedges.
 constexpr uint32_t kEdgeCand = 5;
 constexpr uint32_t kEdgeTotals = kEdgeCand + 3 * kCoreNumCandidates;
+// Rows of more than kWalkShortCols columns among m columns at most, when the
+// offsets are monotone: the room for long_rows. The kernels that number the
+// long rows are also the ones that check the offsets, and rows that overlap
+// (0, m, 0, m, ...) can be long in any number, so ids past the room are
+// dropped and raise kDevRowPtrRange.
+__host__ __device__ inline uint64_t long_rows_room(uint64_t m) {
+  return m / (kWalkShortCols + 1) + 1;
+}
 template <typename Off>
 __global__ void __launch_bounds__(kWalkBlock)
     k_edge_vertices(const Off *__restrict__ rp, uint64_t n, uint64_t m,
@@ -167,7 +175,10 @@ __global__ void __launch_bounds__(kWalkBlock)
       id = __shfl_sync(0xffffffffu, id, 0) + __popc(mask & ((1u << lane) - 1u));
       if (v < n) number[v] = is_long ? id : kWalkShort;
       if (is_long) {
-        long_rows[id] = (uint32_t)v;
+        if (id < long_rows_room(m))
+          long_rows[id] = (uint32_t)v;
+        else
+          atomicCAS(err, 0u, (uint32_t)kDevRowPtrRange);
         long_w += w;
       }
     }
