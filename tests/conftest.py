@@ -1,7 +1,9 @@
 """Shared test setup: import paths, the `gpu` marker, small graph builders."""
 from __future__ import annotations
 
+import ctypes
 import os
+import subprocess
 import sys
 
 import numpy as np
@@ -69,3 +71,17 @@ def wetric_mod():
     import wetric
 
     return wetric
+
+
+@pytest.fixture(scope="session")
+def probe(wetric_mod, tmp_path_factory):
+    """tests/kernel_probe.cu, compiled beside the library it links to."""
+    lib = tmp_path_factory.mktemp("probe") / "libprobe.so"
+    subprocess.check_call(
+        [os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-gencode",
+         "arch=compute_100a,code=sm_100a", "-ccbin", "/usr/bin/g++", "-std=c++17", "-O2",
+         "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-shared", "-cudart", "static",
+         "-I", os.path.join(PKG, "csrc"), "-o", str(lib),
+         os.path.join(ROOT, "tests", "kernel_probe.cu"), "-L", os.path.join(PKG, "wetric"),
+         "-lwetric", "-Xlinker", "-rpath," + os.path.join(PKG, "wetric")])
+    return ctypes.CDLL(str(lib))

@@ -67,14 +67,16 @@ struct Arena {
 };
 
 // Exclusive scan with its look-back words taken from the arena (same kernel
-// as the allocating scan in primitives.cuh).
+// as the allocating scan in primitives.cuh). *words: the words of an earlier
+// scan of as many elements or more, which serve as the second words of a
+// 64-bit scan; the new ones on return.
 template <typename InT, typename OutT>
 int scan_in_arena(Arena *ar, cudaStream_t st, const InT *in, OutT *out,
-                  uint64_t n, uint32_t *err) {
+                  uint64_t n, uint32_t *err, uint64_t **words) {
   using namespace wetric::prim;
   const uint64_t tiles = n == 0 ? 1 : wetric::ceil_div(n, kScanChunk);
   if (tiles == 1) {
-    k_scan<InT, OutT><<<1, kScanThreads, 0, st>>>(in, n, out, nullptr, nullptr, err);
+    k_scan<InT, OutT><<<1, kScanThreads, 0, st>>>(in, n, out, nullptr, nullptr, nullptr, err);
     WETRIC_LAUNCH_CHECK();
     return WETRIC_OK;
   }
@@ -84,8 +86,11 @@ int scan_in_arena(Arena *ar, cudaStream_t st, const InT *in, OutT *out,
     return WETRIC_ERANGE;
   }
   WETRIC_CUDA_TRY(cudaMemsetAsync(state, 0, (tiles + 1) * sizeof(uint64_t), st));
+  uint64_t *rest = kScanWide<InT> ? *words : nullptr;
+  if (rest) WETRIC_CUDA_TRY(cudaMemsetAsync(rest, 0, tiles * sizeof(uint64_t), st));
+  *words = state;
   k_scan<InT, OutT><<<(unsigned)tiles, kScanThreads, 0, st>>>(
-      in, n, out, state + 1, reinterpret_cast<uint32_t *>(state), err);
+      in, n, out, state + 1, rest, reinterpret_cast<uint32_t *>(state), err);
   WETRIC_LAUNCH_CHECK();
   return WETRIC_OK;
 }
@@ -184,7 +189,8 @@ int count_noalloc_impl(int device, cudaStream_t st, const Off *rp,
   WETRIC_CUDA_TRY(cudaMemsetAsync(acc, 0, 4 * sizeof(unsigned long long), st));
   k_vertex_wedges<Off><<<grid_cap(sms, n), 256, 0, st>>>(rp, n, m, active, acc, small);
   WETRIC_LAUNCH_CHECK();
-  WETRIC_TRY((scan_in_arena<uint32_t, uint64_t>(&ar, st, active, pos, n, small)));
+  uint64_t *look = nullptr;  // the scans' look-back words
+  WETRIC_TRY((scan_in_arena<uint32_t, uint64_t>(&ar, st, active, pos, n, small, &look)));
   uint64_t K = 0;
   unsigned long long maxdeg = 0;
   uint32_t err = 0;
@@ -213,7 +219,7 @@ int count_noalloc_impl(int device, cudaStream_t st, const Off *rp,
                                                            act_rb, act_d);
     WETRIC_LAUNCH_CHECK();
   }
-  WETRIC_TRY((scan_in_arena<uint64_t, uint64_t>(&ar, st, act_wp, act_wp, K, small)));
+  WETRIC_TRY((scan_in_arena<uint64_t, uint64_t>(&ar, st, act_wp, act_wp, K, small, &look)));
   uint64_t W = 0;
   WETRIC_CUDA_TRY(cudaMemcpyAsync(&W, act_wp + K, 8, cudaMemcpyDeviceToHost, st));
   WETRIC_CUDA_TRY(cudaMemcpyAsync(&err, small, 4, cudaMemcpyDeviceToHost, st));

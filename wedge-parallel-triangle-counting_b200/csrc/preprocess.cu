@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kThreads)
     const uint32_t c = lane < kThreads / 32 ? s_warp[lane] : 0u;
     const uint32_t total = __reduce_add_sync(0xffffffffu, c);
     uint64_t excl = 0;
-    const bool ok = prim::tile_prefix(state, tile, total, err, &excl);
+    const bool ok = prim::tile_prefix<false>(state, nullptr, tile, total, err, &excl);
     if (lane == 0) {
       s_excl = excl;
       s_ok = ok;

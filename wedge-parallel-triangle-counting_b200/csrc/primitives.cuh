@@ -22,17 +22,34 @@ namespace prim {
 
 // Published words: value in the low 48 bits, (epoch << 2 | flag) above it.
 // A word of another epoch reads as "not published yet", so one clearing of
-// the words serves every pass of a sort.
+// the words serves every pass of a sort. 48 bits hold any number of keys,
+// rows or columns; the wedge prefixes are 64 bits wide (one row of 2^25
+// columns has 2^49 wedges) and take two words, each with its flag: the low
+// 48 bits and the rest (tile_rest). Every word is written once per flag, so
+// two words with the same flag are of one value.
 constexpr uint32_t kTileAgg = 1, kTileIncl = 2, kTilePoison = 3;
 constexpr uint64_t kTileValueMask = (1ull << 48) - 1;
 constexpr uint32_t kLookbackSpins = 1u << 22;
 
-__device__ __forceinline__ uint64_t tile_word(uint32_t epoch, uint32_t flag, uint64_t value) {
-  return ((uint64_t)(epoch << 2 | flag) << 48) | value;
+__host__ __device__ __forceinline__ uint64_t tile_word(uint32_t epoch, uint32_t flag,
+                                                       uint64_t value) {
+  return ((uint64_t)(epoch << 2 | flag) << 48) | (value & kTileValueMask);
 }
-__device__ __forceinline__ uint32_t tile_flag(uint64_t w, uint32_t epoch) {
+__host__ __device__ __forceinline__ uint32_t tile_flag(uint64_t w, uint32_t epoch) {
   const uint32_t tag = (uint32_t)(w >> 48);
   return (tag >> 2) == epoch ? (tag & 3u) : 0u;
+}
+// The second word of a 64-bit value, and the flag and value of a pair: no
+// flag while the two differ, poison as soon as one has it.
+__host__ __device__ __forceinline__ uint64_t tile_rest(uint32_t flag, uint64_t value) {
+  return tile_word(0, flag, value >> 48);
+}
+__host__ __device__ __forceinline__ uint32_t tile_pair_flag(uint64_t w, uint64_t rest) {
+  const uint32_t a = tile_flag(w, 0), b = tile_flag(rest, 0);
+  return a == kTilePoison || b == kTilePoison ? kTilePoison : a == b ? a : 0u;
+}
+__host__ __device__ __forceinline__ uint64_t tile_pair_value(uint64_t w, uint64_t rest) {
+  return (w & kTileValueMask) | (rest << 48);
 }
 __device__ __forceinline__ uint64_t ld_tile(const uint64_t *p) {
   uint64_t v;
@@ -44,24 +61,30 @@ __device__ __forceinline__ void st_tile(uint64_t *p, uint64_t v) {
 }
 
 // Exclusive prefix of `agg` over the tiles before `tile` (a whole warp
-// calls it; one word per tile). A step looks at 128 predecessors, four per
+// calls it; one word per tile, with kWide another in rest). A step looks at 128 predecessors, four per
 // lane: all tiles of a short scan start together, so the last one walks back
 // over all of them. Returns false when a wait ran out.
 constexpr int kLookWide = 4;
-__device__ __forceinline__ bool tile_prefix(uint64_t *state, uint64_t tile, uint64_t agg,
-                                            uint32_t *err, uint64_t *excl) {
+template <bool kWide>
+__device__ __forceinline__ bool tile_prefix(uint64_t *state, uint64_t *rest, uint64_t tile,
+                                            uint64_t agg, uint32_t *err, uint64_t *excl) {
   const uint32_t lane = threadIdx.x & 31;
+  auto publish = [&](uint32_t flag, uint64_t value) {
+    if (lane != 0) return;
+    st_tile(state + tile, tile_word(0, flag, value));
+    if (kWide) st_tile(rest + tile, tile_rest(flag, value));
+  };
   *excl = 0;
   if (tile == 0) {
-    if (lane == 0) st_tile(state, tile_word(0, kTileIncl, agg));
+    publish(kTileIncl, agg);
     return true;
   }
-  if (lane == 0) st_tile(state + tile, tile_word(0, kTileAgg, agg));
+  publish(kTileAgg, agg);
   uint64_t sum = 0;
   for (int64_t hi = (int64_t)tile - 1;; hi -= 32 * kLookWide) {
     // word j of the lane: predecessor j * 32 + lane of the window
     uint64_t w[kLookWide];
-    uint32_t spins = 0;
+    uint32_t flag[kLookWide], spins = 0;
     bool bad = false;
     for (;;) {
       bool ready = true;
@@ -69,12 +92,17 @@ __device__ __forceinline__ bool tile_prefix(uint64_t *state, uint64_t tile, uint
       for (int j = 0; j < kLookWide; ++j) {
         const int64_t at = hi - j * 32 - lane;
         w[j] = at >= 0 ? ld_tile(state + at) : tile_word(0, kTileIncl, 0);
+        flag[j] = tile_flag(w[j], 0);
+        if (kWide) {
+          const uint64_t r = at >= 0 ? ld_tile(rest + at) : tile_rest(kTileIncl, 0);
+          flag[j] = tile_pair_flag(w[j], r);
+          w[j] = tile_pair_value(w[j], r);
+        }
       }
 #pragma unroll
       for (int j = 0; j < kLookWide; ++j) {
-        const uint32_t f = tile_flag(w[j], 0);
-        ready = ready && f != 0;
-        bad = bad || f == kTilePoison;
+        ready = ready && flag[j] != 0;
+        bad = bad || flag[j] == kTilePoison;
       }
       if (__any_sync(0xffffffffu, bad) || __all_sync(0xffffffffu, ready)) break;
       if (++spins > kLookbackSpins) {
@@ -85,7 +113,7 @@ __device__ __forceinline__ bool tile_prefix(uint64_t *state, uint64_t tile, uint
     if (__any_sync(0xffffffffu, bad)) {
       if (lane == 0) {
         atomicCAS(err, 0u, (uint32_t)kDevLookbackTimeout);
-        st_tile(state + tile, tile_word(0, kTilePoison, 0));
+        publish(kTilePoison, 0);
       }
       return false;
     }
@@ -94,9 +122,9 @@ __device__ __forceinline__ bool tile_prefix(uint64_t *state, uint64_t tile, uint
     uint64_t v = 0;
 #pragma unroll
     for (int j = 0; j < kLookWide; ++j) {
-      const uint32_t incl = __ballot_sync(0xffffffffu, tile_flag(w[j], 0) == kTileIncl);
+      const uint32_t incl = __ballot_sync(0xffffffffu, flag[j] == kTileIncl);
       const uint32_t last = incl ? __ffs(incl) - 1 : 31;
-      if (!found && lane <= last) v += w[j] & kTileValueMask;
+      if (!found && lane <= last) v += kWide ? w[j] : w[j] & kTileValueMask;
       found = found || incl;
     }
 #pragma unroll
@@ -104,7 +132,7 @@ __device__ __forceinline__ bool tile_prefix(uint64_t *state, uint64_t tile, uint
     sum += v;
     if (found) break;
   }
-  if (lane == 0) st_tile(state + tile, tile_word(0, kTileIncl, sum + agg));
+  publish(kTileIncl, sum + agg);
   *excl = sum;
   return true;
 }
@@ -144,6 +172,10 @@ __device__ __forceinline__ T block_inclusive_scan(T v, T *smem_warp, T *total) {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanChunk = kScanThreads * kScanItems;
+// A 64-bit input is summed in 64 bits (wedges); 32-bit ones are flags,
+// buckets or columns, whose sums stay below 2^48.
+template <typename InT>
+constexpr bool kScanWide = sizeof(InT) == 8;
 
 // out[i] = exclusive prefix of in, out[n] = total, in one pass, the tile's
 // offset by look-back (state null: a single tile). Item j of lane l is
@@ -154,8 +186,8 @@ constexpr int kScanChunk = kScanThreads * kScanItems;
 // saves the host two launches of three.
 template <typename InT, typename OutT>
 __global__ void __launch_bounds__(kScanThreads)
-    k_scan(const InT *in, uint64_t n, OutT *out, uint64_t *state, uint32_t *ticket,
-           uint32_t *err) {
+    k_scan(const InT *in, uint64_t n, OutT *out, uint64_t *state, uint64_t *rest,
+           uint32_t *ticket, uint32_t *err) {
   __shared__ OutT s_warp[kScanThreads / 32];
   __shared__ uint64_t s_excl;
   __shared__ uint32_t s_tile, s_ok;
@@ -197,7 +229,7 @@ __global__ void __launch_bounds__(kScanThreads)
   if (state) {
     if (warp == 0) {
       uint64_t excl = 0;
-      const bool ok = tile_prefix(state, tile, (uint64_t)total, err, &excl);
+      const bool ok = tile_prefix<kScanWide<InT>>(state, rest, tile, (uint64_t)total, err, &excl);
       if (lane == 0) {
         s_excl = excl;
         s_ok = ok;
@@ -224,15 +256,17 @@ int exclusive_scan(DeviceContext *ctx, cudaStream_t st, const InT *in,
                    OutT *out, uint64_t n, uint32_t *err) {
   const uint64_t tiles = n == 0 ? 1 : ceil_div(n, kScanChunk);
   if (tiles == 1) {
-    k_scan<InT, OutT><<<1, kScanThreads, 0, st>>>(in, n, out, nullptr, nullptr, err);
+    k_scan<InT, OutT><<<1, kScanThreads, 0, st>>>(in, n, out, nullptr, nullptr, nullptr, err);
     WETRIC_LAUNCH_CHECK();
     return WETRIC_OK;
   }
-  Scratch<uint64_t> state;  // [0] the ticket, then one word per tile
-  WETRIC_TRY(state.alloc(ctx, st, tiles + 1));
-  WETRIC_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (tiles + 1) * sizeof(uint64_t), st));
+  Scratch<uint64_t> state;  // [0] the ticket, then one or two words per tile
+  const uint64_t words = 1 + (kScanWide<InT> ? 2 : 1) * tiles;
+  WETRIC_TRY(state.alloc(ctx, st, words));
+  WETRIC_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, words * sizeof(uint64_t), st));
   k_scan<InT, OutT><<<(unsigned)tiles, kScanThreads, 0, st>>>(
-      in, n, out, state.ptr + 1, reinterpret_cast<uint32_t *>(state.ptr), err);
+      in, n, out, state.ptr + 1, state.ptr + 1 + tiles, reinterpret_cast<uint32_t *>(state.ptr),
+      err);
   WETRIC_LAUNCH_CHECK();
   return WETRIC_OK;
 }
