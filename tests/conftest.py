@@ -73,15 +73,24 @@ def wetric_mod():
     return wetric
 
 
-@pytest.fixture(scope="session")
-def probe(wetric_mod, tmp_path_factory):
-    """tests/kernel_probe.cu, compiled beside the library it links to."""
-    lib = tmp_path_factory.mktemp("probe") / "libprobe.so"
+def build_probe(tmp, name):
+    """tests/<name>.cu as a library of its own, linked to libwetric.so."""
+    lib = tmp / f"lib{name}.so"
     subprocess.check_call(
         [os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-gencode",
          "arch=compute_100a,code=sm_100a", "-ccbin", "/usr/bin/g++", "-std=c++17", "-O2",
          "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-shared", "-cudart", "static",
          "-I", os.path.join(PKG, "csrc"), "-o", str(lib),
-         os.path.join(ROOT, "tests", "kernel_probe.cu"), "-L", os.path.join(PKG, "wetric"),
+         os.path.join(ROOT, "tests", f"{name}.cu"), "-L", os.path.join(PKG, "wetric"),
          "-lwetric", "-Xlinker", "-rpath," + os.path.join(PKG, "wetric")])
     return ctypes.CDLL(str(lib))
+
+
+@pytest.fixture(scope="session")
+def probe(wetric_mod, tmp_path_factory):
+    return build_probe(tmp_path_factory.mktemp("probe"), "kernel_probe")
+
+
+@pytest.fixture(scope="session")
+def preprocess_probe(wetric_mod, tmp_path_factory):
+    return build_probe(tmp_path_factory.mktemp("probe"), "preprocess_probe")

@@ -1,6 +1,9 @@
 // Device code of the library as tests call it: the words that look-back
-// scans publish, and scans of given values.
+// scans publish, scans of given values, and the kernels that follow a scan or
+// a sort, run with a given error word.
+#include "pair_streams.cuh"
 #include "primitives.cuh"
+#include "walk.cuh"
 
 using namespace wetric;
 
@@ -31,5 +34,71 @@ extern "C" int probe_scan_u64(const uint64_t *in, uint64_t n, uint64_t *out, uin
   PROBE(cudaMemsetAsync(e.ptr, 0, 4, ctx->stream));
   PROBE((prim::exclusive_scan<uint64_t, uint64_t>(ctx, ctx->stream, in, out, n, e.ptr)));
   PROBE(cudaMemcpyAsync(err, e.ptr, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  return (int)cudaStreamSynchronize(ctx->stream);
+}
+
+// The rest take device arrays and the device error word *err.
+
+// keys[0..n) sorted on their bits [0, bits) into out, by way of a and b.
+extern "C" int probe_sort(const uint64_t *keys, uint64_t n, uint32_t bits, uint64_t *a,
+                          uint64_t *b, uint64_t *out, uint32_t *err) {
+  DeviceContext *ctx = nullptr;
+  PROBE(get_context(0, &ctx));
+  const prim::KeysFrom from{keys};
+  PROBE((prim::radix_sort_into(ctx, ctx->stream, from, from, a, b, prim::KeysTo{out}, n, 0, bits,
+                               err)));
+  return (int)cudaStreamSynchronize(ctx->stream);
+}
+
+// The kernels behind the scans of the wedge-check path; every output is an
+// element of `out` (room for 4 n each).
+extern "C" int probe_after_scan(const uint32_t *rp, uint64_t n, const uint32_t *active,
+                                const uint64_t *pos, uint64_t *out, const uint32_t *err) {
+  DeviceContext *ctx = nullptr;
+  PROBE(get_context(0, &ctx));
+  uint64_t *wp = out, *rb = out + n;
+  k_compact_active<uint32_t><<<8, 256, 0, ctx->stream>>>(
+      rp, n, active, pos, wp, rb, reinterpret_cast<uint32_t *>(out + 2 * n), err);
+  CoreStarts cs{};
+  cs.v0[cs.c++] = n / 2;
+  k_core_prefix<<<1, 32, 0, ctx->stream>>>(wp, pos, cs, out + 3 * n, err);
+  ChunkRows rows{};
+  rows.v[rows.c++] = n / 2;
+  k_chunk_prefix<<<1, 32, 0, ctx->stream>>>(wp, pos, rows, out + 3 * n + 2, err);
+  PROBE(cudaGetLastError());
+  return (int)cudaStreamSynchronize(ctx->stream);
+}
+
+// The walk behind its sort: `keys` are m sorted entries, one per middle
+// vertex x = 0, 1, ... (its column row[x]), tails of one column each.
+extern "C" int probe_walk(const uint32_t *rp, const uint32_t *split, const uint32_t *long_rows,
+                          const uint32_t *ci, uint64_t m, const uint64_t *keys, uint32_t entries,
+                          uint32_t rows, uint32_t bits_start, uint32_t bits_len, uint32_t *start,
+                          uint32_t *items, uint32_t *counts, unsigned long long *out,
+                          const uint32_t *err) {
+  DeviceContext *ctx = nullptr;
+  PROBE(get_context(0, &ctx));
+  const WalkBits bits{1, bits_start, bits_len};
+  uint2 *big = reinterpret_cast<uint2 *>(items), *small = big + 2 * rows;
+  k_walk_starts<<<1, kWalkBlock, 0, ctx->stream>>>(keys, entries, 2 * rows, bits.shift(), start,
+                                                   err);
+  k_walk_plan<<<1, kWalkBlock, 0, ctx->stream>>>(rp, split, long_rows, start, 2 * rows, big, small,
+                                                 counts, err);
+  k_walk_count<kWalkSmallBlock, kWalkSmallBlocks, false><<<4, kWalkSmallBlock, 0, ctx->stream>>>(
+      rp, split, long_rows, walk_columns(ci, m), 0, keys, start, bits, small, counts + 1,
+      counts + 2, 0, out, WalkGroups{}, nullptr, err);
+  PROBE(cudaGetLastError());
+  return (int)cudaStreamSynchronize(ctx->stream);
+}
+
+// A vertex of two columns counted by pair streams (one tile of all columns).
+extern "C" int probe_pairs(const uint32_t *rp, const uint32_t *ci, const uint32_t *pv,
+                           const uint64_t *ps, const uint32_t *tile_k, uint64_t cols,
+                           unsigned long long *total, const uint32_t *err) {
+  DeviceContext *ctx = nullptr;
+  PROBE(get_context(0, &ctx));
+  k_count_pairs<false><<<1, kPairWarps * 32, 0, ctx->stream>>>(rp, ci, pv, ps, nullptr, 1, tile_k,
+                                                               1, cols, total, nullptr, err);
+  PROBE(cudaGetLastError());
   return (int)cudaStreamSynchronize(ctx->stream);
 }

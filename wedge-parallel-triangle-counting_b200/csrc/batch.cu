@@ -682,6 +682,17 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
   }
   WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, active.ptr,
                                                        pos.ptr, NT, err.ptr)));
+  // Read at every wait behind a scan, before its values are used.
+  uint32_t herr = 0;
+  auto read_err = [&]() {
+    return cudaMemcpyAsync(&herr, err.ptr, 4, cudaMemcpyDeviceToHost, st);
+  };
+  auto scans_done = [&]() -> int {
+    if (herr == kDevOk) return WETRIC_OK;
+    const int code = herr == kDevLookbackTimeout ? WETRIC_ETIMEDOUT : WETRIC_EINVAL;
+    set_error(code, "batch rows (device code %u)", herr);
+    return code;
+  };
   uint64_t K = 0, Kp = 0;
   unsigned long long maxdeg = 0, Wp = 0;
   WETRIC_CUDA_TRY(cudaMemcpyAsync(&K, pos.ptr + NT, 8, cudaMemcpyDeviceToHost, st));
@@ -691,7 +702,9 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
     WETRIC_CUDA_TRY(cudaMemcpyAsync(&Kp, ppos.ptr + NT, 8, cudaMemcpyDeviceToHost, st));
     WETRIC_CUDA_TRY(cudaMemcpyAsync(pacc, pw.ptr, 24, cudaMemcpyDeviceToHost, st));
   }
+  WETRIC_CUDA_TRY(read_err());
   WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  WETRIC_TRY(scans_done());
   if (maxdeg >= (1ull << 30)) {
     set_error(WETRIC_ERANGE, "max out-degree %llu >= 2^30", maxdeg);
     return WETRIC_ERANGE;
@@ -728,7 +741,9 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
     WETRIC_CUDA_TRY(cudaMemcpyAsync(&Rp, b->ps.ptr + Kp, 8, cudaMemcpyDeviceToHost, st));
     WETRIC_CUDA_TRY(cudaMemcpyAsync(b->pair_w.data(), gw.ptr, G * 8ull,
                                     cudaMemcpyDeviceToHost, st));
+    WETRIC_CUDA_TRY(read_err());
     WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+    WETRIC_TRY(scans_done());
     const uint64_t Tp = pair_tile_cols(Rp, ctx->sm_count);
     b->ptile_cols = Tp;
     b->ptiles = Rp ? ceil_div(Rp, Tp) : 0;
@@ -750,11 +765,11 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
     if (b->off32)
       k_compact_active<uint32_t><<<grid_for(ctx, NT), 256, 0, st>>>(
           b->rp32.ptr, NT, active.ptr, pos.ptr, b->act_wp.ptr, b->act_rb.ptr,
-          b->act_d.ptr);
+          b->act_d.ptr, err.ptr);
     else
       k_compact_active<uint64_t><<<grid_for(ctx, NT), 256, 0, st>>>(
           b->csr.row_ptr, NT, active.ptr, pos.ptr, b->act_wp.ptr,
-          b->act_rb.ptr, b->act_d.ptr);
+          b->act_rb.ptr, b->act_d.ptr, err.ptr);
     WETRIC_LAUNCH_CHECK();
     k_active_graph<<<grid_for(ctx, NT), 256, 0, st>>>(
         active.ptr, NT, pos.ptr, d_vbase.ptr, G, b->act_g.ptr);
@@ -770,7 +785,9 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
   b->wbase.assign(G + 1, 0);
   WETRIC_CUDA_TRY(cudaMemcpyAsync(b->wbase.data(), d_wbase.ptr, (G + 1) * 8,
                                   cudaMemcpyDeviceToHost, st));
+  WETRIC_CUDA_TRY(read_err());
   WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  WETRIC_TRY(scans_done());
   b->W = b->wbase[G];
   active.release();
   pos.release();
@@ -840,15 +857,11 @@ int batch_create(DeviceContext *ctx, const uint32_t *src, const uint32_t *dst,
     WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, nb.ptr,
                                                          b->hoff.ptr, NT, err.ptr)));
     uint64_t buckets = 0;
-    uint32_t herr = 0;
     WETRIC_CUDA_TRY(cudaMemcpyAsync(&buckets, b->hoff.ptr + NT, 8,
                                     cudaMemcpyDeviceToHost, st));
-    WETRIC_CUDA_TRY(cudaMemcpyAsync(&herr, err.ptr, 4, cudaMemcpyDeviceToHost, st));
+    WETRIC_CUDA_TRY(read_err());
     WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
-    if (herr == kDevLookbackTimeout) {
-      set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
-      return WETRIC_ETIMEDOUT;
-    }
+    WETRIC_TRY(scans_done());
     nb.release();
     // The sets stay resident with the batch: take at most half of the
     // device memory that is free now.
@@ -935,7 +948,7 @@ static int batch_enqueue(Batch *b, cudaStream_t st, uint32_t *launches) {
     // the walk's item counters (counts[3], counts[4])
     WETRIC_CUDA_TRY(cudaMemsetAsync(w.run.counts.ptr + 3, 0, 2 * sizeof(uint32_t), st));
     return w.run.count<true>(ctx, st, b->rp32.ptr, b->csr.col_ind, w.long_rows.ptr,
-                             b->opt.persistent, nullptr, &most, launches, groups,
+                             b->opt.persistent, nullptr, err, &most, launches, groups,
                              w.long_graph.ptr);
   }
   WETRIC_CUDA_TRY(cudaMemsetAsync(b->total.ptr, 0, 8, st));

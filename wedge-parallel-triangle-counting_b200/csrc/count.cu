@@ -182,7 +182,7 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
   WETRIC_TRY(act_d.alloc(ctx, st, n));
   WETRIC_CUDA_TRY(cudaMemsetAsync(act_wp.ptr, 0, (n + 1) * sizeof(uint64_t), st));
   k_compact_active<Off><<<grid_for(ctx, n), 256, 0, st>>>(
-      rp, n, active.ptr, pos.ptr, act_wp.ptr, act_rb.ptr, act_d.ptr);
+      rp, n, active.ptr, pos.ptr, act_wp.ptr, act_rb.ptr, act_d.ptr, small.ptr);
   WETRIC_LAUNCH_CHECK();
   ++launches;
   WETRIC_TRY((prim::exclusive_scan<uint64_t, uint64_t>(ctx, st, act_wp.ptr,
@@ -253,7 +253,7 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
       push(a.core_len < kCoreMaxLen ? a.core_len : kCoreMaxLen);
     }
     WETRIC_TRY(cstart.alloc(ctx, st, 2 * (2 * kCoreNumCandidates + 2)));
-    k_core_prefix<<<1, 32, 0, st>>>(act_wp.ptr, pos.ptr, cs, cstart.ptr);
+    k_core_prefix<<<1, 32, 0, st>>>(act_wp.ptr, pos.ptr, cs, cstart.ptr, small.ptr);
     WETRIC_LAUNCH_CHECK();
     ++launches;
   }
@@ -266,7 +266,7 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
     for (uint32_t i = 0; i < C_in; ++i) cr.v[i] = a.chunk_lo[i];
     cr.c = C_in;
     WETRIC_TRY(cpre.alloc(ctx, st, kMaxColChunks));
-    k_chunk_prefix<<<1, 32, 0, st>>>(act_wp.ptr, pos.ptr, cr, cpre.ptr);
+    k_chunk_prefix<<<1, 32, 0, st>>>(act_wp.ptr, pos.ptr, cr, cpre.ptr, small.ptr);
     WETRIC_LAUNCH_CHECK();
     ++launches;
   }
@@ -619,7 +619,7 @@ int count_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
     WETRIC_CUDA_TRY(cudaEventRecord(ev_pair.a, st));
     k_count_pairs<false><<<(unsigned)ceil_div(ptiles, kPairWarps), kPairWarps * 32, 0, st>>>(
         reinterpret_cast<const uint32_t *>(rp), a.col_ind, pv.ptr, ps.ptr, nullptr, Kp,
-        ptile.ptr, ptiles, Tp, acc.ptr + 1, nullptr);
+        ptile.ptr, ptiles, Tp, acc.ptr + 1, nullptr, small.ptr);
     WETRIC_LAUNCH_CHECK();
     WETRIC_CUDA_TRY(cudaEventRecord(ev_pair.b, st));
     launches += 5;
@@ -893,6 +893,10 @@ static int wedge_total_impl(DeviceContext *ctx, cudaStream_t st,
   WETRIC_CUDA_TRY(cudaMemcpyAsync(&herr, err.ptr, sizeof(uint32_t),
                                   cudaMemcpyDeviceToHost, st));
   WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  if (herr == kDevLookbackTimeout) {
+    set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
+    return WETRIC_ETIMEDOUT;
+  }
   if (herr != kDevOk) {
     set_error(WETRIC_EINVAL, "row offsets check failed (device code %u)", herr);
     return WETRIC_EINVAL;
@@ -904,7 +908,7 @@ static int wedge_total_impl(DeviceContext *ctx, cudaStream_t st,
   WETRIC_TRY(act_d.alloc(ctx, st, K));
   if (K > 0) {
     k_compact_active<Off><<<grid_for(ctx, n), 256, 0, st>>>(
-        rp, n, active.ptr, wc.ptr, act_wp.ptr, act_rb.ptr, act_d.ptr);
+        rp, n, active.ptr, wc.ptr, act_wp.ptr, act_rb.ptr, act_d.ptr, err.ptr);
     WETRIC_LAUNCH_CHECK();
   }
   WETRIC_TRY((prim::exclusive_scan<uint64_t, uint64_t>(ctx, st, act_wp.ptr,

@@ -135,7 +135,9 @@ __global__ void k_compact_active(const Off *__restrict__ rp, uint64_t n,
                                  const uint64_t *__restrict__ pos,
                                  uint64_t *__restrict__ act_wc,
                                  uint64_t *__restrict__ act_rb,
-                                 uint32_t *__restrict__ act_d) {
+                                 uint32_t *__restrict__ act_d,
+                                 const uint32_t *__restrict__ err) {
+  if (*err != kDevOk) return;  // the scan that made pos may have run out
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
        v += (uint64_t)gridDim.x * blockDim.x) {
     if (active[v]) {
@@ -157,7 +159,8 @@ struct ChunkRows {
 };
 __global__ void k_chunk_prefix(const uint64_t *__restrict__ act_wp,
                                const uint64_t *__restrict__ pos, ChunkRows rows,
-                               uint64_t *__restrict__ out) {
+                               uint64_t *__restrict__ out, const uint32_t *__restrict__ err) {
+  if (*err != kDevOk) return;
   const uint32_t i = threadIdx.x;
   if (i < rows.c) out[i] = act_wp[pos[rows.v[i]]];
 }
@@ -1553,7 +1556,8 @@ struct CoreStarts {
 };
 __global__ void k_core_prefix(const uint64_t *__restrict__ act_wp,
                               const uint64_t *__restrict__ pos, CoreStarts cs,
-                              uint64_t *__restrict__ out) {
+                              uint64_t *__restrict__ out, const uint32_t *__restrict__ err) {
+  if (*err != kDevOk) return;
   const uint32_t i = threadIdx.x;
   if (i < cs.c) {
     const uint64_t k = pos[cs.v0[i]];

@@ -350,7 +350,7 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
       WETRIC_TRY(walk.sort(ctx, st, rp32, long_rows.ptr, entries, err, &launches));
       WETRIC_TRY(ev_walk.start(st));
       WETRIC_TRY(walk.count(ctx, st, rp32, a.col_ind, long_rows.ptr, a.persistent, words.ptr,
-                            &grid, &launches));
+                            err, &grid, &launches));
       WETRIC_TRY(ev_walk.stop(st));
     }
   }

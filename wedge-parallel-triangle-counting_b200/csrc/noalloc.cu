@@ -216,7 +216,7 @@ int count_noalloc_impl(int device, cudaStream_t st, const Off *rp,
   if (!act_wp || !act_rb || !act_d) return too_big();
   if (K > 0) {
     k_compact_active<Off><<<grid_cap(sms, n), 256, 0, st>>>(rp, n, active, pos, act_wp,
-                                                           act_rb, act_d);
+                                                           act_rb, act_d, small);
     WETRIC_LAUNCH_CHECK();
   }
   WETRIC_TRY((scan_in_arena<uint64_t, uint64_t>(&ar, st, act_wp, act_wp, K, small, &look)));

@@ -199,7 +199,9 @@ __global__ void __launch_bounds__(kPairWarps * 32, 8)
                   const uint32_t *__restrict__ pg, uint64_t Kp,
                   const uint32_t *__restrict__ tile_k, uint64_t tiles, uint64_t T,
                   unsigned long long *__restrict__ total,
-                  unsigned long long *__restrict__ counts) {
+                  unsigned long long *__restrict__ counts,
+                  const uint32_t *__restrict__ err = nullptr) {
+  if (err && *err != kDevOk) return;  // the scan that made ps may have run out
   __shared__ uint32_t s_set[kPairWarps][kPairSlots];
   // entry e: column index of its stream position 0 (row start minus stream
   // start, mod 2^32: position q reads column s_off[e] + q) and its start

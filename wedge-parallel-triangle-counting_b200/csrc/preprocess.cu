@@ -228,7 +228,9 @@ struct BothDirections {
 constexpr uint32_t kGapByThread = 8;
 __global__ void __launch_bounds__(kThreads)
     k_keys_to_csr(const uint64_t *__restrict__ keys, uint64_t m, uint64_t n, uint32_t b,
-                  uint64_t *__restrict__ rp, uint32_t *__restrict__ ci) {
+                  uint64_t *__restrict__ rp, uint32_t *__restrict__ ci,
+                  const uint32_t *__restrict__ err) {
+  if (*err != kDevOk) return;  // the keys may not be there
   __shared__ uint32_t s_from[kThreads], s_to[kThreads], s_gaps;
   const uint64_t mask = (1ull << b) - 1;
   const uint64_t gid = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -281,7 +283,9 @@ __global__ void k_row_lengths(const uint64_t *__restrict__ rp, uint64_t n,
 __global__ void k_kept_per_row(const uint64_t *__restrict__ rp,
                                const uint32_t *__restrict__ ci, uint64_t n,
                                const uint32_t *__restrict__ rank,
-                               uint32_t *__restrict__ kept, uint64_t *__restrict__ most) {
+                               uint32_t *__restrict__ kept, uint64_t *__restrict__ most,
+                               const uint32_t *__restrict__ err) {
+  if (*err != kDevOk) return;  // the ranks may not be there
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -496,12 +500,12 @@ int degree_rank(DeviceContext *ctx, cudaStream_t st, const uint32_t *deg, uint64
 // Sorted packed (row, col) keys -> CSR arrays.
 int keys_to_csr(DeviceContext *ctx, cudaStream_t st, const uint64_t *keys,
                 uint64_t m, uint64_t n, uint32_t b, uint64_t *row_ptr,
-                uint32_t *col_ind) {
+                uint32_t *col_ind, const uint32_t *err) {
   if (m == 0) {
     WETRIC_CUDA_TRY(cudaMemsetAsync(row_ptr, 0, (n + 1) * sizeof(uint64_t), st));
     return WETRIC_OK;
   }
-  k_keys_to_csr<<<grid_for(ctx, m), kThreads, 0, st>>>(keys, m, n, b, row_ptr, col_ind);
+  k_keys_to_csr<<<grid_for(ctx, m), kThreads, 0, st>>>(keys, m, n, b, row_ptr, col_ind, err);
   WETRIC_LAUNCH_CHECK();
   return WETRIC_OK;
 }
@@ -651,7 +655,7 @@ int orient_pairs(DeviceContext *ctx, cudaStream_t st, const uint32_t *src,
       ukeys.ptr, okeys.ptr, prim::KeysTo{sorted}, m, 0, 2 * b, err, &space.last)));
   rank.release();
   WETRIC_TRY(alloc_csr(ctx, st, n, m, out));
-  WETRIC_TRY(keys_to_csr(ctx, st, sorted, m, n, b, out->row_ptr, out->col_ind));
+  WETRIC_TRY(keys_to_csr(ctx, st, sorted, m, n, b, out->row_ptr, out->col_ind, err));
   return checked_words(st, words.ptr, "orientation", &h);
 }
 
@@ -699,7 +703,8 @@ int symmetric_from_pairs(DeviceContext *ctx, cudaStream_t st,
   ukeys.release();
   WETRIC_TRY(alloc_csr(ctx, st, n, 2 * m, out));
   WETRIC_TRY(
-      keys_to_csr(ctx, st, sorted, 2 * m, n, b, out->row_ptr, out->col_ind));
+      keys_to_csr(ctx, st, sorted, 2 * m, n, b, out->row_ptr, out->col_ind,
+                  &words.ptr->err));
   return checked_words(st, words.ptr, "symmetric CSR", &h);
 }
 
@@ -734,7 +739,8 @@ int orient_csr(DeviceContext *ctx, cudaStream_t st, const uint64_t *rp,
   // deg is reused as the kept count of every oriented row.
   const unsigned warps_grid = grid_for(ctx, n * 32);
   WETRIC_CUDA_TRY(cudaMemsetAsync(&words.ptr->maxdeg, 0, sizeof(uint64_t), st));
-  k_kept_per_row<<<warps_grid, 256, 0, st>>>(rp, ci, n, rank.ptr, deg.ptr, &words.ptr->maxdeg);
+  k_kept_per_row<<<warps_grid, 256, 0, st>>>(rp, ci, n, rank.ptr, deg.ptr, &words.ptr->maxdeg,
+                                          err);
   WETRIC_LAUNCH_CHECK();
   Scratch<uint64_t> off;
   WETRIC_TRY(off.alloc(ctx, st, n + 1));
@@ -767,7 +773,7 @@ int orient_csr(DeviceContext *ctx, cudaStream_t st, const uint64_t *rp,
                                     prim::KeysTo{sorted}, kept, 0, 2 * b, err)));
   WETRIC_TRY(alloc_csr(ctx, st, n, kept, out));
   WETRIC_TRY(
-      keys_to_csr(ctx, st, sorted, kept, n, b, out->row_ptr, out->col_ind));
+      keys_to_csr(ctx, st, sorted, kept, n, b, out->row_ptr, out->col_ind, err));
   return checked_words(st, words.ptr, "csr", &h);
 }
 

@@ -10,7 +10,13 @@
 // Tickets are handed out in order to running blocks, so a block only ever
 // waits on blocks that are already running. Every wait is bounded all the
 // same: on running out it records kDevLookbackTimeout, publishes a poison
-// word that ends its successors' waits, and the block leaves.
+// word that ends its successors' waits, and the block leaves. What such a
+// pass leaves is not complete, and kernels behind it may be queued already:
+// those that index with it look at the error word first and leave. In a pass
+// with a look-back the first tile looks: every other one waits for a word
+// that follows from the first's, so its poison keeps all of them from writing
+// (orientation of R-MAT scale 22: without any look 7.03-7.07 ms, this way
+// 7.08, by every block 7.12).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -76,8 +82,11 @@ __device__ __forceinline__ bool tile_prefix(uint64_t *state, uint64_t *rest, uin
   };
   *excl = 0;
   if (tile == 0) {
-    publish(kTileIncl, agg);
-    return true;
+    uint32_t on = 1;
+    if (lane == 0) on = *err == kDevOk;
+    on = __shfl_sync(0xffffffffu, on, 0);
+    publish(on ? kTileIncl : kTilePoison, agg);
+    return on;
   }
   publish(kTileAgg, agg);
   uint64_t sum = 0;
@@ -335,11 +344,12 @@ constexpr int kHistAhead = 4;
 template <class Load>
 __global__ void __launch_bounds__(256)
     k_radix_hist(Load load, uint64_t n, const __grid_constant__ DigitPlan plan,
-                 unsigned long long *__restrict__ hist) {
+                 unsigned long long *__restrict__ hist, const uint32_t *err) {
   extern __shared__ uint32_t s_hist[];  // [pass][digit][copy]
   const uint32_t total = plan.passes * kRadix * kHistCopies;
   for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) s_hist[i] = 0;
-  __syncthreads();
+  // (load itself may set the word, hence one verdict per block)
+  if (__syncthreads_or(*err != kDevOk)) return;
   const uint32_t copy = threadIdx.x & (kHistCopies - 1);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -498,8 +508,10 @@ __global__ void __launch_bounds__(kSortThreads, kSortBlocks)
     const unsigned long long i64 =
         block_inclusive_scan<kSortThreads, unsigned long long>(h, s_warp64, &t64);
     if (threadIdx.x < kRadix) {
-      st_tile(word, tile_word(epoch, kTileIncl, i64 - h + c));
+      const bool on = *err == kDevOk;  // else the keys may not be there
+      st_tile(word, tile_word(epoch, on ? kTileIncl : kTilePoison, i64 - h + c));
       s_goff[threadIdx.x] = i64 - h - (incl - c);
+      if (!on) s_bad = 1;
     }
   } else if (threadIdx.x < kRadix) {
     uint64_t sum = 0;
@@ -639,7 +651,7 @@ int radix_sort_into(DeviceContext *ctx, cudaStream_t st, const Counted &counted,
   const uint64_t cap = (uint64_t)ctx->sm_count * 8;
   if (blocks > cap) blocks = cap;
   const size_t hs = (size_t)plan.passes * kRadix * kHistCopies * sizeof(uint32_t);
-  k_radix_hist<Counted><<<(unsigned)blocks, 256, hs, st>>>(counted, n, plan, ws.hist);
+  k_radix_hist<Counted><<<(unsigned)blocks, 256, hs, st>>>(counted, n, plan, ws.hist, err);
   WETRIC_LAUNCH_CHECK();
   if (plan.passes == 1) return onesweep_pass(st, first, sink, n, plan, 0, ws, err);
   WETRIC_TRY((onesweep_pass(st, first, KeysTo{a}, n, plan, 0, ws, err)));

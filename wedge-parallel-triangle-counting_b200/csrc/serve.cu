@@ -283,7 +283,8 @@ int serve_prepare(DeviceContext *ctx, cudaStream_t st, uint32_t spread,
   WETRIC_TRY(p->act_d.alloc(ctx, st, n));
   WETRIC_CUDA_TRY(cudaMemsetAsync(p->act_wp.ptr, 0, (n + 1) * sizeof(uint64_t), st));
   k_compact_active<uint32_t><<<grid_for(ctx, n), 256, 0, st>>>(
-      rp, n, active.ptr, pos.ptr, p->act_wp.ptr, p->act_rb.ptr, p->act_d.ptr);
+      rp, n, active.ptr, pos.ptr, p->act_wp.ptr, p->act_rb.ptr, p->act_d.ptr,
+      small.ptr);
   WETRIC_LAUNCH_CHECK();
   WETRIC_TRY((prim::exclusive_scan<uint64_t, uint64_t>(ctx, st, p->act_wp.ptr,
                                                        p->act_wp.ptr, n, small.ptr)));
@@ -328,7 +329,8 @@ int serve_prepare(DeviceContext *ctx, cudaStream_t st, uint32_t spread,
       cs.v0[cs.c++] = n - h;  // no shell: the wedge checks are faster there
     }
     WETRIC_TRY(cstart.alloc(ctx, st, 2 * cs.c));
-    k_core_prefix<<<1, 32, 0, st>>>(p->act_wp.ptr, pos.ptr, cs, cstart.ptr);
+    k_core_prefix<<<1, 32, 0, st>>>(p->act_wp.ptr, pos.ptr, cs, cstart.ptr,
+                                  small.ptr);
     WETRIC_LAUNCH_CHECK();
   }
   unsigned long long plan[2 * kCoreNumCandidates] = {};

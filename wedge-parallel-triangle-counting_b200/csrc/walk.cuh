@@ -248,7 +248,8 @@ __global__ void __launch_bounds__(kWalkBlock)
 // A lane fills a gap of up to 8 vertices, the warp a longer one.
 __global__ void __launch_bounds__(kWalkBlock)
     k_walk_starts(const uint64_t *__restrict__ keys, uint32_t m, uint32_t n, uint32_t shift,
-                  uint32_t *__restrict__ start) {
+                  uint32_t *__restrict__ start, const uint32_t *__restrict__ err) {
+  if (*err != kDevOk) return;  // the sort may have run out
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t stride = (uint64_t)gridDim.x * kWalkBlock;
   const uint64_t gid = (uint64_t)blockIdx.x * kWalkBlock + threadIdx.x;
@@ -290,7 +291,8 @@ __global__ void __launch_bounds__(kWalkBlock)
     k_walk_plan(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ split,
                 const uint32_t *__restrict__ long_rows, const uint32_t *__restrict__ start,
                 uint32_t x_end, uint2 *__restrict__ big, uint2 *__restrict__ small,
-                uint32_t *__restrict__ counts) {
+                uint32_t *__restrict__ counts, const uint32_t *__restrict__ err) {
+  if (*err != kDevOk) return;
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t stride = (uint64_t)gridDim.x * kWalkBlock;
   for (uint64_t x0 = (uint64_t)blockIdx.x * kWalkBlock + threadIdx.x - lane; x0 < x_end;
@@ -967,7 +969,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
                  const uint2 *__restrict__ items, const uint32_t *__restrict__ count,
                  uint32_t *__restrict__ ticket, uint32_t per_block,
                  unsigned long long *__restrict__ out, const __grid_constant__ WalkGroups groups,
-                 const uint32_t *__restrict__ long_graph) {
+                 const uint32_t *__restrict__ long_graph, const uint32_t *__restrict__ err) {
+  if (*err != kDevOk) return;
   struct Entry {
     uint32_t first, len;
   };
@@ -1169,11 +1172,11 @@ struct WalkRun {
                                       entries, bits.shift(), bits.w, err, &ws)));
     sorted = to;
     k_walk_starts<<<grid(ctx, entries), kWalkBlock, 0, st>>>(
-        sorted, (uint32_t)entries, (uint32_t)(2 * rows), bits.shift(), start.ptr);
+        sorted, (uint32_t)entries, (uint32_t)(2 * rows), bits.shift(), start.ptr, err);
     WETRIC_LAUNCH_CHECK();
     k_walk_plan<<<grid(ctx, 2 * rows), kWalkBlock, 0, st>>>(
         rp, split.ptr, long_rows, start.ptr, (uint32_t)(2 * rows), big.ptr, small.ptr,
-        counts.ptr + 1);
+        counts.ptr + 1, err);
     WETRIC_LAUNCH_CHECK();
     *launches += 3 + prim::digit_plan(bits.shift(), bits.w).passes;
     return WETRIC_OK;
@@ -1183,8 +1186,8 @@ struct WalkRun {
   // start at zero (alloc) and are the caller's to clear for another count.
   template <bool kBatch = false>
   int count(DeviceContext *ctx, cudaStream_t st, const uint32_t *rp, const uint32_t *ci,
-            const uint32_t *long_rows, bool persistent, unsigned long long *out, uint64_t *most,
-            uint32_t *launches, const WalkGroups &groups = WalkGroups{},
+            const uint32_t *long_rows, bool persistent, unsigned long long *out, const uint32_t *err,
+            uint64_t *most, uint32_t *launches, const WalkGroups &groups = WalkGroups{},
             const uint32_t *long_graph = nullptr) {
     constexpr uint32_t kPerBlock = 16;
     const auto big_fn = k_walk_count<kWalkBigBlock, kWalkBigBlocks, kBatch>;
@@ -1204,11 +1207,11 @@ struct WalkRun {
         small_fn, cudaFuncAttributePreferredSharedMemoryCarveout, kWalkCarveout));
     big_fn<<<(unsigned)g, kWalkBigBlock, 0, st>>>(
         rp, split.ptr, long_rows, cols, t0, sorted, start.ptr, bits, big.ptr, counts.ptr + 1,
-        counts.ptr + 3, persistent ? 0 : kPerBlock, out, groups, long_graph);
+        counts.ptr + 3, persistent ? 0 : kPerBlock, out, groups, long_graph, err);
     WETRIC_LAUNCH_CHECK();
     small_fn<<<(unsigned)gs, kWalkSmallBlock, 0, st>>>(
         rp, split.ptr, long_rows, cols, t0, sorted, start.ptr, bits, small.ptr, counts.ptr + 2,
-        counts.ptr + 4, persistent ? 0 : kPerBlock, out, groups, long_graph);
+        counts.ptr + 4, persistent ? 0 : kPerBlock, out, groups, long_graph, err);
     WETRIC_LAUNCH_CHECK();
     *launches += 2;
     if (g > *most) *most = g;
