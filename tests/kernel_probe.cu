@@ -102,3 +102,9 @@ extern "C" int probe_pairs(const uint32_t *rp, const uint32_t *ci, const uint32_
   PROBE(cudaGetLastError());
   return (int)cudaStreamSynchronize(ctx->stream);
 }
+
+// The form that counts a graph: 0 intersections, 1 with the walk, 2 neither.
+extern "C" int probe_walk_form(uint64_t n, uint64_t m, uint64_t edges, uint64_t long_rows,
+                               uint64_t longest, uint64_t long_wedges) {
+  return (int)walk_form(n, m, edges, long_rows, longest, long_wedges);
+}

@@ -441,7 +441,8 @@ static int autotune_spreads(Batch *b, std::vector<uint32_t> *sg, cudaStream_t st
 }
 
 // Rows and, where they pay, the long rows' entries of a batch counted by row
-// intersections and the walk; b->whole stays false when there is no room.
+// intersections and the walk; b->whole stays false when there is no room, or
+// entries would not fit their bits.
 static int make_whole(Batch *b, cudaStream_t st) {
   DeviceContext *ctx = b->ctx;
   const uint32_t G = b->G;
@@ -489,9 +490,11 @@ static int make_whole(Batch *b, cudaStream_t st) {
   b->max_out_degree = longest;
   b->Kp = rows;
   b->pair_wedges = b->W;
-  if (walk_wanted(long_rows, longest, long_w, m) && w->run.fits(n, m, long_rows, longest)) {
+  const WalkForm form = walk_form(n, m, m, long_rows, longest, long_w);
+  if (form == WalkForm::kNone) return WETRIC_OK;
+  if (form == WalkForm::kWalk) {
     WalkRun &run = w->run;
-    if (run.alloc(ctx, st, m + m / 4) != WETRIC_OK) {
+    if (run.alloc(ctx, st, n, m, long_rows, longest, m + m / 4) != WETRIC_OK) {
       clear_error();
       return WETRIC_OK;
     }

@@ -89,8 +89,8 @@ int count_oriented(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
                    CountResult *r);
 
 // The default count of a whole graph (count_whole.cu). count_oriented sends
-// the calls it takes there; *declined: not counted (no room, or too many
-// entries), the wedge-check path takes the call.
+// the calls it takes there; *declined: not counted (no room, entries that
+// would not fit their bits, or too many), the wedge-check path takes the call.
 bool count_whole_takes(const CountArgs &a);
 int count_whole(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
                 CountResult *r, bool *declined);

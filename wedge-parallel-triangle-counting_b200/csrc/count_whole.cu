@@ -244,13 +244,19 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
       core_rows = tot[kEdgeCand + 3 * pick + 2];
       r->core_len = (uint32_t)core_h;
     }
-    emit = walk_wanted(tot[3], tot[1], tot[4], below_m) && walk.fits(n, m, tot[3], tot[1]);
+    const WalkForm form = walk_form(n, m, below_m, tot[3], tot[1], tot[4]);
+    if (form == WalkForm::kNone) {
+      *declined = true;
+      return WETRIC_OK;
+    }
+    emit = form == WalkForm::kWalk;
     sets = row_sets_wanted(below_m, W - r->core_wedges, tot[1], emit ? tot[4] : 0);
     // Room for an entry per edge below the core and a quarter more: tails
     // with two entries are rare (they need a long row with more than 48
     // columns outside the window), and a graph with more of them starts over
     // on the wedge-check path.
-    if (emit && walk.alloc(ctx, st, below_m + below_m / 4) != WETRIC_OK) {
+    if (emit &&
+        walk.alloc(ctx, st, n, m, tot[3], tot[1], below_m + below_m / 4) != WETRIC_OK) {
       // no room for the walk: the wedge-check path counts (and searches
       // where it has no room for its sets)
       clear_error();

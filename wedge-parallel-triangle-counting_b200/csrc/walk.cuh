@@ -819,6 +819,28 @@ inline bool walk_wanted(uint64_t long_rows, uint64_t longest, uint64_t long_wedg
   return long_rows > 0 && edges >= kWalkMinEdges && (longest > 128 || long_wedges >= (1ull << 25));
 }
 
+// How an entry's fields lie when m columns, long_rows rows of up to `longest`
+// columns have to fit them; 64 bits or fewer in all, or there is no walk.
+inline WalkBits walk_bits(uint64_t m, uint64_t long_rows, uint64_t longest) {
+  return WalkBits{1 + (long_rows > 1 ? bits_for(long_rows - 1) : 1), bits_for(m),
+                  bits_for(longest)};
+}
+
+// What counts a graph (or batch) below its core: intersections alone, with
+// the walk, or neither -- the walk is wanted, so intersecting the long rows
+// edge by edge is the slower way by far, but its entries do not fit, as from
+// about 2^30 columns on in graphs with hubs: the wedge checks take it (R-MAT
+// scale 26, 1.05e9 columns, one bit too many: 584 ms a count, 2,917 when its
+// long rows were intersected).
+enum class WalkForm { kMerge, kWalk, kNone };
+inline WalkForm walk_form(uint64_t n, uint64_t m, uint64_t edges, uint64_t long_rows,
+                          uint64_t longest, uint64_t long_wedges) {
+  if (!walk_wanted(long_rows, longest, long_wedges, edges)) return WalkForm::kMerge;
+  const WalkBits b = walk_bits(m, long_rows, longest);
+  return n < (1ull << 31) && m < (1ull << 31) && b.w + b.start + b.len <= 64 ? WalkForm::kWalk
+                                                                             : WalkForm::kNone;
+}
+
 // Whether k_edge_merge counts by sets: a set pays when many wedges share it,
 // that is from some mean tail (wedges per edge) on. Measured, sets /
 // intersections in us: Erdos-Renyi, 6M edges, tail 4.2 207 / 192, 5.4 200 /
@@ -1137,18 +1159,13 @@ struct WalkRun {
     const uint64_t most = (uint64_t)ctx->sm_count * 32, g = ceil_div(threads, kWalkBlock);
     return (unsigned)(g == 0 ? 1 : g < most ? g : most);
   }
-  // Whether an entry fits 64 bits.
-  bool fits(uint64_t n_, uint64_t m_, uint64_t long_rows, uint64_t longest) {
+  // Room for `most` entries of a graph that walk_form has walked.
+  int alloc(DeviceContext *ctx, cudaStream_t st, uint64_t n_, uint64_t m_, uint64_t long_rows,
+            uint64_t longest, uint64_t most) {
     n = n_;
     m = m_;
     rows = long_rows;
-    bits.w = 1 + (rows > 1 ? bits_for(rows - 1) : 1);
-    bits.start = bits_for(m);
-    bits.len = bits_for(longest);
-    return n < (1ull << 31) && m < (1ull << 31) && bits.w + bits.start + bits.len <= 64;
-  }
-  // Room for `most` entries.
-  int alloc(DeviceContext *ctx, cudaStream_t st, uint64_t most) {
+    bits = walk_bits(m, rows, longest);
     cap = walk_room(most);
     const uint64_t room = walk_room(2 * rows);
     WETRIC_TRY(split.alloc(ctx, st, n));
