@@ -108,3 +108,13 @@ extern "C" int probe_walk_form(uint64_t n, uint64_t m, uint64_t edges, uint64_t 
                                uint64_t longest, uint64_t long_wedges) {
   return (int)walk_form(n, m, edges, long_rows, longest, long_wedges);
 }
+
+// One warp's hits, hits[lane] each, added to *sum (device).
+__global__ void add_hits(const unsigned long long *hits, unsigned long long *sum) {
+  walk_add_hits(sum, hits[threadIdx.x], threadIdx.x);
+}
+extern "C" int probe_add_hits(const unsigned long long *hits, unsigned long long *sum) {
+  add_hits<<<1, 32>>>(hits, sum);
+  PROBE(cudaGetLastError());
+  return (int)cudaDeviceSynchronize();
+}

@@ -29,3 +29,18 @@ def test_overlapping_rows_are_rejected(wetric_mod, dtype, n, m):
             assert e.value.status == 1, e.value
     # the device still counts
     assert wetric_mod.count(np.array([0, 2, 3, 3], np.uint64), np.array([1, 2, 2], np.uint32))[0] == 1
+
+
+@pytest.mark.parametrize("most", [0, 1, 1 << 27, (1 << 32) - 1, 1 << 40])
+def test_a_warps_hits_are_summed_in_64_bits(probe, wetric_mod, most):
+    import ctypes as C
+
+    import torch
+
+    hits = np.random.default_rng(1).integers(0, most + 1, 32)
+    hits[0] = most
+    d = torch.from_numpy(hits).cuda()
+    total = torch.full((1,), 5, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    assert probe.probe_add_hits(C.c_void_p(d.data_ptr()), C.c_void_p(total.data_ptr())) == 0
+    assert total.item() == 5 + int(hits.sum())

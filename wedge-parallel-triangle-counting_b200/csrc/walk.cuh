@@ -89,6 +89,15 @@ __device__ __forceinline__ uint32_t walk_scan(uint32_t x, uint32_t lane) {
   return x;
 }
 
+// The warp's hits added to *to, in 64 bits: a block that stays with one dense
+// graph of a batch can pass 2^32 (a clique of 60,000: 6e9 a warp).
+__device__ __forceinline__ void walk_add_hits(unsigned long long *to, unsigned long long hits,
+                                              uint32_t lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, o);
+  if (lane == 0 && hits) atomicAdd(to, hits);
+}
+
 // Core lengths to size up, at most n each.
 struct EdgeCores {
   uint32_t len[kCoreNumCandidates];
@@ -1037,8 +1046,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
     if (kBatch) {
       const uint32_t now = __ldg(long_graph + (x >> 1));
       if (now != g) {
-        const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)hits);
-        if (lane == 0 && c) atomicAdd(groups.counts + g, (unsigned long long)c);
+        walk_add_hits(groups.counts + g, hits, lane);
         hits = 0;
         g = now;
       }
@@ -1131,8 +1139,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
       fill(kWalkSetSlots, 0u);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, o);
-  if (lane == 0 && hits) atomicAdd(kBatch ? groups.counts + g : out, hits);
+  walk_add_hits(kBatch ? groups.counts + g : out, hits, lane);
 }
 
 // Room for at least x elements, in eighths of a power of two: graphs of one
