@@ -188,10 +188,19 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
                                                                    ? a.core_len
                                                                    : kCoreMaxLen);
   }
-  Scratch<uint32_t> number, long_rows;
+  // No room for a part of this way: the wedge-check path counts (and searches
+  // where it has no room for its sets).
+  const auto without_room = [&](int rc) {
+    if (rc != WETRIC_ENOMEM) return rc;
+    clear_error();
+    *declined = true;
+    return (int)WETRIC_OK;
+  };
+  Scratch<uint32_t> number, long_rows, core;
   if (!small) {
-    WETRIC_TRY(number.alloc(ctx, st, n));
-    WETRIC_TRY(long_rows.alloc(ctx, st, long_rows_room(m)));
+    int rc = number.alloc(ctx, st, n);
+    if (rc == WETRIC_OK) rc = long_rows.alloc(ctx, st, long_rows_room(m));
+    if (rc != WETRIC_OK) return without_room(rc);
   }
   if (n > 0) {
     const uint64_t most = (uint64_t)ctx->sm_count * 8, need = ceil_div(n, kWalkBlock);
@@ -209,7 +218,8 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
     ++launches;
   }
 
-  uint64_t core_h = 0, core_v0 = n, below_m = m, core_rows = 0;
+  uint64_t core_h = 0, core_v0 = n, below_m = m, core_rows = 0, core_words = 0;
+  uint32_t core_H4 = 0;
   uint64_t local[kReadWords];
   uint64_t W = 0, rows = 0;
   bool emit = false, sets = false;
@@ -255,27 +265,18 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
     // with two entries are rare (they need a long row with more than 48
     // columns outside the window), and a graph with more of them starts over
     // on the wedge-check path.
-    if (emit &&
-        walk.alloc(ctx, st, n, m, tot[3], tot[1], below_m + below_m / 4) != WETRIC_OK) {
-      // no room for the walk: the wedge-check path counts (and searches
-      // where it has no room for its sets)
-      clear_error();
-      *declined = true;
-      return WETRIC_OK;
-    }
+    int rc = WETRIC_OK;
+    if (emit) rc = walk.alloc(ctx, st, n, m, tot[3], tot[1], below_m + below_m / 4);
+    if (core_h) core_H4 = (uint32_t)(4 * ceil_div(core_h, 128));
+    core_words = core_h ? core_row_off(core_H4, (uint32_t)core_h) + 4 : 0;
+    if (rc == WETRIC_OK && core_h) rc = core.alloc(ctx, st, core_words);
+    if (rc != WETRIC_OK) return without_room(rc);
     r->copies_issued = a.issue_copies != nullptr;
     if (a.issue_copies) WETRIC_TRY(a.issue_copies(a.issue_ctx));
   }
 
-  Scratch<uint32_t> core;
-  uint32_t core_H4 = 0;
   const bool tma_ok = (reinterpret_cast<uintptr_t>(a.col_ind) & 15) == 0;
-  if (core_h) {
-    core_H4 = (uint32_t)(4 * ceil_div(core_h, 128));
-    const uint64_t cwords = core_row_off(core_H4, (uint32_t)core_h);
-    WETRIC_TRY(core.alloc(ctx, st, cwords + 4));
-    WETRIC_CUDA_TRY(cudaMemsetAsync(core.ptr, 0, (cwords + 4) * sizeof(uint32_t), st));
-  }
+  if (core_h) WETRIC_CUDA_TRY(cudaMemsetAsync(core.ptr, 0, core_words * sizeof(uint32_t), st));
 
   NvtxRange nvtx_launch("wetric count: structures and kernels");
   EventPair ev_merge[kMaxColChunks], ev_core[kMaxColChunks], ev_walk;
