@@ -107,6 +107,8 @@ __device__ __forceinline__ ServeGraph load_graph(const ServeGraph *p) {
   return g;
 }
 
+constexpr int kServeCarveout = 30;  // percent of an SM's memory that is shared (serve_engine_create)
+
 template <bool kNear>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kServeMaxBlocksPerSm)
     k_serve(const ServeGraph *graphs, const volatile ServeItem *items,
@@ -702,6 +704,15 @@ int serve_engine_create(DeviceContext *ctx, const ServeEngineOptions &o,
   WETRIC_CUDA_TRY(cudaMalloc(&e->slot_count, S * sizeof(unsigned long long)));
   WETRIC_CUDA_TRY(cudaMalloc(&e->slot_tiles, S * sizeof(unsigned long long)));
   WETRIC_CUDA_TRY(cudaMalloc(&e->exit_code, 8));  // [0] exit status, [1] quit
+  // The resident kernel uses no shared memory, and without a wish of its own
+  // it starts on whatever split of the SM the last kernel left. On a split
+  // with much of it (the sorts' tiles, the walk) kernels that want less wait
+  // until it ends: beside a large request one of 400,000 pairs took 18 or 77
+  // ms, a program's own count 9 or 73. Wishes of 0 to 55% all gave 16-17 and
+  // 8 ms, 60 and 100% the former; a large request alone 190 ms for 186 without
+  // one.
+  WETRIC_CUDA_TRY(cudaFuncSetAttribute(
+      k_serve<true>, cudaFuncAttributePreferredSharedMemoryCarveout, kServeCarveout));
   int occ = 0;
   WETRIC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &occ, k_serve<true>, kWarpsPerBlock * 32, 0));
