@@ -27,6 +27,7 @@
 #include <memory>
 #include <new>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "batch.cuh"
@@ -502,7 +503,7 @@ static int make_whole(Batch *b, cudaStream_t st) {
         b->rp32.ptr, b->csr.col_ind, n, 0, n, run.split.ptr, groups);
     WETRIC_LAUNCH_CHECK();
     const uint32_t T = merge_tile(m, ctx->sm_count);
-    k_edge_merge<uint32_t, true, true, false>
+    k_edge_merge<uint32_t, true, true, false, false>
         <<<(unsigned)ceil_div(ceil_div(m, T), kMergeBlock / 32), kMergeBlock, 0, st>>>(
             b->rp32.ptr, walk_columns(b->csr.col_ind, m), n, 0, n, T, w->number.ptr,
             run.split.ptr, run.bits, run.keys.ptr, (uint32_t)run.cap, run.counts.ptr,
@@ -938,14 +939,22 @@ static int batch_enqueue(Batch *b, cudaStream_t st, uint32_t *launches) {
                                            w.run.split.ptr, w.run.bits, nullptr, 0, nullptr,
                                            w.words.ptr, err, groups, kMergeCount);
     };
-    if (w.entries && w.sets)
-      merge(k_edge_merge<uint32_t, true, true, true>);
-    else if (w.entries)
-      merge(k_edge_merge<uint32_t, true, true, false>);
-    else if (w.sets)
-      merge(k_edge_merge<uint32_t, false, true, true>);
+    // (a graph of m columns in its order by degree has rows of up to sqrt(2 m))
+    const auto form = [&](auto search) {
+      constexpr bool kSearch = decltype(search)::value;
+      if (w.entries && w.sets)
+        merge(k_edge_merge<uint32_t, true, true, true, kSearch>);
+      else if (w.entries)
+        merge(k_edge_merge<uint32_t, true, true, false, kSearch>);
+      else if (w.sets)
+        merge(k_edge_merge<uint32_t, false, true, true, kSearch>);
+      else
+        merge(k_edge_merge<uint32_t, false, true, false, kSearch>);
+    };
+    if (b->max_out_degree > kSearchOver)
+      form(std::true_type());
     else
-      merge(k_edge_merge<uint32_t, false, true, false>);
+      form(std::false_type());
     WETRIC_LAUNCH_CHECK();
     if (!w.entries) return WETRIC_OK;
     // the walk's item counters (counts[3], counts[4])

@@ -20,6 +20,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "count.cuh"
 #include "count_kernels.cuh"
 #include "primitives.cuh"
@@ -313,14 +315,22 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
             (uint32_t)walk.cap, walk.counts.ptr, words.ptr, err, WalkGroups{},
             kMergeCount | kMergeEmit);
       };
-      if (emit && sets)
-        merge(k_edge_merge<uint32_t, true, false, true>, rp32);
-      else if (emit)
-        merge(k_edge_merge<uint32_t, true, false, false>, rp32);
-      else if (sets)
-        merge(k_edge_merge<uint32_t, false, false, true>, rp32);
+      const auto form = [&](auto search) {
+        constexpr bool kSearch = decltype(search)::value;
+        if (emit && sets)
+          merge(k_edge_merge<uint32_t, true, false, true, kSearch>, rp32);
+        else if (emit)
+          merge(k_edge_merge<uint32_t, true, false, false, kSearch>, rp32);
+        else if (sets)
+          merge(k_edge_merge<uint32_t, false, false, true, kSearch>, rp32);
+        else
+          merge(k_edge_merge<Off, false, false, false, kSearch>, rp);
+      };
+      // (a small graph's longest row is not known here)
+      if (small || r->max_out_degree > kSearchOver)
+        form(std::true_type());
       else
-        merge(k_edge_merge<Off, false, false, false>, rp);
+        form(std::false_type());
       WETRIC_LAUNCH_CHECK();
       ++launches;
       WETRIC_TRY(ev_merge[i].stop(st));

@@ -67,6 +67,8 @@ constexpr uint32_t kRowSetRows = 4;
 constexpr uint32_t kRowSetTries = 8;
 constexpr uint32_t kRowSetMin = 8;            // edges that are worth a set
 constexpr uint32_t kRowSetLong = 64;          // columns of a row w streamed at most
+constexpr uint32_t kSearchOver = 2048;        // columns that are searched for few others
+constexpr uint32_t kSearchRatio = 16;
 constexpr uint32_t kMergeStage = 128;         // entries a warp gathers (64 or more)
 constexpr uint32_t kWalkBig = 64;             // entries from which a block takes a vertex
 constexpr uint32_t kWalkBigCols = 128;        // or columns
@@ -368,16 +370,47 @@ __device__ __forceinline__ void walk_half(const WalkColumns &cols, uint32_t a, u
   }
 }
 
+// |[t0, t1) & [s0, s1)| where the second is much shorter: each of its columns
+// by bisection of what the ones before it left of the first.
+__device__ __forceinline__ uint32_t search_rows(const WalkColumns &cols, uint32_t t0, uint32_t t1,
+                                                uint32_t s0, uint32_t s1) {
+  uint32_t hits = 0;
+  for (; s0 < s1 && t0 < t1; ++s0) {
+    const uint32_t x = __ldg(cols.base + s0);
+    uint32_t len = t1 - t0;
+    while (len > 0) {
+      const uint32_t half = len >> 1;
+      const bool below = __ldg(cols.base + t0 + half) < x;
+      t0 = below ? t0 + half + 1 : t0;
+      len = below ? len - half - 1 : half;
+    }
+    hits += t0 < t1 && __ldg(cols.base + t0) == x;
+  }
+  return hits;
+}
+
 // |[t0, t1) & [s0, s1)| of the column array (both sorted, indices with mis,
 // neither empty), four columns of each at a time: all pairs of them, then
 // the four with the smaller last column move on. (Eight at a time: fewer
 // loads, four times the pairs; Erdos-Renyi, 13.3M edges: 670 us against
-// 551.)
+// 551.) kSearch: more than kSearchOver columns against less than a sixteenth
+// of them are searched instead, which only rows of a hub have that comes
+// early in the order (a graph's own order by degree keeps rows short). One
+// thread merged such a row with each of its short ones: 262,144 vertices in
+// id order, skewed, 53.8 ms a count, by search 7.5 (wedge checks 13.2); four
+// hubs of 200,000 columns 134 and 1.2 (180). Limits of 240 to 2,048 differ by
+// 2%. The kernels have a form without it, 1% faster on short rows (a batch of
+// 96 graphs 7.71 ms, 7.79 with it).
 struct MergeTask {
   uint32_t t0, t1, s0, s1;
 };
+template <bool kSearch>
 __device__ __forceinline__ uint32_t merge_rows(const WalkColumns &cols, const MergeTask &task) {
   const uint32_t t0 = task.t0, t1 = task.t1, s0 = task.s0, s1 = task.s1;
+  if (kSearch && max(t1 - t0, s1 - s0) > kSearchOver) {
+    if (t1 - t0 > kSearchRatio * (s1 - s0)) return search_rows(cols, t0, t1, s0, s1);
+    if (s1 - s0 > kSearchRatio * (t1 - t0)) return search_rows(cols, s0, s1, t0, t1);
+  }
   const uint32_t t_last = __ldg(cols.base + t1 - 1), s_last = __ldg(cols.base + s1 - 1);
   uint32_t a = t0 & ~3u, b = s0 & ~3u, hits = 0;
   uint32_t x[4], y[4];
@@ -460,7 +493,7 @@ __device__ __forceinline__ uint64_t row_of_edge(const Off *__restrict__ rp, uint
 // with kEmit, `what` says whether it is the count (the long rows' entries
 // were made before) or the making of the entries.
 enum MergeWhat : uint32_t { kMergeCount = 1, kMergeEmit = 2 };
-template <typename Off, bool kEmit, bool kBatch, bool kSets>
+template <typename Off, bool kEmit, bool kBatch, bool kSets, bool kSearch>
 __global__ void __launch_bounds__(kMergeBlock, kSets ? 7 : 8)
     k_edge_merge(const Off *__restrict__ rp, const __grid_constant__ WalkColumns cols, uint64_t n,
                  uint64_t row_lo, uint64_t row_hi, uint32_t T,
@@ -511,7 +544,7 @@ __global__ void __launch_bounds__(kMergeBlock, kSets ? 7 : 8)
   };
   uint32_t g = 0;
   auto drain = [&]() {  // kBatch: the graph's hits so far
-    if (kGather && lane < tasks) hits += merge_rows(cols, s_task[kGather ? wid : 0][lane]);
+    if (kGather && lane < tasks) hits += merge_rows<kSearch>(cols, s_task[kGather ? wid : 0][lane]);
     tasks = 0;
     const uint32_t c = __reduce_add_sync(0xffffffffu, hits);
     if (lane == 0 && c) atomicAdd(groups.counts + g, (unsigned long long)c);
@@ -613,7 +646,7 @@ __global__ void __launch_bounds__(kMergeBlock, kSets ? 7 : 8)
       if (kBatch && !(what & kMergeCount)) continue;
       const MergeTask task{first + cols.mis, t1 + cols.mis, s0 + cols.mis, s1 + cols.mis};
       if (!kGather) {
-        if (s0 < s1) hits += merge_rows(cols, task);
+        if (s0 < s1) hits += merge_rows<kSearch>(cols, task);
         if (!kEmit) next_row(edge + len < stop);
         continue;
       }
@@ -702,7 +735,7 @@ __global__ void __launch_bounds__(kMergeBlock, kSets ? 7 : 8)
       tasks += __popc(mm);
       __syncwarp();
       if (tasks >= 32) {
-        hits += merge_rows(cols, s_task[wid][lane]);
+        hits += merge_rows<kSearch>(cols, s_task[wid][lane]);
         tasks -= 32;
         const MergeTask moved = s_task[wid][32 + lane];
         __syncwarp();
@@ -713,7 +746,7 @@ __global__ void __launch_bounds__(kMergeBlock, kSets ? 7 : 8)
     j = stop;
   }
   if (kBatch) drain();
-  if (kGather && lane < tasks) hits += merge_rows(cols, s_task[kGather ? wid : 0][lane]);
+  if (kGather && lane < tasks) hits += merge_rows<kSearch>(cols, s_task[kGather ? wid : 0][lane]);
   if (kEmit && staged) flush();
   unsigned long long h = hits;
   for (int o = 16; o > 0; o >>= 1) {
@@ -792,7 +825,7 @@ __global__ void __launch_bounds__(kWalkBlock)
         if (w < n) {
           const uint64_t s0 = ld_off(rp, (uint64_t)w), s1 = ld_off(rp, (uint64_t)w + 1);
           if (s0 < s1 && s1 <= m)
-            hits += merge_rows(cols, MergeTask{edge + 1 + cols.mis, end + cols.mis,
+            hits += merge_rows<true>(cols, MergeTask{edge + 1 + cols.mis, end + cols.mis,
                                                (uint32_t)s0 + cols.mis, (uint32_t)s1 + cols.mis});
         }
       }
