@@ -26,8 +26,8 @@ def far_graph(oracle_mod, kind):
     rng = np.random.default_rng(11)
     n = 270_000
     share = 0.2  # of the vertices have window columns (all: no room for the entries)
-    if kind == "parts":  # rows of up to 1,800 columns outside the window, 60 in it
-        k, p, win = 3000, 0.6, 60
+    if kind in ("parts", "heavy"):  # rows of up to 1,150 or 1,800 columns outside the window
+        k, p, win = 3000, 0.36 if kind == "parts" else 0.6, 60
         i, j = np.triu_indices(k, 1)
         keep = rng.random(i.size) < p
         i, j = i[keep], j[keep]
@@ -70,6 +70,12 @@ def entries(g):
 KINDS = ["parts", "light", "hub"]
 
 
+def heavy(g, far):
+    """Wedges outside the window of rows that take several hash sets."""
+    far = far[far > PART]
+    return int((far * (far - 1) // 2).sum())
+
+
 @pytest.mark.parametrize("kind", KINDS)
 def test_far_columns(wetric_mod, oracle_mod, kind):
     import torch
@@ -80,6 +86,7 @@ def test_far_columns(wetric_mod, oracle_mod, kind):
     assert rest.sum() > 10_000 and win > 10_000
     assert rest.sum() + win < g.m + g.m // 4  # they have room
     assert g.m >= 1 << 19 and (d.max() > 128 or (d * (d - 1) // 2)[d > SHORT].sum() >= 1 << 25)
+    assert heavy(g, far) <= oracle_mod.wedge_total(g) // 5
     one_warp = (rest > 0) & (rest <= FEW) & (far <= 128)
     if kind == "parts":
         assert (far[rest > 0] > PART).sum() > 100  # sets in two parts
@@ -147,6 +154,52 @@ def test_more_entries_than_room(wetric_mod, oracle_mod, k):
         for r, c in ((rp, ci), (rp.int(), ci), (g.row_ptr, g.col_ind), pinned):
             got, st = wetric_mod.count(r, c, 5, 8192, core_len=core)
             assert got == want and st.wedges == st.wedges_counted == oracle_mod.wedge_total(g)
+
+
+def test_large_sets_go_to_the_wedge_checks(wetric_mod, oracle_mod):
+    """More than a fifth of the wedges on rows of several hash sets, from the
+    device and in row chunks from the host."""
+    import torch
+
+    g = far_graph(oracle_mod, "heavy")
+    assert heavy(g, entries(g)[2]) > oracle_mod.wedge_total(g) // 5
+    want = oracle_mod.count_merge(g)
+    rp = torch.from_numpy(g.row_ptr.view(np.int64)).cuda()
+    ci = torch.from_numpy(g.col_ind.view(np.int32)).cuda()
+    torch.cuda.synchronize()
+    for core in (wetric_mod.CORE_OFF, 0, 1000, 65_536):
+        for r, c in ((rp, ci), (g.row_ptr, g.col_ind)):
+            got, st = wetric_mod.count(r, c, 5, 8192, core_len=core)
+            assert got == want and st.wedges == st.wedges_counted == oracle_mod.wedge_total(g)
+
+
+@pytest.mark.parametrize("order", ["id", "random"])
+def test_an_order_of_its_own_does_not_slow_the_count(wetric_mod, order):
+    """R-MAT scale 18 as drawn and shuffled, oriented by id: the hubs' columns lie
+    anywhere. The default count against the wedge checks (it took 3 to 5
+    times as long when every rest set was walked)."""
+    import torch
+
+    n = 1 << 18
+    src, dst = (x.long() for x in wetric_mod.gen_rmat_device(18, 16 << 18, seed=3))
+    if order == "random":
+        gen = torch.Generator(device="cuda")
+        gen.manual_seed(2)
+        at = torch.randperm(n, device="cuda", generator=gen)
+        src, dst = at[src], at[dst]
+    key = torch.unique((torch.minimum(src, dst) * n + torch.maximum(src, dst))[src != dst])
+    rp = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    rp[1:] = torch.cumsum(torch.bincount(key // n, minlength=n), 0)
+    ci = (key % n).int()
+    torch.cuda.synchronize()
+
+    def ms(**kw):
+        runs = [wetric_mod.count(rp, ci, 5, 8192, **kw) for _ in range(6)]
+        assert len({c for c, _ in runs}) == 1
+        return runs[0][0], sorted(st.exec_ms for _, st in runs)[2]
+
+    (a, default), (b, checks) = ms(), ms(kernel=8)
+    assert a == b and default < 1.5 * checks, (default, checks)
 
 
 def test_batch_far_columns(wetric_mod, oracle_mod):

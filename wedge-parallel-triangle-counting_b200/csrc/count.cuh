@@ -90,7 +90,8 @@ int count_oriented(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
 
 // The default count of a whole graph (count_whole.cu). count_oriented sends
 // the calls it takes there; *declined: not counted (no room, entries that
-// would not fit their bits, or too many), the wedge-check path takes the call.
+// would not fit their bits, too many of them, or sets too large), the
+// wedge-check path takes the call.
 bool count_whole_takes(const CountArgs &a);
 int count_whole(DeviceContext *ctx, cudaStream_t st, const CountArgs &a,
                 CountResult *r, bool *declined);
