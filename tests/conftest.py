@@ -79,7 +79,7 @@ def build_probe(tmp, name):
     subprocess.check_call(
         [os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-gencode",
          "arch=compute_100a,code=sm_100a", "-ccbin", "/usr/bin/g++", "-std=c++17", "-O2",
-         "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-shared", "-cudart", "static",
+         "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC,-pthread", "-shared", "-cudart", "static",
          "-I", os.path.join(PKG, "csrc"), "-o", str(lib),
          os.path.join(ROOT, "tests", f"{name}.cu"), "-L", os.path.join(PKG, "wetric"),
          "-lwetric", "-Xlinker", "-rpath," + os.path.join(PKG, "wetric")])

@@ -3,6 +3,7 @@
 // a sort, run with a given error word.
 #include "pair_streams.cuh"
 #include "primitives.cuh"
+#include "stage_workers.h"
 #include "walk.cuh"
 
 using namespace wetric;
@@ -117,4 +118,30 @@ extern "C" int probe_add_hits(const unsigned long long *hits, unsigned long long
   add_hits<<<1, 32>>>(hits, sum);
   PROBE(cudaGetLastError());
   return (int)cudaDeviceSynchronize();
+}
+
+// `callers` threads copy pieces of the given sizes at once, `rounds` times
+// each, `gap_ms` apart; 0 when every copy is whole and nothing else changed.
+extern "C" int probe_stage_copies(const uint64_t *sizes, int n, int callers, int rounds,
+                                  int gap_ms) {
+  StageWorkers workers;
+  workers.start();
+  std::atomic<int> bad{0};
+  std::vector<std::thread> threads;
+  for (int c = 0; c < callers; ++c)
+    threads.emplace_back([&, c] {
+      for (int r = 0; r < rounds; ++r)
+        for (int i = 0; i < n; ++i) {
+          const size_t size = sizes[i], pad = 64;
+          std::vector<unsigned char> src(size), dst(size + 2 * pad, 0xAB);
+          for (size_t k = 0; k < size; ++k) src[k] = (unsigned char)(k * 31 + (k >> 13) + c + r + i);
+          workers.copy(src.data(), dst.data() + pad, size);
+          bool ok = size == 0 || memcmp(src.data(), dst.data() + pad, size) == 0;
+          for (size_t k = 0; k < pad; ++k) ok = ok && dst[k] == 0xAB && dst[pad + size + k] == 0xAB;
+          if (!ok) ++bad;
+          if (gap_ms) std::this_thread::sleep_for(std::chrono::milliseconds(gap_ms));
+        }
+    });
+  for (std::thread &t : threads) t.join();
+  return bad;
 }

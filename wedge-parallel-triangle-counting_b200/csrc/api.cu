@@ -9,12 +9,10 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include <condition_variable>
 #include <memory>
 #include <mutex>
 #include <new>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "batch.cuh"
@@ -22,6 +20,7 @@
 #include "count.cuh"
 #include "graph_io.h"
 #include "preprocess.cuh"
+#include "stage_workers.h"
 
 namespace wetric {
 
@@ -285,88 +284,6 @@ int stage_buffers(DeviceContext *ctx) {
   ctx->stage_bytes = kStageBytes;
   return WETRIC_OK;
 }
-
-// Threads that share the copying of staged pieces for the length of one
-// call. They sleep between pieces: an OpenMP team spins at its barriers, and
-// the two teams that the driver's callback threads made spun against each
-// other's copies (R-MAT scale 20 from pageable arrays on 16 cores: 50 ms a
-// call, 45 of them the device waiting for 64 MB of copies; now 6 ms).
-class StageWorkers {
- public:
-  static constexpr size_t kBlock = 1ull << 20;
-  struct Job {
-    const char *src = nullptr;
-    char *dst = nullptr;
-    size_t bytes = 0, blocks = 0, next = 0, done = 0;  // under mu_
-  };
-  ~StageWorkers() {
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      stop_ = true;
-    }
-    work_.notify_all();
-    for (std::thread &t : threads_) t.join();
-  }
-  void start() {
-    const unsigned cores = std::thread::hardware_concurrency();
-    const unsigned want = cores > 15 ? 7 : cores / 2;
-    try {
-      for (unsigned i = 0; i < want; ++i) threads_.emplace_back([this] { loop(); });
-    } catch (...) {  // fewer threads: the caller of copy() copies too
-    }
-  }
-  // Copies a piece; returns when it is done.
-  void copy(const void *src, void *dst, size_t bytes) {
-    Job job;
-    job.src = static_cast<const char *>(src);
-    job.dst = static_cast<char *>(dst);
-    job.bytes = bytes;
-    job.blocks = (bytes + kBlock - 1) / kBlock;
-    std::unique_lock<std::mutex> lk(mu_);
-    job.next = 0;
-    Job *mine = &job, **slot = nullptr;
-    for (Job *&j : jobs_)
-      if (!j) slot = &j;
-    if (slot) *slot = mine;  // else both slots are taken: copied here alone
-    work_.notify_all();
-    while (take(lk, mine)) {
-    }
-    done_.wait(lk, [&] { return job.done == job.blocks; });
-    if (slot) *slot = nullptr;
-  }
-
- private:
-  // Copies the job's next block, if there is one.
-  bool take(std::unique_lock<std::mutex> &lk, Job *job) {
-    if (job->next >= job->blocks) return false;
-    const size_t o = job->next++ * kBlock;
-    lk.unlock();
-    memcpy(job->dst + o, job->src + o, o + kBlock <= job->bytes ? kBlock : job->bytes - o);
-    lk.lock();
-    if (++job->done == job->blocks) done_.notify_all();
-    return true;
-  }
-  void loop() {
-    std::unique_lock<std::mutex> lk(mu_);
-    for (;;) {
-      Job *job = nullptr;
-      for (Job *j : jobs_)
-        if (j && j->next < j->blocks) job = j;
-      if (job) {
-        take(lk, job);
-      } else if (stop_) {
-        return;
-      } else {
-        work_.wait(lk);
-      }
-    }
-  }
-  std::mutex mu_;
-  std::condition_variable work_, done_;
-  Job *jobs_[2] = {};
-  bool stop_ = false;
-  std::vector<std::thread> threads_;
-};
 
 struct StagePiece {
   StageWorkers *workers = nullptr;
