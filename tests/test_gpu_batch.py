@@ -168,3 +168,23 @@ def test_batch_autotune(wetric_mod, oracle_mod):
     assert set(b3.spreads().tolist()) == {3}
     assert np.array_equal(b3.count()[0], counts)
     b3.free()
+
+
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_batch_without_wedges(wetric_mod, use_graph):
+    """Paths and stars have no wedge in their order by degree: nothing is
+    launched for them, and a batch that holds one triangle beside them counts."""
+    n = 5000
+    path = (np.arange(n - 1, dtype=np.uint32), np.arange(1, n, dtype=np.uint32))
+    star = (np.zeros(n - 1, np.uint32), np.arange(1, n, dtype=np.uint32))
+    tri = (np.array([0, 1, 2], np.uint32), np.array([1, 2, 0], np.uint32))
+    for parts, want in (([path, star], [0, 0]), ([path, tri, star], [0, 1, 0])):
+        src, dst = (np.concatenate([p[k] for p in parts]) for k in (0, 1))
+        off = np.concatenate([[0], np.cumsum([p[0].size for p in parts])]).astype(np.uint64)
+        b = wetric_mod.Batch(src, dst, off, np.full(len(parts), n, np.uint64),
+                             use_cuda_graph=use_graph)
+        for _ in range(2):
+            counts, st = b.count()
+            assert [int(x) for x in counts] == want
+            assert st.wedges == sum(want) and (st.launches > 0) == bool(sum(want))
+        b.free()

@@ -929,6 +929,8 @@ static int batch_enqueue(Batch *b, cudaStream_t st, uint32_t *launches) {
     BatchWalk &w = *b->walk;
     DeviceContext *ctx = b->ctx;
     const uint64_t n = b->vbase[b->G], m = b->m_total;
+    *launches = 0;
+    if (b->W + b->pair_wedges == 0) return WETRIC_OK;  // (every row has one column or none)
     const WalkGroups groups{b->vbase_d.ptr, b->G, b->counts.ptr};
     const uint32_t T = merge_tile(m, ctx->sm_count);
     const unsigned grid = (unsigned)ceil_div(ceil_div(m, T), kMergeBlock / 32);
