@@ -885,14 +885,17 @@ static int wedge_total_impl(DeviceContext *ctx, cudaStream_t st,
     WETRIC_TRY((prim::exclusive_scan<uint32_t, uint64_t>(ctx, st, active.ptr,
                                                          wc.ptr, n, err.ptr)));
   }
-  uint64_t K = 0;
+  uint64_t K = 0, local[4];
   uint32_t herr = 0;
-  if (n > 0)
-    WETRIC_CUDA_TRY(cudaMemcpyAsync(&K, wc.ptr + n, sizeof(uint64_t),
-                                    cudaMemcpyDeviceToHost, st));
-  WETRIC_CUDA_TRY(cudaMemcpyAsync(&herr, err.ptr, sizeof(uint32_t),
-                                  cudaMemcpyDeviceToHost, st));
-  WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
+  const uint64_t *got = nullptr;
+  {
+    ReadPlan rd;
+    rd.add(err.ptr, 1, 4);
+    if (n > 0) rd.add(wc.ptr + n, 1, 8);
+    WETRIC_TRY(read_back(ctx, st, rd, local, &got));
+    herr = (uint32_t)got[0];
+    K = n > 0 ? got[1] : 0;
+  }
   if (herr == kDevLookbackTimeout) {
     set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
     return WETRIC_ETIMEDOUT;
@@ -913,19 +916,17 @@ static int wedge_total_impl(DeviceContext *ctx, cudaStream_t st,
   }
   WETRIC_TRY((prim::exclusive_scan<uint64_t, uint64_t>(ctx, st, act_wp.ptr,
                                                        act_wp.ptr, K, err.ptr)));
-  unsigned long long hmd = 0;
-  WETRIC_CUDA_TRY(cudaMemcpyAsync(&herr, err.ptr, sizeof(uint32_t),
-                                  cudaMemcpyDeviceToHost, st));
-  WETRIC_CUDA_TRY(cudaMemcpyAsync(W, act_wp.ptr + K, sizeof(uint64_t),
-                                  cudaMemcpyDeviceToHost, st));
-  WETRIC_CUDA_TRY(cudaMemcpyAsync(&hmd, md.ptr, sizeof(hmd),
-                                  cudaMemcpyDeviceToHost, st));
-  WETRIC_CUDA_TRY(cudaStreamSynchronize(st));
-  if (herr != kDevOk) {
+  ReadPlan rd;
+  rd.add(err.ptr, 1, 4);
+  rd.add(act_wp.ptr + K, 1, 8);
+  rd.add(md.ptr, 1, 8);
+  WETRIC_TRY(read_back(ctx, st, rd, local, &got));
+  if (got[0] != kDevOk) {
     set_error(WETRIC_ETIMEDOUT, "a scan's look-back did not complete in time");
     return WETRIC_ETIMEDOUT;
   }
-  *maxdeg = hmd;
+  *W = got[1];
+  *maxdeg = got[2];
   return WETRIC_OK;
 }
 
