@@ -49,3 +49,22 @@ def test_symmetric_rows_around_the_row_sort(wetric_mod, oracle_mod, size):
     ci = torch.from_numpy(sym.col_ind.view(np.int32)).cuda()
     assert wetric_mod.count(rp, ci, 5, 64, oriented=False)[0] == tri
     assert wetric_mod.count(rp.int(), ci, 5, 64, oriented=False)[0] == tri
+
+
+@pytest.mark.parametrize("hubs", [1, 2, 7])
+@pytest.mark.parametrize("leaves", [1, 30, 126, 127, 128, 129, 161, 5000])
+def test_symmetric_hubs_in_place(wetric_mod, oracle_mod, hubs, leaves):
+    """Rows of hubs that keep nothing or little of many columns, around the
+    128 columns from which such rows are skipped."""
+    rng = np.random.default_rng(hubs * 7 + leaves)
+    n = hubs + leaves + 40
+    ids = rng.permutation(n)
+    i, j = np.triu_indices(hubs, 1)
+    src = np.concatenate([np.repeat(np.arange(hubs), leaves), i, hubs + rng.integers(0, leaves, 20)])
+    dst = np.concatenate([np.tile(hubs + np.arange(leaves), hubs), j,
+                          hubs + rng.integers(0, leaves, 20)])
+    sym = oracle_mod.csr_from_pairs(ids[src].astype(np.uint32), ids[dst].astype(np.uint32), n)
+    want = oracle_mod.preprocess(sym)
+    got = wetric_mod.preprocess(wetric_mod.Graph(sym.row_ptr, sym.col_ind))
+    assert np.array_equal(got.row_ptr, want.row_ptr)
+    assert np.array_equal(got.col_ind, want.col_ind)
