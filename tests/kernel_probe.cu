@@ -84,7 +84,7 @@ extern "C" int probe_walk(const uint32_t *rp, const uint32_t *split, const uint3
   k_walk_starts<<<1, kWalkBlock, 0, ctx->stream>>>(keys, entries, 2 * rows, bits.shift(), start,
                                                    err);
   k_walk_plan<<<1, kWalkBlock, 0, ctx->stream>>>(rp, split, long_rows, start, 2 * rows, big, small,
-                                                 counts, err);
+                                                 counts, false, err);
   k_walk_count<kWalkSmallBlock, kWalkSmallBlocks, false><<<4, kWalkSmallBlock, 0, ctx->stream>>>(
       rp, split, long_rows, walk_columns(ci, m), 0, keys, start, bits, small, counts + 1,
       counts + 2, 0, out, WalkGroups{}, nullptr, err);

@@ -96,3 +96,31 @@ def test_hubs_in_front_do_not_slow_the_count(wetric_mod):
 
     (a, default), (b, checks) = ms(), ms(kernel=8)
     assert a == b and default < 1.5 * checks, (default, checks)
+
+
+def test_a_star_in_front_takes_no_wedge_checks(wetric_mod):
+    """Vertex 0 with 400,000 leaves among other edges: 8e10 wedges that close
+    nothing, on one row outside the window, and no long row for its tails to
+    go to."""
+    import torch
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    n, leaves = 500_000, 400_000
+    s = torch.cat([torch.zeros(leaves, dtype=torch.int64, device="cuda"),
+                   torch.randint(1, n, (2_000_000,), device="cuda", generator=gen)])
+    d = torch.cat([torch.arange(1, leaves + 1, device="cuda"),
+                   torch.randint(1, n, (2_000_000,), device="cuda", generator=gen)])
+    key = torch.unique((torch.minimum(s, d) * n + torch.maximum(s, d))[s != d])
+    rp = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    rp[1:] = torch.cumsum(torch.bincount(key // n, minlength=n), 0)
+    ci = (key % n).int()
+    torch.cuda.synchronize()
+
+    def ms(**kw):
+        runs = [wetric_mod.count(rp, ci, 5, 8192, **kw) for _ in range(4)]
+        assert len({c for c, _ in runs}) == 1
+        return runs[0][0], sorted(st.exec_ms for _, st in runs)[1]
+
+    (a, default), (b, checks) = ms(), ms(kernel=8)
+    assert a == b and default < checks / 4, (default, checks)

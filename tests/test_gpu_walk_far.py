@@ -27,7 +27,7 @@ def far_graph(oracle_mod, kind):
     n = 270_000
     share = 0.2  # of the vertices have window columns (all: no room for the entries)
     if kind in ("parts", "heavy"):  # rows of up to 1,150 or 1,800 columns outside the window
-        k, p, win = 3000, 0.36 if kind == "parts" else 0.6, 60
+        k, p, win = 3000, 0.35 if kind == "parts" else 0.6, 60
         i, j = np.triu_indices(k, 1)
         keep = rng.random(i.size) < p
         i, j = i[keep], j[keep]
@@ -71,9 +71,10 @@ KINDS = ["parts", "light", "hub"]
 
 
 def heavy(g, far):
-    """Wedges outside the window of rows that take several hash sets."""
+    """Bound of the wedges outside the window between rows that take several
+    hash sets there."""
     far = far[far > PART]
-    return int((far * (far - 1) // 2).sum())
+    return min(int((far * (far - 1) // 2).sum()), int(far.sum()) * far.size)
 
 
 @pytest.mark.parametrize("kind", KINDS)
@@ -86,10 +87,10 @@ def test_far_columns(wetric_mod, oracle_mod, kind):
     assert rest.sum() > 10_000 and win > 10_000
     assert rest.sum() + win < g.m + g.m // 4  # they have room
     assert g.m >= 1 << 19 and (d.max() > 128 or (d * (d - 1) // 2)[d > SHORT].sum() >= 1 << 25)
-    assert heavy(g, far) <= oracle_mod.wedge_total(g) // 5
+    assert heavy(g, far) <= oracle_mod.wedge_total(g) // 10
     one_warp = (rest > 0) & (rest <= FEW) & (far <= 128)
     if kind == "parts":
-        assert (far[rest > 0] > PART).sum() > 100  # sets in two parts
+        assert (far[rest > 0] > PART).sum() > 30  # sets in two parts
     elif kind == "light":
         assert one_warp.sum() > 1000 and ((rest > 0) & ~one_warp).sum() > 1000
     else:
@@ -157,12 +158,12 @@ def test_more_entries_than_room(wetric_mod, oracle_mod, k):
 
 
 def test_large_sets_go_to_the_wedge_checks(wetric_mod, oracle_mod):
-    """More than a fifth of the wedges on rows of several hash sets, from the
+    """More than a tenth of the wedges on rows of several hash sets, from the
     device and in row chunks from the host."""
     import torch
 
     g = far_graph(oracle_mod, "heavy")
-    assert heavy(g, entries(g)[2]) > oracle_mod.wedge_total(g) // 5
+    assert heavy(g, entries(g)[2]) > oracle_mod.wedge_total(g) // 10
     want = oracle_mod.count_merge(g)
     rp = torch.from_numpy(g.row_ptr.view(np.int64)).cuda()
     ci = torch.from_numpy(g.col_ind.view(np.int32)).cuda()
@@ -224,3 +225,39 @@ def test_batch_far_columns(wetric_mod, oracle_mod):
     og = wetric_mod.orient_edges(*big, n=n)
     got, st = og.count(5, 8192)
     assert got == want and st.pair_wedges + st.core_wedges < st.wedges
+
+
+def test_hub_rows_are_shared_out(wetric_mod, oracle_mod):
+    """Hubs with up to 60 hash sets among rows of one, few enough that the graph
+    is walked: their entries and sets go to several blocks."""
+    import torch
+
+    rng = np.random.default_rng(21)
+    n, hubs, k = 330_000, 40, 3000
+    at = np.sort(rng.choice(n - WINDOW - 70_000, k, replace=False))  # the middle vertices' range
+    lengths = rng.choice([900, 1023, 1024, 1025, 2048, 2049, 9000, 33_000, 60_000], hubs)
+    src, dst = [], []
+    for h, x in zip(rng.choice(at, hubs, replace=False), lengths):
+        src.append(np.full(x, h))
+        dst.append(h + 1 + rng.choice(n - WINDOW - h - 2, x, replace=False))
+    # everybody before a hub points at it and at a few hundred others
+    i = np.repeat(at, 300)
+    j = rng.choice(at, i.size)
+    src += [i, np.repeat(at, hubs)]
+    dst += [j, np.tile(np.array([s[0] for s in src[:hubs]]), k)]
+    s, d = np.concatenate(src), np.concatenate(dst)
+    g = csr(oracle_mod, n, np.minimum(s, d)[s != d], np.maximum(s, d)[s != d])
+    rest, win, far = entries(g)
+    sets = -(-far[(rest > 0) & (far > PART)] // PART)
+    assert sets.max() > 32 and sets.size > 15 and rest[far > PART].max() > 512
+    assert g.m >= 1 << 19 and rest.sum() + win < g.m + g.m // 4
+    assert heavy(g, far) <= oracle_mod.wedge_total(g) // 10
+    want, W = oracle_mod.count_merge(g), oracle_mod.wedge_total(g)
+    rp = torch.from_numpy(g.row_ptr.astype(np.int32)).cuda()
+    ci = torch.from_numpy(g.col_ind.view(np.int32)).cuda()
+    torch.cuda.synchronize()
+    for kw in ({}, {"one_pass": True}, {"core_len": 1000}, {"kernel": 8}):
+        got, st = wetric_mod.count(rp, ci, 5, 8192, **kw)
+        assert got == want and st.wedges == st.wedges_counted == W, kw
+        if "kernel" not in kw:
+            assert st.pair_wedges + st.core_wedges < W

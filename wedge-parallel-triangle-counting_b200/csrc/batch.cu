@@ -442,8 +442,8 @@ static int autotune_spreads(Batch *b, std::vector<uint32_t> *sg, cudaStream_t st
 }
 
 // Rows and, where they pay, the long rows' entries of a batch counted by row
-// intersections and the walk; b->whole stays false when there is no room,
-// entries would not fit their bits or the sets are too large.
+// intersections and the walk; b->whole stays false when there is no room, or
+// entries would not fit their bits.
 static int make_whole(Batch *b, cudaStream_t st) {
   DeviceContext *ctx = b->ctx;
   const uint32_t G = b->G;
@@ -500,8 +500,8 @@ static int make_whole(Batch *b, cudaStream_t st) {
       return WETRIC_OK;
     }
     k_walk_split<true><<<WalkRun::grid(ctx, n), kWalkBlock, 0, st>>>(
-        b->rp32.ptr, b->csr.col_ind, n, 0, n, run.split.ptr, run.heavy(), 0, nullptr,
-        groups);
+        b->rp32.ptr, b->csr.col_ind, n, 0, n, run.split.ptr, groups, nullptr, 0,
+        nullptr);
     WETRIC_LAUNCH_CHECK();
     const uint32_t T = merge_tile(m, ctx->sm_count);
     k_edge_merge<uint32_t, true, true, false, false>
@@ -515,11 +515,10 @@ static int make_whole(Batch *b, cudaStream_t st) {
     ReadPlan rd;
     rd.add(run.counts.ptr, 1, 4);
     rd.add(w->words.ptr + 1, 1, 8);
-    rd.add(run.heavy(), 1, 8);
     WETRIC_TRY(read_back(ctx, st, rd, local, &got));
     const uint64_t made = got[0];
     b->pair_wedges = got[1];
-    if (made > run.cap || got[2] > walk_most_heavy(b->W)) return WETRIC_OK;
+    if (made > run.cap) return WETRIC_OK;
     w->entries = made > 0;
     uint32_t launches = 0;
     if (made) {

@@ -293,15 +293,15 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
   if (!made) made = local;
   const WalkColumns cols = walk_columns(a.col_ind, m);
   const uint32_t *rp32 = reinterpret_cast<const uint32_t *>(rp);  // unless small
-  const uint64_t most_heavy = walk_most_heavy(W - r->core_wedges);
+  const uint64_t most_far = walk_most_far(W - r->core_wedges);
   for (uint32_t i = 0; i < C && n > 0; ++i) {
     const uint64_t lo = C_in ? a.chunk_lo[i] : 0, hi = i ? a.chunk_lo[i - 1] : n;
     const cudaEvent_t ready = C_in ? a.chunk_ready[i] : a.ci_ready;
     if (ready && !small) WETRIC_CUDA_TRY(cudaStreamWaitEvent(st, ready, 0));
     if (emit) {
       k_walk_split<false><<<WalkRun::grid(ctx, hi - lo), kWalkBlock, 0, st>>>(
-          rp32, a.col_ind, n, lo, hi, walk.split.ptr, walk.heavy(), most_heavy, err + 1,
-          WalkGroups{});
+          rp32, a.col_ind, n, lo, hi, walk.split.ptr, WalkGroups{}, walk.far(), most_far,
+          err + 1);
       WETRIC_LAUNCH_CHECK();
       ++launches;
     }
@@ -339,7 +339,7 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
       WETRIC_TRY(ev_merge[i].stop(st));
     }
     if (emit && i + 1 == C) {
-      WETRIC_CUDA_TRY(cudaMemcpyAsync(made, walk.counts.ptr, 4 * sizeof(uint64_t),
+      WETRIC_CUDA_TRY(cudaMemcpyAsync(made, walk.counts.ptr, WalkRun::kCounts * 4,
                                       cudaMemcpyDeviceToHost, st));
       WETRIC_CUDA_TRY(cudaEventCreateWithFlags(&ev_made.e, cudaEventDisableTiming));
       WETRIC_CUDA_TRY(cudaEventRecord(ev_made.e, st));
@@ -362,10 +362,13 @@ static int whole_impl(DeviceContext *ctx, cudaStream_t st, const CountArgs &a, C
   if (emit) {
     WETRIC_CUDA_TRY(cudaEventSynchronize(ev_made.e));
     const uint64_t entries = (uint32_t)*made;
-    if (entries > walk.cap || made[3] > most_heavy) {
+    const WalkFar far{made[WalkRun::kFar / 2], made[WalkRun::kFar / 2 + 1],
+                      made[WalkRun::kFar / 2 + 2], 0};
+    if (entries > walk.cap || far.past(most_far)) {
       *declined = true;
       return WETRIC_OK;
     }
+    if (far.rows) walk.share(ctx, st);
     if (entries > 0) {
       WETRIC_TRY(walk.sort(ctx, st, rp32, long_rows.ptr, entries, err, &launches));
       WETRIC_TRY(ev_walk.start(st));

@@ -78,6 +78,8 @@ constexpr uint32_t kWalkBigBlock = 128, kWalkSmallBlock = 32;
 constexpr int kWalkBigBlocks = 10, kWalkSmallBlocks = 28;  // per SM
 constexpr uint32_t kWalkSmallSlots = 512;
 constexpr uint32_t kWalkSetCols = 1024;  // columns per hash set
+constexpr uint32_t kWalkSetGroups = 32;  // items that share the sets of a row at most (2^k)
+constexpr uint32_t kWalkSetPiece = 512;  // entries per item of a row of several sets
 constexpr uint32_t kWalkSetSlots = 2048;
 constexpr int kWalkCarveout = 70;  // percent of an SM's memory that is shared
 
@@ -232,17 +234,40 @@ __global__ void __launch_bounds__(kWalkBlock)
     if (ld_off(rp, 0) != 0 || ld_off(rp, n) != m) atomicCAS(err, 0u, (uint32_t)kDevRowPtrRange);
 }
 
+// The rows with more than kWalkSetCols columns outside the window, which take
+// several hash sets: their wedges there, columns there and number, and the
+// blocks that are through with them. At most min(wedges, columns * rows) of a
+// graph's wedges have their tail on one such row and their middle vertex on
+// another; with more than a tenth of those below the core (`most`) it is not
+// walked. Half full sets cost several tries a column and the tails stream
+// once for each set, where a bit row costs one lookup. In an order by degree
+// the columns of long rows lie in the window, and a batch, always in that
+// order, does without this; in another order they need not. Walk / wedge checks
+// in ms and that share: R-MAT scale 20 in id order 73 / 57 (0.71), in random
+// order 31 / 27 (0.53), Chung-Lu 300,000 vertices, mean degree 20, exponent
+// 2.2 5.9 / 4.3 (0.13), in random order 2.2 / 1.9 (0.02), 1,000,000, 40, 2.8
+// 5.8 / 7.6 (0.25), 3.8 / 5.0 (0.06); dense parts of 3,000 vertices 9 / 6
+// (0.82); skewed draws in id order 4.5 / 13 (0.01); Erdos-Renyi 150,000, 1300
+// 36 / 127 (0); four hubs of 200,000 columns, all wedges theirs, 1.2 / 180 (0).
+struct WalkFar {
+  unsigned long long wedges, columns, rows, blocks;
+  __host__ __device__ bool past(unsigned long long most) const {
+    return wedges > most && columns * rows > most;
+  }
+};
+inline uint64_t walk_most_far(uint64_t wedges) { return wedges / 10; }
+
 // split[v] = index of row v's first window column (rows are sorted), rows
-// [lo, hi), and *heavy += the wedges outside the window of rows with more
-// than kWalkSetCols columns there; past most_heavy (walk_most_heavy) *stop is
-// set. kBatch: the window of the row's own graph, and no *stop.
+// [lo, hi), and their part of *far; *stop is set when it is past `most`.
+// kBatch: of the row's own graph, and no *far.
 template <bool kBatch>
 __global__ void __launch_bounds__(kWalkBlock)
     k_walk_split(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ci, uint64_t n,
                  uint64_t lo_row, uint64_t hi_row, uint32_t *__restrict__ split,
-                 unsigned long long *__restrict__ heavy, unsigned long long most_heavy,
-                 uint32_t *__restrict__ stop, const WalkGroups groups) {
-  unsigned long long far_w = 0;
+                 const WalkGroups groups, WalkFar *far, unsigned long long most,
+                 uint32_t *__restrict__ stop) {
+  unsigned long long wedges = 0, columns = 0;
+  uint32_t rows = 0;
   uint32_t t0 = n > kWalkWindow ? (uint32_t)(n - kWalkWindow) : 0u;
   for (uint64_t v = lo_row + (uint64_t)blockIdx.x * kWalkBlock + threadIdx.x; v < hi_row;
        v += (uint64_t)gridDim.x * kWalkBlock) {
@@ -256,12 +281,29 @@ __global__ void __launch_bounds__(kWalkBlock)
       else lo = mid + 1;
     }
     split[v] = lo;
-    const unsigned long long far = lo - begin;
-    if (far > kWalkSetCols) far_w += far * (far - 1) / 2;
+    const unsigned long long d = lo - begin;
+    if (!kBatch && d > kWalkSetCols) {
+      wedges += d * (d - 1) / 2;
+      columns += d;
+      ++rows;
+    }
   }
-  if (!__any_sync(0xffffffffu, far_w != 0)) return;
-  for (int o = 16; o > 0; o >>= 1) far_w += __shfl_down_sync(0xffffffffu, far_w, o);
-  if ((threadIdx.x & 31) == 0 && atomicAdd(heavy, far_w) + far_w > most_heavy && !kBatch) *stop = 1;
+  if (kBatch) return;
+  if (rows) {  // few threads have any
+    atomicAdd(&far->wedges, wedges);
+    atomicAdd(&far->columns, columns);
+    atomicAdd(&far->rows, (unsigned long long)rows);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {  // the last block has all of them
+    __threadfence();
+    uint32_t *blocks = reinterpret_cast<uint32_t *>(&far->blocks);
+    if (atomicInc(blocks, gridDim.x - 1) == gridDim.x - 1) {
+      __threadfence();
+      const volatile WalkFar *all = far;
+      if (WalkFar{all->wedges, all->columns, all->rows, 0}.past(most)) *stop = 1;
+    }
+  }
 }
 
 // start[x] = the first of the sorted entries of middle vertex x or more, x in
@@ -305,14 +347,38 @@ __device__ __forceinline__ uint2 walk_set(const uint32_t *__restrict__ rp,
   return x & 1 ? make_uint2(s, __ldg(rp + w + 1)) : make_uint2(__ldg(rp + w), s);
 }
 
-// The work items over the x_end middle vertices: counts[0] pieces of those
+// A row of several hash sets is shared out by entries and by sets: a hub's, with
+// a set for each 1,024 of its columns outside the window, was one block's
+// for 2,048 long tails at a time, and the rest of the device waited for it
+// (Chung-Lu in random order, as above, 5.0 ms; 1,000,000, 20, 2.4 11.2, now
+// 4.3; R-MAT scale 20 in id order 271). The kernel has a form without it (R-MAT
+// scale 22 5.88 ms, 5.97 with it), taken when no row has several sets.
+// An item's word: its piece of the entries (of kWalkSetPiece when the top bit
+// is set), its group of sets.
+constexpr uint32_t kWalkSeveral = 1u << 31, kWalkGroupShift = 24;
+__device__ __forceinline__ bool walk_several(uint32_t x, uint32_t d) {
+  return !(x & 1) && d > kWalkSetCols;
+}
+// Columns of a group: a multiple of kWalkSetCols, kWalkSetGroups of them or
+// fewer make d.
+__device__ __forceinline__ uint32_t walk_group_cols(uint32_t d) {
+  return (d + kWalkSetGroups * kWalkSetCols - 1) / (kWalkSetGroups * kWalkSetCols) * kWalkSetCols;
+}
+// Items of the big blocks at most, with `cap` entries and m columns.
+inline uint64_t walk_most_items(uint64_t cap, uint64_t m, bool share_sets) {
+  return cap / kWalkPiece + cap / kWalkBig + m / kWalkBigCols + 1 +
+         (share_sets ? kWalkSetGroups * (cap / kWalkSetPiece + m / kWalkSetCols + 1) : 0);
+}
+
+// The work items over the x_end middle vertices: counts[0] shares of those
 // with more than kWalkBig entries or kWalkBigCols columns, counts[1] of the
 // others (whole).
 __global__ void __launch_bounds__(kWalkBlock)
     k_walk_plan(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ split,
                 const uint32_t *__restrict__ long_rows, const uint32_t *__restrict__ start,
                 uint32_t x_end, uint2 *__restrict__ big, uint2 *__restrict__ small,
-                uint32_t *__restrict__ counts, const uint32_t *__restrict__ err) {
+                uint32_t *__restrict__ counts, bool share_sets,
+                const uint32_t *__restrict__ err) {
   if (*err != kDevOk) return;
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t stride = (uint64_t)gridDim.x * kWalkBlock;
@@ -321,11 +387,17 @@ __global__ void __launch_bounds__(kWalkBlock)
     const uint64_t x = x0 + lane;
     const uint32_t E = x < x_end ? start[x + 1] - start[x] : 0u;
     bool few = false;
-    if (E && E <= kWalkBig) {
+    uint32_t groups = 1, piece = kWalkPiece;
+    if (E && (E <= kWalkBig || (share_sets && !(x & 1)))) {
       const uint2 set = walk_set(rp, split, long_rows, (uint32_t)x);
-      few = set.y - set.x <= kWalkBigCols;
+      const uint32_t d = set.y - set.x;
+      few = E <= kWalkBig && d <= kWalkBigCols;
+      if (share_sets && walk_several((uint32_t)x, d)) {
+        groups = (d + walk_group_cols(d) - 1) / walk_group_cols(d);
+        piece = kWalkSetPiece;
+      }
     }
-    const uint32_t pieces = E && !few ? (E + kWalkPiece - 1) / kWalkPiece : 0u;
+    const uint32_t each = E && !few ? (E + piece - 1) / piece : 0u, pieces = groups * each;
     const uint32_t incl = walk_scan(pieces, lane);
     const uint32_t sm = __ballot_sync(0xffffffffu, few);
     const uint32_t sum = __shfl_sync(0xffffffffu, incl, 31);
@@ -334,7 +406,10 @@ __global__ void __launch_bounds__(kWalkBlock)
     if (lane < 2 && add) got = atomicAdd(counts + lane, add);
     const uint32_t base = __shfl_sync(0xffffffffu, got, 0) + incl - pieces;
     const uint32_t at = __shfl_sync(0xffffffffu, got, 1) + __popc(sm & ((1u << lane) - 1u));
-    for (uint32_t p = 0; p < pieces; ++p) big[base + p] = make_uint2((uint32_t)x, p);
+    for (uint32_t p = 0, g = 0; g < groups; ++g)
+      for (uint32_t q = 0; q < each; ++q, ++p)
+        big[base + p] = make_uint2(
+            (uint32_t)x, piece == kWalkPiece ? q : q | g << kWalkGroupShift | kWalkSeveral);
     if (few) small[at] = make_uint2((uint32_t)x, 0u);
   }
 }
@@ -896,18 +971,6 @@ inline WalkForm walk_form(uint64_t n, uint64_t m, uint64_t edges, uint64_t long_
                                                                              : WalkForm::kNone;
 }
 
-// A graph is walked while its wedges on rows that take several hash sets
-// (*heavy of k_walk_split) are at most this many of those below the core. Sets that are half full cost several tries a column, and the tails
-// stream once for each; a bit row costs one. In an order by degree the
-// columns of long rows lie in the window. In another order they need not:
-// default / wedge checks in ms without this rule, share of heavy wedges, R-MAT
-// scale 20 in id order 272 / 57 (0.93), in random order 102 / 30 (0.72),
-// Chung-Lu 1,000,000 vertices, mean degree 20, exponent 2.4 16 / 9 (0.80), 40,
-// 2.8 6.3 / 7.6 (0.52) and in random order 6.6 / 5.0 (0.31), dense parts of
-// 12,000 vertices 8.7 / 10.2 (0.38), Chung-Lu 300,000, 60, 3.0 in random order
-// 2.4 / 2.3 (0.07), Erdos-Renyi 150,000, 1300 36 / 127 (0).
-inline uint64_t walk_most_heavy(uint64_t wedges) { return wedges / 5; }
-
 // Whether k_edge_merge counts by sets: a set pays when many wedges share it,
 // that is from some mean tail (wedges per edge) on. Measured, sets /
 // intersections in us: Erdos-Renyi, 6M edges, tail 4.2 207 / 192, 5.4 200 /
@@ -1049,7 +1112,7 @@ __device__ __forceinline__ uint32_t walk_find8(const uint32_t *set, uint32_t slo
 // R-MAT scale 22: 1.87 ms for the blocks' vertices (shared-memory pipe 86%
 // busy, DRAM 5.4 GB) and 0.38 ms for the others, where the wedge checks of
 // the same edges took 7.6 ms and 0.58 for the hash sets.
-template <uint32_t kThreads, int kBlocks, bool kBatch>
+template <uint32_t kThreads, int kBlocks, bool kBatch, bool kShare = false>
 __global__ void __launch_bounds__(kThreads, kBlocks)
     k_walk_count(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ split,
                  const uint32_t *__restrict__ long_rows, const __grid_constant__ WalkColumns cols,
@@ -1097,10 +1160,16 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
       next = per_block ? (turn < per_block ? it + 1 : n_items) : atomicAdd(ticket, 1u);
     const uint2 item = items[it];
     const uint32_t x = item.x;
-    const uint32_t e0 = start[x] + item.y * kWalkPiece;
-    const uint32_t e1 = min(start[x + 1], e0 + kWalkPiece);
+    const bool several = kShare && (item.y & kWalkSeveral);
+    const uint32_t piece = several ? kWalkSetPiece : kWalkPiece;
+    const uint32_t e0 = start[x] + (several ? item.y & ((1u << kWalkGroupShift) - 1) : item.y) * piece;
+    const uint32_t e1 = min(start[x + 1], e0 + piece);
     const uint2 set = walk_set(rp, split, long_rows, x);
     const uint32_t d = set.y - set.x;
+    const uint32_t group_cols = several ? walk_group_cols(d) : d;
+    const uint32_t part0 =
+        several ? (item.y >> kWalkGroupShift & (kWalkSetGroups - 1)) * group_cols : 0u;
+    const uint32_t part1 = min(d, part0 + group_cols);
     if (kBatch) {
       const uint32_t now = __ldg(long_graph + (x >> 1));
       if (now != g) {
@@ -1112,12 +1181,12 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
       not_t0 = t0 - 1;
     }
     const bool window = kBits && (x & 1);
-    for (uint32_t part = 0; part < d; part += window || !kBits ? d : kWalkSetCols) {
+    for (uint32_t part = part0; part < part1; part += window || !kBits ? d : kWalkSetCols) {
       const uint32_t ncols = window || !kBits ? d : min(d - part, kWalkSetCols);
       const uint32_t slots = min(1u << (32 - __clz(max(ncols * 4u, 256u) - 1u)), kSlots);
       const uint32_t shift = __clz(slots - 1);
       for (uint32_t at = e0; at < e1; at += kGroup) {
-        if (part || at > e0) __syncthreads();  // the last group is done with
+        if (part > part0 || at > e0) __syncthreads();  // the last group is done with
         const bool fresh = at == e0;           // the set is built with the first group
         if (fresh && !window) fill(slots, kWalkEmpty);
         Entry en[kWalkPer];
@@ -1214,16 +1283,16 @@ inline uint64_t walk_room(uint64_t x) {
 struct WalkRun {
   WalkBits bits{};
   uint64_t n = 0, m = 0, rows = 0, cap = 0, entries = 0, big_cap = 0;
+  bool share_sets = false;  // there are rows of several sets (WalkFar), shared out
   Scratch<uint64_t> keys, alt;
-  // [0] entries made, [1] big, [2] small items, [3, 4] tickets, [6, 7] heavy
+  // [0] entries made, [1] big, [2] small items, [3, 4] tickets, [6...] WalkFar
   Scratch<uint32_t> split, start, counts;
   Scratch<uint2> big, small;
   prim::SortSpace ws;
   const uint64_t *sorted = nullptr;
 
-  unsigned long long *heavy() const {
-    return reinterpret_cast<unsigned long long *>(counts.ptr + 6);
-  }
+  static constexpr uint32_t kFar = 6, kCounts = kFar + sizeof(WalkFar) / 4;
+  WalkFar *far() const { return reinterpret_cast<WalkFar *>(counts.ptr + kFar); }
   static unsigned grid(DeviceContext *ctx, uint64_t threads) {
     const uint64_t most = (uint64_t)ctx->sm_count * 32, g = ceil_div(threads, kWalkBlock);
     return (unsigned)(g == 0 ? 1 : g < most ? g : most);
@@ -1240,13 +1309,29 @@ struct WalkRun {
     WETRIC_TRY(split.alloc(ctx, st, n));
     WETRIC_TRY(keys.alloc(ctx, st, cap));
     WETRIC_TRY(alt.alloc(ctx, st, cap));
-    WETRIC_TRY(counts.alloc(ctx, st, 8));
-    WETRIC_CUDA_TRY(cudaMemsetAsync(counts.ptr, 0, 8 * sizeof(uint32_t), st));
-    big_cap = cap / kWalkPiece + cap / kWalkBig + m / kWalkBigCols + 1;
+    WETRIC_TRY(counts.alloc(ctx, st, kCounts));
+    WETRIC_CUDA_TRY(cudaMemsetAsync(counts.ptr, 0, kCounts * sizeof(uint32_t), st));
+    big_cap = walk_most_items(cap, m, false);
     WETRIC_TRY(start.alloc(ctx, st, room + 1));
     WETRIC_TRY(small.alloc(ctx, st, room));
     WETRIC_TRY(ws.alloc(ctx, st, cap));
     return big.alloc(ctx, st, big_cap);
+  }
+  // Rows of several sets will be shared out (before sort); not without room
+  // for their items.
+  void share(DeviceContext *ctx, cudaStream_t st) {
+    Scratch<uint2> more;
+    if (more.alloc(ctx, st, walk_most_items(cap, m, true)) != WETRIC_OK) {
+      clear_error();
+      return;
+    }
+    big.release();
+    big.ctx = more.ctx;
+    big.stream = more.stream;
+    big.bytes = more.bytes;
+    big.ptr = more.detach();
+    share_sets = true;
+    big_cap = walk_most_items(cap, m, true);
   }
   // The entries made, sorted by middle vertex, and the work items.
   int sort(DeviceContext *ctx, cudaStream_t st, const uint32_t *rp, const uint32_t *long_rows,
@@ -1262,7 +1347,7 @@ struct WalkRun {
     WETRIC_LAUNCH_CHECK();
     k_walk_plan<<<grid(ctx, 2 * rows), kWalkBlock, 0, st>>>(
         rp, split.ptr, long_rows, start.ptr, (uint32_t)(2 * rows), big.ptr, small.ptr,
-        counts.ptr + 1, err);
+        counts.ptr + 1, share_sets, err);
     WETRIC_LAUNCH_CHECK();
     *launches += 3 + prim::digit_plan(bits.shift(), bits.w).passes;
     return WETRIC_OK;
@@ -1276,7 +1361,9 @@ struct WalkRun {
             uint64_t *most, uint32_t *launches, const WalkGroups &groups = WalkGroups{},
             const uint32_t *long_graph = nullptr) {
     constexpr uint32_t kPerBlock = 16;
-    const auto big_fn = k_walk_count<kWalkBigBlock, kWalkBigBlocks, kBatch>;
+    const auto big_fn = !kBatch && share_sets
+                            ? k_walk_count<kWalkBigBlock, kWalkBigBlocks, kBatch, !kBatch>
+                            : k_walk_count<kWalkBigBlock, kWalkBigBlocks, kBatch>;
     const auto small_fn = k_walk_count<kWalkSmallBlock, kWalkSmallBlocks, kBatch>;
     const uint64_t g = persistent ? (uint64_t)ctx->sm_count * kWalkBigBlocks
                                   : ceil_div(big_cap, kPerBlock);
