@@ -210,7 +210,7 @@ def run_ours(args):
     stream = torch.cuda.current_stream()
 
     # one GPU counts the whole graph (wedge_end 0), which lets the count
-    # take pair streams for its short rows
+    # go by middle vertex instead of by wedge checks
     hi_arg = hi if world > 1 else 0
 
     def step():
@@ -1077,7 +1077,8 @@ def main():
                     help="batch: spread from the size table instead of the autotuner")
     ap.add_argument("--sub-batch-pairs", type=float, default=1.2e9)
     ap.add_argument("--pair-streams", type=int, default=1,
-                    help="1 = pair streams for short rows (the library default), 0 = off")
+                    help="1 = short rows are counted row by row (the library default), "
+                         "0 = every wedge below the core is checked")
     ap.add_argument("--plain-every", type=int, default=1,
                     help="batch: plain per-graph calls on every k-th graph (1 = all)")
     args = ap.parse_args()

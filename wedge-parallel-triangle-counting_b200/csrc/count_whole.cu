@@ -9,14 +9,16 @@
 // the host (k_small_count; with validation k_edge_vertices, k_validate,
 // k_edge_merge and a copy), a large one
 //
-//   k_edge_vertices                                               [read]
+//   k_edge_vertices                                                 [read]
 //   per row chunk: k_walk_split k_edge_merge k_core_bitmap k_core_count
-//   the entries made                                              [read]
-//   sort  k_walk_starts  k_walk_plan  k_walk_heavy                [read]
+//   the entries made                                                [read]
+//   sort  k_walk_starts  k_walk_plan  k_walk_count (two block sizes) [read]
 //
 // Wedge ranges, u64 offsets of large graphs and the options that name another
 // kernel (CountArgs::kernel, pair_streams off, a shell, l2_persist) keep to
-// count.cu.
+// count.cu. So do graphs that are declined here: no room for a part, entries of
+// more than 64 bits (walk_form), more entries than room, or too many wedges
+// between rows of several hash sets (WalkFar).
 #include <cuda_runtime.h>
 #include <stdint.h>
 

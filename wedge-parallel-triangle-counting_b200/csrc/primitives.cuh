@@ -294,7 +294,7 @@ constexpr int kSortItems = 16;  // per thread
 // shared-memory split they were started with: a large tile could wait there
 // until that kernel ended.
 constexpr int kSortFewItems = 4;
-constexpr uint64_t kSortFewTiles = 148;
+constexpr uint64_t kSortFewTiles = 148;  // the B200's SMs
 constexpr uint64_t kSortFewKeys = kSortFewTiles * kSortThreads * kSortFewItems;
 // Most tiles of a sort of up to n keys.
 inline uint64_t sort_tiles(uint64_t n) {

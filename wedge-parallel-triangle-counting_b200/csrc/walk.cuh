@@ -24,13 +24,15 @@
 //
 //   k_edge_vertices  row checks, W, the longest row, core sizing, and the
 //                    numbers of the long rows
-//   k_walk_split     where a row's window columns start
+//   k_walk_split     where a row's window columns start, and the wedges of
+//                    rows with several hash sets
 //   k_edge_merge     the short rows' edges counted, the others' entries:
 //                    middle vertex, the tail's first column index and its
 //                    length in 64 bits
 //   radix sort       by middle vertex (primitives.cuh)
 //   k_walk_starts    the first entry of every middle vertex
-//   k_walk_plan      work items: a vertex, a piece of its entries
+//   k_walk_plan      work items: a vertex, a piece of its entries and, with
+//                    several hash sets, a group of them
 //   k_walk_count     a block per item: the bit row, or a hash set
 //   k_small_count    a small graph's whole count
 #pragma once
@@ -1107,8 +1109,9 @@ __device__ __forceinline__ uint32_t walk_find8(const uint32_t *set, uint32_t slo
 // for each part). The block's threads share the sectors of up to four tails
 // each equally, so they meet at the barriers together: with tails handed to
 // warps in groups of 64 the kernel spent half its time there. Vertices of up
-// to 256 entries have blocks of one warp: most of the vertices of R-MAT scale
-// 22, whose set-up by four warps took two thirds of the instructions.
+// to kWalkBig entries and kWalkBigCols columns have blocks of one warp: most of
+// the vertices of R-MAT scale 22, whose set-up by four warps took two thirds of
+// the instructions.
 // R-MAT scale 22: 1.87 ms for the blocks' vertices (shared-memory pipe 86%
 // busy, DRAM 5.4 GB) and 0.38 ms for the others, where the wedge checks of
 // the same edges took 7.6 ms and 0.58 for the hash sets.
