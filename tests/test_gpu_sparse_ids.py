@@ -56,3 +56,15 @@ def test_few_pairs_among_many_ids(wetric_mod):
         return sorted(t)[2]
 
     assert ms(*few) < 1.5 * ms(*many)
+
+
+@pytest.mark.parametrize("dtype", ["int32", "int64"])
+def test_no_vertices_launch_nothing(wetric_mod, dtype):
+    import torch
+
+    rp = torch.zeros(1, dtype=getattr(torch, dtype), device="cuda")
+    ci = torch.zeros(0, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for kw in ({}, {"validate": True}, {"core_len": wetric_mod.CORE_OFF}, {"kernel": 8}):
+        count, st = wetric_mod.count(rp, ci, 5, 8192, **kw)
+        assert count == 0 and st.wedges == 0 and st.launches == 0, kw

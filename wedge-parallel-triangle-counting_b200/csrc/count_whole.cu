@@ -92,7 +92,7 @@ int check_words(uint64_t err, uint64_t longest) {
 }  // namespace
 
 bool count_whole_takes(const CountArgs &a) {
-  return a.kernel == 0 && a.pair_streams && !a.l2_persist && a.wedge_begin == 0 &&
+  return a.n > 0 && a.kernel == 0 && a.pair_streams && !a.l2_persist && a.wedge_begin == 0 &&
          a.wedge_end == 0 && (a.shell_len == 0 || a.shell_len == kCoreOff) &&
          a.n < (1ull << 31) && a.m < (1ull << 31) &&
          (a.offsets32 || (a.m < kSmallColumns && (a.core_len == 0 || a.core_len == kCoreOff)));
