@@ -124,3 +124,30 @@ def test_a_star_in_front_takes_no_wedge_checks(wetric_mod):
 
     (a, default), (b, checks) = ms(), ms(kernel=8)
     assert a == b and default < checks / 4, (default, checks)
+
+
+def test_hubs_with_many_sets_in_front(wetric_mod):
+    """300 hubs, then 300,000 vertices with up to 12 columns to them: few wedges
+    have both ends on hubs, but each hub has a dozen hash sets (the count took
+    2.4 times as long as the wedge checks)."""
+    import torch
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    k, n = 300, 300_300
+    i, j = torch.triu_indices(k, k, 1, device="cuda")
+    hub = torch.randint(0, k, (12 * (n - k),), device="cuda", generator=gen)
+    leaf = torch.arange(k, n, device="cuda").repeat_interleave(12)
+    key = torch.unique(torch.cat([i * n + j, hub * n + leaf]))
+    rp = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    rp[1:] = torch.cumsum(torch.bincount(key // n, minlength=n), 0)
+    ci = (key % n).int()
+    torch.cuda.synchronize()
+
+    def ms(**kw):
+        runs = [wetric_mod.count(rp, ci, 5, 8192, **kw) for _ in range(4)]
+        assert len({c for c, _ in runs}) == 1
+        return runs[0][0], sorted(st.exec_ms for _, st in runs)[1]
+
+    (a, default), (b, checks) = ms(), ms(kernel=8)
+    assert a == b and default < 1.5 * checks, (default, checks)

@@ -240,8 +240,9 @@ __global__ void __launch_bounds__(kWalkBlock)
 // several hash sets: their wedges there, columns there and number, and the
 // blocks that are through with them. At most min(wedges, columns * rows) of a
 // graph's wedges have their tail on one such row and their middle vertex on
-// another; with more than a tenth of those below the core (`most`) it is not
-// walked. Half full sets cost several tries a column and the tails stream
+// another, and such a wedge is looked up once for each set of that vertex, at
+// most columns^2 / kWalkSetCols times in all; with more than a tenth (`most`) of
+// those below the core, or a third as many lookups, it is not walked. Half full sets cost several tries a column and the tails stream
 // once for each set, where a bit row costs one lookup. In an order by degree
 // the columns of long rows lie in the window, and a batch, always in that
 // order, does without this; in another order they need not. Walk / wedge checks
@@ -251,10 +252,14 @@ __global__ void __launch_bounds__(kWalkBlock)
 // 5.8 / 7.6 (0.25), 3.8 / 5.0 (0.06); dense parts of 3,000 vertices 9 / 6
 // (0.82); skewed draws in id order 4.5 / 13 (0.01); Erdos-Renyi 150,000, 1300
 // 36 / 127 (0); four hubs of 200,000 columns, all wedges theirs, 1.2 / 180 (0).
+// With the lookups per wedge: 300 hubs in front of 300,000 vertices with 12
+// columns to them 28 / 12 (0.36), of 1,000,000 354 / 130 (0.51); in random
+// order 48 / 157 (0.33); Chung-Lu 2,000,000, 8, 2.1 13 / 14 (0.27).
 struct WalkFar {
   unsigned long long wedges, columns, rows, blocks;
   __host__ __device__ bool past(unsigned long long most) const {
-    return wedges > most && columns * rows > most;
+    return (wedges > most && columns * rows > most) ||
+           columns / kWalkSetCols * columns > most / 3 * 10;
   }
 };
 inline uint64_t walk_most_far(uint64_t wedges) { return wedges / 10; }
