@@ -1368,7 +1368,11 @@ struct WalkRun {
             const uint32_t *long_rows, bool persistent, unsigned long long *out, const uint32_t *err,
             uint64_t *most, uint32_t *launches, const WalkGroups &groups = WalkGroups{},
             const uint32_t *long_graph = nullptr) {
-    constexpr uint32_t kPerBlock = 16;
+    // Items per block when blocks are to be short (one pass): the last block is
+    // the one with most work, so few, but not a block each (1.5e6 at scale 22).
+    // R-MAT scale 18 / 20 / 22 in us: 16 items 793 / 1890 / 6455, 4 574 / 1636 /
+    // 6101, 1 561 / 1739 / 6925; from a counter 540 / 1548 / 5900.
+    constexpr uint32_t kPerBlock = 4;
     const auto big_fn = !kBatch && share_sets
                             ? k_walk_count<kWalkBigBlock, kWalkBigBlocks, kBatch, !kBatch>
                             : k_walk_count<kWalkBigBlock, kWalkBigBlocks, kBatch>;
